@@ -2,13 +2,15 @@
 
 ``build_all()`` runs nvcc on every source under ``csrc/`` for sm_100a only
 (``-gencode arch=compute_100a,code=sm_100a``), links ``libjq_b200.so`` next to this file and
-builds ``python/q8_1_me*.so`` and ``python/mm_q4_0_q8_1_me*.so`` against it.  nvcc
+builds ``python/q8_1_me*.so`` and ``python/mm_q4_0_q8_1_me*.so`` against it, and ``_torch_calls*.so`` (the
+native part of ``capi.py``) against torch.  nvcc
 cross-compiles without a GPU, so this also serves as the "does it build" check.  The
 top-level ``CMakeLists.txt`` describes the same targets for CMake users.
 """
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -58,6 +60,10 @@ def _nvcc() -> str:
         if cand and os.path.exists(cand):
             return cand
     raise RuntimeError("nvcc not found: the CUDA toolkit is required to build jjjetson_ops_b200")
+
+
+def _cuda_include() -> str:
+    return os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
 
 
 def _host_cxx() -> str:
@@ -127,6 +133,20 @@ def build_all(force: bool = False, verbose: bool = False) -> str:
                     "-L", PKG_DIR, "-ljq_b200", "-Wl,-rpath,$ORIGIN/..",
                 ]
             )
+
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    torch_lib = os.path.join(torch_dir, "lib")
+    src_path = os.path.join(CSRC, "bindings", "torch_calls.cpp")
+    out = os.path.join(PKG_DIR, "_torch_calls" + ext)
+    if force or _mtime(out) < max(_mtime(src_path), hdr_time):
+        _run(
+            [
+                _host_cxx(), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                "-I", os.path.join(torch_dir, "include"), "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+                "-I", _cuda_include(), "-I", py_inc, "-I", INCLUDE_DIR, src_path, "-o", out,
+                "-L", torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath," + torch_lib,
+            ]
+        )
     return LIB_PATH
 
 

@@ -1,8 +1,9 @@
 """ctypes binding of ``libjq_b200.so`` with torch tensors as device memory.
 
 Every function here is a direct call through the C ABI declared in ``include/jq_b200.h``; torch
-only provides allocations and the current stream.  The library is loaded at import time and a
-missing build is an error, never a fallback.
+only provides allocations and the current stream.  The calls of a forward pass go through the native
+module ``_torch_calls``, which checks the tensors, looks up the stream and makes the C call; the rest
+goes through ctypes.  Both are loaded at import time and a missing build is an error, never a fallback.
 """
 from __future__ import annotations
 
@@ -104,6 +105,13 @@ for _name, (_res, _args) in _SIGS.items():
     _fn.argtypes = _args
 
 
+try:
+    from . import _torch_calls as _calls
+except ImportError as _e:
+    raise ImportError("%s: build it with `python -m jjjetson_ops_b200._build`" % _e) from _e
+_calls.bind({_name: ctypes.cast(getattr(_lib, _name), ctypes.c_void_p).value for _name in _SIGS})
+
+
 def lib() -> ctypes.CDLL:
     return _lib
 
@@ -157,12 +165,12 @@ def _dev(t: torch.Tensor, dtype: torch.dtype, name: str) -> int:
 def quantize_q8_1(x: torch.Tensor, order: int = ORDER_COL_KSUPER, s_mode: int = S_SUM_X,
                   out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 ``[M, K]`` -> raw ``block_q8_1_mmq`` bytes on the same device."""
-    M, K = x.shape
     if out is None:
+        M, K = x.shape
         out = torch.empty(q8_1_bytes(K, M), dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        check(_lib.jq_quantize_q8_1_device(_stream(x), _dev(x, torch.float32, "x"), _dev(out, torch.uint8, "out"),
-                                           K, M, order, s_mode))
+    rc = _calls.quantize(x, out, order, s_mode)
+    if rc:
+        check(rc)
     return out
 
 
@@ -172,23 +180,23 @@ def mul_mat_q4_0_q8_1(w: torch.Tensor, xq: torch.Tensor, K: int, N: int, M: int,
     """Q4_0 weights x Q8_1 activations -> fp32 ``[M, N]``."""
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=w.device)
-    with torch.cuda.device(w.device):
-        check(_lib.jq_mul_mat_q4_0_q8_1_device_ex(_stream(w), _dev(w, torch.uint8, "w"), _dev(xq, torch.uint8, "xq"),
-                                                  _dev(out, torch.float32, "out"), K, N, M, order, kernel))
+    rc = _calls.mul_mat(w, xq, out, K, N, M, order, kernel)
+    if rc:
+        check(rc)
     return out
 
 
 def linear_q4_0(w: torch.Tensor, x: torch.Tensor, N: int, s_mode: int = S_D_SUM_Q,
                 ws: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """fp32 activations ``[M, K]`` -> quantize -> multiply -> fp32 ``[M, N]`` in one call."""
-    M, K = x.shape
     if ws is None:
+        M, K = x.shape
         ws = torch.empty(max(q8_1_bytes(K, M), 16), dtype=torch.uint8, device=x.device)
     if out is None:
-        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        check(_lib.jq_linear_q4_0_device(_stream(x), _dev(w, torch.uint8, "w"), _dev(x, torch.float32, "x"),
-                                         _dev(ws, torch.uint8, "ws"), _dev(out, torch.float32, "out"), K, N, M, s_mode))
+        out = torch.empty((x.shape[0], N), dtype=torch.float32, device=x.device)
+    rc = _calls.linear(w, x, ws, out, N, s_mode)
+    if rc:
+        check(rc)
     return out
 
 
@@ -202,16 +210,11 @@ def linear_q4_0_multi(ws_list, N_list, x: Optional[torch.Tensor] = None, xq: Opt
         M, K = x.shape
         if ws is None:
             ws = torch.empty(max(q8_1_bytes(K, M), 16), dtype=torch.uint8, device=dev)
-    n = len(ws_list)
     if outs is None:
         outs = [torch.empty((M, int(Ni)), dtype=torch.float32, device=dev) for Ni in N_list]
-    wp = (_vp * n)(*[_dev(w, torch.uint8, "w") for w in ws_list])
-    yp = (_vp * n)(*[_dev(y, torch.float32, "out") for y in outs])
-    np_ = (_i64 * n)(*[int(v) for v in N_list])
-    with torch.cuda.device(dev):
-        check(_lib.jq_linear_q4_0_multi_device(
-            _stream(ws_list[0]), n, wp, np_, yp, None if x is None else _dev(x, torch.float32, "x"),
-            None if xq is None else _dev(xq, torch.uint8, "xq"), None if ws is None else _dev(ws, torch.uint8, "ws"), K, M, s_mode))
+    rc = _calls.multi(ws_list, N_list, outs, x, xq, ws, K, M, s_mode)
+    if rc:
+        check(rc)
     return outs
 
 
@@ -221,16 +224,14 @@ def rms_norm_q8_1(x: torch.Tensor, weight: torch.Tensor, epsilon: float, residua
     """RMSNorm of ``x`` ``[T, H]`` (with ``residual`` given: z = x + residual, residual <- z first) with the
     Q8_1 quantizer folded in.  ``normed`` (may be ``x`` itself) receives the fp32 result; the returned uint8
     tensor holds the Q8_1 blocks of it (``None`` when ``want_q8`` is false)."""
-    T, H = x.shape
     if want_q8 and xq is None:
+        T, H = x.shape
         xq = torch.empty(max(q8_1_bytes(H, T), 16), dtype=torch.uint8, device=x.device)
     if not want_q8:
         xq = None
-    with torch.cuda.device(x.device):
-        check(_lib.jq_rms_norm_q8_1_device(
-            _stream(x), _dev(x, torch.float32, "x"), None if residual is None else _dev(residual, torch.float32, "residual"),
-            _dev(weight, torch.float32, "weight"), None if normed is None else _dev(normed, torch.float32, "normed"),
-            None if xq is None else xq.data_ptr(), H, T, float(epsilon), order, s_mode))
+    rc = _calls.rms_norm(x, weight, epsilon, residual, normed, xq, order, s_mode)
+    if rc:
+        check(rc)
     return xq
 
 
@@ -238,15 +239,14 @@ def swiglu_q8_1(gate: torch.Tensor, up: torch.Tensor, mid: Optional[torch.Tensor
                 order: int = ORDER_COL_KSUPER, s_mode: int = S_D_SUM_Q,
                 xq: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """silu(gate) * up over ``[T, I]`` with the Q8_1 quantizer folded in; ``mid`` receives the fp32 result."""
-    T, I = gate.shape
     if want_q8 and xq is None:
+        T, I = gate.shape
         xq = torch.empty(max(q8_1_bytes(I, T), 16), dtype=torch.uint8, device=gate.device)
     if not want_q8:
         xq = None
-    with torch.cuda.device(gate.device):
-        check(_lib.jq_swiglu_q8_1_device(
-            _stream(gate), _dev(gate, torch.float32, "gate"), _dev(up, torch.float32, "up"),
-            None if mid is None else _dev(mid, torch.float32, "mid"), None if xq is None else xq.data_ptr(), I, T, order, s_mode))
+    rc = _calls.swiglu(gate, up, mid, xq, order, s_mode)
+    if rc:
+        check(rc)
     return xq
 
 

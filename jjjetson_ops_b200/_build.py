@@ -32,6 +32,7 @@ CUDA_SOURCES = [
     "producers.cu",
     "mmq_generic.cu",
     "mmq_gemv_sm100.cu",
+    "mmq_stream_sm100.cu",
     "mmq_gemm_sm100.cu",
     "mmq_gemm_tc_sm100.cu",
     "mmq_gemm_f16_sm100.cu",

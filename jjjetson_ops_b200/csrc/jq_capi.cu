@@ -184,6 +184,14 @@ int check_mul_mat_shape(int64_t K, int64_t N, int64_t M) {
 // Smallest batch the automatic choice gives to the fp16-operand GEMM (unless JQ_OPT_PREFILL_EXACT): half a 128-column tile.
 constexpr int64_t FP16_OPERANDS_MIN_COLUMNS = 64;
 
+// The small-batch kernel takes what the decode kernels above it refuse, up to 63 columns, and every batch whose K is an
+// odd multiple of 128 (the GEMMs need K % 256 == 0).  Multiply alone, cold weights, what was taken before / this kernel:
+// K = 4096, N = 11008, M = 16 18.8 / 14.9 us, M = 24 28.0 / 18.0 us (passes of eight columns), M = 48 44 / 26 us (integer
+// GEMM); K = 11008, N = 4096, M = 8 60 / 17.6 us (integer GEMM); K = 1408, N = 1003, M = 1 3.15 / 2.9 us, M = 45
+// 13.6 / 4.4 us; K = 4224, N = 11008, M = 2 23.7 / 16.3 us (generic kernel).  Where the decode kernel runs (3 to 8 columns,
+// K <= 6144) it is the faster one at K = 4096: N = 11008 9.5 against 13.1 us.
+inline bool small_batch_kernel_pays(int64_t K, int64_t M) { return M < FP16_OPERANDS_MIN_COLUMNS || K % (2 * SUPER) != 0; }
+
 int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N,
                      int64_t M, int order, int kernel) {
     if (N == 0 || M == 0) return JQ_OK;
@@ -204,19 +212,7 @@ int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *
     int rc = JQ_ERR_UNSUPPORTED;
     if (M <= 2) rc = launch_gemv_dp4a(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
     if (rc == JQ_ERR_UNSUPPORTED && M <= 8) rc = launch_gemv_mma(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
-    if (M > 8 && M <= 32 && order == JQ_ORDER_COL_KSUPER && K <= 6144) {
-        // A handful of columns more than one GEMV pass takes: passes of eight columns (the weights of the
-        // later passes come from L2) beat a GEMM tile that would be mostly padding (cfg2 shape: M = 16 in
-        // 18.8 us against 41.7 us, M = 32 in 37 us against 44 us; from M = 40 on the GEMM wins).
-        const size_t col_bytes = (size_t)(K / SUPER) * Q8_BYTES;  // one column's blocks are contiguous in this order
-        for (int64_t m0 = 0; m0 < M; m0 += 8) {
-            const int64_t mc = M - m0 < 8 ? M - m0 : 8;
-            rc = launch_gemv_mma(st, d_w, static_cast<const uint8_t *>(d_xq) + (size_t)m0 * col_bytes, nullptr, nullptr,
-                                 d_y + (size_t)m0 * N, K, N, mc, order, 0);
-            if (rc != JQ_OK) break;
-        }
-        if (rc != JQ_OK && rc != JQ_ERR_UNSUPPORTED) return rc;
-    }
+    if (rc == JQ_ERR_UNSUPPORTED && small_batch_kernel_pays(K, M)) rc = launch_mmq_stream(st, d_w, d_xq, d_y, K, N, M, order);
     if (rc == JQ_ERR_UNSUPPORTED && M >= FP16_OPERANDS_MIN_COLUMNS && option_value(JQ_OPT_PREFILL_EXACT) == 0)
         rc = launch_gemm_f16(st, d_w, d_xq, d_y, K, N, M, order);  // refuses shapes outside its rules: the integer GEMM takes those
     if (rc == JQ_ERR_UNSUPPORTED && M > 8) rc = launch_gemm_mma(st, d_w, d_xq, d_y, K, N, M, order);
@@ -442,7 +438,7 @@ int jq_linear_q4_0_multi_device(void *stream, int n_mats, const void *const *d_w
     // one launch over the concatenated rows while the decode kernels take the shape
     bool all_rows = true;
     for (int i = 0; i < n_mats; ++i) all_rows = all_rows && N[i] > 0;
-    if (K > 0 && M <= 8 && all_rows) {
+    if (K > 0 && M < FP16_OPERANDS_MIN_COLUMNS && all_rows) {
         MultiMat mm{};
         mm.n = n_mats;
         for (int i = 0; i < n_mats; ++i) {
@@ -450,7 +446,7 @@ int jq_linear_q4_0_multi_device(void *stream, int n_mats, const void *const *d_w
             mm.y[i] = d_y[i];
             mm.rows[i] = N[i];
         }
-        const bool fuse_quantizer = d_x != nullptr && fuse_quantizer_pays(M, K);
+        const bool fuse_quantizer = d_x != nullptr && M <= 8 && fuse_quantizer_pays(M, K);
         if (d_x != nullptr && !fuse_quantizer) {
             if (int rc = launch_quantize_q8_1(st, d_x, d_ws, K, M, JQ_ORDER_COL_KSUPER, s_mode)) return rc;
         }
@@ -459,9 +455,12 @@ int jq_linear_q4_0_multi_device(void *stream, int n_mats, const void *const *d_w
         int rc = JQ_ERR_UNSUPPORTED;
         if (M <= 2) rc = launch_gemv_dp4a(st, nullptr, xq, xf, fuse_quantizer ? d_ws : nullptr, nullptr, K, n_total, M,
                                           JQ_ORDER_COL_KSUPER, s_mode, nullptr, &mm);
-        if (rc == JQ_ERR_UNSUPPORTED)
+        if (rc == JQ_ERR_UNSUPPORTED && M <= 8)
             rc = launch_gemv_mma(st, nullptr, xq, xf, fuse_quantizer ? d_ws : nullptr, nullptr, K, n_total, M, JQ_ORDER_COL_KSUPER,
                                  s_mode, &mm);
+        if (rc == JQ_ERR_UNSUPPORTED && !fuse_quantizer)
+            rc = launch_mmq_stream(st, nullptr, xq, nullptr, K, n_total, M, JQ_ORDER_COL_KSUPER, &mm);
+        if (rc == JQ_OK) t_last_error.clear();  // what the kernels tried before had to say
         if (rc != JQ_ERR_UNSUPPORTED) return rc;
         // not a shape for the decode kernels: the activations may already be quantized in d_ws, go on below
         if (d_x != nullptr && !fuse_quantizer) {

@@ -156,6 +156,9 @@ int launch_gemv_dp4a(cudaStream_t st, const void *d_w, const void *d_xq, const f
 int launch_gemv_mma(cudaStream_t st, const void *d_w, const void *d_xq, const float *d_x_f32,
                     void *d_xq_out, float *d_y, int64_t K, int64_t N, int64_t M, int order,
                     int s_mode, const MultiMat *multi = nullptr);
+// Small batches on ready Q8_1 blocks, any K % 128 == 0 (16-byte aligned weights).
+int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N, int64_t M,
+                      int order, const MultiMat *multi = nullptr);
 int launch_gemm_mma(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K,
                     int64_t N, int64_t M, int order, const GatherArgs *gather = nullptr);
 int launch_gemm_tc(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K,

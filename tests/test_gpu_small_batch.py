@@ -1,0 +1,76 @@
+"""GPU parity of the small-batch multiply, which the automatic choice takes for 3 to 63 columns (where the decode kernels
+refuse the shape) and for any batch when K is an odd multiple of 128.
+
+The bar against the oracle's reference-formula multiply is the integer kernels' 1e-5: block sums are exact, only the
+order of the fp32 additions differs (K / 32 <= 344 terms of relative rounding 2^-24 each, 2.1e-5 at the very worst and
+a few 1e-7 as a rule).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+@pytest.fixture(scope="module")
+def env(native_lib, oracle, cuda_device):
+    import torch
+
+    class Env:
+        c, O, t, dev = native_lib, oracle, torch, cuda_device
+
+    yield Env()
+    assert native_lib.device_fault(clear=True) == 0
+
+
+def _problem(K, N, M):
+    rng = np.random.default_rng(5 * K + 3 * N + M)
+    w = (rng.standard_normal((N, K), dtype=np.float32) * np.float32(0.02)).astype(np.float32)
+    return w, rng.standard_normal((M, K), dtype=np.float32)
+
+
+# Row tiles of 32 and (from 17 columns on, with enough of them) 64, column tiles of 8 to 32 in equal groups, stages of 512
+# or 256 values with a shorter last one; more stages than the ring holds; an odd K with every remainder of four.
+@pytest.mark.parametrize("K,N,M", [(128, 1, 1), (128, 31, 3), (384, 33, 9), (640, 32, 33), (1408, 65, 45), (896, 100, 130), (4224, 20, 2),
+                                   (256, 31, 9), (512, 33, 16), (768, 64, 17), (6400, 40, 8), (6400, 10, 3), (4608, 97, 32),
+                                   (256, 9500, 24), (512, 4800, 63), (1280, 9473, 31), (11008, 35, 63)])
+@pytest.mark.parametrize("order", [0, 1])
+def test_small_batch_shapes(env, K, N, M, order):
+    c, O = env.c, env.O
+    w, x = _problem(K, N, M)
+    wq = O.quantize_q4_0(w)
+    xq = O.quantize_q8_1(x, order, c.S_SUM_X)
+    d_w, d_x = env.t.from_numpy(wq).to(env.dev), env.t.from_numpy(xq).to(env.dev)
+    y = env.t.full((M, N), float("nan"), device=env.dev)
+    c.mul_mat_q4_0_q8_1(d_w, d_x, K, N, M, order, out=y)
+    assert O.err_max_rel(y.cpu().numpy(), O.mul_mat_ref(wq, xq, K, N, M, order)) <= TOL
+
+
+@pytest.mark.parametrize("K", [512, 640])
+@pytest.mark.parametrize("shift", [2, 8])
+def test_small_batch_weights_off_alignment(env, K, shift):
+    """Weights that are not 16-byte aligned go to another kernel: same answer."""
+    c, O = env.c, env.O
+    N, M = 70, 20
+    w, x = _problem(K, N, M)
+    wq = O.quantize_q4_0(w)
+    xq = O.quantize_q8_1(x, O.ORDER_COL_KSUPER, c.S_SUM_X)
+    buf = env.t.zeros(wq.nbytes + 16, dtype=env.t.uint8, device=env.dev)
+    d_w = buf[shift:shift + wq.nbytes]
+    d_w.copy_(env.t.from_numpy(wq.reshape(-1)))
+    y = c.mul_mat_q4_0_q8_1(d_w, env.t.from_numpy(xq).to(env.dev), K, N, M)
+    assert O.err_max_rel(y.cpu().numpy(), O.mul_mat_ref(wq, xq, K, N, M)) <= TOL
+
+
+@pytest.mark.parametrize("K,M", [(512, 12), (6400, 5), (640, 7), (512, 40)])
+def test_small_batch_several_matrices(env, K, M):
+    """Several matrices in one launch give the bits of separate calls."""
+    c, O = env.c, env.O
+    rows = [40, 1, 96, 33]
+    x = _problem(K, 1, M)[1]
+    ws = [env.t.from_numpy(O.quantize_q4_0(_problem(K, n, M + i)[0])).to(env.dev) for i, n in enumerate(rows)]
+    xq = env.t.from_numpy(O.quantize_q8_1(x, O.ORDER_COL_KSUPER, c.S_D_SUM_Q)).to(env.dev)
+    outs = c.linear_q4_0_multi(ws, rows, xq=xq, K=K, M=M)
+    for w, n, y in zip(ws, rows, outs):
+        assert env.t.equal(y, c.mul_mat_q4_0_q8_1(w, xq, K, n, M))

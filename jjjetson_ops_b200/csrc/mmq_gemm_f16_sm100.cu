@@ -20,7 +20,10 @@
 // by name only.  Operands must stay inside fp16's range: |x| <= 65504 for the activations, and
 // scales whose products are not subnormal (|d| * |q| >= 6.1e-5) keep full precision.
 //
-// A CTA owns a 128 (activation columns) x 128 (weight rows) tile of Y.  K advances in stages of 128
+// A CTA owns a 128 (activation columns) x 128 (weight rows) tile of Y, or two CTAs on neighbouring SMs own 256 x 256:
+// each converts 128 columns and 128 rows, and cta_group::2 MMAs, issued by the first, multiply all with all, so that a
+// converted operand is used twice as often (the conversion is what bounds the single CTA: 57 % of the issue slots, tensor
+// pipe 37 %).  K advances in stages of 128
 // values (one Q8_1 block per column, four Q4_0 blocks per row) through three rings:
 //   raw rings       the quantized bytes as they lie in global memory, brought in by the copy engine:
 //                   one tiled tensor copy per stage for the 128 activation blocks (128 rows x 144
@@ -81,7 +84,9 @@ static_assert(HF_RAWX_SLOTS == HF_STAGES, "stage c uses slot c % 3 of both the o
 // column, 64 columns of two fp16 values = the 128 values of K in order
 constexpr uint32_t HF_TMEM_A_COL = 128, HF_TMEM_A_STAGE_COLS = 64;
 constexpr uint32_t HF_TMEM_COLS = 512;
-static_assert(HF_TMEM_A_COL + HF_STAGES * HF_TMEM_A_STAGE_COLS <= HF_TMEM_COLS, "tensor memory too small");
+// A pair of CTAs (two SMs, cta_group::2) shares a 256 x 256 tile: its accumulator is 256 columns wide in each
+constexpr uint32_t HF_TMEM_A_COL_PAIR = 256;
+static_assert(HF_TMEM_A_COL_PAIR + HF_STAGES * HF_TMEM_A_STAGE_COLS <= HF_TMEM_COLS, "tensor memory too small");
 static_assert(HF_SMEM_BYTES <= 227 * 1024, "stages do not fit in shared memory");
 static_assert(HF_PROD_WARPS * 32 * HF_OUT_PITCH * 4 <= HF_STAGES * HF_STAGE_BYTES, "output staging does not fit in the operand stages");
 
@@ -149,6 +154,54 @@ __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, 
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
         "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// ---- the same for a pair of CTAs: A's 256 rows and B's 256 rows are 128 in each CTA, at the same addresses ----------
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// completion of this thread's tensor-core operations arrives on the barrier at this offset in both CTAs
+__device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+// arrive on the barrier at this offset in the pair's first CTA (which issues the MMAs)
+__device__ __forceinline__ void mbar_arrive_leader(uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %0, 0;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_bounded_cluster(uint64_t *bar, uint32_t parity, int *fault, uint32_t limit = (1u << 22)) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    report_fault(fault, 1);
+    return false;
+}
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
@@ -246,6 +299,7 @@ __device__ __forceinline__ void hf_convert_activation_col(uint32_t st, int r, co
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(HF_THREADS, 1)
 gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -262,14 +316,18 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
     static_assert((2 * HF_STAGES + 1 + 2 * HF_RAWX_SLOTS + 2 * HF_RAWW_SLOTS) * 8 + 4 <= 256, "barrier block too small");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t n0 = (int64_t)blockIdx.x * HF_BN, m0 = (int64_t)blockIdx.y * HF_BM;
+    // what this CTA converts: 128 weight rows from n0, 128 activation columns from m0.  It also multiplies just these
+    // with one another, or, as one of a pair (blockIdx.x even: first, odd: second), its columns with the rows of both.
+    const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
+    const int64_t n0 = (int64_t)blockIdx.x * HF_BN, m0 = (int64_t)blockIdx.y * (PAIR ? 2 * HF_BM : HF_BM) + rank * HF_BM;
+    constexpr uint32_t A_COL = PAIR ? HF_TMEM_A_COL_PAIR : HF_TMEM_A_COL;
     // this CTA's chunks of K: c counts them from 0 (ring slots, parities), c0 + c is the chunk of the matrix (copies)
     const int c0 = (int)blockIdx.z * p.chunks_per_split;
     const int n_chunks = min(p.chunks_per_split, p.K / SUPER - c0);
 
     if (tid == 0) {
         for (int s = 0; s < HF_STAGES; ++s) {
-            mbar_init(&stage_full[s], HF_GROUP_WARPS);
+            mbar_init(&stage_full[s], PAIR ? 2 * HF_GROUP_WARPS : HF_GROUP_WARPS);
             mbar_init(&stage_empty[s], 1);
         }
         mbar_init(acc_full, 1);
@@ -292,13 +350,19 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read by the tensor core
     }
     if (warp == HF_MMA_WARP) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(HF_TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(HF_TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(HF_TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();  // both CTAs' barriers are set up before the other arrives on them
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
     // Programmatic dependent launch: everything above ran while the previous kernel (the activation quantizer, as a
@@ -348,7 +412,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
                     uint4 v[9];
 #pragma unroll
                     for (int i = 0; i < 9; ++i) v[i] = lds_v4(raw + i * 16);
-                    hf_convert_activation_col(st, row, v, tmem + ((uint32_t)((gw & 3) * 32) << 16) + HF_TMEM_A_COL + s * HF_TMEM_A_STAGE_COLS);
+                    hf_convert_activation_col(st, row, v, tmem + ((uint32_t)((gw & 3) * 32) << 16) + A_COL + s * HF_TMEM_A_STAGE_COLS);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&rawx_empty[s]);
                     tc_fence_before();
@@ -356,65 +420,73 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
                 if (stamps) hf_stamp(p, gw >> 2, c, 4);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // tiles are read by the tensor core
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&stage_full[s]);
+                if (lane == 0) {
+                    if (PAIR)
+                        mbar_arrive_leader(&stage_full[s]);
+                    else
+                        mbar_arrive(&stage_full[s]);
+                }
                 if (stamps) hf_stamp(p, gw >> 2, c, 5);
             }
         }
 
-        // epilogue: warp w reads TMEM lanes 32 * (w % 4) .. (activation columns) and 32 of the 128 weight rows, and
-        // turns the 32 x 32 block around in shared memory (the operand stages are free by now) so that a store
-        // instruction writes 128 contiguous bytes of one output row
+        // epilogue: warp w reads TMEM lanes 32 * (w % 4) .. (activation columns) and 32 (of a pair's 256: twice 32) of the
+        // tile's weight rows, and turns each 32 x 32 block around in shared memory (the operand stages are free by now)
+        // so that a store instruction writes 128 contiguous bytes of one output row.  K is only split without pairs.
         if (alive && __all_sync(0xFFFFFFFFu, mbar_wait_bounded(acc_full, 0u, p.fault))) {
             tc_fence_after();
             asm volatile("griddepcontrol.wait;" ::: "memory");  // (long past: orders the stores to y after the previous kernel)
-            const int cb = warp >> 2;  // which 32 of the 128 weight rows
+            constexpr int BLOCKS = PAIR ? 2 : 1;
             const uint32_t stage_blk = sbase + warp * (32 * HF_OUT_PITCH * 4);
             const int64_t m_first = m0 + (warp & 3) * 32;
-            uint32_t v[32];
-            tmem_ld32_nowait(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(cb * 32), v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) sts_f32(stage_blk + (lane * HF_OUT_PITCH + j) * 4, __uint_as_float(v[j]));
-            __syncwarp();
-            const int64_t n = n0 + cb * 32 + lane;
-            const int z = (int)blockIdx.z;
-            int *sem = p.k_splits > 1 ? p.tile_sem + (blockIdx.y * gridDim.x + blockIdx.x) : nullptr;
+            const int z = PAIR ? 0 : (int)blockIdx.z;
+            int *sem = !PAIR && p.k_splits > 1 ? p.tile_sem + (blockIdx.y * gridDim.x + blockIdx.x) : nullptr;
             bool go = true;
-            if (z > 0) {
-                // the splits below this one have added their parts: all sixteen warps of each
-                if (lane == 0) {
-                    go = false;
-                    for (uint32_t spin = 0; spin < p.poll_limit && !go; ++spin) {
-                        int seen;
-                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(sem) : "memory");
-                        go = seen >= HF_PROD_WARPS * z;
+#pragma unroll 1
+            for (int blk = 0; blk < BLOCKS; ++blk) {
+                const int cb = (warp >> 2) * BLOCKS + blk;  // which 32 of the tile's weight rows
+                uint32_t v[32];
+                tmem_ld32_nowait(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(cb * 32), v);
+                tmem_ld_wait();
+                __syncwarp();  // the block before has been read
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sts_f32(stage_blk + (lane * HF_OUT_PITCH + j) * 4, __uint_as_float(v[j]));
+                __syncwarp();
+                const int64_t n = n0 - rank * HF_BN + cb * 32 + lane;
+                if (z > 0) {
+                    // the splits below this one have added their parts: all sixteen warps of each
+                    if (lane == 0) {
+                        go = false;
+                        for (uint32_t spin = 0; spin < p.poll_limit && !go; ++spin) {
+                            int seen;
+                            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(sem) : "memory");
+                            go = seen >= HF_PROD_WARPS * z;
+                        }
+                        if (!go) report_fault(p.fault, 1);
                     }
-                    if (!go) report_fault(p.fault, 1);
-                }
-                go = __shfl_sync(0xFFFFFFFFu, go ? 1 : 0, 0) != 0;
-                __threadfence();  // every lane's reads of y come after the count was seen
-            }
-            if (z > 0) {
-                // all of this lane's partial sums of the earlier splits are requested before the first is used
-                float prev[32];
+                    go = __shfl_sync(0xFFFFFFFFu, go ? 1 : 0, 0) != 0;
+                    __threadfence();  // every lane's reads of y come after the count was seen
+                    // all of this lane's partial sums of the earlier splits are requested before the first is used
+                    float prev[32];
 #pragma unroll
-                for (int rr = 0; rr < 32; ++rr) {
-                    prev[rr] = 0.0f;
-                    if (go && m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
-                        prev[rr] = __ldcg(p.y + (m_first + rr) * p.N + n);
-                }
+                    for (int rr = 0; rr < 32; ++rr) {
+                        prev[rr] = 0.0f;
+                        if (go && m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
+                            prev[rr] = __ldcg(p.y + (m_first + rr) * p.N + n);
+                    }
 #pragma unroll
-                for (int rr = 0; rr < 32; ++rr) {
-                    const float val = __uint_as_float(lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4)) + prev[rr];
-                    if (go && m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
-                        p.y[(m_first + rr) * p.N + n] = val;
-                }
-            } else {
+                    for (int rr = 0; rr < 32; ++rr) {
+                        const float val = __uint_as_float(lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4)) + prev[rr];
+                        if (go && m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
+                            p.y[(m_first + rr) * p.N + n] = val;
+                    }
+                } else {
 #pragma unroll 8
-                for (int rr = 0; rr < 32; ++rr) {
-                    const uint32_t val = lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4);
-                    if (m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
-                        p.y[(m_first + rr) * p.N + n] = __uint_as_float(val);
+                    for (int rr = 0; rr < 32; ++rr) {
+                        const uint32_t val = lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4);
+                        if (m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
+                            p.y[(m_first + rr) * p.N + n] = __uint_as_float(val);
+                    }
                 }
             }
             if (sem != nullptr) {
@@ -459,42 +531,62 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
                 }
             }
         }
-    } else if (lane == 0) {
+    } else if (lane == 0 && rank == 0) {
         // =============================== MMA issuer ============================================
-
-        const uint32_t idesc = tc_idesc_f16(HF_BM, HF_BN);
+        // (of a pair: the first CTA's, for both)
+        const uint32_t idesc = PAIR ? tc_idesc_f16(2 * HF_BM, 2 * HF_BN) : tc_idesc_f16(HF_BM, HF_BN);
         int s = 0;
         uint32_t parity = 0;
         bool alive = true;
         for (int c = 0; c < n_chunks; ++c) {
-            if (!mbar_wait_bounded(&stage_full[s], parity, p.fault)) {
+            if (!(PAIR ? mbar_wait_bounded_cluster(&stage_full[s], parity, p.fault) : mbar_wait_bounded(&stage_full[s], parity, p.fault))) {
                 alive = false;
                 break;
             }
-            const uint32_t st = sbase + s * HF_STAGE_BYTES;
+            const uint32_t st = sbase + s * HF_STAGE_BYTES, a_tmem = tmem + A_COL + s * HF_TMEM_A_STAGE_COLS;
             tc_fence_after();
             hf_stamp(p, 2, c, 0);
-            tc_mma_f16(tmem, tc_desc(st + HF_ZA_OFF), tc_desc(st + HF_ZB_OFF), idesc, c > 0 ? 1u : 0u);
+            const uint32_t more = c > 0 ? 1u : 0u;
+            if (PAIR)
+                tc_mma_f16_pair(tmem, tc_desc(st + HF_ZA_OFF), tc_desc(st + HF_ZB_OFF), idesc, more);
+            else
+                tc_mma_f16(tmem, tc_desc(st + HF_ZA_OFF), tc_desc(st + HF_ZB_OFF), idesc, more);
 #pragma unroll
             for (int t = 0; t < HF_KT; ++t) {
-                tc_mma_f16_ts(tmem, tmem + HF_TMEM_A_COL + s * HF_TMEM_A_STAGE_COLS + t * 8, tc_desc(st + HF_B_OFF + t * TC_TILE), idesc, 1u);
+                if (PAIR)
+                    tc_mma_f16_ts_pair(tmem, a_tmem + t * 8, tc_desc(st + HF_B_OFF + t * TC_TILE), idesc, 1u);
+                else
+                    tc_mma_f16_ts(tmem, a_tmem + t * 8, tc_desc(st + HF_B_OFF + t * TC_TILE), idesc, 1u);
             }
-            tc_commit(&stage_empty[s]);  // the stage may be overwritten once these MMAs have read it
+            // the stage may be overwritten once these MMAs have read it
+            if (PAIR)
+                tc_commit_pair(&stage_empty[s]);
+            else
+                tc_commit(&stage_empty[s]);
             hf_stamp(p, 2, c, 1);
             if (++s == HF_STAGES) {
                 s = 0;
                 parity ^= 1u;
             }
         }
-        if (alive) tc_commit(acc_full);
+        if (alive) {
+            if (PAIR)
+                tc_commit_pair(acc_full);
+            else
+                tc_commit(acc_full);
+        }
     }
 
     // common exit: nobody touches tensor memory any more, release it
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();  // nor does the other CTA, which may still arrive on this one's barriers until here
     if (warp == HF_MMA_WARP) {
         __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HF_TMEM_COLS) : "memory");
+        if (PAIR)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HF_TMEM_COLS) : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HF_TMEM_COLS) : "memory");
     }
 }
 
@@ -543,7 +635,17 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     // 46.5; three and four splits are no faster (44.3, 46.4 us at K = 11008): every further split adds an ordered
     // pass over the tile in y.
     const int n_chunks = (int)(K / SUPER);
-    const int splits = gx * gy * 2 <= caps.sm_count && gx * gy <= HF_MAX_SPLIT_TILES && n_chunks >= 32 ? 2 : 1;
+    int splits = gx * gy * 2 <= caps.sm_count && gx * gy <= HF_MAX_SPLIT_TILES && n_chunks >= 32 ? 2 : 1;
+    // A pair of CTAs converts as many operands per stage as two CTAs on their own and multiplies twice as much, in 1.05 us
+    // a stage against 0.73: pairs are taken where that makes up for fewer waves (stages per SM: waves times chunks, or
+    // half of them with two CTAs per tile).  Single / pairs, K = 4096: N = 4096, M = 1024 57 / 40 us; N = 11008, M = 256
+    // 57 / 40, M = 512 84 / 77; K = 8192, N = 28672: M = 256 205 / 147, M = 2048 1326 / 997.  Pairs that also split K were
+    // slower than single CTAs that need not (K = N = 4096, M = 512 35.8 against 29.6 us).
+    const int64_t pair_gx = (N + 2 * HF_BN - 1) / (2 * HF_BN) * 2, pair_gy = (M + 2 * HF_BM - 1) / (2 * HF_BM);
+    const int64_t waves = (gx * gy * splits + caps.sm_count - 1) / caps.sm_count;
+    const int64_t pair_waves = (pair_gx * pair_gy + caps.sm_count - 1) / caps.sm_count;
+    const bool pair = pair_waves * splits * 13 < waves * 9;
+    if (pair) splits = 1;
     p.chunks_per_split = ((n_chunks + splits - 1) / splits + 1) / 2 * 2;
     p.k_splits = (n_chunks + p.chunks_per_split - 1) / p.chunks_per_split;
     p.tile_sem = nullptr;
@@ -559,19 +661,23 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
                      ? encode_byte_map(&x_map, d_xq, Q8_BYTES, (uint64_t)p.n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, 128)
                      : encode_byte_map(&x_map, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, 128))
         return rc;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(gemm_q4_0_q8_1_f16_kernel), HF_SMEM_BYTES)) return rc;
+    const auto kernel = pair ? gemm_q4_0_q8_1_f16_kernel<true> : gemm_q4_0_q8_1_f16_kernel<false>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
     (void)cudaGetLastError();  // a stale error of an earlier, unrelated call must not be taken for this launch's
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)gx, (unsigned)gy, (unsigned)p.k_splits);
+    cfg.gridDim = pair ? dim3((unsigned)pair_gx, (unsigned)pair_gy, 1u) : dim3((unsigned)gx, (unsigned)gy, (unsigned)p.k_splits);
     cfg.blockDim = dim3(HF_THREADS);
     cfg.dynamicSmemBytes = HF_SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_q4_0_q8_1_f16_kernel, p, w_map, x_map));
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = pair ? 2 : 1;
+    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, w_map, x_map));
     return JQ_OK;
 }
 

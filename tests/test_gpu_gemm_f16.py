@@ -101,6 +101,18 @@ def test_gemm_f16_matches_integer_kernel_closely(env):
     assert env.O.err_max_rel(y_f16, y_int) <= TOL_F16_FORMULA
 
 
+# More tiles than SMs, so that pairs of CTAs share 256 x 256 tiles: the last pair's second CTA without rows (18690 = 73 * 256
+# + 2) or with one, its columns a few or all but one; one stage pair, and more stages than the ring holds.
+@pytest.mark.parametrize("K,N,M", [(256, 18690, 130), (768, 18690, 255), (1280, 18817, 256), (512, 9473, 400)])
+@pytest.mark.parametrize("order", [0, 1])
+def test_gemm_f16_pairs_of_ctas(env, K, N, M, order):
+    rng = np.random.default_rng(K + N + M + order)
+    w = (rng.standard_normal((N, K), dtype=np.float32) * np.float32(0.02)).astype(np.float32)
+    x = rng.standard_normal((M, K), dtype=np.float32)
+    rows = np.unique(np.concatenate([rng.choice(N, size=96, replace=False), [0, 127, 128, 255, 256, N - 2, N - 1]]))
+    _check(env, env.O.quantize_q4_0(w), x, K, N, M, order, env.c.S_SUM_X, rows)
+
+
 @pytest.mark.parametrize("K,N,M", [(4096, 4096, 128), (11008, 4096, 128), (8192, 300, 70), (2048, 1000, 64)])
 def test_gemm_f16_split_k_is_ordered(env, K, N, M):
     """Few output tiles and a long K: the kernel splits K over several CTAs per tile, which add their parts to y in a

@@ -435,17 +435,17 @@ int jq_linear_q4_0_multi_device(void *stream, int n_mats, const void *const *d_w
     if (((uintptr_t)d_x & 15u) != 0 || ((uintptr_t)d_xq & 15u) != 0 || ((uintptr_t)d_ws & 15u) != 0)
         return set_error(JQ_ERR_ALIGN, "activations, Q8_1 blocks and workspace must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // one launch over the concatenated rows while the decode kernels take the shape
+    // one launch over the concatenated rows where a kernel takes the shape
     bool all_rows = true;
     for (int i = 0; i < n_mats; ++i) all_rows = all_rows && N[i] > 0;
+    MultiMat mm{};
+    mm.n = n_mats;
+    for (int i = 0; i < n_mats; ++i) {
+        mm.w[i] = d_w[i];
+        mm.y[i] = d_y[i];
+        mm.rows[i] = N[i];
+    }
     if (K > 0 && M < FP16_OPERANDS_MIN_COLUMNS && all_rows) {
-        MultiMat mm{};
-        mm.n = n_mats;
-        for (int i = 0; i < n_mats; ++i) {
-            mm.w[i] = d_w[i];
-            mm.y[i] = d_y[i];
-            mm.rows[i] = N[i];
-        }
         const bool fuse_quantizer = d_x != nullptr && M <= 8 && fuse_quantizer_pays(M, K);
         if (d_x != nullptr && !fuse_quantizer) {
             if (int rc = launch_quantize_q8_1(st, d_x, d_ws, K, M, JQ_ORDER_COL_KSUPER, s_mode)) return rc;
@@ -471,6 +471,11 @@ int jq_linear_q4_0_multi_device(void *stream, int n_mats, const void *const *d_w
     if (d_x != nullptr && K > 0) {
         if (int rc = launch_quantize_q8_1(st, d_x, d_ws, K, M, JQ_ORDER_COL_KSUPER, s_mode)) return rc;
         d_xq = d_ws;
+    }
+    if (K > 0 && M >= FP16_OPERANDS_MIN_COLUMNS && all_rows && option_value(JQ_OPT_PREFILL_EXACT) == 0) {
+        // together they fill the SMs better than one after the other: a tile takes a CTA as long however many there are
+        const int rc = launch_gemm_f16(st, nullptr, d_xq, nullptr, K, n_total, M, JQ_ORDER_COL_KSUPER, &mm);
+        if (rc != JQ_ERR_UNSUPPORTED) return rc;
     }
     for (int i = 0; i < n_mats; ++i) {
         if (N[i] == 0) continue;

@@ -99,17 +99,26 @@ constexpr uint32_t H2_1152 = 0x64806480u;
 constexpr uint32_t H2_SIXTEENTH = 0x2C002C00u;
 constexpr uint32_t H2_MINUS_72 = 0xD480D480u;
 
+constexpr int HF_MAX_MATS = 4;
+struct HfMaps {
+    CUtensorMap w[HF_MAX_MATS];
+    CUtensorMap x;
+};
+
 struct HfParams {
-    const uint8_t *w;
-    const uint8_t *xq;
-    float *y;
+    // Up to four weight matrices that share K and the activations: the CTAs with blockIdx.x in [tile_begin[i],
+    // tile_begin[i + 1]) have 128 rows each of matrix i (whole pairs of CTAs, if they work in pairs), which goes to y[i],
+    // an [M][rows[i]] array.
+    float *y[HF_MAX_MATS];
+    int64_t rows[HF_MAX_MATS];
+    int tile_begin[HF_MAX_MATS + 1];
+    int n_mats;
     int *fault;
 #ifdef JQ_BOUNDS_CHECK
-    Extent ext_y;  // range-checked debug build (the operand loads are tensor copies: their maps bound them)
+    Extent ext_y[HF_MAX_MATS];  // range-checked debug build (the operand loads are tensor copies: their maps bound them)
 #endif
-    int64_t N, M;
-    int K, order, n_super;
-    uint32_t row_bytes;
+    int64_t M;
+    int K, order;
     unsigned long long *trace;  // tracing aid (or nullptr): SM clock stamps of CTA (0,0), rows of 8
     // Split K (few output tiles, long K): blockIdx.z takes the 128-value chunks [z * chunks_per_split, ...) and the
     // splits of a tile add their partial results to y in the order of z (so the sum is formed the same way every
@@ -301,7 +310,7 @@ __device__ __forceinline__ void hf_convert_activation_col(uint32_t st, int r, co
 
 template <bool PAIR>
 __global__ void __launch_bounds__(HF_THREADS, 1)
-gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map) {
+gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_constant__ HfMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + HF_BAR_OFF);
@@ -319,7 +328,9 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
     // what this CTA converts: 128 weight rows from n0, 128 activation columns from m0.  It also multiplies just these
     // with one another, or, as one of a pair (blockIdx.x even: first, odd: second), its columns with the rows of both.
     const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
-    const int64_t n0 = (int64_t)blockIdx.x * HF_BN, m0 = (int64_t)blockIdx.y * (PAIR ? 2 * HF_BM : HF_BM) + rank * HF_BM;
+    int mat = 0;
+    while (mat + 1 < p.n_mats && (int)blockIdx.x >= p.tile_begin[mat + 1]) ++mat;
+    const int64_t n0 = (int64_t)((int)blockIdx.x - p.tile_begin[mat]) * HF_BN, m0 = (int64_t)blockIdx.y * (PAIR ? 2 * HF_BM : HF_BM) + rank * HF_BM;
     constexpr uint32_t A_COL = PAIR ? HF_TMEM_A_COL_PAIR : HF_TMEM_A_COL;
     // this CTA's chunks of K: c counts them from 0 (ring slots, parities), c0 + c is the chunk of the matrix (copies)
     const int c0 = (int)blockIdx.z * p.chunks_per_split;
@@ -437,6 +448,8 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
             tc_fence_after();
             asm volatile("griddepcontrol.wait;" ::: "memory");  // (long past: orders the stores to y after the previous kernel)
             constexpr int BLOCKS = PAIR ? 2 : 1;
+            float *const y = p.y[mat];
+            const int64_t N = p.rows[mat];
             const uint32_t stage_blk = sbase + warp * (32 * HF_OUT_PITCH * 4);
             const int64_t m_first = m0 + (warp & 3) * 32;
             const int z = PAIR ? 0 : (int)blockIdx.z;
@@ -471,21 +484,21 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
                     for (int rr = 0; rr < 32; ++rr) {
                         prev[rr] = 0.0f;
-                        if (go && m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
-                            prev[rr] = __ldcg(p.y + (m_first + rr) * p.N + n);
+                        if (go && m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[mat], y + (m_first + rr) * N + n, sizeof(float), p.fault))
+                            prev[rr] = __ldcg(y + (m_first + rr) * N + n);
                     }
 #pragma unroll
                     for (int rr = 0; rr < 32; ++rr) {
                         const float val = __uint_as_float(lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4)) + prev[rr];
-                        if (go && m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
-                            p.y[(m_first + rr) * p.N + n] = val;
+                        if (go && m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[mat], y + (m_first + rr) * N + n, sizeof(float), p.fault))
+                            y[(m_first + rr) * N + n] = val;
                     }
                 } else {
 #pragma unroll 8
                     for (int rr = 0; rr < 32; ++rr) {
                         const uint32_t val = lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4);
-                        if (m_first + rr < p.M && n < p.N && JQ_IN_EXTENT(p.ext_y, p.y + (m_first + rr) * p.N + n, sizeof(float), p.fault))
-                            p.y[(m_first + rr) * p.N + n] = __uint_as_float(val);
+                        if (m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[mat], y + (m_first + rr) * N + n, sizeof(float), p.fault))
+                            y[(m_first + rr) * N + n] = __uint_as_float(val);
                     }
                 }
             }
@@ -510,20 +523,20 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ CUtensorMap 
                 if (c == 0 && p.static_weights) {
                     // the first pair of weight chunks is requested ahead of the wait for the previous kernel
                     mbar_arrive_expect_tx(&raww_full[0], HF_RAW_SLOT_BYTES);
-                    tma_load_2d(sbase + HF_RAWW_OFF, &w_map, (c0 >> 1) * Q8_BYTES, (int)n0, &raww_full[0]);
+                    tma_load_2d(sbase + HF_RAWW_OFF, &maps.w[mat], (c0 >> 1) * Q8_BYTES, (int)n0, &raww_full[0]);
                     asm volatile("griddepcontrol.wait;" ::: "memory");
                 } else if ((c & 1) == 0) {
                     const int pair = c >> 1, ws = pair & 1;
                     if (pair >= HF_RAWW_SLOTS && !mbar_wait_bounded(&raww_empty[ws], (uint32_t)((pair >> 1) - 1) & 1u, p.fault)) break;
                     mbar_arrive_expect_tx(&raww_full[ws], HF_RAW_SLOT_BYTES);
-                    tma_load_2d(sbase + HF_RAWW_OFF + ws * HF_RAW_SLOT_BYTES, &w_map, ((c0 + c) >> 1) * Q8_BYTES, (int)n0, &raww_full[ws]);
+                    tma_load_2d(sbase + HF_RAWW_OFF + ws * HF_RAW_SLOT_BYTES, &maps.w[mat], ((c0 + c) >> 1) * Q8_BYTES, (int)n0, &raww_full[ws]);
                 }
                 if (xround > 0 && !mbar_wait_bounded(&rawx_empty[xs], (xround - 1) & 1u, p.fault)) break;
                 mbar_arrive_expect_tx(&rawx_full[xs], HF_RAW_SLOT_BYTES);
                 if (p.order == JQ_ORDER_KSUPER_COL) {  // the tensor is [n_super * M blocks][144 bytes]
-                    tma_load_2d(sbase + HF_RAWX_OFF + xs * HF_RAW_SLOT_BYTES, &x_map, 0, (int)((int64_t)(c0 + c) * p.M + m0), &rawx_full[xs]);
+                    tma_load_2d(sbase + HF_RAWX_OFF + xs * HF_RAW_SLOT_BYTES, &maps.x, 0, (int)((int64_t)(c0 + c) * p.M + m0), &rawx_full[xs]);
                 } else {                               // the tensor is [M columns][n_super * 144 bytes]
-                    tma_load_2d(sbase + HF_RAWX_OFF + xs * HF_RAW_SLOT_BYTES, &x_map, (c0 + c) * Q8_BYTES, (int)m0, &rawx_full[xs]);
+                    tma_load_2d(sbase + HF_RAWX_OFF + xs * HF_RAW_SLOT_BYTES, &maps.x, (c0 + c) * Q8_BYTES, (int)m0, &rawx_full[xs]);
                 }
                 if (++xs == HF_RAWX_SLOTS) {
                     xs = 0;
@@ -600,32 +613,35 @@ int reset_gemm_f16_split_state() {
 }
 
 int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N, int64_t M,
-                    int order) {
+                    int order, const MultiMat *multi) {
     // a weight row's pitch, K / 32 * 18 bytes, must be a multiple of 16 for the tensor copies
     if (K % (2 * SUPER) != 0) return set_error(JQ_ERR_UNSUPPORTED, "fp16-operand tcgen05 GEMM needs K %% 256 == 0 (K = %lld)", (long long)K);
-    if (((uintptr_t)d_w & 15u) != 0 || ((uintptr_t)d_xq & 15u) != 0)
-        return set_error(JQ_ERR_UNSUPPORTED, "fp16-operand tcgen05 GEMM needs 16-byte aligned operands");
+    const void *w[HF_MAX_MATS] = {};
+    HfParams p{};
+    p.n_mats = multi != nullptr ? multi->n : 1;
+    if (p.n_mats < 1 || p.n_mats > HF_MAX_MATS) return set_error(JQ_ERR_INVALID_ARG, "1 to %d weight matrices per launch", HF_MAX_MATS);
+    uintptr_t bits = (uintptr_t)d_xq;
+    int64_t gx = 0, pair_gx = 0;  // CTAs along the weight rows, on their own and in pairs
+    for (int i = 0; i < p.n_mats; ++i) {
+        w[i] = multi != nullptr ? multi->w[i] : d_w;
+        p.y[i] = multi != nullptr ? multi->y[i] : d_y;
+        p.rows[i] = multi != nullptr ? multi->rows[i] : N;
+        bits |= (uintptr_t)w[i];
+        gx += (p.rows[i] + HF_BN - 1) / HF_BN;
+        pair_gx += (p.rows[i] + 2 * HF_BN - 1) / (2 * HF_BN) * 2;
+    }
+    if ((bits & 15u) != 0) return set_error(JQ_ERR_UNSUPPORTED, "fp16-operand tcgen05 GEMM needs 16-byte aligned operands");
     if (N == 0 || M == 0) return JQ_OK;
     DeviceCaps caps;
     if (int rc = device_caps(&caps)) return rc;
     if (caps.cc / 10 != 10) return set_error(JQ_ERR_UNSUPPORTED, "tcgen05 needs an sm_100-class device");
-    const int64_t gx = (N + HF_BN - 1) / HF_BN, gy = (M + HF_BM - 1) / HF_BM;
+    const int64_t gy = (M + HF_BM - 1) / HF_BM;
     if (gy > 65535 || K > (1 << 24) || (K / SUPER) * M >= ((int64_t)1 << 31) || N >= ((int64_t)1 << 31))
         return set_error(JQ_ERR_UNSUPPORTED, "shape too large for the tcgen05 GEMM");
-    HfParams p{};
-    p.w = static_cast<const uint8_t *>(d_w);
-    p.xq = static_cast<const uint8_t *>(d_xq);
-    p.y = d_y;
     p.fault = device_fault_ptr();
-#ifdef JQ_BOUNDS_CHECK
-    p.ext_y = make_extent(d_y, (unsigned long long)M * (unsigned long long)N * sizeof(float));
-#endif
-    p.N = N;
     p.M = M;
     p.K = (int)K;
     p.order = order;
-    p.n_super = (int)(K / SUPER);
-    p.row_bytes = (uint32_t)(K / QK * Q4_BYTES);
     p.trace = static_cast<unsigned long long *>(next_trace_slot());
     p.poll_limit = wait_poll_limit();
     p.static_weights = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 1 : 0;
@@ -641,7 +657,7 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     // half of them with two CTAs per tile).  Single / pairs, K = 4096: N = 4096, M = 1024 57 / 40 us; N = 11008, M = 256
     // 57 / 40, M = 512 84 / 77; K = 8192, N = 28672: M = 256 205 / 147, M = 2048 1326 / 997.  Pairs that also split K were
     // slower than single CTAs that need not (K = N = 4096, M = 512 35.8 against 29.6 us).
-    const int64_t pair_gx = (N + 2 * HF_BN - 1) / (2 * HF_BN) * 2, pair_gy = (M + 2 * HF_BM - 1) / (2 * HF_BM);
+    const int64_t pair_gy = (M + 2 * HF_BM - 1) / (2 * HF_BM);
     const int64_t waves = (gx * gy * splits + caps.sm_count - 1) / caps.sm_count;
     const int64_t pair_waves = (pair_gx * pair_gy + caps.sm_count - 1) / caps.sm_count;
     const bool pair = pair_waves * splits * 13 < waves * 9;
@@ -654,12 +670,22 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
         JQ_CUDA_TRY(cudaGetSymbolAddress(&sem, g_tile_sem));
         p.tile_sem = static_cast<int *>(sem);
     }
-    CUtensorMap w_map, x_map;
-    if (int rc = encode_byte_map(&w_map, d_w, p.row_bytes, (uint64_t)N, p.row_bytes, Q8_BYTES, 128)) return rc;
-    const uint64_t x_row = (uint64_t)p.n_super * Q8_BYTES;
+    const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
+    HfMaps maps{};
+    p.tile_begin[0] = 0;
+    for (int i = 0; i < p.n_mats; ++i) {
+        const int64_t per = pair ? 2 : 1;
+        p.tile_begin[i + 1] = p.tile_begin[i] + (int)((p.rows[i] + per * HF_BN - 1) / (per * HF_BN) * per);
+        if (int rc = encode_byte_map(&maps.w[i], w[i], row_bytes, (uint64_t)p.rows[i], row_bytes, Q8_BYTES, 128)) return rc;
+#ifdef JQ_BOUNDS_CHECK
+        p.ext_y[i] = make_extent(p.y[i], (unsigned long long)M * (unsigned long long)p.rows[i] * sizeof(float));
+#endif
+    }
+    const int64_t n_super = K / SUPER;
+    const uint64_t x_row = (uint64_t)n_super * Q8_BYTES;
     if (int rc = order == JQ_ORDER_KSUPER_COL
-                     ? encode_byte_map(&x_map, d_xq, Q8_BYTES, (uint64_t)p.n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, 128)
-                     : encode_byte_map(&x_map, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, 128))
+                     ? encode_byte_map(&maps.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, 128)
+                     : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, 128))
         return rc;
     const auto kernel = pair ? gemm_q4_0_q8_1_f16_kernel<true> : gemm_q4_0_q8_1_f16_kernel<false>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
@@ -677,7 +703,7 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     attr[1].val.clusterDim.x = 2;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = pair ? 2 : 1;
-    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, w_map, x_map));
+    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, maps));
     return JQ_OK;
 }
 

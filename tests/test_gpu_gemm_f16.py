@@ -113,6 +113,20 @@ def test_gemm_f16_pairs_of_ctas(env, K, N, M, order):
     _check(env, env.O.quantize_q4_0(w), x, K, N, M, order, env.c.S_SUM_X, rows)
 
 
+@pytest.mark.parametrize("K,rows,M", [(512, [300, 1, 128, 257], 64), (256, [9400, 9290], 130), (4096, [128, 200], 100)])
+def test_gemm_f16_several_matrices(env, K, rows, M):
+    """Several matrices in one launch (single CTAs, pairs, split K): each row against separate calls, whose sums over K may
+    be split elsewhere (fp32 additions in another order)."""
+    c = env.c
+    rng = np.random.default_rng(K + M)
+    ws = [c.quantize_q4_0(env.up((rng.standard_normal((n, K), dtype=np.float32) * np.float32(0.02)))) for n in rows]
+    xq = c.quantize_q8_1(env.up(rng.standard_normal((M, K), dtype=np.float32)), c.ORDER_COL_KSUPER, c.S_D_SUM_Q)
+    outs = c.linear_q4_0_multi(ws, rows, xq=xq, K=K, M=M)
+    for w, n, y in zip(ws, rows, outs):
+        want = c.mul_mat_q4_0_q8_1(w, xq, K, n, M, c.ORDER_COL_KSUPER, c.KERNEL_GEMM_F16)
+        assert env.O.err_max_rel(y.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+
+
 @pytest.mark.parametrize("K,N,M", [(4096, 4096, 128), (11008, 4096, 128), (8192, 300, 70), (2048, 1000, 64)])
 def test_gemm_f16_split_k_is_ordered(env, K, N, M):
     """Few output tiles and a long K: the kernel splits K over several CTAs per tile, which add their parts to y in a

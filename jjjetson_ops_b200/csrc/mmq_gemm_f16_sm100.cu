@@ -99,46 +99,44 @@ constexpr uint32_t H2_1152 = 0x64806480u;
 constexpr uint32_t H2_SIXTEENTH = 0x2C002C00u;
 constexpr uint32_t H2_MINUS_72 = 0xD480D480u;
 
+constexpr int HF_MAX_SPLITS = 8;    // CTAs per tile along K: the largest portable cluster
 constexpr int HF_MAX_MATS = 4;
+template <int MATS>
 struct HfMaps {
-    CUtensorMap w[HF_MAX_MATS];
+    CUtensorMap w[MATS];
     CUtensorMap x;
 };
 
+// The kernel has an instance for one matrix and one for up to four, and takes these by value: a look-up by matrix needs
+// them addressable (__grid_constant__), and then fields are read again in every turn of the conversion loop, 2 to 4 % of a
+// launch (K = 4096, N = 11008, M = 128 30.4 against 31.5 us).
+template <int MATS>
 struct HfParams {
     // Up to four weight matrices that share K and the activations: the CTAs with blockIdx.x in [tile_begin[i],
     // tile_begin[i + 1]) have 128 rows each of matrix i (whole pairs of CTAs, if they work in pairs), which goes to y[i],
     // an [M][rows[i]] array.
-    float *y[HF_MAX_MATS];
-    int64_t rows[HF_MAX_MATS];
-    int tile_begin[HF_MAX_MATS + 1];
+    float *y[MATS];
+    int64_t rows[MATS];
+    int tile_begin[MATS + 1];
     int n_mats;
     int *fault;
 #ifdef JQ_BOUNDS_CHECK
-    Extent ext_y[HF_MAX_MATS];  // range-checked debug build (the operand loads are tensor copies: their maps bound them)
+    Extent ext_y[MATS];  // range-checked debug build (the operand loads are tensor copies: their maps bound them)
 #endif
     int64_t M;
     int K, order;
     unsigned long long *trace;  // tracing aid (or nullptr): SM clock stamps of CTA (0,0), rows of 8
-    // Split K (few output tiles, long K): blockIdx.z takes the 128-value chunks [z * chunks_per_split, ...) and the
-    // splits of a tile add their partial results to y in the order of z (so the sum is formed the same way every
-    // time): tile_sem[tile] counts the epilogue warps that have finished, split z goes ahead at 16 * z, the last
-    // warp of the last split puts the count back to zero.
+    // Split K (few output tiles): the CTAs of a tile, blockIdx.z of k_splits, are a cluster and take the 128-value chunks
+    // [z * chunks_per_split, ...) each; their partial tiles meet in shared memory.
     int k_splits, chunks_per_split;
-    int *tile_sem;
-    uint32_t poll_limit;
     int static_weights;  // the weight copies may start before the previous kernel in the stream has finished
 };
-
-// Counts of finished epilogue warps per output tile (split K); zero between launches.  Part of the library image, like
-// the fault word: launches that split K must not overlap on one device (they do not on one stream).
-constexpr int HF_MAX_SPLIT_TILES = 128;
-__device__ int g_tile_sem[HF_MAX_SPLIT_TILES];
 
 // Tracing aid.  Row c (stage, < 64) of block `who`: 0 = weight warp 0, 1 = activation warp 4, 2 = the MMA thread.
 // Producer columns: 0 loop top, 1 past the barrier, 2 copies of stage c + 2 issued, 3 operand stage free,
 // 4 converted, 5 published.  MMA columns: 0 stage seen full, 1 MMAs and commit issued.
-__device__ __forceinline__ void hf_stamp(const HfParams &p, int who, int c, int slot) {
+template <int MATS>
+__device__ __forceinline__ void hf_stamp(const HfParams<MATS> &p, int who, int c, int slot) {
     if (p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && c < 64) {
         p.trace[((who * 64 + c) * 8) + slot] = (unsigned long long)clock64();
     }
@@ -207,6 +205,17 @@ __device__ __forceinline__ bool mbar_wait_bounded_cluster(uint64_t *bar, uint32_
     }
     report_fault(fault, 1);
     return false;
+}
+// shared-memory word of CTA `rank` of the cluster, at this CTA's address of it
+__device__ __forceinline__ float lds_f32_of(uint32_t addr, int rank) {
+    float v;
+    asm volatile(
+        "{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %1, %2;\n\t"
+        "ld.shared::cluster.f32 %0, [remote];\n\t}"
+        : "=f"(v)
+        : "r"(addr), "r"(rank)
+        : "memory");
+    return v;
 }
 __device__ __forceinline__ void cluster_sync() {
     __syncwarp();
@@ -308,9 +317,19 @@ __device__ __forceinline__ void hf_convert_activation_col(uint32_t st, int r, co
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-template <bool PAIR>
+// the matrix this CTA works on
+template <int MATS>
+__device__ __forceinline__ int hf_matrix(const HfParams<MATS> &p) {
+    int mat = 0;
+    if (MATS > 1) {
+        while (mat + 1 < p.n_mats && (int)blockIdx.x >= p.tile_begin[mat + 1]) ++mat;
+    }
+    return mat;
+}
+
+template <bool PAIR, bool SPLIT, int MATS>
 __global__ void __launch_bounds__(HF_THREADS, 1)
-gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_constant__ HfMaps maps) {
+gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps<MATS> maps) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + HF_BAR_OFF);
@@ -328,12 +347,11 @@ gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_const
     // what this CTA converts: 128 weight rows from n0, 128 activation columns from m0.  It also multiplies just these
     // with one another, or, as one of a pair (blockIdx.x even: first, odd: second), its columns with the rows of both.
     const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
-    int mat = 0;
-    while (mat + 1 < p.n_mats && (int)blockIdx.x >= p.tile_begin[mat + 1]) ++mat;
-    const int64_t n0 = (int64_t)((int)blockIdx.x - p.tile_begin[mat]) * HF_BN, m0 = (int64_t)blockIdx.y * (PAIR ? 2 * HF_BM : HF_BM) + rank * HF_BM;
+    const int mat = hf_matrix(p);
+    const int64_t n0 = (int64_t)((int)blockIdx.x - (MATS > 1 ? p.tile_begin[mat] : 0)) * HF_BN, m0 = (int64_t)blockIdx.y * (PAIR ? 2 * HF_BM : HF_BM) + rank * HF_BM;
     constexpr uint32_t A_COL = PAIR ? HF_TMEM_A_COL_PAIR : HF_TMEM_A_COL;
     // this CTA's chunks of K: c counts them from 0 (ring slots, parities), c0 + c is the chunk of the matrix (copies)
-    const int c0 = (int)blockIdx.z * p.chunks_per_split;
+    const int c0 = SPLIT ? (int)blockIdx.z * p.chunks_per_split : 0;
     const int n_chunks = min(p.chunks_per_split, p.K / SUPER - c0);
 
     if (tid == 0) {
@@ -379,6 +397,8 @@ gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_const
     // Programmatic dependent launch: everything above ran while the previous kernel (the activation quantizer, as a
     // rule) was still finishing; the activations are read, and the outputs written, only after it has.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    bool finished = false;  // this epilogue warp has seen the tile complete
 
     if (warp < HF_PROD_WARPS) {
         // =============================== producers, then epilogue ==============================
@@ -448,14 +468,12 @@ gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_const
             tc_fence_after();
             asm volatile("griddepcontrol.wait;" ::: "memory");  // (long past: orders the stores to y after the previous kernel)
             constexpr int BLOCKS = PAIR ? 2 : 1;
-            float *const y = p.y[mat];
-            const int64_t N = p.rows[mat];
+            finished = true;
+            const int out = hf_matrix(p);
+            float *const y = p.y[out];
+            const int64_t N = p.rows[out], m_first = m0 + (warp & 3) * 32;
             const uint32_t stage_blk = sbase + warp * (32 * HF_OUT_PITCH * 4);
-            const int64_t m_first = m0 + (warp & 3) * 32;
-            const int z = PAIR ? 0 : (int)blockIdx.z;
-            int *sem = !PAIR && p.k_splits > 1 ? p.tile_sem + (blockIdx.y * gridDim.x + blockIdx.x) : nullptr;
-            bool go = true;
-#pragma unroll 1
+#pragma unroll
             for (int blk = 0; blk < BLOCKS; ++blk) {
                 const int cb = (warp >> 2) * BLOCKS + blk;  // which 32 of the tile's weight rows
                 uint32_t v[32];
@@ -465,49 +483,13 @@ gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_const
 #pragma unroll
                 for (int j = 0; j < 32; ++j) sts_f32(stage_blk + (lane * HF_OUT_PITCH + j) * 4, __uint_as_float(v[j]));
                 __syncwarp();
+                if (SPLIT) break;  // the parts are added below
                 const int64_t n = n0 - rank * HF_BN + cb * 32 + lane;
-                if (z > 0) {
-                    // the splits below this one have added their parts: all sixteen warps of each
-                    if (lane == 0) {
-                        go = false;
-                        for (uint32_t spin = 0; spin < p.poll_limit && !go; ++spin) {
-                            int seen;
-                            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(sem) : "memory");
-                            go = seen >= HF_PROD_WARPS * z;
-                        }
-                        if (!go) report_fault(p.fault, 1);
-                    }
-                    go = __shfl_sync(0xFFFFFFFFu, go ? 1 : 0, 0) != 0;
-                    __threadfence();  // every lane's reads of y come after the count was seen
-                    // all of this lane's partial sums of the earlier splits are requested before the first is used
-                    float prev[32];
-#pragma unroll
-                    for (int rr = 0; rr < 32; ++rr) {
-                        prev[rr] = 0.0f;
-                        if (go && m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[mat], y + (m_first + rr) * N + n, sizeof(float), p.fault))
-                            prev[rr] = __ldcg(y + (m_first + rr) * N + n);
-                    }
-#pragma unroll
-                    for (int rr = 0; rr < 32; ++rr) {
-                        const float val = __uint_as_float(lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4)) + prev[rr];
-                        if (go && m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[mat], y + (m_first + rr) * N + n, sizeof(float), p.fault))
-                            y[(m_first + rr) * N + n] = val;
-                    }
-                } else {
 #pragma unroll 8
-                    for (int rr = 0; rr < 32; ++rr) {
-                        const uint32_t val = lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4);
-                        if (m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[mat], y + (m_first + rr) * N + n, sizeof(float), p.fault))
-                            y[(m_first + rr) * N + n] = __uint_as_float(val);
-                    }
-                }
-            }
-            if (sem != nullptr) {
-                __syncwarp();
-                if (lane == 0) {
-                    __threadfence();
-                    const int before = atomicAdd(sem, 1);
-                    if (before == HF_PROD_WARPS * p.k_splits - 1) atomicExch(sem, 0);  // the last warp of the last split re-arms the tile
+                for (int rr = 0; rr < 32; ++rr) {
+                    const uint32_t val = lds_u32(stage_blk + (rr * HF_OUT_PITCH + lane) * 4);
+                    if (m_first + rr < p.M && n < N && JQ_IN_EXTENT(p.ext_y[out], y + (m_first + rr) * N + n, sizeof(float), p.fault))
+                        y[(m_first + rr) * N + n] = __uint_as_float(val);
                 }
             }
         }
@@ -590,6 +572,42 @@ gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_const
         }
     }
 
+    if (SPLIT) {
+        // The parts of K: every CTA of the cluster has its partial tile in shared memory and adds up its share of the output
+        // rows over all of them, in the order of z (the same bits every time).
+        const int parts = p.k_splits, z = (int)blockIdx.z;
+        cluster_sync();
+        if (finished) {
+            const int out = hf_matrix(p);
+            float *const y = p.y[out];
+            const int64_t N = p.rows[out], m_first = m0 + (warp & 3) * 32;
+            const uint32_t stage_blk = sbase + warp * (32 * HF_OUT_PITCH * 4);
+            const int64_t n = n0 + (warp >> 2) * 32 + lane;
+            const int end = 32 * (z + 1) / parts;
+#pragma unroll 1
+            for (int r0 = 32 * z / parts; r0 < end; r0 += 4) {
+                float part[4][HF_MAX_SPLITS];
+#pragma unroll
+                for (int q = 0; q < HF_MAX_SPLITS; ++q) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        part[u][q] = 0.0f;
+                        if (q < parts && r0 + u < end) part[u][q] = lds_f32_of(stage_blk + ((r0 + u) * HF_OUT_PITCH + lane) * 4, q);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float v = part[u][0];
+#pragma unroll
+                    for (int q = 1; q < HF_MAX_SPLITS; ++q) v += part[u][q];
+                    const int64_t m = m_first + r0 + u;
+                    if (r0 + u < end && m < p.M && n < N && JQ_IN_EXTENT(p.ext_y[out], y + m * N + n, sizeof(float), p.fault)) y[m * N + n] = v;
+                }
+            }
+        }
+        cluster_sync();  // nobody leaves while another still reads its part
+    }
+
     // common exit: nobody touches tensor memory any more, release it
     tc_fence_before();
     __syncthreads();
@@ -603,21 +621,44 @@ gemm_q4_0_q8_1_f16_kernel(const __grid_constant__ HfParams p, const __grid_const
     }
 }
 
-}  // namespace
-
-int reset_gemm_f16_split_state() {
-    void *sem = nullptr;
-    JQ_CUDA_TRY(cudaGetSymbolAddress(&sem, g_tile_sem));
-    JQ_CUDA_TRY(cudaMemset(sem, 0, sizeof(int) * HF_MAX_SPLIT_TILES));
+template <bool PAIR, bool SPLIT, int MATS>
+int launch_kernel(cudaStream_t st, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
+    const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, MATS>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
+    (void)cudaGetLastError();  // a stale error of an earlier, unrelated call must not be taken for this launch's
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(HF_THREADS);
+    cfg.dynamicSmemBytes = HF_SMEM_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = PAIR ? 2 : 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = (unsigned)p.k_splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = PAIR || SPLIT ? 2 : 1;
+    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, maps));
     return JQ_OK;
 }
+// form: 0 pairs of CTAs, 1 split K, 2 neither
+template <int MATS>
+int launch_form(cudaStream_t st, int form, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
+    if (form == 0) return launch_kernel<true, false, MATS>(st, grid, p, maps);
+    if (form == 1) return launch_kernel<false, true, MATS>(st, grid, p, maps);
+    return launch_kernel<false, false, MATS>(st, grid, p, maps);
+}
+
+}  // namespace
 
 int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N, int64_t M,
                     int order, const MultiMat *multi) {
     // a weight row's pitch, K / 32 * 18 bytes, must be a multiple of 16 for the tensor copies
     if (K % (2 * SUPER) != 0) return set_error(JQ_ERR_UNSUPPORTED, "fp16-operand tcgen05 GEMM needs K %% 256 == 0 (K = %lld)", (long long)K);
     const void *w[HF_MAX_MATS] = {};
-    HfParams p{};
+    HfParams<HF_MAX_MATS> p{};
     p.n_mats = multi != nullptr ? multi->n : 1;
     if (p.n_mats < 1 || p.n_mats > HF_MAX_MATS) return set_error(JQ_ERR_INVALID_ARG, "1 to %d weight matrices per launch", HF_MAX_MATS);
     uintptr_t bits = (uintptr_t)d_xq;
@@ -643,35 +684,38 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     p.K = (int)K;
     p.order = order;
     p.trace = static_cast<unsigned long long *>(next_trace_slot());
-    p.poll_limit = wait_poll_limit();
     p.static_weights = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 1 : 0;
-    // Few tiles and a long K: two CTAs per tile, each half of K (whole pairs of chunks), so that twice as many SMs
-    // convert operands; both are resident at once (the second adds to what the first stored, and waits for it).
-    // Measured at M = 128, N = 4096 (32 tiles): K = 4096 28.9 -> 26.1 us, K = 8192 52.1 -> 37.9, K = 11008 68.2 ->
-    // 46.5; three and four splits are no faster (44.3, 46.4 us at K = 11008): every further split adds an ordered
-    // pass over the tile in y.
+    // What a launch takes, in hundredths of a us: per wave of CTAs 73 for each 128-value stage and 600 to fill the pipeline
+    // and write the tile; 200 more where the CTAs of a cluster split K and add up their parts; 105 per stage where pairs of
+    // CTAs share 256 x 256 (they convert as much per stage as single CTAs and multiply twice as much).  Few tiles take the
+    // split, many the pairs.  Whole linear, before / now: K = N = 4096: M = 64 27.0 / 16.5 us, M = 256 30.1 / 23.9; K = 11008,
+    // N = 4096, M = 128 48.5 / 28.7; K = 4096, N = 1024, M = 300 27.3 / 16.3 (two CTAs per tile that added to y one after the
+    // other, or one); pairs, multiply alone: K = 4096: N = 4096, M = 1024 57 / 40, N = 11008, M = 256 57 / 40, M = 512 84 / 77;
+    // K = 8192, N = 28672, M = 2048 1326 / 997.
     const int n_chunks = (int)(K / SUPER);
-    int splits = gx * gy * 2 <= caps.sm_count && gx * gy <= HF_MAX_SPLIT_TILES && n_chunks >= 32 ? 2 : 1;
-    // A pair of CTAs converts as many operands per stage as two CTAs on their own and multiplies twice as much, in 1.05 us
-    // a stage against 0.73: pairs are taken where that makes up for fewer waves (stages per SM: waves times chunks, or
-    // half of them with two CTAs per tile).  Single / pairs, K = 4096: N = 4096, M = 1024 57 / 40 us; N = 11008, M = 256
-    // 57 / 40, M = 512 84 / 77; K = 8192, N = 28672: M = 256 205 / 147, M = 2048 1326 / 997.  Pairs that also split K were
-    // slower than single CTAs that need not (K = N = 4096, M = 512 35.8 against 29.6 us).
+    const int64_t sms = caps.sm_count, tiles = gx * gy;
+    int64_t best = 0;
+    for (const int s : {1, 2, 3, 4, 6, 8}) {
+        const int chunks = ((n_chunks + s - 1) / s + 1) / 2 * 2;  // whole pairs of chunks
+        const int parts = (n_chunks + chunks - 1) / chunks;
+        if (parts != s) continue;
+        // clusters of more than two leave some SMs of a GPC over
+        const int64_t per_wave = (s <= 2 ? sms : sms * 7 / 8) / s;
+        const int64_t cost = (tiles + per_wave - 1) / per_wave * (chunks * 73 + (s > 1 ? 800 : 600));
+        if (best == 0 || cost < best) {
+            best = cost;
+            p.k_splits = s;
+            p.chunks_per_split = chunks;
+        }
+    }
     const int64_t pair_gy = (M + 2 * HF_BM - 1) / (2 * HF_BM);
-    const int64_t waves = (gx * gy * splits + caps.sm_count - 1) / caps.sm_count;
-    const int64_t pair_waves = (pair_gx * pair_gy + caps.sm_count - 1) / caps.sm_count;
-    const bool pair = pair_waves * splits * 13 < waves * 9;
-    if (pair) splits = 1;
-    p.chunks_per_split = ((n_chunks + splits - 1) / splits + 1) / 2 * 2;
-    p.k_splits = (n_chunks + p.chunks_per_split - 1) / p.chunks_per_split;
-    p.tile_sem = nullptr;
-    if (p.k_splits > 1) {
-        void *sem = nullptr;
-        JQ_CUDA_TRY(cudaGetSymbolAddress(&sem, g_tile_sem));
-        p.tile_sem = static_cast<int *>(sem);
+    const bool pair = (pair_gx * pair_gy + sms - 1) / sms * (n_chunks * 105 + 600) < best;
+    if (pair) {
+        p.k_splits = 1;
+        p.chunks_per_split = n_chunks;
     }
     const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
-    HfMaps maps{};
+    HfMaps<HF_MAX_MATS> maps{};
     p.tile_begin[0] = 0;
     for (int i = 0; i < p.n_mats; ++i) {
         const int64_t per = pair ? 2 : 1;
@@ -687,24 +731,28 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
                      ? encode_byte_map(&maps.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, 128)
                      : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, 128))
         return rc;
-    const auto kernel = pair ? gemm_q4_0_q8_1_f16_kernel<true> : gemm_q4_0_q8_1_f16_kernel<false>;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
-    (void)cudaGetLastError();  // a stale error of an earlier, unrelated call must not be taken for this launch's
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = pair ? dim3((unsigned)pair_gx, (unsigned)pair_gy, 1u) : dim3((unsigned)gx, (unsigned)gy, (unsigned)p.k_splits);
-    cfg.blockDim = dim3(HF_THREADS);
-    cfg.dynamicSmemBytes = HF_SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = pair ? 2 : 1;
-    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, maps));
-    return JQ_OK;
+    const int form = pair ? 0 : p.k_splits > 1 ? 1 : 2;
+    const dim3 grid = pair ? dim3((unsigned)pair_gx, (unsigned)pair_gy, 1u) : dim3((unsigned)gx, (unsigned)gy, (unsigned)p.k_splits);
+    if (p.n_mats > 1) return launch_form(st, form, grid, p, maps);
+    HfParams<1> p1{};
+    p1.y[0] = p.y[0];
+    p1.rows[0] = p.rows[0];
+    p1.n_mats = 1;
+    p1.fault = p.fault;
+#ifdef JQ_BOUNDS_CHECK
+    p1.ext_y[0] = p.ext_y[0];
+#endif
+    p1.M = p.M;
+    p1.K = p.K;
+    p1.order = p.order;
+    p1.trace = p.trace;
+    p1.k_splits = p.k_splits;
+    p1.chunks_per_split = p.chunks_per_split;
+    p1.static_weights = p.static_weights;
+    HfMaps<1> maps1{};
+    maps1.w[0] = maps.w[0];
+    maps1.x = maps.x;
+    return launch_form(st, form, grid, p1, maps1);
 }
 
 }  // namespace jq

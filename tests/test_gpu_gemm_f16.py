@@ -113,6 +113,14 @@ def test_gemm_f16_pairs_of_ctas(env, K, N, M, order):
     _check(env, env.O.quantize_q4_0(w), x, K, N, M, order, env.c.S_SUM_X, rows)
 
 
+# K in 2, 3, 4, 6 and 8 parts, equal and with a shorter last one, added up over shared memory by the CTAs of a cluster
+@pytest.mark.parametrize("K,N,M", [(512, 130, 64), (768, 200, 66), (1024, 129, 200), (1536, 1, 130), (2816, 300, 65), (2048, 257, 9)])
+def test_gemm_f16_parts_of_k(env, K, N, M):
+    rng = np.random.default_rng(K + N + M)
+    w = (rng.standard_normal((N, K), dtype=np.float32) * np.float32(0.02)).astype(np.float32)
+    _check(env, env.O.quantize_q4_0(w), rng.standard_normal((M, K), dtype=np.float32), K, N, M, env.c.ORDER_KSUPER_COL, env.c.S_SUM_X)
+
+
 @pytest.mark.parametrize("K,rows,M", [(512, [300, 1, 128, 257], 64), (256, [9400, 9290], 130), (4096, [128, 200], 100)])
 def test_gemm_f16_several_matrices(env, K, rows, M):
     """Several matrices in one launch (single CTAs, pairs, split K): each row against separate calls, whose sums over K may

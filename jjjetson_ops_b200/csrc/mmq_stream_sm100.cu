@@ -35,8 +35,9 @@ namespace jq {
 namespace {
 
 constexpr int SK_MAX_STAGES = 8;
-constexpr int SK_WARPS = 8;             // consumer warps
-constexpr int SK_THREADS = (SK_WARPS + 1) * 32;
+// Consumer warps: 8 with two CTAs per SM, 16 with one, for grids that would leave the second place empty anyway (K = 11008,
+// N = 4096, M = 8 17.6 -> 10.6 us, whole linears of K = N = 4096: M = 24 12 -> 9.5 us)
+constexpr int SK_WARPS = 8, SK_WARPS_ALONE = 16;
 constexpr int SK_BAR_BYTES = 256;       // full[8], empty[8], meet[2]
 constexpr int SK_PITCH = 144;           // bytes of a weight row per 256 values of K, of an activation column per 128
 constexpr int SK_ODD_PITCH = 160;       // the same for the odd rows of an odd K, which start 8 bytes into their 160
@@ -72,17 +73,17 @@ struct StreamParams {
 #endif
 };
 
-template <int CT, int WR, bool ODD>
+template <int CT, int WR, bool ODD, int WARPS>
 struct StreamTile {
     static constexpr int ROWS = 32 * WR, COLS = 8 * CT;
-    static constexpr int KW = SK_WARPS / WR;  // warps along K = pairs of blocks per stage
+    static constexpr int KW = WARPS / WR;  // warps along K = pairs of blocks per stage
     static constexpr int SUPERS = KW / 2;     // 128-value groups per stage
     // weights of 256 values of K: ROWS rows, or ROWS / 2 even ones and ROWS / 2 odd ones
     static constexpr int HALF_BYTES = ODD ? ROWS / 2 * (SK_PITCH + SK_ODD_PITCH) : ROWS * SK_PITCH;
     static constexpr int SUPER_BYTES = COLS * SK_PITCH;  // activations of 128 values of K
     static constexpr int W_BYTES = (SUPERS / 2) * HALF_BYTES;
     static constexpr int STAGE_BYTES = W_BYTES + SUPERS * SUPER_BYTES;
-    static constexpr int RED_BYTES = SK_WARPS * COLS * SK_RED_PITCH * 4;
+    static constexpr int RED_BYTES = WARPS * COLS * SK_RED_PITCH * 4;
     static_assert(HALF_BYTES % 128 == 0 && SUPER_BYTES % 128 == 0, "tensor copies land on 128-byte boundaries");
     static_assert(ROWS / 2 * SK_PITCH % 128 == 0, "tensor copies land on 128-byte boundaries");
 };
@@ -124,10 +125,10 @@ __device__ __forceinline__ bool stream_meet(uint64_t *bar, int lane, int *fault,
 }
 
 // Weights of stage c (one thread).
-template <int CT, int WR, bool ODD>
+template <int CT, int WR, bool ODD, int WARPS>
 __device__ __forceinline__ void stream_load_weights(const StreamParams &p, const StreamMaps &maps, int mat, int64_t n0, int c, uint32_t stage,
                                                     uint64_t *full) {
-    using T = StreamTile<CT, WR, ODD>;
+    using T = StreamTile<CT, WR, ODD, WARPS>;
 #pragma unroll
     for (int h = 0; h < T::SUPERS / 2; ++h) {
         const int ks = c * T::SUPERS + 2 * h;  // first 128-value group of this half
@@ -143,10 +144,10 @@ __device__ __forceinline__ void stream_load_weights(const StreamParams &p, const
 }
 
 // Activations of stage c (lane 0).
-template <int CT, int WR, bool ODD>
+template <int CT, int WR, bool ODD, int WARPS>
 __device__ __forceinline__ void stream_load_activations(const StreamParams &p, const CUtensorMap *map, int64_t m0, int c, uint32_t stage,
                                                         uint64_t *full) {
-    using T = StreamTile<CT, WR, ODD>;
+    using T = StreamTile<CT, WR, ODD, WARPS>;
 #pragma unroll
     for (int i = 0; i < T::SUPERS; ++i) {
         const int ks = c * T::SUPERS + i;
@@ -159,9 +160,9 @@ __device__ __forceinline__ void stream_load_activations(const StreamParams &p, c
     }
 }
 
-template <int CT, int WR, bool ODD>
-__global__ void __launch_bounds__(SK_THREADS, 2) mmq_stream_kernel(const StreamParams p, const __grid_constant__ StreamMaps maps) {
-    using T = StreamTile<CT, WR, ODD>;
+template <int CT, int WR, bool ODD, int WARPS>
+__global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) mmq_stream_kernel(const __grid_constant__ StreamParams p, const __grid_constant__ StreamMaps maps) {
+    using T = StreamTile<CT, WR, ODD, WARPS>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *empty = full + SK_MAX_STAGES;
@@ -172,10 +173,10 @@ __global__ void __launch_bounds__(SK_THREADS, 2) mmq_stream_kernel(const StreamP
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], SK_WARPS);
+            mbar_init(&empty[s], WARPS);
         }
-        mbar_init(&meet[0], SK_WARPS);
-        mbar_init(&meet[1], SK_WARPS);
+        mbar_init(&meet[0], WARPS);
+        mbar_init(&meet[1], WARPS);
         fence_mbar_init();
     }
     __syncthreads();
@@ -187,14 +188,14 @@ __global__ void __launch_bounds__(SK_THREADS, 2) mmq_stream_kernel(const StreamP
     const int64_t m0 = (int64_t)blockIdx.y * T::COLS;
     const int n_chunks = (p.n_super + T::SUPERS - 1) / T::SUPERS;
 
-    if (warp == SK_WARPS) {
+    if (warp == WARPS) {
         // ---- producer: the weights of the first stages may be on their way before the previous kernel is done ------
         if (lane != 0) return;
         const int early = min(p.early_stages, n_chunks);  // at most `stages`: no slot is waited for below
         const auto arm = [&](int c, int s) {
             const int supers = min(T::SUPERS, p.n_super - c * T::SUPERS);
             mbar_arrive_expect_tx(&full[s], (uint32_t)(supers * T::SUPER_BYTES + (supers + 1) / 2 * T::HALF_BYTES));
-            stream_load_weights<CT, WR, ODD>(p, maps, mat, n0, c, ring + (uint32_t)s * T::STAGE_BYTES, &full[s]);
+            stream_load_weights<CT, WR, ODD, WARPS>(p, maps, mat, n0, c, ring + (uint32_t)s * T::STAGE_BYTES, &full[s]);
         };
         for (int c = 0; c < early; ++c) arm(c, c);
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) mmq_stream_kernel(const StreamP
         for (int c = 0; c < n_chunks; ++c) {
             if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1u, p.fault, p.poll_limit)) return;
             if (c >= early) arm(c, s);
-            stream_load_activations<CT, WR, ODD>(p, &maps.x, m0, c, ring + (uint32_t)s * T::STAGE_BYTES, &full[s]);
+            stream_load_activations<CT, WR, ODD, WARPS>(p, &maps.x, m0, c, ring + (uint32_t)s * T::STAGE_BYTES, &full[s]);
             if (++s == p.stages) {
                 s = 0;
                 ++round;
@@ -306,11 +307,11 @@ __global__ void __launch_bounds__(SK_THREADS, 2) mmq_stream_kernel(const StreamP
     }
 }
 
-template <int CT, int WR, bool ODD>
+template <int CT, int WR, bool ODD, int WARPS>
 int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps) {
-    using T = StreamTile<CT, WR, ODD>;
-    // two CTAs share an SM (1 KB of its shared memory is reserved per CTA)
-    const int budget = min(caps.smem_optin, caps.smem_per_sm / 2 - 1024);
+    using T = StreamTile<CT, WR, ODD, WARPS>;
+    // two CTAs may share an SM (1 KB of its shared memory is reserved per CTA)
+    const int budget = WARPS == SK_WARPS ? min(caps.smem_optin, caps.smem_per_sm / 2 - 1024) : caps.smem_optin;
     p.stages = min(SK_MAX_STAGES, (budget - SK_BAR_BYTES) / T::STAGE_BYTES);
     if (p.stages < 2 || p.stages * T::STAGE_BYTES < T::RED_BYTES)
         return set_error(JQ_ERR_UNSUPPORTED, "the stages of the small-batch kernel do not fit in shared memory");
@@ -320,11 +321,11 @@ int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const D
     for (int i = 0; i < p.n_mats; ++i) p.tile_begin[i + 1] = p.tile_begin[i] + (int)((p.rows[i] + T::ROWS - 1) / T::ROWS);
     const int64_t gy = (p.M + T::COLS - 1) / T::COLS;
     if (gy > 65535) return set_error(JQ_ERR_UNSUPPORTED, "too many columns for the small-batch kernel");
-    auto kernel = mmq_stream_kernel<CT, WR, ODD>;
+    auto kernel = mmq_stream_kernel<CT, WR, ODD, WARPS>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), bytes, true)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)p.tile_begin[p.n_mats], (unsigned)gy);
-    cfg.blockDim = dim3(SK_THREADS);
+    cfg.blockDim = dim3((WARPS + 1) * 32);
     cfg.dynamicSmemBytes = (size_t)bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -337,10 +338,14 @@ int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const D
     return JQ_OK;
 }
 
+template <int CT, bool ODD>
+int run_stream_shape(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps, int wr, bool alone) {
+    if (alone) return run_stream<CT, 1, ODD, SK_WARPS_ALONE>(st, p, maps, caps);
+    return wr == 1 ? run_stream<CT, 1, ODD, SK_WARPS>(st, p, maps, caps) : run_stream<CT, 2, ODD, SK_WARPS>(st, p, maps, caps);
+}
 template <int CT>
-int run_stream_columns(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps, int wr, bool odd) {
-    if (odd) return wr == 1 ? run_stream<CT, 1, true>(st, p, maps, caps) : run_stream<CT, 2, true>(st, p, maps, caps);
-    return wr == 1 ? run_stream<CT, 1, false>(st, p, maps, caps) : run_stream<CT, 2, false>(st, p, maps, caps);
+int run_stream_columns(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps, int wr, bool alone, bool odd) {
+    return odd ? run_stream_shape<CT, true>(st, p, maps, caps, wr, alone) : run_stream_shape<CT, false>(st, p, maps, caps, wr, alone);
 }
 
 // The maps of one weight matrix.  Row pitch (of two rows, if odd) and bases are multiples of 16 bytes, and no map covers
@@ -371,13 +376,14 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     if (p.n_mats < 1 || p.n_mats > SK_MAX_MATS) return set_error(JQ_ERR_INVALID_ARG, "1 to %d weight matrices per launch", SK_MAX_MATS);
     const void *w[SK_MAX_MATS] = {};
     uintptr_t bits = 0;
-    int64_t wide_tiles = 0;
+    int64_t tiles = 0, wide_tiles = 0;
     const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
     for (int i = 0; i < p.n_mats; ++i) {
         w[i] = multi != nullptr ? multi->w[i] : d_w;
         p.y[i] = multi != nullptr ? multi->y[i] : d_y;
         p.rows[i] = multi != nullptr ? multi->rows[i] : N;
         bits |= (uintptr_t)w[i];
+        tiles += (p.rows[i] + 31) / 32;
         wide_tiles += (p.rows[i] + 63) / 64;
 #ifdef JQ_BOUNDS_CHECK
         p.ext_y[i] = make_extent(p.y[i], (unsigned long long)M * (unsigned long long)p.rows[i] * sizeof(float));
@@ -397,6 +403,7 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     // 64 rows per CTA halve the activation traffic, which from three column tiles on exceeds the weights'; 32 rows
     // keep more SMs at work when there are few
     const int wr = ct >= 3 && wide_tiles * groups >= caps.sm_count ? 2 : 1;
+    const bool alone = wr == 1 && tiles * groups <= caps.sm_count;
     StreamMaps maps{};
     for (int i = 0; i < p.n_mats; ++i)
         if (int rc = encode_weight_maps(&maps.w[i], &maps.w_odd[i], w[i], p.rows[i], row_bytes, 32 * wr, odd)) return rc;
@@ -406,10 +413,10 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
                      : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, 8u * (uint32_t)ct))
         return rc;
     switch (ct) {
-        case 1: return run_stream_columns<1>(st, p, maps, caps, wr, odd);
-        case 2: return run_stream_columns<2>(st, p, maps, caps, wr, odd);
-        case 3: return run_stream_columns<3>(st, p, maps, caps, wr, odd);
-        default: return run_stream_columns<4>(st, p, maps, caps, wr, odd);
+        case 1: return run_stream_columns<1>(st, p, maps, caps, wr, alone, odd);
+        case 2: return run_stream_columns<2>(st, p, maps, caps, wr, alone, odd);
+        case 3: return run_stream_columns<3>(st, p, maps, caps, wr, alone, odd);
+        default: return run_stream_columns<4>(st, p, maps, caps, wr, alone, odd);
     }
 }
 

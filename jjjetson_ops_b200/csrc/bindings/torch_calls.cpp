@@ -14,6 +14,7 @@
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
@@ -55,6 +56,12 @@ PyObject *bind(PyObject *, PyObject *addresses) {
     }
     Py_RETURN_NONE;
 }
+
+// a reference that is given back on every way out, an exception's included
+struct Owned {
+    PyObject *p = nullptr;
+    ~Owned() { Py_XDECREF(p); }
+};
 
 // ---- arguments -------------------------------------------------------------------------------------
 const char *dtype_text(at::ScalarType t) { return t == at::kFloat ? "torch.float32" : "torch.uint8"; }
@@ -116,7 +123,12 @@ class OnDevice {
         if (had_ != want_) c10::cuda::set_device(want_);
     }
     ~OnDevice() {
-        if (had_ != want_) c10::cuda::set_device(had_);
+        if (had_ != want_) (void)c10::cuda::SetDevice(had_);  // no exception from here: restore() has reported the error
+    }
+    void restore() {
+        const c10::DeviceIndex back = had_;
+        had_ = want_;
+        if (back != want_) c10::cuda::set_device(back);
     }
     void *stream() const { return c10::cuda::getCurrentCUDAStream(want_).stream(); }
 
@@ -124,21 +136,28 @@ class OnDevice {
     c10::DeviceIndex want_, had_;
 };
 
-// Runs `call` (which returns a jq_status) and hands the status to Python; C++ exceptions of torch become RuntimeError.
+// Runs `call` (which returns a jq_status) and hands the status to Python.
 template <typename F>
 PyObject *status_of(const at::Tensor &on, F &&call) {
-    try {
-        OnDevice device(on);
-        return PyLong_FromLong(call(device.stream()));
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
-    }
+    OnDevice device(on);
+    const int status = call(device.stream());
+    device.restore();
+    return PyLong_FromLong(status);
+}
+
+// What Python calls.  Almost everything of torch can throw, is_contiguous() and data_ptr() of a tensor without storage
+// (under vmap, for instance) included, and no exception may leave a C function: each becomes the Python exception that
+// torch's own functions raise for it.
+template <PyObject *(*Call)(PyObject *const *, Py_ssize_t)>
+PyObject *entry(PyObject *, PyObject *const *a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    return Call(a, n);
+    END_HANDLE_TH_ERRORS
 }
 
 // ---- the calls: every one returns the library's status -------------------------------------------------
 // (x, out, order, s_mode)
-PyObject *quantize(PyObject *, PyObject *const *a, Py_ssize_t n) {
+PyObject *quantize(PyObject *const *a, Py_ssize_t n) {
     int64_t M, K, order, s_mode;
     void *xp, *op;
     if (!argument_count(n, 4)) return nullptr;
@@ -151,7 +170,7 @@ PyObject *quantize(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // (w, xq, out, K, N, M, order, kernel)
-PyObject *mul_mat(PyObject *, PyObject *const *a, Py_ssize_t n) {
+PyObject *mul_mat(PyObject *const *a, Py_ssize_t n) {
     int64_t K, N, M, order, kernel;
     void *xp, *yp;
     if (!argument_count(n, 8)) return nullptr;
@@ -165,7 +184,7 @@ PyObject *mul_mat(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // (w, x, ws, out, N, s_mode)
-PyObject *linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
+PyObject *linear(PyObject *const *a, Py_ssize_t n) {
     int64_t K, N, M, s_mode;
     void *wp, *wsp, *yp;
     if (!argument_count(n, 6)) return nullptr;
@@ -180,7 +199,7 @@ PyObject *linear(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // (ws_list, N_list, outs, x or None, xq or None, ws or None, K, M, s_mode); the first three are sequences of one length
-PyObject *multi(PyObject *, PyObject *const *a, Py_ssize_t n) {
+PyObject *multi(PyObject *const *a, Py_ssize_t n) {
     constexpr Py_ssize_t MOST = 16;  // the library says how many it takes; this only bounds the arrays here
     const void *w[MOST];
     float *y[MOST];
@@ -188,40 +207,37 @@ PyObject *multi(PyObject *, PyObject *const *a, Py_ssize_t n) {
     int64_t K, M, s_mode;
     void *xp, *xqp, *wsp;
     if (!argument_count(n, 9)) return nullptr;
-    PyObject *seq[3] = {nullptr, nullptr, nullptr};
-    PyObject *result = nullptr;
-    const at::Tensor *first = nullptr;
-    bool ok = true;
-    for (int i = 0; i < 3 && ok; ++i) ok = (seq[i] = PySequence_Fast(a[i], "a sequence is expected")) != nullptr;
-    const Py_ssize_t n_mats = ok ? PySequence_Fast_GET_SIZE(seq[0]) : 0;
-    if (ok && (n_mats < 1 || n_mats > MOST || PySequence_Fast_GET_SIZE(seq[1]) != n_mats || PySequence_Fast_GET_SIZE(seq[2]) != n_mats)) {
-        PyErr_SetString(PyExc_ValueError, "weights, row counts and outputs must be sequences of one length (1 to 16)");
-        ok = false;
+    Owned seq[3];
+    for (int i = 0; i < 3; ++i) {
+        seq[i].p = PySequence_Fast(a[i], "a sequence is expected");
+        if (seq[i].p == nullptr) return nullptr;
     }
-    for (Py_ssize_t i = 0; i < n_mats && ok; ++i) {
+    const Py_ssize_t n_mats = PySequence_Fast_GET_SIZE(seq[0].p);
+    if (n_mats < 1 || n_mats > MOST || PySequence_Fast_GET_SIZE(seq[1].p) != n_mats || PySequence_Fast_GET_SIZE(seq[2].p) != n_mats) {
+        PyErr_SetString(PyExc_ValueError, "weights, row counts and outputs must be sequences of one length (1 to 16)");
+        return nullptr;
+    }
+    const at::Tensor *first = nullptr;
+    for (Py_ssize_t i = 0; i < n_mats; ++i) {
         void *yp = nullptr;
-        const at::Tensor *t = tensor_arg(PySequence_Fast_GET_ITEM(seq[0], i), at::kByte, "w");
-        PyObject *r = nullptr;
-        ok = t != nullptr && pointer_arg(PySequence_Fast_GET_ITEM(seq[2], i), at::kFloat, "out", &yp) &&
-             (r = PyNumber_Long(PySequence_Fast_GET_ITEM(seq[1], i))) != nullptr && size_arg(r, &rows[i]);
-        Py_XDECREF(r);
-        if (!ok) break;
+        const at::Tensor *t = tensor_arg(PySequence_Fast_GET_ITEM(seq[0].p, i), at::kByte, "w");
+        if (t == nullptr || !pointer_arg(PySequence_Fast_GET_ITEM(seq[2].p, i), at::kFloat, "out", &yp)) return nullptr;
+        Owned r{PyNumber_Long(PySequence_Fast_GET_ITEM(seq[1].p, i))};
+        if (r.p == nullptr || !size_arg(r.p, &rows[i])) return nullptr;
         if (i == 0) first = t;
         w[i] = t->data_ptr();
         y[i] = static_cast<float *>(yp);
     }
-    if (ok && optional_pointer_arg(a[3], at::kFloat, "x", &xp) && optional_pointer_arg(a[4], at::kByte, "xq", &xqp) &&
-        optional_pointer_arg(a[5], at::kByte, "ws", &wsp) && size_arg(a[6], &K) && size_arg(a[7], &M) && size_arg(a[8], &s_mode)) {
-        result = status_of(*first, [&](void *st) {
-            return f_multi(st, (int)n_mats, w, rows, y, static_cast<const float *>(xp), xqp, wsp, K, M, (int)s_mode);
-        });
-    }
-    for (PyObject *s : seq) Py_XDECREF(s);
-    return result;
+    if (!optional_pointer_arg(a[3], at::kFloat, "x", &xp) || !optional_pointer_arg(a[4], at::kByte, "xq", &xqp) ||
+        !optional_pointer_arg(a[5], at::kByte, "ws", &wsp) || !size_arg(a[6], &K) || !size_arg(a[7], &M) || !size_arg(a[8], &s_mode))
+        return nullptr;
+    return status_of(*first, [&](void *st) {
+        return f_multi(st, (int)n_mats, w, rows, y, static_cast<const float *>(xp), xqp, wsp, K, M, (int)s_mode);
+    });
 }
 
 // (x, weight, epsilon, residual or None, normed or None, xq or None, order, s_mode)
-PyObject *rms_norm(PyObject *, PyObject *const *a, Py_ssize_t n) {
+PyObject *rms_norm(PyObject *const *a, Py_ssize_t n) {
     int64_t T, H, order, s_mode;
     void *wp, *rp, *np, *qp;
     if (!argument_count(n, 8)) return nullptr;
@@ -239,7 +255,7 @@ PyObject *rms_norm(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // (gate, up, mid or None, xq or None, order, s_mode)
-PyObject *swiglu(PyObject *, PyObject *const *a, Py_ssize_t n) {
+PyObject *swiglu(PyObject *const *a, Py_ssize_t n) {
     int64_t T, I, order, s_mode;
     void *up, *mp, *qp;
     if (!argument_count(n, 6)) return nullptr;
@@ -254,7 +270,7 @@ PyObject *swiglu(PyObject *, PyObject *const *a, Py_ssize_t n) {
     });
 }
 
-#define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)), METH_FASTCALL
+#define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<f>)), METH_FASTCALL
 PyMethodDef methods[] = {
     {"bind", bind, METH_O, "Addresses of the library's functions, by name."},
     {"quantize", FAST(quantize), "(x, out, order, s_mode) -> status"},

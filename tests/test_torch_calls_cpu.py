@@ -1,0 +1,44 @@
+"""CPU checks of the native module behind capi.py's tensor calls: what it refuses, it refuses with a Python exception."""
+import os
+import subprocess
+import sys
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+# Fake CUDA tensors reach the native argument checks without a GPU.
+FAKE = """
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from jjjetson_ops_b200 import capi as c
+
+def f32(*shape):
+    return torch.empty(shape, device="cuda")
+
+def u8(n, *batch):
+    return torch.empty(batch + (n,), dtype=torch.uint8, device="cuda")
+
+K, N, M = 256, 64, 2
+nw, nq = c.q4_0_bytes(N, K), c.q8_1_bytes(K, M)
+"""
+
+
+def _raised(calls, setup=""):
+    """The names of the exceptions that the calls raise, in a process of its own that has to outlive all of them."""
+    code = FAKE + setup + "for call in %r:\n    with FakeTensorMode():\n        try:\n            eval(call)\n            print('nothing')\n" \
+        "        except Exception as e:\n            print('RuntimeError' if isinstance(e, RuntimeError) else type(e).__name__)\n" % (calls,)
+    r = subprocess.run([sys.executable, "-W", "ignore", "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=300)
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr[-2000:])
+    return r.stdout.split()
+
+
+def test_tensor_without_storage_is_a_runtime_error(native_lib):
+    """A tensor whose data pointer torch refuses to give: an exception, not the end of the process."""
+    calls = [
+        "torch.vmap(lambda v: c.quantize_q8_1(v, out=u8(nq)))(f32(3, M, K))",
+        "torch.vmap(lambda v: c.mul_mat_q4_0_q8_1(u8(nw), v, K, N, M, out=f32(M, N)))(u8(nq, 3))",
+        "torch.vmap(lambda v: c.linear_q4_0(v, f32(M, K), N, ws=u8(nq), out=f32(M, N)))(u8(nw, 3))",
+        "torch.vmap(lambda v: c.linear_q4_0_multi([v], [N], xq=u8(nq), K=K, M=M, outs=[f32(M, N)]))(u8(nw, 3))",
+        "torch.vmap(lambda v: c.rms_norm_q8_1(f32(M, K), f32(K), 1e-6, xq=v))(u8(nq, 3))",
+        "torch.vmap(lambda v: c.swiglu_q8_1(f32(M, K), v, xq=u8(nq)))(f32(3, M, K))",
+    ]
+    assert _raised(calls) == ["RuntimeError"] * len(calls)

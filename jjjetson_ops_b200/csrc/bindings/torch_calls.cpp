@@ -207,22 +207,22 @@ PyObject *multi(PyObject *const *a, Py_ssize_t n) {
     int64_t K, M, s_mode;
     void *xp, *xqp, *wsp;
     if (!argument_count(n, 9)) return nullptr;
-    Owned seq[3];
+    Owned seq[3];  // tuples of the call's own: converting a row count may run Python code that changes the caller's lists
     for (int i = 0; i < 3; ++i) {
-        seq[i].p = PySequence_Fast(a[i], "a sequence is expected");
+        seq[i].p = PySequence_Tuple(a[i]);
         if (seq[i].p == nullptr) return nullptr;
     }
-    const Py_ssize_t n_mats = PySequence_Fast_GET_SIZE(seq[0].p);
-    if (n_mats < 1 || n_mats > MOST || PySequence_Fast_GET_SIZE(seq[1].p) != n_mats || PySequence_Fast_GET_SIZE(seq[2].p) != n_mats) {
+    const Py_ssize_t n_mats = PyTuple_GET_SIZE(seq[0].p);
+    if (n_mats < 1 || n_mats > MOST || PyTuple_GET_SIZE(seq[1].p) != n_mats || PyTuple_GET_SIZE(seq[2].p) != n_mats) {
         PyErr_SetString(PyExc_ValueError, "weights, row counts and outputs must be sequences of one length (1 to 16)");
         return nullptr;
     }
     const at::Tensor *first = nullptr;
     for (Py_ssize_t i = 0; i < n_mats; ++i) {
         void *yp = nullptr;
-        const at::Tensor *t = tensor_arg(PySequence_Fast_GET_ITEM(seq[0].p, i), at::kByte, "w");
-        if (t == nullptr || !pointer_arg(PySequence_Fast_GET_ITEM(seq[2].p, i), at::kFloat, "out", &yp)) return nullptr;
-        Owned r{PyNumber_Long(PySequence_Fast_GET_ITEM(seq[1].p, i))};
+        const at::Tensor *t = tensor_arg(PyTuple_GET_ITEM(seq[0].p, i), at::kByte, "w");
+        if (t == nullptr || !pointer_arg(PyTuple_GET_ITEM(seq[2].p, i), at::kFloat, "out", &yp)) return nullptr;
+        Owned r{PyNumber_Long(PyTuple_GET_ITEM(seq[1].p, i))};
         if (r.p == nullptr || !size_arg(r.p, &rows[i])) return nullptr;
         if (i == 0) first = t;
         w[i] = t->data_ptr();

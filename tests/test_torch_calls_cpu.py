@@ -42,3 +42,26 @@ def test_tensor_without_storage_is_a_runtime_error(native_lib):
         "torch.vmap(lambda v: c.swiglu_q8_1(f32(M, K), v, xq=u8(nq)))(f32(3, M, K))",
     ]
     assert _raised(calls) == ["RuntimeError"] * len(calls)
+
+
+def test_lists_that_change_during_the_call(native_lib):
+    """A row count whose conversion empties the caller's lists: the call works on what the lists held."""
+    setup = """
+ws_list, N_list, outs = [], [], []
+
+class Rows:
+    def __int__(self):
+        for l in (ws_list, N_list, outs):
+            l.clear()
+        return 2**70  # refused, with OverflowError, once the lists are gone
+
+def multi(*rows):
+    ws_list[:], N_list[:], outs[:] = [u8(nw) for _ in rows], rows, [f32(M, N) for _ in rows]
+    return c.linear_q4_0_multi(ws_list, N_list, xq=u8(nq), K=K, M=M, outs=outs)
+
+class Small(Rows):
+    def __int__(self):
+        super().__int__()
+        return N
+"""
+    assert _raised(["multi(Rows(), N, N)", "multi(Small(), N, Rows())"], setup) == ["OverflowError"] * 2

@@ -136,11 +136,27 @@ class OnDevice {
     c10::DeviceIndex want_, had_;
 };
 
-// Runs `call` (which returns a jq_status) and hands the status to Python.
+// Other Python threads run while this is in scope: no Python object and no tensor is touched meanwhile.
+class WithoutGil {
+  public:
+    WithoutGil() : state_(PyEval_SaveThread()) {}
+    ~WithoutGil() { PyEval_RestoreThread(state_); }
+
+  private:
+    PyThreadState *state_;
+};
+
+// Runs `call` (which returns a jq_status) and hands the status to Python.  A launch can wait: for room in the queue, for a
+// kernel's module to be loaded on its first use.  So `call` has only plain values left to pass on, and runs without the GIL.
 template <typename F>
 PyObject *status_of(const at::Tensor &on, F &&call) {
     OnDevice device(on);
-    const int status = call(device.stream());
+    void *const stream = device.stream();
+    int status;
+    {
+        const WithoutGil released;
+        status = call(stream);
+    }
     device.restore();
     return PyLong_FromLong(status);
 }
@@ -178,8 +194,9 @@ PyObject *mul_mat(PyObject *const *a, Py_ssize_t n) {
     if (w == nullptr || !pointer_arg(a[1], at::kByte, "xq", &xp) || !pointer_arg(a[2], at::kFloat, "out", &yp) || !size_arg(a[3], &K) ||
         !size_arg(a[4], &N) || !size_arg(a[5], &M) || !size_arg(a[6], &order) || !size_arg(a[7], &kernel))
         return nullptr;
+    const void *wp = w->data_ptr();
     return status_of(*w, [&](void *st) {
-        return f_mul_mat(st, w->data_ptr(), xp, static_cast<float *>(yp), K, N, M, (int)order, (int)kernel);
+        return f_mul_mat(st, wp, xp, static_cast<float *>(yp), K, N, M, (int)order, (int)kernel);
     });
 }
 
@@ -193,8 +210,9 @@ PyObject *linear(PyObject *const *a, Py_ssize_t n) {
     if (x == nullptr || !two_sizes(*x, "x", &M, &K) || !pointer_arg(a[2], at::kByte, "ws", &wsp) ||
         !pointer_arg(a[3], at::kFloat, "out", &yp) || !size_arg(a[4], &N) || !size_arg(a[5], &s_mode))
         return nullptr;
+    const void *xp = x->data_ptr();
     return status_of(*x, [&](void *st) {
-        return f_linear(st, wp, static_cast<const float *>(x->data_ptr()), wsp, static_cast<float *>(yp), K, N, M, (int)s_mode);
+        return f_linear(st, wp, static_cast<const float *>(xp), wsp, static_cast<float *>(yp), K, N, M, (int)s_mode);
     });
 }
 
@@ -248,8 +266,9 @@ PyObject *rms_norm(PyObject *const *a, Py_ssize_t n) {
     if (!optional_pointer_arg(a[3], at::kFloat, "residual", &rp) || !optional_pointer_arg(a[4], at::kFloat, "normed", &np) ||
         !optional_bytes_arg(a[5], "xq", &qp) || !size_arg(a[6], &order) || !size_arg(a[7], &s_mode))
         return nullptr;
+    void *xp = x->data_ptr();
     return status_of(*x, [&](void *st) {
-        return f_rms_norm(st, static_cast<float *>(x->data_ptr()), static_cast<float *>(rp), static_cast<const float *>(wp),
+        return f_rms_norm(st, static_cast<float *>(xp), static_cast<float *>(rp), static_cast<const float *>(wp),
                           static_cast<float *>(np), qp, H, T, (float)epsilon, (int)order, (int)s_mode);
     });
 }
@@ -264,8 +283,9 @@ PyObject *swiglu(PyObject *const *a, Py_ssize_t n) {
         !optional_pointer_arg(a[2], at::kFloat, "mid", &mp) || !optional_bytes_arg(a[3], "xq", &qp) || !size_arg(a[4], &order) ||
         !size_arg(a[5], &s_mode))
         return nullptr;
+    const void *gp = g->data_ptr();
     return status_of(*g, [&](void *st) {
-        return f_swiglu(st, static_cast<const float *>(g->data_ptr()), static_cast<const float *>(up), static_cast<float *>(mp), qp, I, T,
+        return f_swiglu(st, static_cast<const float *>(gp), static_cast<const float *>(up), static_cast<float *>(mp), qp, I, T,
                         (int)order, (int)s_mode);
     });
 }

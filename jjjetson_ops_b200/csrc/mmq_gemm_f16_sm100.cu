@@ -47,6 +47,10 @@
 // around in shared memory and store 128 contiguous bytes of an output row per instruction.
 // Every mbarrier wait is a bounded poll; a wait that runs out sets the device fault word, and every
 // warp still reaches the common exit where tensor memory is released.
+#include <mutex>
+#include <vector>
+
+#include "gemm_f16_plan.h"
 #include "tc_common.cuh"
 
 namespace jq {
@@ -99,7 +103,6 @@ constexpr uint32_t H2_1152 = 0x64806480u;
 constexpr uint32_t H2_SIXTEENTH = 0x2C002C00u;
 constexpr uint32_t H2_MINUS_72 = 0xD480D480u;
 
-constexpr int HF_MAX_SPLITS = 8;    // CTAs per tile along K: the largest portable cluster
 constexpr int HF_MAX_MATS = 4;
 template <int MATS>
 struct HfMaps {
@@ -643,6 +646,55 @@ int launch_kernel(cudaStream_t st, dim3 grid, const HfParams<MATS> &p, const HfM
     JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, maps));
     return JQ_OK;
 }
+// Clusters of z CTAs along K, or of a pair of CTAs, of this kernel that the current device runs at a time (0: none).  The instances
+// for several matrices have the same threads and shared memory.
+template <bool PAIR, bool SPLIT>
+int clusters_at_a_time(unsigned z, int *out) {
+    const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, 1>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(PAIR ? 2 : 1, 1, z);
+    cfg.blockDim = dim3(HF_THREADS);
+    cfg.dynamicSmemBytes = HF_SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = z;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(out, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        *out = 0;
+    }
+    return JQ_OK;
+}
+// ... for every form, asked once per device
+int form_widths(const DeviceCaps &caps, GemmF16Widths *out) {
+    struct Entry {
+        int dev;
+        GemmF16Widths width;
+    };
+    static std::vector<Entry> table;
+    static std::mutex table_mutex;
+    int dev = 0;
+    JQ_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(table_mutex);
+    for (const Entry &e : table) {
+        if (e.dev == dev) {
+            *out = e.width;
+            return JQ_OK;
+        }
+    }
+    GemmF16Widths w{};
+    w.splits[1] = caps.sm_count;
+    for (int s = 2; s <= HF_MAX_SPLITS; ++s)
+        if (int rc = clusters_at_a_time<false, true>((unsigned)s, &w.splits[s])) return rc;
+    if (int rc = clusters_at_a_time<true, false>(1, &w.pairs)) return rc;
+    table.push_back(Entry{dev, w});
+    *out = w;
+    return JQ_OK;
+}
 // form: 0 pairs of CTAs, 1 split K, 2 neither
 template <int MATS>
 int launch_form(cudaStream_t st, int form, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
@@ -685,35 +737,13 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     p.order = order;
     p.trace = static_cast<unsigned long long *>(next_trace_slot());
     p.static_weights = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 1 : 0;
-    // What a launch takes, in hundredths of a us: per wave of CTAs 73 for each 128-value stage and 600 to fill the pipeline
-    // and write the tile; 200 more where the CTAs of a cluster split K and add up their parts; 105 per stage where pairs of
-    // CTAs share 256 x 256 (they convert as much per stage as single CTAs and multiply twice as much).  Few tiles take the
-    // split, many the pairs.  Whole linear, before / now: K = N = 4096: M = 64 27.0 / 16.5 us, M = 256 30.1 / 23.9; K = 11008,
-    // N = 4096, M = 128 48.5 / 28.7; K = 4096, N = 1024, M = 300 27.3 / 16.3 (two CTAs per tile that added to y one after the
-    // other, or one); pairs, multiply alone: K = 4096: N = 4096, M = 1024 57 / 40, N = 11008, M = 256 57 / 40, M = 512 84 / 77;
-    // K = 8192, N = 28672, M = 2048 1326 / 997.
-    const int n_chunks = (int)(K / SUPER);
-    const int64_t sms = caps.sm_count, tiles = gx * gy;
-    int64_t best = 0;
-    for (const int s : {1, 2, 3, 4, 6, 8}) {
-        const int chunks = ((n_chunks + s - 1) / s + 1) / 2 * 2;  // whole pairs of chunks
-        const int parts = (n_chunks + chunks - 1) / chunks;
-        if (parts != s) continue;
-        // clusters of more than two leave some SMs of a GPC over
-        const int64_t per_wave = (s <= 2 ? sms : sms * 7 / 8) / s;
-        const int64_t cost = (tiles + per_wave - 1) / per_wave * (chunks * 73 + (s > 1 ? 800 : 600));
-        if (best == 0 || cost < best) {
-            best = cost;
-            p.k_splits = s;
-            p.chunks_per_split = chunks;
-        }
-    }
+    GemmF16Widths width;
+    if (int rc = form_widths(caps, &width)) return rc;
     const int64_t pair_gy = (M + 2 * HF_BM - 1) / (2 * HF_BM);
-    const bool pair = (pair_gx * pair_gy + sms - 1) / sms * (n_chunks * 105 + 600) < best;
-    if (pair) {
-        p.k_splits = 1;
-        p.chunks_per_split = n_chunks;
-    }
+    const GemmF16Plan plan = plan_gemm_f16((int)(K / SUPER), gx * gy, pair_gx / 2 * pair_gy, width);
+    const bool pair = plan.pair;
+    p.k_splits = plan.k_splits;
+    p.chunks_per_split = plan.chunks_per_split;
     const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
     HfMaps<HF_MAX_MATS> maps{};
     p.tile_begin[0] = 0;

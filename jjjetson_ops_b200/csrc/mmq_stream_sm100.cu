@@ -24,6 +24,15 @@
 // 22.5 against 18.0 us at M = 24; weights of four or eight stages ahead of the previous kernel's end instead of two, no
 // difference.
 //
+// Rounding.  A running sum rounds at every addition, and most when it is long: with one per warp over all of its blocks and the
+// warps' parts added one after the other the error against 64 bits was 1.2 to 1.55 times that of the kernels that took these shapes
+// before (K = 4224: 7.3e-8 of the result in the generic kernel, 11.4e-8 here at 64 rows per CTA).  So the parts are added as a tree;
+// up to eight columns, where registers are left, a warp sums in two levels; the two blocks of a pair are added to each other first
+// where the sums are long for their kind (64 rows per CTA have four warps along K, odd K replaces the generic kernel); and odd K
+// beyond 2048 keeps to 32 rows per CTA and adds the parts of eight warps with the rounded-off remainders.  The error is then 0.85 to
+// 1.02 times the former kernels' on average over each group of shapes, and the multiply takes (of its time with plain running sums)
+// 1.00 to 1.03 on average: 64 rows per CTA 1.02 to 1.05, odd K beyond 2048 with many rows 1.04, at most 1.18.
+//
 // A tensor copy wants a row pitch of whole 16-byte units, which K % 256 == 0 gives.  When K is an odd multiple of 128 a
 // row is 8 bytes short of that but two rows are not: the even rows are one tensor and the odd rows another (its base 8
 // bytes before the first odd row, so that it is aligned), each with the pitch of two rows; the even rows of a group of 32
@@ -44,6 +53,8 @@ constexpr int SK_ODD_PITCH = 160;       // the same for the odd rows of an odd K
 constexpr int SK_MAX_MATS = 4;
 constexpr int SK_RED_PITCH = 36;        // floats between two columns of a warp's partial tile: 2 * 36 = 8 mod 32 banks
 constexpr int SK_COLUMNS = 32;          // most columns a CTA takes
+constexpr int SK_FLUSH = 4;             // stages per running sum
+constexpr int SK_SHORT_SUPERS = 16;     // K up to 2048: short running sums
 constexpr uint32_t SK_MASK4 = 0x0F0F0F0Fu;
 constexpr int SK_MAGIC_I = 0x4B400000;  // bit pattern of 1.5 * 2^23
 constexpr float SK_MAGIC_F = 12582912.0f;
@@ -76,6 +87,8 @@ struct StreamParams {
 template <int CT, int WR, bool ODD, int WARPS>
 struct StreamTile {
     static constexpr int ROWS = 32 * WR, COLS = 8 * CT;
+    static constexpr bool PAIR_FIRST = ODD || WR == 2;  // the blocks of a pair are added before they join the running sum
+    static constexpr bool LEVELS = CT == 1;             // running sums of SK_FLUSH stages, and one of those
     static constexpr int KW = WARPS / WR;  // warps along K = pairs of blocks per stage
     static constexpr int SUPERS = KW / 2;     // 128-value groups per stage
     // weights of 256 values of K: ROWS rows, or ROWS / 2 even ones and ROWS / 2 odd ones
@@ -95,6 +108,13 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
         : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
     return d;
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<uint64_t &>(d))
+        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
+    return d;
+}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -104,17 +124,37 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return d;
 }
 
-// acc[2 rows g, g + 8][2 columns] += d4 * (sumi * d8 - 8 * s8) of one block
-__device__ __forceinline__ void accumulate_block(float2 (&acc)[2], const uint32_t (&a)[4], const uint32_t (&b)[2], float d4_lo,
-                                                 float d4_hi, float2 d8, float2 m8s) {
+// Sums of the warps' parts, in an order that is always the same: as a tree, or (odd K) with what each addition rounds off
+// added up as well (Knuth's two-sum), so that only the result is rounded.
+template <int N>
+__device__ __forceinline__ float sum_tree(float (&v)[N]) {
+#pragma unroll
+    for (int step = 1; step < N; step *= 2) {
+#pragma unroll
+        for (int k = 0; k < N; k += 2 * step) v[k] += v[k + step];
+    }
+    return v[0];
+}
+template <int N>
+__device__ __forceinline__ float sum_compensated(const float (&v)[N]) {
+    float sum = v[0], lost = 0.0f;
+#pragma unroll
+    for (int k = 1; k < N; ++k) {
+        const float s = sum + v[k], got = s - sum;
+        lost += (sum - (s - got)) + (v[k] - got);
+        sum = s;
+    }
+    return isfinite(sum) ? sum + lost : sum;
+}
+
+// sumi * d8 - 8 * s8 of one block for the rows g and g + 8 and two columns
+__device__ __forceinline__ void block_terms(float2 (&t)[2], const uint32_t (&a)[4], const uint32_t (&b)[2], float2 d8, float2 m8s) {
     const int magic4[4] = {SK_MAGIC_I, SK_MAGIC_I, SK_MAGIC_I, SK_MAGIC_I};
     const float2 minus = make_float2(-SK_MAGIC_F, -SK_MAGIC_F);
     int c[4];
     mma_u8s8_16832(c, a, b, magic4);
-    const float2 lo = add2(make_float2(__int_as_float(c[0]), __int_as_float(c[1])), minus);  // exact
-    const float2 hi = add2(make_float2(__int_as_float(c[2]), __int_as_float(c[3])), minus);
-    acc[0] = fma2(make_float2(d4_lo, d4_lo), fma2(lo, d8, m8s), acc[0]);
-    acc[1] = fma2(make_float2(d4_hi, d4_hi), fma2(hi, d8, m8s), acc[1]);
+    t[0] = fma2(add2(make_float2(__int_as_float(c[0]), __int_as_float(c[1])), minus), d8, m8s);  // the sum is exact
+    t[1] = fma2(add2(make_float2(__int_as_float(c[2]), __int_as_float(c[3])), minus), d8, m8s);
 }
 
 // The consumer warps meet on an mbarrier with a bounded wait: a warp whose wait for a stage ran out has left.
@@ -224,11 +264,11 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
                                    : w_pair + (uint32_t)((wr * 32 + 16 + g) * SK_PITCH)};
     const uint32_t x_head = (uint32_t)(T::W_BYTES + (kw >> 1) * T::SUPER_BYTES + (kw & 1) * 8 + 2 * t * SK_PITCH);
     const uint32_t x_off = (uint32_t)(T::W_BYTES + (kw >> 1) * T::SUPER_BYTES + g * SK_PITCH + Q8_QS_OFFSET + (kw & 1) * 2 * QK + 4 * t);
-    float2 acc[2][CT][2];
+    float2 acc[2][CT][2], sum[2][CT][2];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < CT; ++j) acc[i][j][0] = acc[i][j][1] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < CT; ++j) acc[i][j][0] = acc[i][j][1] = sum[i][j][0] = sum[i][j][1] = make_float2(0.0f, 0.0f);
 
     int s = 0;
     uint32_t parity = 0;
@@ -264,13 +304,36 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
                 const float2 me = make_float2(-8.0f * half_bits_to_float(s0.x >> 16), -8.0f * half_bits_to_float(s1.x >> 16));
                 const float2 mo = make_float2(-8.0f * half_bits_to_float(s0.y >> 16), -8.0f * half_bits_to_float(s1.y >> 16));
 #pragma unroll
-                for (int i = 0; i < 2; ++i) accumulate_block(acc[i][j], a_e[i], b_e, d_e[i][0], d_e[i][1], de, me);
+                for (int i = 0; i < 2; ++i) {
+                    float2 te[2], to[2];
+                    block_terms(te, a_e[i], b_e, de, me);
+                    block_terms(to, a_o[i], b_o, dq, mo);
 #pragma unroll
-                for (int i = 0; i < 2; ++i) accumulate_block(acc[i][j], a_o[i], b_o, d_o[i][0], d_o[i][1], dq, mo);
+                    for (int h = 0; h < 2; ++h) {
+                        const float2 de2 = make_float2(d_e[i][h], d_e[i][h]), do2 = make_float2(d_o[i][h], d_o[i][h]);
+                        if (T::PAIR_FIRST)
+                            acc[i][j][h] = add2(acc[i][j][h], fma2(de2, te[h], mul2(do2, to[h])));
+                        else
+                            acc[i][j][h] = fma2(de2, te[h], fma2(do2, to[h], acc[i][j][h]));
+                    }
+                }
             }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
+        if (T::LEVELS && (c % SK_FLUSH == SK_FLUSH - 1 || c == n_chunks - 1)) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                for (int j = 0; j < CT; ++j) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        sum[i][j][h] = add2(sum[i][j][h], acc[i][j][h]);
+                        acc[i][j][h] = make_float2(0.0f, 0.0f);
+                    }
+                }
+            }
+        }
         if (++s == p.stages) {
             s = 0;
             parity ^= 1u;
@@ -285,10 +348,11 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
 #pragma unroll
         for (int j = 0; j < CT; ++j) {
             const uint32_t at = mine + (uint32_t)(((j * 8 + 2 * t) * SK_RED_PITCH + i * 16 + g) * 4);
-            sts_f32(at, acc[i][j][0].x);
-            sts_f32(at + SK_RED_PITCH * 4, acc[i][j][0].y);
-            sts_f32(at + 32, acc[i][j][1].x);
-            sts_f32(at + SK_RED_PITCH * 4 + 32, acc[i][j][1].y);
+            const float2(&out)[2] = T::LEVELS ? sum[i][j] : acc[i][j];
+            sts_f32(at, out[0].x);
+            sts_f32(at + SK_RED_PITCH * 4, out[0].y);
+            sts_f32(at + 32, out[1].x);
+            sts_f32(at + SK_RED_PITCH * 4 + 32, out[1].y);
         }
     }
     if (!stream_meet(&meet[1], lane, p.fault, p.poll_limit)) return;
@@ -298,12 +362,13 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
     const int64_t rows = p.rows[mat];
 #pragma unroll
     for (int col = kw; col < T::COLS; col += T::KW) {
-        float v = 0.0f;
+        float v[T::KW];
 #pragma unroll
         for (int k = 0; k < T::KW; ++k)
-            v += __uint_as_float(lds_u32(ring + (uint32_t)((((wr * T::KW + k) * T::COLS + col) * SK_RED_PITCH + lane) * 4)));
+            v[k] = __uint_as_float(lds_u32(ring + (uint32_t)((((wr * T::KW + k) * T::COLS + col) * SK_RED_PITCH + lane) * 4)));
+        const float total = ODD && WARPS == SK_WARPS && p.n_super > SK_SHORT_SUPERS ? sum_compensated(v) : sum_tree(v);
         const int64_t m = m0 + col;
-        if (n < rows && m < p.M && JQ_IN_EXTENT(p.ext_y[mat], p.y[mat] + m * rows + n, sizeof(float), p.fault)) p.y[mat][m * rows + n] = v;
+        if (n < rows && m < p.M && JQ_IN_EXTENT(p.ext_y[mat], p.y[mat] + m * rows + n, sizeof(float), p.fault)) p.y[mat][m * rows + n] = total;
     }
 }
 
@@ -401,8 +466,8 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     const int64_t groups = (M + SK_COLUMNS - 1) / SK_COLUMNS;
     const int ct = (int)(((M + groups - 1) / groups + 7) / 8);
     // 64 rows per CTA halve the activation traffic, which from three column tiles on exceeds the weights'; 32 rows
-    // keep more SMs at work when there are few
-    const int wr = ct >= 3 && wide_tiles * groups >= caps.sm_count ? 2 : 1;
+    // keep more SMs at work when there are few, and running sums half as long (odd K, see the top)
+    const int wr = !(odd && n_super > SK_SHORT_SUPERS) && ct >= 3 && wide_tiles * groups >= caps.sm_count ? 2 : 1;
     const bool alone = wr == 1 && tiles * groups <= caps.sm_count;
     StreamMaps maps{};
     for (int i = 0; i < p.n_mats; ++i)

@@ -186,11 +186,18 @@ constexpr int64_t FP16_OPERANDS_MIN_COLUMNS = 64;
 
 // The small-batch kernel takes what the decode kernels above it refuse, up to 63 columns, and every batch whose K is an
 // odd multiple of 128 (the GEMMs need K % 256 == 0).  Multiply alone, cold weights, what was taken before / this kernel:
-// K = 4096, N = 11008, M = 16 18.8 / 14.9 us, M = 24 28.0 / 18.0 us (passes of eight columns), M = 48 44 / 26 us (integer
-// GEMM); K = 11008, N = 4096, M = 8 60 / 17.6 us (integer GEMM); K = 1408, N = 1003, M = 1 3.15 / 2.9 us, M = 45
-// 13.6 / 4.4 us; K = 4224, N = 11008, M = 2 23.7 / 16.3 us (generic kernel).  Where the decode kernel runs (3 to 8 columns,
+// K = 4096, N = 11008, M = 16 18.7 / 14.1 us, M = 24 27.8 / 17.8 us (passes of eight columns), M = 48 44.7 / 26.0 us (integer
+// GEMM); K = 11008, N = 4096, M = 8 61.6 / 11.0 us (generic kernel); K = 1408, N = 1003, M = 1 3.4 / 2.8 us, M = 48
+// 13.9 / 3.9 us; K = 4224, N = 11008, M = 2 24.2 / 14.1 us (generic kernel).  Where the decode kernel runs (3 to 8 columns,
 // K <= 6144) it is the faster one at K = 4096: N = 11008 9.5 against 13.1 us.
-inline bool small_batch_kernel_pays(int64_t K, int64_t M) { return M < FP16_OPERANDS_MIN_COLUMNS || K % (2 * SUPER) != 0; }
+// One column of a long odd K and few rows stays with the generic kernel: a CTA's stages of K are a chain however few the rows,
+// and there a warp per row still has an SM almost to itself.  Quantizer and multiply, generic / small-batch kernel: K = 10880,
+// N = 64 11.2 / 13.8 us, N = 600 12.8 / 14.2 us; K = 8320, N = 300 10.5 / 11.5 us, N = 800 11.1 / 11.5 us (with static weights
+// 3 % the other way); K = 5504, N = 1003 8.8 / 8.9 us.
+inline bool small_batch_kernel_pays(int64_t K, int64_t N, int64_t M) {
+    if (K % (2 * SUPER) == 0) return M < FP16_OPERANDS_MIN_COLUMNS;
+    return !(M == 1 && K > 8192 && N * K <= (int64_t)6 << 20);
+}
 
 int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N,
                      int64_t M, int order, int kernel) {
@@ -212,7 +219,7 @@ int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *
     int rc = JQ_ERR_UNSUPPORTED;
     if (M <= 2) rc = launch_gemv_dp4a(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
     if (rc == JQ_ERR_UNSUPPORTED && M <= 8) rc = launch_gemv_mma(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
-    if (rc == JQ_ERR_UNSUPPORTED && small_batch_kernel_pays(K, M)) rc = launch_mmq_stream(st, d_w, d_xq, d_y, K, N, M, order);
+    if (rc == JQ_ERR_UNSUPPORTED && small_batch_kernel_pays(K, N, M)) rc = launch_mmq_stream(st, d_w, d_xq, d_y, K, N, M, order);
     if (rc == JQ_ERR_UNSUPPORTED && M >= FP16_OPERANDS_MIN_COLUMNS && option_value(JQ_OPT_PREFILL_EXACT) == 0)
         rc = launch_gemm_f16(st, d_w, d_xq, d_y, K, N, M, order);  // refuses shapes outside its rules: the integer GEMM takes those
     if (rc == JQ_ERR_UNSUPPORTED && M > 8) rc = launch_gemm_mma(st, d_w, d_xq, d_y, K, N, M, order);

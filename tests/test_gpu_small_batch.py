@@ -76,6 +76,20 @@ def test_small_batch_several_matrices(env, K, M):
         assert env.t.equal(y, c.mul_mat_q4_0_q8_1(w, xq, K, n, M))
 
 
+@pytest.mark.parametrize("K,N,M,generic", [(8320, 756, 1, True), (8320, 757, 1, False), (10880, 31, 1, True), (8320, 64, 2, False),
+                                           (8064, 64, 1, False), (10752, 64, 1, False)])
+def test_one_column_of_a_long_odd_k(env, K, N, M, generic):
+    """Which side of its line a shape is on shows in the bits: the kernels add in different orders."""
+    c, O = env.c, env.O
+    w, x = _problem(K, N, M)
+    wq = O.quantize_q4_0(w)
+    xq = O.quantize_q8_1(x, O.ORDER_COL_KSUPER, c.S_SUM_X)
+    d_w, d_x = env.t.from_numpy(wq).to(env.dev), env.t.from_numpy(xq).to(env.dev)
+    y = c.mul_mat_q4_0_q8_1(d_w, d_x, K, N, M)
+    assert O.err_max_rel(y.cpu().numpy(), O.mul_mat_ref(wq, xq, K, N, M)) <= TOL
+    assert env.t.equal(y, c.mul_mat_q4_0_q8_1(d_w, d_x, K, N, M, kernel=c.KERNEL_GENERIC)) == generic
+
+
 def _error_against_64_bits(t, w, xq, y, K, rows):
     """2-norm of the difference over 2-norm of sum(d4 * (sumi * d8 - 8 * s8)) in 64 bits, over some weight rows."""
     M = y.shape[0]

@@ -3,7 +3,7 @@
 ``build_all()`` runs nvcc on every source under ``csrc/`` for sm_100a only
 (``-gencode arch=compute_100a,code=sm_100a``), links ``libjq_b200.so`` next to this file and
 builds ``python/q8_1_me*.so`` and ``python/mm_q4_0_q8_1_me*.so`` against it, and ``_torch_calls*.so`` (the
-native part of ``capi.py``) against torch.  nvcc
+native part of ``capi.py``) against torch, where there is one.  nvcc
 cross-compiles without a GPU, so this also serves as the "does it build" check.  The
 top-level ``CMakeLists.txt`` describes the same targets for CMake users.
 """
@@ -112,6 +112,34 @@ def build_check(force: bool = False, verbose: bool = False) -> str:
     return CHECK_LIB_PATH
 
 
+def _torch_dir() -> str | None:
+    spec = importlib.util.find_spec("torch")
+    return os.path.dirname(spec.origin) if spec is not None and spec.origin else None
+
+
+def _build_torch_calls(force: bool, verbose: bool) -> None:
+    """The native part of ``capi.py``.  Without torch there is nothing to build it against and nothing that imports it: the
+    library and the two reference-named modules do without."""
+    torch_dir = _torch_dir()
+    if torch_dir is None:
+        if verbose:
+            print("[jq build] no torch: _torch_calls is left out", file=sys.stderr)
+        return
+    src_path = os.path.join(CSRC, "bindings", "torch_calls.cpp")
+    out = os.path.join(PKG_DIR, "_torch_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if not force and _mtime(out) >= max(_mtime(src_path), _newest_header()):
+        return
+    torch_lib = os.path.join(torch_dir, "lib")
+    _run(
+        [
+            _host_cxx(), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+            "-I", os.path.join(torch_dir, "include"), "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+            "-I", _cuda_include(), "-I", sysconfig.get_paths()["include"], "-I", INCLUDE_DIR, src_path, "-o", out,
+            "-L", torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath," + torch_lib,
+        ]
+    )
+
+
 def build_all(force: bool = False, verbose: bool = False) -> str:
     """Compile what is out of date; returns the path of ``libjq_b200.so``."""
     os.makedirs(PY_DIR, exist_ok=True)
@@ -135,19 +163,7 @@ def build_all(force: bool = False, verbose: bool = False) -> str:
                 ]
             )
 
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
-    torch_lib = os.path.join(torch_dir, "lib")
-    src_path = os.path.join(CSRC, "bindings", "torch_calls.cpp")
-    out = os.path.join(PKG_DIR, "_torch_calls" + ext)
-    if force or _mtime(out) < max(_mtime(src_path), hdr_time):
-        _run(
-            [
-                _host_cxx(), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-                "-I", os.path.join(torch_dir, "include"), "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
-                "-I", _cuda_include(), "-I", py_inc, "-I", INCLUDE_DIR, src_path, "-o", out,
-                "-L", torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath," + torch_lib,
-            ]
-        )
+    _build_torch_calls(force, verbose)
     return LIB_PATH
 
 

@@ -1,0 +1,30 @@
+"""What the build does with and without torch, with the compiler replaced by a list of its command lines."""
+import importlib.util
+
+import pytest
+
+from jjjetson_ops_b200 import _build
+
+
+@pytest.fixture
+def commands(monkeypatch, tmp_path):
+    """A package folder whose library and binding modules are up to date, and what is compiled there."""
+    ran = []
+
+    def run(cmd):
+        ran.append(cmd)
+        with open(cmd[cmd.index("-o") + 1], "w"):
+            pass
+
+    monkeypatch.setattr(_build, "_run", run)
+    monkeypatch.setattr(_build, "_build_library", lambda *a: None)
+    monkeypatch.setattr(_build, "BINDINGS", {})
+    for name, folder in (("PKG_DIR", tmp_path), ("PY_DIR", tmp_path / "python"), ("OBJ_DIR", tmp_path / "build")):
+        monkeypatch.setattr(_build, name, str(folder))
+    return ran
+
+
+def test_without_torch_the_rest_is_built(commands, monkeypatch):
+    find = importlib.util.find_spec
+    monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
+    assert _build.build_all() == _build.LIB_PATH and commands == []

@@ -10,6 +10,7 @@ top-level ``CMakeLists.txt`` describes the same targets for CMake users.
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.metadata
 import importlib.util
 import os
 import shutil
@@ -127,8 +128,17 @@ def _build_torch_calls(force: bool, verbose: bool) -> None:
         return
     src_path = os.path.join(CSRC, "bindings", "torch_calls.cpp")
     out = os.path.join(PKG_DIR, "_torch_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
-    if not force and _mtime(out) >= max(_mtime(src_path), _newest_header()):
-        return
+    # another torch needs another build, whatever the age of the files
+    stamp = os.path.join(OBJ_DIR, "torch_calls.txt")
+    try:
+        version = importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:
+        version = "unknown"
+    built_for = "%s %s\n" % (version, torch_dir)
+    if not force and _mtime(out) >= max(_mtime(src_path), _newest_header()) and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read() == built_for:
+                return
     torch_lib = os.path.join(torch_dir, "lib")
     _run(
         [
@@ -138,6 +148,9 @@ def _build_torch_calls(force: bool, verbose: bool) -> None:
             "-L", torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath," + torch_lib,
         ]
     )
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(built_for)
 
 
 def build_all(force: bool = False, verbose: bool = False) -> str:

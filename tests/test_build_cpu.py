@@ -1,5 +1,6 @@
 """What the build does with and without torch, with the compiler replaced by a list of its command lines."""
 import importlib.util
+import os
 
 import pytest
 
@@ -28,3 +29,13 @@ def test_without_torch_the_rest_is_built(commands, monkeypatch):
     find = importlib.util.find_spec
     monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
     assert _build.build_all() == _build.LIB_PATH and commands == []
+
+
+def test_another_torch_is_another_build(commands, monkeypatch):
+    _build.build_all()
+    assert len(commands) == 1 and os.path.basename(commands[0][commands[0].index("-o") + 1]).startswith("_torch_calls")
+    _build.build_all()
+    assert len(commands) == 1
+    monkeypatch.setattr(_build.importlib.metadata, "version", lambda name: "0.0.0")
+    _build.build_all()
+    assert len(commands) == 2

@@ -24,14 +24,17 @@
 // 22.5 against 18.0 us at M = 24; weights of four or eight stages ahead of the previous kernel's end instead of two, no
 // difference.
 //
-// Rounding.  A running sum rounds at every addition, and most when it is long: with one per warp over all of its blocks and the
-// warps' parts added one after the other the error against 64 bits was 1.2 to 1.55 times that of the kernels that took these shapes
-// before (K = 4224: 7.3e-8 of the result in the generic kernel, 11.4e-8 here at 64 rows per CTA).  So the parts are added as a tree;
-// up to eight columns, where registers are left, a warp sums in two levels; the two blocks of a pair are added to each other first
-// where the sums are long for their kind (64 rows per CTA have four warps along K, odd K replaces the generic kernel); and odd K
-// beyond 2048 keeps to 32 rows per CTA and adds the parts of eight warps with the rounded-off remainders.  The error is then 0.85 to
-// 1.02 times the former kernels' on average over each group of shapes, and the multiply takes (of its time with plain running sums)
-// 1.00 to 1.03 on average: 64 rows per CTA 1.02 to 1.05, odd K beyond 2048 with many rows 1.04, at most 1.18.
+// Rounding.  K % 256 == 0: a warp keeps one running sum over all of its blocks and the warps' parts are added one after the other,
+// 1.0 to 1.4 times the error against 64 bits of the kernels that took these shapes up to 32 columns (8e-8 to 12e-8 of the result)
+// and a seventh to a half of the integer GEMM's beyond.  An odd multiple of 128 replaces the generic kernel, whose 32 lanes round off
+// little (7.3e-8): there the same sums were 1.2 to 1.55 times as far off, so they are kept short.  The two blocks of a pair are added
+// to each other first; up to eight columns, where registers are left, a warp sums in two levels; the parts are added as a tree;
+// beyond K = 2048 a CTA keeps to 32 rows (eight warps along K, not four) and adds the parts of eight warps with the rounded-off
+// remainders.  That is 0.94 to 1.03 times the generic kernel's error on average over each group of shapes, for 1.00 to 1.05 of the
+// time (K beyond 2048 with thousands of rows 1.04 on average, 1.18 at most; the generic kernel takes three to eight times as long).
+// The same for K % 256 == 0 was measured (1.00 to 1.05 of the time, the former kernels' error) and left out: a decode step turns a
+// last bit into a step of the int8 quantizer here and there, up to 4e-3 of its logits, for no gain in their own error (6.2e-3 against
+// a chain in 64 bits either way).
 //
 // A tensor copy wants a row pitch of whole 16-byte units, which K % 256 == 0 gives.  When K is an odd multiple of 128 a
 // row is 8 bytes short of that but two rows are not: the even rows are one tensor and the odd rows another (its base 8
@@ -87,8 +90,8 @@ struct StreamParams {
 template <int CT, int WR, bool ODD, int WARPS>
 struct StreamTile {
     static constexpr int ROWS = 32 * WR, COLS = 8 * CT;
-    static constexpr bool PAIR_FIRST = ODD || WR == 2;  // the blocks of a pair are added before they join the running sum
-    static constexpr bool LEVELS = CT == 1;             // running sums of SK_FLUSH stages, and one of those
+    static constexpr bool PAIR_FIRST = ODD;        // the blocks of a pair are added before they join the running sum
+    static constexpr bool LEVELS = ODD && CT == 1;  // running sums of SK_FLUSH stages, and one of those
     static constexpr int KW = WARPS / WR;  // warps along K = pairs of blocks per stage
     static constexpr int SUPERS = KW / 2;     // 128-value groups per stage
     // weights of 256 values of K: ROWS rows, or ROWS / 2 even ones and ROWS / 2 odd ones
@@ -124,8 +127,15 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return d;
 }
 
-// Sums of the warps' parts, in an order that is always the same: as a tree, or (odd K) with what each addition rounds off
-// added up as well (Knuth's two-sum), so that only the result is rounded.
+// Sums of the warps' parts, in an order that is always the same: one after the other, as a tree, or with what each addition
+// rounds off added up as well (Knuth's two-sum), so that only the result is rounded.
+template <int N>
+__device__ __forceinline__ float sum_in_order(const float (&v)[N]) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) sum += v[k];
+    return sum;
+}
 template <int N>
 __device__ __forceinline__ float sum_tree(float (&v)[N]) {
 #pragma unroll
@@ -314,7 +324,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
                         if (T::PAIR_FIRST)
                             acc[i][j][h] = add2(acc[i][j][h], fma2(de2, te[h], mul2(do2, to[h])));
                         else
-                            acc[i][j][h] = fma2(de2, te[h], fma2(do2, to[h], acc[i][j][h]));
+                            acc[i][j][h] = fma2(do2, to[h], fma2(de2, te[h], acc[i][j][h]));
                     }
                 }
             }
@@ -366,7 +376,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
 #pragma unroll
         for (int k = 0; k < T::KW; ++k)
             v[k] = __uint_as_float(lds_u32(ring + (uint32_t)((((wr * T::KW + k) * T::COLS + col) * SK_RED_PITCH + lane) * 4)));
-        const float total = ODD && WARPS == SK_WARPS && p.n_super > SK_SHORT_SUPERS ? sum_compensated(v) : sum_tree(v);
+        const float total = !ODD ? sum_in_order(v) : WARPS == SK_WARPS && p.n_super > SK_SHORT_SUPERS ? sum_compensated(v) : sum_tree(v);
         const int64_t m = m0 + col;
         if (n < rows && m < p.M && JQ_IN_EXTENT(p.ext_y[mat], p.y[mat] + m * rows + n, sizeof(float), p.fault)) p.y[mat][m * rows + n] = total;
     }

@@ -28,10 +28,10 @@
 // 1.0 to 1.4 times the error against 64 bits of the kernels that took these shapes up to 32 columns (8e-8 to 12e-8 of the result)
 // and a seventh to a half of the integer GEMM's beyond.  An odd multiple of 128 replaces the generic kernel, whose 32 lanes round off
 // little (7.3e-8): there the same sums were 1.2 to 1.55 times as far off, so they are kept short.  The two blocks of a pair are added
-// to each other first; up to eight columns, where registers are left, a warp sums in two levels; the parts are added as a tree;
-// beyond K = 2048 a CTA keeps to 32 rows (eight warps along K, not four) and adds the parts of eight warps with the rounded-off
-// remainders.  That is 0.94 to 1.03 times the generic kernel's error on average over each group of shapes, for 1.00 to 1.05 of the
-// time (K beyond 2048 with thousands of rows 1.04 on average, 1.18 at most; the generic kernel takes three to eight times as long).
+// to each other first, unless sixteen warps share K; up to eight columns, where registers are left, each of eight warps sums in two
+// levels; the parts are added as a tree; beyond K = 2048 a CTA keeps to 32 rows (eight warps along K, not four) and adds the parts of
+// eight warps with the rounded-off remainders.  That is 0.93 to 1.06 times the generic kernel's error on average over each group of
+// shapes, for 0.98 to 1.06 of the time (at most 1.18: K = 4224, N = 32000, M = 24, where the generic kernel takes eight times as long).
 // The same for K % 256 == 0 was measured (1.00 to 1.05 of the time, the former kernels' error) and left out: a decode step turns a
 // last bit into a step of the int8 quantizer here and there, up to 4e-3 of its logits, for no gain in their own error (6.2e-3 against
 // a chain in 64 bits either way).
@@ -90,8 +90,10 @@ struct StreamParams {
 template <int CT, int WR, bool ODD, int WARPS>
 struct StreamTile {
     static constexpr int ROWS = 32 * WR, COLS = 8 * CT;
-    static constexpr bool PAIR_FIRST = ODD;        // the blocks of a pair are added before they join the running sum
-    static constexpr bool LEVELS = ODD && CT == 1;  // running sums of SK_FLUSH stages, and one of those
+    // the blocks of a pair are added before they join the running sum (sixteen warps' are short without that: it then only
+    // stays where the copies hide it)
+    static constexpr bool PAIR_FIRST = ODD && (WARPS == SK_WARPS || CT <= 2);
+    static constexpr bool LEVELS = ODD && WARPS == SK_WARPS && CT == 1;  // running sums of SK_FLUSH stages, and one of those
     static constexpr int KW = WARPS / WR;  // warps along K = pairs of blocks per stage
     static constexpr int SUPERS = KW / 2;     // 128-value groups per stage
     // weights of 256 values of K: ROWS rows, or ROWS / 2 even ones and ROWS / 2 odd ones

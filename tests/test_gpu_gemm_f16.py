@@ -9,6 +9,8 @@ when the quantizer stored s = d * sum(q).
 import numpy as np
 import pytest
 
+from launch_forms import gemm_f16_form
+
 pytestmark = pytest.mark.gpu
 
 TOL_F16_FORMULA = 1e-3  # operands rounded to fp16 (2^-11 relative each), fp32 accumulation
@@ -102,10 +104,13 @@ def test_gemm_f16_matches_integer_kernel_closely(env):
 
 
 # More tiles than SMs, so that pairs of CTAs share 256 x 256 tiles: the last pair's second CTA without rows (18690 = 73 * 256
-# + 2) or with one, its columns a few or all but one; one stage pair, and more stages than the ring holds.
-@pytest.mark.parametrize("K,N,M", [(256, 18690, 130), (768, 18690, 255), (1280, 18817, 256), (512, 9473, 400)])
+# + 2) or with one, its columns a few or all but one; one stage pair, and more stages than the ring holds.  With 300 tiles on 148
+# SMs and a short K single CTAs are as quick: several waves of those.
+@pytest.mark.parametrize("K,N,M,form", [(256, 18690, 130, "pair"), (768, 18690, 255, "pair"), (1280, 18817, 256, "pair"), (512, 8960, 400, "pair"),
+                                        (512, 9473, 400, 1)])
 @pytest.mark.parametrize("order", [0, 1])
-def test_gemm_f16_pairs_of_ctas(env, K, N, M, order):
+def test_gemm_f16_pairs_of_ctas(env, K, N, M, form, order):
+    assert gemm_f16_form(K, [N], M) == form
     rng = np.random.default_rng(K + N + M + order)
     w = (rng.standard_normal((N, K), dtype=np.float32) * np.float32(0.02)).astype(np.float32)
     x = rng.standard_normal((M, K), dtype=np.float32)
@@ -113,18 +118,45 @@ def test_gemm_f16_pairs_of_ctas(env, K, N, M, order):
     _check(env, env.O.quantize_q4_0(w), x, K, N, M, order, env.c.S_SUM_X, rows)
 
 
-# K in 2, 3, 4, 6 and 8 parts, equal and with a shorter last one, added up over shared memory by the CTAs of a cluster
-@pytest.mark.parametrize("K,N,M", [(512, 130, 64), (768, 200, 66), (1024, 129, 200), (1536, 1, 130), (2816, 300, 65), (2048, 257, 9)])
-def test_gemm_f16_parts_of_k(env, K, N, M):
+# K in one to eight parts, equal and with a shorter last one, added up over shared memory by the CTAs of a cluster
+@pytest.mark.parametrize("K,N,M,parts", [(512, 130, 64, 1), (768, 200, 66, 1), (2048, 4096, 200, 2), (2304, 4096, 256, 2), (2304, 300, 65, 3),
+                                         (1024, 129, 200, 4), (2048, 257, 9, 4), (1536, 1, 130, 6), (2816, 300, 65, 6), (4096, 300, 65, 8)])
+def test_gemm_f16_parts_of_k(env, K, N, M, parts):
+    assert gemm_f16_form(K, [N], M) == parts
     rng = np.random.default_rng(K + N + M)
     w = (rng.standard_normal((N, K), dtype=np.float32) * np.float32(0.02)).astype(np.float32)
-    _check(env, env.O.quantize_q4_0(w), rng.standard_normal((M, K), dtype=np.float32), K, N, M, env.c.ORDER_KSUPER_COL, env.c.S_SUM_X)
+    rows = None if N <= 300 else np.unique(np.concatenate([rng.choice(N, size=96, replace=False), [0, 127, 128, N - 1]]))
+    _check(env, env.O.quantize_q4_0(w), rng.standard_normal((M, K), dtype=np.float32), K, N, M, env.c.ORDER_KSUPER_COL, env.c.S_SUM_X, rows)
 
 
-@pytest.mark.parametrize("K,rows,M", [(512, [300, 1, 128, 257], 64), (256, [9400, 9290], 130), (4096, [128, 200], 100)])
-def test_gemm_f16_several_matrices(env, K, rows, M):
+def test_gemm_f16_parts_of_k_on_two_streams(env):
+    """Launches that split K on two streams at once: each keeps its parts to itself."""
+    c, t = env.c, env.t
+    g = t.Generator(device=env.dev)
+    g.manual_seed(12)
+    problems = []
+    for K, N, M in [(4096, 2048, 100), (2048, 1003, 70)]:
+        assert gemm_f16_form(K, [N], M) > 1
+        w = c.quantize_q4_0(t.randn((N, K), generator=g, device=env.dev).mul_(0.02))
+        xqs = [c.quantize_q8_1(t.randn((M, K), generator=g, device=env.dev)) for _ in range(8)]
+        want = [c.mul_mat_q4_0_q8_1(w, xq, K, N, M, kernel=c.KERNEL_GEMM_F16) for xq in xqs]
+        problems.append((K, N, M, w, xqs, want, [t.empty_like(y) for y in want], t.cuda.Stream(env.dev)))
+    t.cuda.synchronize()
+    for i in range(8):
+        for K, N, M, w, xqs, _, got, stream in problems:
+            with t.cuda.stream(stream):
+                c.mul_mat_q4_0_q8_1(w, xqs[i], K, N, M, kernel=c.KERNEL_GEMM_F16, out=got[i])
+    t.cuda.synchronize()
+    for p in problems:
+        assert all(t.equal(a, b) for a, b in zip(p[5], p[6]))
+
+
+@pytest.mark.parametrize("K,rows,M,form", [(512, [300, 1, 128, 257], 64, 1), (256, [9400, 9290], 130, "pair"), (4096, [128, 200], 100, 8),
+                                           (4096, [1024, 1024, 1024], 128, 4)])
+def test_gemm_f16_several_matrices(env, K, rows, M, form):
     """Several matrices in one launch (single CTAs, pairs, split K): each row against separate calls, whose sums over K may
     be split elsewhere (fp32 additions in another order)."""
+    assert gemm_f16_form(K, rows, M) == form
     c = env.c
     rng = np.random.default_rng(K + M)
     ws = [c.quantize_q4_0(env.up((rng.standard_normal((n, K), dtype=np.float32) * np.float32(0.02)))) for n in rows]
@@ -137,7 +169,7 @@ def test_gemm_f16_several_matrices(env, K, rows, M):
 
 @pytest.mark.parametrize("K,N,M", [(4096, 4096, 128), (11008, 4096, 128), (8192, 300, 70), (2048, 1000, 64)])
 def test_gemm_f16_split_k_is_ordered(env, K, N, M):
-    """Few output tiles and a long K: the kernel splits K over several CTAs per tile, which add their parts to y in a
+    """Few output tiles and a long K: the kernel splits K over the CTAs of a cluster, which add up their parts in a
     fixed order.  Right against the oracle (a sample of rows at the large sizes), and bit-equal from run to run."""
     c = env.c
     rng = np.random.default_rng(K + N + M)

@@ -8,6 +8,8 @@ a few 1e-7 as a rule).
 import numpy as np
 import pytest
 
+from launch_forms import small_batch_form
+
 pytestmark = pytest.mark.gpu
 
 TOL = 1e-5
@@ -30,8 +32,8 @@ def _problem(K, N, M):
     return w, rng.standard_normal((M, K), dtype=np.float32)
 
 
-# Row tiles of 32 and (from 17 columns on, with enough of them) 64, column tiles of 8 to 32 in equal groups, stages of 512
-# or 256 values with a shorter last one; more stages than the ring holds; an odd K with every remainder of four.
+# Row tiles of 32 (one CTA per SM, sixteen warps along K) and (from 17 columns on, with enough of them) 64, column tiles of 8 to 32
+# in equal groups, stages of 1024 or 256 values with a shorter last one; an odd K with every remainder of eight.
 @pytest.mark.parametrize("K,N,M", [(128, 1, 1), (128, 31, 3), (384, 33, 9), (640, 32, 33), (1408, 65, 45), (896, 100, 130), (4224, 20, 2),
                                    (256, 31, 9), (512, 33, 16), (768, 64, 17), (6400, 40, 8), (6400, 10, 3), (4608, 97, 32),
                                    (256, 9500, 24), (512, 4800, 63), (1280, 9473, 31), (11008, 35, 63)])
@@ -63,17 +65,46 @@ def test_small_batch_weights_off_alignment(env, K, shift):
     assert O.err_max_rel(y.cpu().numpy(), O.mul_mat_ref(wq, xq, K, N, M)) <= TOL
 
 
-@pytest.mark.parametrize("K,M", [(512, 12), (6400, 5), (640, 7), (512, 40)])
-def test_small_batch_several_matrices(env, K, M):
-    """Several matrices in one launch give the bits of separate calls."""
+# The other forms: eight warps, two CTAs per SM, with 32 and 64 rows each, at even and odd K; a ring that goes round several times.
+@pytest.mark.parametrize("K,N,M,form", [
+    (640, 4900, 5, (True, 1, 32, False)), (1408, 4801, 16, (True, 2, 32, False)), (2688, 9473, 20, (True, 3, 32, False)),
+    (1152, 4740, 30, (True, 4, 32, False)), (384, 9473, 24, (True, 3, 64, False)), (1152, 9473, 31, (True, 4, 64, False)),
+    (6400, 4900, 8, (False, 1, 32, False)), (512, 5000, 12, (False, 2, 32, False)), (512, 5000, 24, (False, 3, 32, False)),
+    (3072, 4740, 30, (False, 4, 32, False)), (4096, 9473, 24, (False, 3, 64, False)), (4352, 9473, 31, (False, 4, 64, False))])
+@pytest.mark.parametrize("order", [0, 1])
+def test_small_batch_two_ctas_per_sm(env, K, N, M, form, order):
+    assert small_batch_form(K, [N], M) == form
     c, O = env.c, env.O
-    rows = [40, 1, 96, 33]
+    w, x = _problem(K, N, M)
+    d_w = c.quantize_q4_0(env.t.from_numpy(w).to(env.dev))
+    wq = d_w.cpu().numpy().reshape(N, -1)
+    rows = np.unique(np.concatenate([np.random.default_rng(N).choice(N, size=120, replace=False), [0, 31, 32, 63, 64, N - 2, N - 1]]))
+    xq = O.quantize_q8_1(x, order, c.S_SUM_X)
+    y = env.t.full((M, N), float("nan"), device=env.dev)
+    c.mul_mat_q4_0_q8_1(d_w, env.t.from_numpy(xq).to(env.dev), K, N, M, order, out=y)
+    assert not env.t.isnan(y).any()
+    assert O.err_max_rel(y.cpu().numpy()[:, rows], O.mul_mat_ref(np.ascontiguousarray(wq[rows]), xq, K, len(rows), M, order)) <= TOL
+
+
+@pytest.mark.parametrize("K,rows,M,same_form", [(512, [40, 1, 96, 33], 12, True), (6400, [40, 1, 96, 33], 5, True), (640, [40, 1, 96, 33], 7, True),
+                                                (512, [40, 1, 96, 33], 40, True), (4096, [2000, 2000, 2000], 16, False),
+                                                (4096, [4096, 4096, 4096], 20, False), (1408, [4096, 64], 45, False)])
+def test_small_batch_several_matrices(env, K, rows, M, same_form):
+    """Several matrices in one launch against separate calls: the same bits where both are divided in the same way.  Where the
+    launch has more tiles than each matrix alone, K may be shared by fewer warps, and the fp32 additions are in another order."""
+    forms = [small_batch_form(K, [n], M) for n in rows]
+    assert all(f == small_batch_form(K, rows, M) for f in forms) == same_form
+    c, O = env.c, env.O
     x = _problem(K, 1, M)[1]
-    ws = [env.t.from_numpy(O.quantize_q4_0(_problem(K, n, M + i)[0])).to(env.dev) for i, n in enumerate(rows)]
+    ws = [c.quantize_q4_0(env.t.from_numpy(_problem(K, n, M + i)[0]).to(env.dev)) for i, n in enumerate(rows)]
     xq = env.t.from_numpy(O.quantize_q8_1(x, O.ORDER_COL_KSUPER, c.S_D_SUM_Q)).to(env.dev)
     outs = c.linear_q4_0_multi(ws, rows, xq=xq, K=K, M=M)
     for w, n, y in zip(ws, rows, outs):
-        assert env.t.equal(y, c.mul_mat_q4_0_q8_1(w, xq, K, n, M))
+        apart = c.mul_mat_q4_0_q8_1(w, xq, K, n, M)
+        if same_form:
+            assert env.t.equal(y, apart)
+        else:
+            assert O.err_max_rel(y.cpu().numpy(), apart.cpu().numpy()) <= TOL
 
 
 @pytest.mark.parametrize("K,N,M,generic", [(8320, 756, 1, True), (8320, 757, 1, False), (10880, 31, 1, True), (8320, 64, 2, False),

@@ -65,3 +65,24 @@ class Small(Rows):
         return N
 """
     assert _raised(["multi(Rows(), N, N)", "multi(Small(), N, Rows())"], setup) == ["OverflowError"] * 2
+
+
+def test_refused_arguments(native_lib):
+    """Wrong type, layout, device, dimensions or counts: ValueError, as before the calls were native."""
+    calls = [
+        "c.quantize_q8_1(f32(M, K).half(), out=u8(nq))",
+        "c.quantize_q8_1(f32(K, M).t(), out=u8(nq))",
+        "c.quantize_q8_1(f32(M, K), out=f32(nq))",
+        "c.quantize_q8_1(f32(1, M, K), out=u8(nq))",
+        "c.mul_mat_q4_0_q8_1(f32(nw), u8(nq), K, N, M, out=f32(M, N))",
+        "c.mul_mat_q4_0_q8_1(u8(nw), u8(nq).cpu(), K, N, M, out=f32(M, N))",
+        "c.mul_mat_q4_0_q8_1(u8(nw), u8(nq), K, N, M, out=f32(M, 2 * N)[:, ::2])",
+        "c.linear_q4_0(u8(nw), f32(M * K), N, ws=u8(nq), out=f32(M, N))",
+        "c.linear_q4_0(None, f32(M, K), N, ws=u8(nq), out=f32(M, N))",
+        "c.linear_q4_0_multi([u8(nw)], [N, N], xq=u8(nq), K=K, M=M, outs=[f32(M, N)])",
+        "c.linear_q4_0_multi([u8(nw)] * 17, [N] * 17, xq=u8(nq), K=K, M=M, outs=[f32(M, N)] * 17)",
+        "c.rms_norm_q8_1(f32(M, K), f32(K), 1e-6, xq=[0])",
+        "c.rms_norm_q8_1(f32(M, K), f32(K).double(), 1e-6, xq=u8(nq))",
+        "c.swiglu_q8_1(f32(M, K), f32(K, M).t(), xq=u8(nq))",
+    ]
+    assert _raised(calls) == ["ValueError"] * len(calls)

@@ -90,7 +90,8 @@ typedef enum jq_option {
     JQ_OPT_PREFILL_EXACT = 1,
     /* Number of polls after which a bounded device-side wait (for a bulk copy, or for the bands of an
      * all-gather) gives up, sets the fault word read by jq_device_fault() and lets its kernel return.
-     * It applies to the decode kernels' waits and to jq_allgather_wait_device.
+     * It applies to the decode kernels' waits, where it counts as at least 2^16 (a kernel must not end
+     * before its copies into shared memory have landed), and to jq_allgather_wait_device.
      * 0 (default): 2^22 polls, far beyond any wait of a healthy run.  The value is read when a kernel is
      * launched.  There is no counterpart in the reference (its kernels never wait on one another). */
     JQ_OPT_WAIT_POLL_LIMIT = 2,

@@ -51,6 +51,11 @@ uint32_t wait_poll_limit() {
     return v > 0 ? (uint32_t)v : (1u << 22);
 }
 
+uint32_t copy_wait_poll_limit() {
+    const uint32_t v = wait_poll_limit();
+    return v < MIN_COPY_POLLS ? MIN_COPY_POLLS : v;
+}
+
 int option_value(int option) {
     return option >= 0 && option < JQ_OPT_COUNT_ ? g_options[option].load(std::memory_order_relaxed) : 0;
 }

@@ -54,6 +54,11 @@ int ensure_dynamic_smem(const void *kernel, int bytes, bool max_carveout = false
 int option_value(int option);       // process-wide settings of jq_set_option()
 // Polls after which a bounded device-side wait gives up (JQ_OPT_WAIT_POLL_LIMIT; 2^22 by default).
 uint32_t wait_poll_limit();
+// The same for kernels that copy into shared memory, at least 2^16.  A CTA must not end while copies into its shared memory are
+// under way: the SM gives that memory to the next one.  So many polls of an mbarrier take many times what a copy does, so that a
+// CTA which gives up has none left.
+constexpr uint32_t MIN_COPY_POLLS = 1u << 16;
+uint32_t copy_wait_poll_limit();
 // Tracing aid (jq_trace_enable): device address where the next traced launch may write its
 // per-CTA timestamps, or nullptr when tracing is off or the buffer is full.
 void *next_trace_slot();

@@ -1209,7 +1209,7 @@ int fill_params(GemvParams &p, const void *d_w, const void *d_xq, const float *d
     // Ahead of the previous kernel's end only two stages are requested (more would delay the
     // activation loads that follow the wait).
     p.early_stages = p.prefetch_early ? 2 : (1 << 30);
-    p.poll_limit = wait_poll_limit();
+    p.poll_limit = copy_wait_poll_limit();
 #ifdef JQ_BOUNDS_CHECK
     const unsigned long long blocks_bytes = (unsigned long long)M * (unsigned long long)p.n_super * Q8_BYTES;
     p.ext_w[0] = make_extent(d_w, (unsigned long long)N * p.row_bytes);

@@ -176,19 +176,6 @@ __device__ __forceinline__ bool stream_meet(uint64_t *bar, int lane, int *fault,
     return mbar_wait_bounded(bar, 0u, fault, limit);
 }
 
-// A CTA must not end while copies into its shared memory are under way: the SM gives that memory to the next one.  Every consumer
-// waits for the stages in turn, so one that gives up on a stage stays some 100 us longer, many times what a copy takes.  (The
-// default limit of 2^22 polls is longer than that by itself; a caller may have set a short one.)
-__device__ __forceinline__ void linger() {
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    for (int i = 0; i < 1024; ++i) {
-        __nanosleep(1000);
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        if (t - t0 > 100000ull) break;
-    }
-}
-
 // Weights of stage c (one thread).
 template <int CT, int WR, bool ODD, int WARPS>
 __device__ __forceinline__ void stream_load_weights(const StreamParams &p, const StreamMaps &maps, int mat, int64_t n0, int c, uint32_t stage,
@@ -298,10 +285,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
     int s = 0;
     uint32_t parity = 0;
     for (int c = 0; c < n_chunks; ++c) {
-        if (!mbar_wait_bounded(&full[s], parity, p.fault, p.poll_limit)) {
-            linger();
-            return;
-        }
+        if (!mbar_wait_bounded(&full[s], parity, p.fault, p.poll_limit)) return;
         if (c * T::KW + kw < n_pairs) {
             const uint32_t stage = ring + (uint32_t)s * T::STAGE_BYTES;
             uint32_t a_e[2][4], a_o[2][4];
@@ -488,7 +472,7 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     p.n_super = (int)n_super;
     p.order = order;
     p.fault = device_fault_ptr();
-    p.poll_limit = wait_poll_limit();
+    p.poll_limit = copy_wait_poll_limit();
     p.early_stages = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 2 : 0;
     // columns in equal groups of at most 32
     const int64_t groups = (M + SK_COLUMNS - 1) / SK_COLUMNS;

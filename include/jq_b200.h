@@ -74,9 +74,10 @@ typedef enum jq_kernel {
 /* Process-wide switches. */
 typedef enum jq_option {
     /* 1: the caller promises that weight buffers are never written by work queued just ahead of a
-     * multiply on the same stream (true for inference: weights are uploaded once).  The decode
-     * kernels then start streaming weights while the previous kernel on the stream is still
-     * draining, before they wait for it; activations and outputs are always ordered normally.
+     * multiply on the same stream (true for inference: weights are uploaded once).  The decode and
+     * small-batch kernels and the fp16-operand GEMM then start streaming weights while the previous
+     * kernel on the stream is still draining, before they wait for it; activations and outputs are
+     * always ordered normally.
      * 0 (default): the weight stream, too, waits for the previous kernel. */
     JQ_OPT_STATIC_WEIGHTS = 0,
     /* What JQ_KERNEL_AUTO runs for prefill batches (64 activation columns and more).
@@ -90,8 +91,9 @@ typedef enum jq_option {
     JQ_OPT_PREFILL_EXACT = 1,
     /* Number of polls after which a bounded device-side wait (for a bulk copy, or for the bands of an
      * all-gather) gives up, sets the fault word read by jq_device_fault() and lets its kernel return.
-     * It applies to the decode kernels' waits, where it counts as at least 2^16 (a kernel must not end
-     * before its copies into shared memory have landed), and to jq_allgather_wait_device.
+     * It applies to the waits of the decode and small-batch kernels, where it counts as at least 2^16 (a
+     * kernel must not end before its copies into shared memory have landed), and to
+     * jq_allgather_wait_device.
      * 0 (default): 2^22 polls, far beyond any wait of a healthy run.  The value is read when a kernel is
      * launched.  There is no counterpart in the reference (its kernels never wait on one another). */
     JQ_OPT_WAIT_POLL_LIMIT = 2,
@@ -158,11 +160,15 @@ int jq_linear_q4_0_device(void *stream, const void *d_w, const float *d_x, void 
  * whose weights live in separate buffers (src/model/transformer_model.h:13-23).  Matrix i has
  * N[i] rows of K / 32 Q4_0 blocks and writes d_y[i] = [M][N[i]].  Give either d_x (fp32, then
  * d_ws receives the Q8_1 blocks as in jq_linear_q4_0_device) or d_xq (blocks in
- * JQ_ORDER_COL_KSUPER order, e.g. from jq_rms_norm_q8_1_device; d_ws unused).  For M <= 8 and
- * K within the decode kernels' reach the matrices are treated as one matrix of sum(N) rows and
- * multiplied by a single launch, with the same results as separate calls; other shapes quantize
- * once and run one multiply per matrix.  No counterpart in the reference (its linears are
- * separate cuBLAS calls). */
+ * JQ_ORDER_COL_KSUPER order, e.g. from jq_rms_norm_q8_1_device; d_ws unused).  Where a kernel
+ * takes several matrices they are treated as one matrix of sum(N) rows and multiplied by a single
+ * launch: the decode and the small-batch kernel (M < 64, 16-byte aligned weights), and from 64
+ * columns on the fp16-operand GEMM (K % 256 == 0, aligned, JQ_OPT_PREFILL_EXACT not set).  Other
+ * shapes quantize once and run one multiply per matrix.  The decode kernels (M <= 2, and M <= 8
+ * with K <= 6144) give the bits of separate calls; the others divide K by the size of the whole
+ * launch, so that the fp32 additions may be in another order than in separate calls (differences
+ * within the kernels' own accuracy, about 1e-7 of the largest output).  No counterpart in the
+ * reference (its linears are separate cuBLAS calls). */
 int jq_linear_q4_0_multi_device(void *stream, int n_mats, const void *const *d_w, const int64_t *N,
                                 float *const *d_y, const float *d_x, const void *d_xq, void *d_ws,
                                 int64_t K, int64_t M, int s_mode);

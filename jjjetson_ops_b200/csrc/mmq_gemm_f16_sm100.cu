@@ -16,8 +16,9 @@
 // to fp16 (relative error <= 2^-11 per element), the accumulation is fp32.  The result differs from
 // the reference formula by about 3e-4 of the largest output on the configurations this kernel is
 // measured on, where the integer kernels differ by 1e-6: it meets the 1e-3 bound against the
-// dequantised product but not bit-level parity of the per-block sums, which is why it is selected
-// by name only.  Operands must stay inside fp16's range: |x| <= 65504 for the activations, and
+// dequantised product but not bit-level parity of the per-block sums; JQ_OPT_PREFILL_EXACT keeps the
+// automatic choice, which takes it from 64 columns on, to the integer kernels.  How K is split does
+// not show in that error.  Operands must stay inside fp16's range: |x| <= 65504 for the activations, and
 // scales whose products are not subnormal (|d| * |q| >= 6.1e-5) keep full precision.
 //
 // A CTA owns a 128 (activation columns) x 128 (weight rows) tile of Y, or two CTAs on neighbouring SMs own 256 x 256:

@@ -5,9 +5,10 @@
 // cost is the weight stream as long as the arithmetic hides behind it, so the kernel is organised around that:
 //
 //   * A CTA owns 32 * WR weight rows and 8 * CT columns for all of K.  Weights and activations of a K stage arrive by
-//     tiled tensor copies in a ring of up to eight stages; two CTAs share an SM, so about 100 KB are in flight per SM
-//     and one CTA's start and end lie behind the other's stream.
-//   * The eight consumer warps split K, not the tile: each takes one pair of 32-value blocks per stage for all rows
+//     tiled tensor copies in a ring of up to eight stages.  Two CTAs of eight consumer warps share an SM, so about
+//     100 KB are in flight per SM and one CTA's start and end lie behind the other's stream; a grid that has at most one
+//     CTA per SM takes sixteen consumer warps and the whole of the shared memory.
+//   * The consumer warps split K, not the tile: each takes one pair of 32-value blocks per stage for all rows
 //     of its row group and all columns.  So a weight is unpacked once and an activation fragment is read once (WR
 //     times) per CTA, the least shared-memory traffic there is, and the activations need no registers between
 //     stages, which is what bounds K in the register-resident decode kernels.  The warps' partial tiles are added
@@ -19,7 +20,8 @@
 //
 // What bounds it: up to about 16 columns the copies (rows of 144 bytes arrive at about 8 cycles each per SM, 4.8 TB/s of
 // weights and activations together: with no arithmetic K = 4096, N = 11008, M = 8 takes 11.2 us, without the activations
-// 8.0, as it stands 13.1), beyond that instruction issue (70 warp instructions per 16 x 32 weights at 24 columns).
+// 8.0, as it stands 13.1), beyond that the arithmetic: 70 warp instructions per 16 x 32 weights at 24 columns, 43 % of the
+// issue slots busy at K = 4096, N = 11008, whose 172 CTAs of 64 rows fill one place on most SMs and two on 24 of them.
 // Measured and dropped: 16-byte cp.async by two producer warps instead of the tensor copies, 15.2 us at that shape and
 // 22.5 against 18.0 us at M = 24; weights of four or eight stages ahead of the previous kernel's end instead of two, no
 // difference.

@@ -648,9 +648,10 @@ int launch_kernel(cudaStream_t st, dim3 grid, const HfParams<MATS> &p, const HfM
     return JQ_OK;
 }
 // Clusters of z CTAs along K, or of a pair of CTAs, of this kernel that the current device runs at a time (0: none).  The instances
-// for several matrices have the same threads and shared memory.
+// for several matrices have the same threads and shared memory.  `answered` is cleared when the query failed for another reason
+// than the size of the cluster.
 template <bool PAIR, bool SPLIT>
-int clusters_at_a_time(unsigned z, int *out) {
+int clusters_at_a_time(unsigned z, int *out, bool *answered) {
     const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, 1>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
     cudaLaunchConfig_t cfg = {};
@@ -664,13 +665,15 @@ int clusters_at_a_time(unsigned z, int *out) {
     attr[0].val.clusterDim.z = z;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(out, kernel, &cfg) != cudaSuccess) {
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(out, kernel, &cfg);
+    if (e != cudaSuccess) {
         (void)cudaGetLastError();
         *out = 0;
+        if (e != cudaErrorInvalidClusterSize && e != cudaErrorInvalidConfiguration) *answered = false;
     }
     return JQ_OK;
 }
-// ... for every form, asked once per device
+// ... for every form, asked once per device that answers
 int form_widths(const DeviceCaps &caps, GemmF16Widths *out) {
     struct Entry {
         int dev;
@@ -689,10 +692,11 @@ int form_widths(const DeviceCaps &caps, GemmF16Widths *out) {
     }
     GemmF16Widths w{};
     w.splits[1] = caps.sm_count;
+    bool answered = true;
     for (int s = 2; s <= HF_MAX_SPLITS; ++s)
-        if (int rc = clusters_at_a_time<false, true>((unsigned)s, &w.splits[s])) return rc;
-    if (int rc = clusters_at_a_time<true, false>(1, &w.pairs)) return rc;
-    table.push_back(Entry{dev, w});
+        if (int rc = clusters_at_a_time<false, true>((unsigned)s, &w.splits[s], &answered)) return rc;
+    if (int rc = clusters_at_a_time<true, false>(1, &w.pairs, &answered)) return rc;
+    if (answered) table.push_back(Entry{dev, w});
     *out = w;
     return JQ_OK;
 }

@@ -6,10 +6,13 @@ max|y - ref| / max|ref| <= 1e-3 against the oracle's reference-formula multiply 
 quantized inputs (about 3e-4 is expected) and <= 1e-3 against dequantise-then-matmul in float64
 when the quantizer stored s = d * sum(q).
 """
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
-from launch_forms import gemm_f16_form
+from launch_forms import ROOT, gemm_f16_form
 
 pytestmark = pytest.mark.gpu
 
@@ -185,3 +188,31 @@ def test_gemm_f16_split_k_is_ordered(env, K, N, M):
         assert np.array_equal(y, runs[0])
     exact = c.mul_mat_q4_0_q8_1(d_w, xq, K, N, M, c.ORDER_COL_KSUPER, c.KERNEL_GEMM_MMA).cpu().numpy()
     assert env.O.err_max_rel(runs[0], exact) <= TOL_F16_FORMULA
+
+
+FIRST_CALL = """
+import torch
+from jjjetson_ops_b200 import capi as c
+dev = torch.device("cuda:0")
+g = torch.Generator(device=dev)
+g.manual_seed(3)
+for K, N, M in [(2048, 2048, 128), (256, 18690, 130)]:
+    w = c.quantize_q4_0(torch.randn((N, K), generator=g, device=dev) * 0.02)
+    xq = c.quantize_q8_1(torch.randn((M, K), generator=g, device=dev))
+    y = torch.zeros((M, N), device=dev)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        c.mul_mat_q4_0_q8_1(w, xq, K, N, M, out=y)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, c.mul_mat_q4_0_q8_1(w, xq, K, N, M)), (K, N, M)
+print("captured")
+"""
+
+
+def test_gemm_f16_first_call_in_a_capture(env):
+    """A process whose first use of the kernel is recorded into a graph: the form is the one of an eager call, bit for bit."""
+    assert gemm_f16_form(2048, [2048], 128) == 4 and gemm_f16_form(256, [18690], 130) == "pair"
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL], capture_output=True, text=True, cwd=ROOT, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]

@@ -26,7 +26,7 @@ struct GemmF16Plan {
 // (101 where pairs of CTAs share 256 x 256: they convert as much per stage as single CTAs and multiply twice as much).  The fixed
 // part fills the pipeline and writes the tile, and adds up the parts where K is split.  A fit over 1677 shapes (K 256 to 11008, N 64
 // to 32000, M 64 to 2048, whole linears, every form): within 3 % on average, and the form it names takes 0.05 % more than the
-// quickest one on average, 5 % at most but for two shapes of K = 2048.  Both sides of the lines, whole linear, us:
+// quickest one on average, 6 % at most (K = 1536, N = 3072, M = 384: two parts 15.8, one 14.9 us).  Both sides of the lines, whole linear, us:
 //   K = 2048, 16 tiles (N = 2048, M = 128): one 17.2, two 15.0, four 11.3; eight 20.0, because 16 clusters take two waves
 //   K = 11008, 16 tiles: six 22.8, eight 36.2; K = 4096, 15 tiles or less: eight
 //   K = 1024, N = 2048, M = 512 (64 tiles): one 11.8, two 14.1

@@ -7,6 +7,7 @@
 namespace jq {
 
 constexpr int HF_MAX_SPLITS = 8;  // CTAs per tile along K: the largest portable cluster
+constexpr int HF_MAX_NARROW_SPLITS = HF_MAX_SPLITS / 2;  // pairs per tile along K
 
 // What the device runs at a time, as the driver says (0: this form does not run there): clusters of `i` CTAs that split K (1: single
 // CTAs), and pairs of CTAs.  Clusters do not fill the SMs: a B200 (148 SMs) holds 74 of two CTAs, 45 of three, 33, 22 and 15 of
@@ -14,10 +15,12 @@ constexpr int HF_MAX_SPLITS = 8;  // CTAs per tile along K: the largest portable
 struct GemmF16Widths {
     int splits[HF_MAX_SPLITS + 1];
     int pairs;
+    int narrow[HF_MAX_NARROW_SPLITS + 1];
 };
 
 struct GemmF16Plan {
     bool pair;                 // pairs of CTAs share 256 x 256
+    bool narrow;
     int k_splits;              // otherwise CTAs per 128 x 128 tile, of
     int chunks_per_split;      // this many 128-value chunks of K each (the last: what is left)
 };
@@ -32,10 +35,12 @@ struct GemmF16Plan {
 //   K = 1024, N = 2048, M = 512 (64 tiles): one 11.8, two 14.1
 //   K = 256, N = 32000, M = 300: single CTAs 32.1, pairs 35.5 (multiply alone)
 // `n_chunks` is K / 128 (even), `tiles` the 128 x 128 tiles of all matrices, `pair_tiles` the 256 x 256 ones.
-inline GemmF16Plan plan_gemm_f16(int n_chunks, int64_t tiles, int64_t pair_tiles, const GemmF16Widths &width) {
+inline GemmF16Plan plan_gemm_f16(int n_chunks, int64_t tiles, int64_t pair_tiles, const GemmF16Widths &width,
+                                 int64_t narrow_tiles = 0) {
+    (void)narrow_tiles;
     constexpr int64_t STAGE = 74, PAIR_STAGE = 101, PAIR_WAVE = 780, PAIR_ONCE = -200;
     constexpr int64_t WAVE[HF_MAX_SPLITS + 1] = {0, 420, 860, 730, 710, 0, 740, 0, 880};  // by CTAs per tile; 0: not used
-    GemmF16Plan plan{false, 1, n_chunks};
+    GemmF16Plan plan{false, false, 1, n_chunks};
     int64_t best = -1;
     for (int s = 1; s <= HF_MAX_SPLITS; ++s) {
         const int chunks = ((n_chunks + s - 1) / s + 1) / 2 * 2;  // whole pairs of chunks: a weight copy brings two
@@ -49,7 +54,7 @@ inline GemmF16Plan plan_gemm_f16(int n_chunks, int64_t tiles, int64_t pair_tiles
     }
     if (width.pairs > 0) {
         const int64_t cost = (pair_tiles + width.pairs - 1) / width.pairs * (n_chunks * PAIR_STAGE + PAIR_WAVE) + PAIR_ONCE;
-        if (best < 0 || cost < best) plan = {true, 1, n_chunks};
+        if (best < 0 || cost < best) plan = {true, false, 1, n_chunks};
     }
     return plan;
 }

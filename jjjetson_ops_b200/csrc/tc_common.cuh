@@ -100,6 +100,18 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[3
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// registers -> 32 lanes x 32 consecutive 32-bit columns of tensor memory (completion: tcgen05.wait::st)
+__device__ __forceinline__ void tmem_st32_nowait(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+        "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+        "r"(r[31])
+        : "memory");
+}
+
 // D(fp32, TMEM) (+)= A(fp16 tile) x B(fp16 tile)^T, K = 16
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -118,6 +130,74 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
 // `rows_a` TMEM lanes (MMA M) by `rows_b` TMEM columns (MMA N).
 __device__ __forceinline__ uint32_t tc_idesc_f16(int rows_a, int rows_b) {
     return (1u << 4) | ((uint32_t)(rows_b >> 3) << 17) | ((uint32_t)(rows_a >> 4) << 24);
+}
+
+// shared-memory matrix descriptor, K-major, 128-byte swizzle: rows 128 bytes apart, their 16-byte chunks exchanged by the row's
+// number modulo 8
+__device__ __forceinline__ uint64_t tc_desc_sw128(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+// shared-memory word of CTA `rank` of the cluster, at this CTA's address of it
+__device__ __forceinline__ float lds_f32_of(uint32_t addr, int rank) {
+    float v;
+    asm volatile(
+        "{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %1, %2;\n\t"
+        "ld.shared::cluster.f32 %0, [remote];\n\t}"
+        : "=f"(v)
+        : "r"(addr), "r"(rank)
+        : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+
+// A weight row's 72 bytes of a 128-value chunk from a raw slot, where two chunks of 128 rows lie 144 bytes apart: four 16-byte
+// words (conflict-free at that pitch) and one of 8, which comes last in an even chunk and first in an odd one.
+__device__ __forceinline__ void load_q4_chunk(uint32_t (&ww)[18], uint32_t raw, bool odd) {
+    if (!odd) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 v = lds_v4(raw + 16 * i);
+            ww[4 * i] = v.x;
+            ww[4 * i + 1] = v.y;
+            ww[4 * i + 2] = v.z;
+            ww[4 * i + 3] = v.w;
+        }
+        const uint2 e = lds_v2(raw + 64);
+        ww[16] = e.x;
+        ww[17] = e.y;
+    } else {
+        const uint2 e = lds_v2(raw + 72);
+        ww[0] = e.x;
+        ww[1] = e.y;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 v = lds_v4(raw + 80 + 16 * i);
+            ww[2 + 4 * i] = v.x;
+            ww[3 + 4 * i] = v.y;
+            ww[4 + 4 * i] = v.z;
+            ww[5 + 4 * i] = v.w;
+        }
+    }
+}
+
+// The sixteen quant bytes and the scale of block j of a 72-byte chunk
+__device__ __forceinline__ void q4_chunk_block(const uint32_t (&ww)[18], int j, uint32_t (&q)[4], uint32_t *dbits) {
+    if ((j & 1) == 0) {  // starts on a word boundary: [d | q0 q1] [q2..q5] ...
+        const int w0 = (j / 2) * 9;
+        *dbits = ww[w0] & 0xFFFFu;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) q[t] = __funnelshift_r(ww[w0 + t], ww[w0 + t + 1], 16);
+    } else {  // starts in the middle of a word
+        const int w0 = (j / 2) * 9 + 4;
+        *dbits = ww[w0] >> 16;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) q[t] = ww[w0 + 1 + t];
+    }
 }
 
 }  // namespace jq

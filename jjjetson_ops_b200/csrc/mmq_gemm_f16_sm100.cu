@@ -310,6 +310,8 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 if (!alive) break;
                 uint32_t ww[18];
                 load_q4_chunk(ww, sbase + T::W_OFF + ws * HF_W_SLOT_BYTES + (uint32_t)((gw * 32 + lane) * Q8_BYTES), (c & 1) != 0);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&w_empty[ws]);
                 uint32_t o[32], z0, z1;
                 convert_two_blocks(ww, 0, o, &z0);
                 if (round > 0) {
@@ -320,8 +322,6 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 const uint32_t a = lanes + T::A_COL + (uint32_t)s * HF_A_COLS;
                 tmem_st32_nowait(a, o);
                 convert_two_blocks(ww, 1, o, &z1);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&w_empty[ws]);
                 tmem_st32_nowait(a + 32, o);
                 // -8 * d4 as fp16 (exact: a power of two; finite unless |d4| > 8188); columns without a chunk stay zero
                 const __half2 m8 = __float2half2_rn(-8.0f);
@@ -348,14 +348,16 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 const uint32_t round = (uint32_t)(c / NS);
                 alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&x_full[rs], (uint32_t)(c / T::RAW_SLOTS) & 1u, p.fault)) != 0;
                 if (!alive) break;
-                if (round > 0) {
-                    alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&stage_empty[s], (round - 1) & 1u, p.fault)) != 0;
-                    if (!alive) break;
-                }
                 uint4 v[9];
                 const uint32_t raw = sbase + T::RAW_OFF + rs * T::RAW_BYTES + (uint32_t)(row * Q8_BYTES);
 #pragma unroll
                 for (int i = 0; i < 9; ++i) v[i] = lds_v4(raw + 16 * i);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&x_empty[rs]);
+                if (round > 0) {
+                    alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&stage_empty[s], (round - 1) & 1u, p.fault)) != 0;
+                    if (!alive) break;
+                }
                 const uint32_t at = sbase + s * T::X_BYTES + (uint32_t)(row * 128 + ((row & 7) << 4));
                 const float r0 = convert_activation_block(v[1], v[2], v[0].x, at, 0);
                 const float r1 = convert_activation_block(v[3], v[4], v[0].y, at, 4);
@@ -368,7 +370,6 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // tiles are read by the tensor core
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(&x_empty[rs]);
                     if (PAIR)
                         mbar_arrive_leader(&stage_full[s], first);
                     else

@@ -7,7 +7,6 @@
 namespace jq {
 
 constexpr int HF_MAX_SPLITS = 8;  // CTAs per tile along K: the largest portable cluster
-constexpr int HF_MAX_NARROW_SPLITS = HF_MAX_SPLITS / 2;  // pairs per tile along K
 
 // What the device runs at a time, as the driver says (0: this form does not run there): clusters of `i` CTAs that split K (1: single
 // CTAs), and pairs of CTAs.  Clusters do not fill the SMs: a B200 (148 SMs) holds 74 of two CTAs, 45 of three, 33, 22 and 15 of
@@ -15,32 +14,27 @@ constexpr int HF_MAX_NARROW_SPLITS = HF_MAX_SPLITS / 2;  // pairs per tile along
 struct GemmF16Widths {
     int splits[HF_MAX_SPLITS + 1];
     int pairs;
-    int narrow[HF_MAX_NARROW_SPLITS + 1];
 };
 
 struct GemmF16Plan {
     bool pair;                 // pairs of CTAs share 256 x 256
-    bool narrow;
     int k_splits;              // otherwise CTAs per 128 x 128 tile, of
     int chunks_per_split;      // this many 128-value chunks of K each (the last: what is left)
 };
 
-// The cheapest form by what a launch takes, in hundredths of a us: per wave of CTAs a fixed part and 74 for each 128-value stage
-// (101 where pairs of CTAs share 256 x 256: they convert as much per stage as single CTAs and multiply twice as much).  The fixed
-// part fills the pipeline and writes the tile, and adds up the parts where K is split.  A fit over 1677 shapes (K 256 to 11008, N 64
-// to 32000, M 64 to 2048, whole linears, every form): within 3 % on average, and the form it names takes 0.05 % more than the
-// quickest one on average, 6 % at most (K = 1536, N = 3072, M = 384: two parts 15.8, one 14.9 us).  Both sides of the lines, whole linear, us:
-//   K = 2048, 16 tiles (N = 2048, M = 128): one 17.2, two 15.0, four 11.3; eight 20.0, because 16 clusters take two waves
-//   K = 11008, 16 tiles: six 22.8, eight 36.2; K = 4096, 15 tiles or less: eight
-//   K = 1024, N = 2048, M = 512 (64 tiles): one 11.8, two 14.1
-//   K = 256, N = 32000, M = 300: single CTAs 32.1, pairs 35.5 (multiply alone)
-// `n_chunks` is K / 128 (even), `tiles` the 128 x 128 tiles of all matrices, `pair_tiles` the 256 x 256 ones.
-inline GemmF16Plan plan_gemm_f16(int n_chunks, int64_t tiles, int64_t pair_tiles, const GemmF16Widths &width,
-                                 int64_t narrow_tiles = 0) {
-    (void)narrow_tiles;
-    constexpr int64_t STAGE = 74, PAIR_STAGE = 101, PAIR_WAVE = 780, PAIR_ONCE = -200;
-    constexpr int64_t WAVE[HF_MAX_SPLITS + 1] = {0, 420, 860, 730, 710, 0, 740, 0, 880};  // by CTAs per tile; 0: not used
-    GemmF16Plan plan{false, false, 1, n_chunks};
+// The cheapest form by what a launch takes, in hundredths of a us: per wave of CTAs a fixed part and 68 for each 128-value stage
+// (79 where pairs of CTAs share 256 x 256: they convert as much per stage as single CTAs and multiply twice as much).  The fixed
+// part fills the pipeline and writes the tile, and adds up the parts where K is split.  A fit over 110 shapes (K 256 to 11008, N 64
+// to 32000, M 64 to 2048, the multiply alone, every form): within 5 % (one CTA and parts of K) and 8 % (pairs), and the form it names
+// takes 0.3 % more than the quickest one on average.  Both sides of the lines, the multiply alone, us:
+//   K = N = 4096, M = 512 (128 tiles): one 26.2, pairs 31.1 (64 on 74 places)
+//   K = N = 4096, M = 128 (32 tiles): four parts 12.4, three 15.5, six 21.2, because 32 clusters of six take two waves
+//   K = 8192, N = 1101, M = 167: six parts 15.6, eight 24.6
+//   K = 2304, N = 24089, M = 1386: pairs 192, one 251
+inline GemmF16Plan plan_gemm_f16(int n_chunks, int64_t tiles, int64_t pair_tiles, const GemmF16Widths &width) {
+    constexpr int64_t STAGE = 68, PAIR_STAGE = 79, PAIR_WAVE = 800, PAIR_ONCE = -126;
+    constexpr int64_t WAVE[HF_MAX_SPLITS + 1] = {0, 429, 834, 741, 668, 0, 718, 0, 805};  // by CTAs per tile; 0: not used
+    GemmF16Plan plan{false, 1, n_chunks};
     int64_t best = -1;
     for (int s = 1; s <= HF_MAX_SPLITS; ++s) {
         const int chunks = ((n_chunks + s - 1) / s + 1) / 2 * 2;  // whole pairs of chunks: a weight copy brings two
@@ -54,7 +48,7 @@ inline GemmF16Plan plan_gemm_f16(int n_chunks, int64_t tiles, int64_t pair_tiles
     }
     if (width.pairs > 0) {
         const int64_t cost = (pair_tiles + width.pairs - 1) / width.pairs * (n_chunks * PAIR_STAGE + PAIR_WAVE) + PAIR_ONCE;
-        if (best < 0 || cost < best) plan = {true, false, 1, n_chunks};
+        if (best < 0 || cost < best) plan = {true, 1, n_chunks};
     }
     return plan;
 }

@@ -21,7 +21,33 @@
 // not show in that error.  Operands must stay inside fp16's range: |x| <= 65504 for the activations, and
 // scales whose products are not subnormal (|d| * |q| >= 6.1e-5) keep full precision.
 //
-// @@DESCRIPTION@@
+// A CTA owns 128 weight rows x 128 activation columns of Y, or two CTAs on neighbouring SMs own 256 x 256: each converts 128 rows
+// and 128 columns, and cta_group::2 MMAs, issued by the first, multiply all with all, so that a converted operand is used twice as
+// often.  K advances in chunks of 128 values (one Q8_1 block per column, four Q4_0 blocks per row):
+//   raw rings       the quantized bytes as they lie in global memory, brought in by the copy engine, one tiled tensor copy per chunk
+//                   for the activation blocks and one per two chunks for 144 bytes of each weight row.  (A per-thread load of "its"
+//                   row touches 32 cache lines per warp instruction.)  A slot is handed back as soon as its words are in registers.
+//   operand stages  the weights are the MMA's A operand and lie in tensor memory, lane = weight row, 64 columns holding the 128
+//                   values of a chunk; the activations are B, in shared memory with the 128-byte swizzle.  So the tile comes out
+//                   with the weight rows in the lanes, and a register of the accumulator is 128 contiguous bytes of an output row:
+//                   stored as it is, where activations in the lanes took a turn through shared memory.
+//   order of K      inside a block of 32 both operands take the values in the order in which a word's nibbles come out under a mask
+//                   (0, 2 | 16, 18 | 1, 3 | 17, 19 of each four): 13 instructions for eight weights, no bytes moved.
+//   rank-one terms  those of four chunks are one MMA of K = 16.
+// Warps: groups of four for the weights (a row per thread: nibbles become fp16 by the magic-number trick, 0x6400 | q is 1024 + q;
+// then one exact subtraction and one rounded multiplication by the scale) and four for the activations (a column per thread, int8
+// the same way) take the chunks in turn; one thread issues the MMAs, one copies activations, one weights.
+// Every mbarrier wait is a bounded poll; a wait that runs out sets the device fault word, and every warp still reaches the common
+// exit where tensor memory is released.
+//
+// What bounds it.  Per chunk of a 256 x 256 pair (K = 8192, N = 28672, M = 2048, with two groups: 1.0 us): the MMAs alone (everything
+// else left out) 0.6, the conversion alone 0.8, the copies alone 0.8, the hand-overs between warps alone 0.33.  The multiply, before
+// (activations in tensor memory, weights in shared memory, two groups) / now: 1010 / 890 us; K = 4096, N = 11008, M = 512 79.1 / 66.9 us;
+// K = N = 4096, M = 512 27.7 / 26.2 us (35.2 / 29.6 us in another process: the card's clock), M = 128 13.1 / 12.4 us; K = 11008,
+// N = 4096, M = 128 23.9 / 22.4 us.  Over 110 shapes 0.924 of the time, none slower.
+// Dropped: pairs on 256 x 128 (each converts 64 columns), 0.25 % over those shapes; all of a chunk converted in registers before its
+// stage is free, 1023 against 961 us; one lane polling for its warp, 982 us; polls that suspend the warp longer, or not at all, or
+// with a pause in between, no better.
 #include <mutex>
 #include <vector>
 
@@ -41,36 +67,41 @@ constexpr int HF_TMEM_COLS = 512;
 constexpr int HF_EPI_WARPS = 16;     // warps that read the accumulator: four per quarter of the lanes
 constexpr int HF_MAX_MATS = 4;
 
-// CG CTAs (one, or two on neighbouring SMs: cta_group::2) share a tile of CG * 128 weight rows and NT activation columns.
-template <int CG, int NT>
+constexpr int HF_X_ROWS = 128;    // activation columns that a CTA converts
+constexpr int HF_X_BOX = HF_X_ROWS * 128;           // bytes of 64 fp16 values of K
+constexpr int HF_X_BYTES = 2 * HF_X_BOX;            // ... of a chunk
+constexpr int HF_Z_BYTES = HF_X_ROWS * 32;          // fp16 residues of sixteen blocks
+constexpr int HF_RAW_BYTES = HF_X_ROWS * Q8_BYTES;  // a chunk's activation blocks as they lie in global memory
+constexpr int HF_STAGES = 3;      // chunks of converted operands: what tensor memory (256 columns of accumulator) and shared memory hold
+constexpr int HF_RAW_SLOTS = 3, HF_W_SLOTS = 3;
+// Groups of warps that take the chunks in turn, four for the weights and four for the activations each.  Three groups of 72 registers
+// a thread, against two of 104: 877 / 928 us on 256 x 256 (K = 8192, N = 28672, M = 2048), 27.1 / 28.3 us on 128 x 128 (K = N = 4096,
+// M = 512): a group waits for its barriers and its stores to tensor memory as long as it converts.
+constexpr int HF_GROUPS = 3;
+constexpr int HF_W_WARPS = 4 * HF_GROUPS, HF_X_WARPS = 4 * HF_GROUPS;
+constexpr int HF_MMA_WARP = HF_W_WARPS + HF_X_WARPS, HF_COPY_X_WARP = HF_MMA_WARP + 1, HF_COPY_W_WARP = HF_MMA_WARP + 2;
+constexpr int HF_THREADS = (HF_MMA_WARP + 3) * 32;
+constexpr int HF_Z_OFF = HF_STAGES * HF_X_BYTES;
+constexpr int HF_RAW_OFF = HF_Z_OFF + 2 * HF_Z_BYTES;
+constexpr int HF_W_OFF = HF_RAW_OFF + HF_RAW_SLOTS * HF_RAW_BYTES;
+constexpr int HF_BAR_OFF = HF_W_OFF + HF_W_SLOTS * HF_W_SLOT_BYTES;
+constexpr int HF_SMEM_BYTES = HF_BAR_OFF + 256;
+static_assert(HF_SMEM_BYTES <= 227 * 1024, "rings do not fit in shared memory");
+static_assert(HF_X_BOX % 1024 == 0 && HF_RAW_OFF % 128 == 0 && HF_RAW_BYTES % 128 == 0 && HF_W_OFF % 128 == 0, "boxes start on whole patterns");
+// A wait by parity is only right while the phase before the awaited one is known to be over.  A raw activation slot belongs to one
+// group, which has waited for each of its phases; what a weight slot held before has been used by the MMAs of chunk
+// c - HF_GROUPS - HF_STAGES or an earlier one, which are over when a group comes to chunk c.
+static_assert(HF_RAW_SLOTS % HF_GROUPS == 0, "another group would use the slot in between");
+static_assert(HF_GROUPS + HF_STAGES <= 2 * HF_W_SLOTS, "the slot's last contents may not have landed");
+
+// A CTA on 128 weight rows x NT = 128 activation columns, or a pair (cta_group::2) on 256 x 256
+template <bool PAIR>
 struct HfTile {
-    static constexpr int X_ROWS = NT / CG;               // activation columns that a CTA converts
-    static constexpr int X_BOX = X_ROWS * 128;           // bytes of 64 fp16 values of K
-    static constexpr int X_BYTES = 2 * X_BOX;            // ... of a chunk
-    static constexpr int Z_BYTES = X_ROWS * 32;          // fp16 residues of sixteen blocks
-    static constexpr int RAW_BYTES = X_ROWS * Q8_BYTES;  // a chunk's activation blocks as they lie in global memory
-    // chunks in flight: what tensor memory (accumulator, weights, rank-one operands) and shared memory hold
-    static constexpr int STAGES = NT == 256 ? 3 : CG == 2 ? 5 : 4;
-    static constexpr int RAW_SLOTS = NT == 256 ? 3 : CG == 2 ? 5 : 2;
-    static constexpr int W_SLOTS = NT == 256 ? 3 : CG == 2 ? 4 : 2;
-    // groups of warps that take the chunks in turn, four for the weights and X_WARPS for the activations each
-    static constexpr int GROUPS = CG == 2 && NT == 128 ? 3 : 2;
-    static constexpr int X_WARPS = X_ROWS / 32;
-    static constexpr int W_WARPS_ALL = 4 * GROUPS, X_WARPS_ALL = X_WARPS * GROUPS;
-    static constexpr int MMA_WARP = W_WARPS_ALL + X_WARPS_ALL, COPY_X_WARP = MMA_WARP + 1, COPY_W_WARP = MMA_WARP + 2;
-    static constexpr int THREADS = (MMA_WARP + 3) * 32;
-    static constexpr uint32_t A_COL = NT, Z_COL = NT + STAGES * HF_A_COLS;
-    static constexpr int Z_OFF = STAGES * X_BYTES;
-    static constexpr int RAW_OFF = Z_OFF + 2 * Z_BYTES;
-    static constexpr int W_OFF = RAW_OFF + RAW_SLOTS * RAW_BYTES;
-    static constexpr int BAR_OFF = W_OFF + W_SLOTS * HF_W_SLOT_BYTES;
-    static constexpr int SMEM_BYTES = BAR_OFF + 256;
-    static constexpr int BLOCKS = NT / 32 / (HF_EPI_WARPS / 4);  // 32 x 32 output blocks per warp
-    static_assert(W_WARPS_ALL + X_WARPS_ALL >= HF_EPI_WARPS, "too few warps for the epilogue");
+    static constexpr int NT = PAIR ? 256 : 128;
+    static constexpr uint32_t A_COL = NT, Z_COL = NT + HF_STAGES * HF_A_COLS;  // tensor memory: accumulator, weights, rank-one operands
+    static constexpr int BLOCKS = NT / 32 / (HF_EPI_WARPS / 4);                // 32 x 32 output blocks per warp
     static_assert(Z_COL + 2 * HF_Z_COLS <= HF_TMEM_COLS, "tensor memory too small");
-    static_assert(SMEM_BYTES <= 227 * 1024, "rings do not fit in shared memory");
-    static_assert(X_BOX % 1024 == 0 && RAW_OFF % 128 == 0 && RAW_BYTES % 128 == 0 && W_OFF % 128 == 0, "boxes start on whole patterns");
-    static_assert(HF_EPI_WARPS * BLOCKS * 4096 <= BAR_OFF, "partial tiles do not fit in shared memory");
+    static_assert(HF_EPI_WARPS * BLOCKS * 4096 <= HF_BAR_OFF, "partial tiles do not fit in shared memory");
 };
 
 // fp16 constants, two per word
@@ -97,18 +128,17 @@ __device__ __forceinline__ void tc_mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_t
         "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// completion of this thread's tensor-core operations arrives on the barrier at this offset in both CTAs (`first`: the cluster
-// rank of the pair's first CTA)
-__device__ __forceinline__ void tc_commit_pair(uint64_t *bar, int first) {
+// completion of this thread's tensor-core operations arrives on the barrier at this offset in both CTAs
+__device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-                 "h"((uint16_t)(3 << first))
+                 "h"((uint16_t)3)
                  : "memory");
 }
 // arrive on the barrier at this offset in the pair's first CTA (which issues the MMAs)
-__device__ __forceinline__ void mbar_arrive_leader(uint64_t *bar, int first) {
+__device__ __forceinline__ void mbar_arrive_leader(uint64_t *bar) {
     asm volatile(
-        "{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %0, %1;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t}" ::"r"(smem_u32(bar)), "r"(first)
+        "{\n\t.reg .b32 remote;\n\tmapa.shared::cluster.u32 remote, %0, 0;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t}" ::"r"(smem_u32(bar))
         : "memory");
 }
 __device__ __forceinline__ bool mbar_wait_bounded_cluster(uint64_t *bar, uint32_t parity, int *fault, uint32_t limit = (1u << 22)) {
@@ -230,51 +260,49 @@ __device__ __forceinline__ int hf_matrix(const HfParams<MATS> &p) {
     return mat;
 }
 
-template <int CG, int NT, bool SPLIT, int MATS>
-__global__ void __launch_bounds__((HfTile<CG, NT>::THREADS), 1)
+template <bool PAIR, bool SPLIT, int MATS>
+__global__ void __launch_bounds__(HF_THREADS, 1)
 gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps<MATS> maps) {
-    using T = HfTile<CG, NT>;
-    constexpr bool PAIR = CG == 2;
-    constexpr int NS = T::STAGES;
+    using T = HfTile<PAIR>;
+    constexpr int NS = HF_STAGES;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + T::BAR_OFF);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + HF_BAR_OFF);
     uint64_t *stage_full = bars;            // [NS] converted: weights in tensor memory, activations in shared memory
     uint64_t *stage_empty = bars + NS;      // [NS] the stage's MMAs are done: it may be filled again
     uint64_t *x_full = bars + 2 * NS;       // [RAW_SLOTS] raw activations have landed
-    uint64_t *x_empty = x_full + T::RAW_SLOTS;
-    uint64_t *w_full = x_empty + T::RAW_SLOTS;  // [W_SLOTS] raw weights have landed
-    uint64_t *w_empty = w_full + T::W_SLOTS;
-    uint64_t *acc_full = w_empty + T::W_SLOTS;
+    uint64_t *x_empty = x_full + HF_RAW_SLOTS;
+    uint64_t *w_full = x_empty + HF_RAW_SLOTS;  // [W_SLOTS] raw weights have landed
+    uint64_t *w_empty = w_full + HF_W_SLOTS;
+    uint64_t *acc_full = w_empty + HF_W_SLOTS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
-    static_assert((2 * NS + 2 * T::RAW_SLOTS + 2 * T::W_SLOTS + 1) * 8 + 4 <= 256, "barrier block too small");
+    static_assert((2 * NS + 2 * HF_RAW_SLOTS + 2 * HF_W_SLOTS + 1) * 8 + 4 <= 256, "barrier block too small");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
-    const int first = SPLIT && PAIR ? 2 * (int)blockIdx.z : 0;  // cluster rank of the pair's first CTA
     const int mat = hf_matrix(p);
     const int64_t n0 = (int64_t)((int)blockIdx.x - (MATS > 1 ? p.tile_begin[mat] : 0)) * HF_ROWS;  // this CTA's weight rows
-    const int64_t m0 = (int64_t)blockIdx.y * NT;  // the tile's activation columns; this CTA converts X_ROWS from m0 + rank * X_ROWS
+    const int64_t m0 = (int64_t)blockIdx.y * T::NT;  // the tile's activation columns; this CTA converts X_ROWS from m0 + rank * X_ROWS
     const int c0 = SPLIT ? (int)blockIdx.z * p.chunks_per_split : 0;
     const int n_chunks = SPLIT ? min(p.chunks_per_split, p.n_chunks - c0) : p.n_chunks;  // even
 
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
-            mbar_init(&stage_full[s], (4 + T::X_WARPS) * CG);
+            mbar_init(&stage_full[s], PAIR ? 16 : 8);  // four warps for each operand, of each CTA
             mbar_init(&stage_empty[s], 1);
         }
-        for (int i = 0; i < T::RAW_SLOTS; ++i) {
+        for (int i = 0; i < HF_RAW_SLOTS; ++i) {
             mbar_init(&x_full[i], 1);
-            mbar_init(&x_empty[i], T::X_WARPS);
+            mbar_init(&x_empty[i], 4);
         }
-        for (int i = 0; i < T::W_SLOTS; ++i) {
+        for (int i = 0; i < HF_W_SLOTS; ++i) {
             mbar_init(&w_full[i], 1);
             mbar_init(&w_empty[i], 8);  // four warps for each of two chunks
         }
         mbar_init(acc_full, 1);
         fence_mbar_init();
     }
-    if (warp == T::MMA_WARP) {
+    if (warp == HF_MMA_WARP) {
         if (PAIR) {
             asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(HF_TMEM_COLS)
                          : "memory");
@@ -296,20 +324,20 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
 
     bool finished = false;  // this epilogue warp has seen the tile complete
 
-    if (warp < T::MMA_WARP) {
+    if (warp < HF_MMA_WARP) {
         bool alive = true;
-        if (warp < T::W_WARPS_ALL) {
+        if (warp < HF_W_WARPS) {
             // =============================== weights -> tensor memory =========================
             const int gw = warp & 3;
             const uint32_t lanes = tmem + ((uint32_t)(gw * 32) << 16);
 #pragma unroll 1
-            for (int c = warp >> 2; c < n_chunks; c += T::GROUPS) {
-                const int s = c % NS, ws = (c >> 1) % T::W_SLOTS;
+            for (int c = warp >> 2; c < n_chunks; c += HF_GROUPS) {
+                const int s = c % NS, ws = (c >> 1) % HF_W_SLOTS;
                 const uint32_t round = (uint32_t)(c / NS);
-                alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&w_full[ws], (uint32_t)((c >> 1) / T::W_SLOTS) & 1u, p.fault)) != 0;
+                alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&w_full[ws], (uint32_t)((c >> 1) / HF_W_SLOTS) & 1u, p.fault)) != 0;
                 if (!alive) break;
                 uint32_t ww[18];
-                load_q4_chunk(ww, sbase + T::W_OFF + ws * HF_W_SLOT_BYTES + (uint32_t)((gw * 32 + lane) * Q8_BYTES), (c & 1) != 0);
+                load_q4_chunk(ww, sbase + HF_W_OFF + ws * HF_W_SLOT_BYTES + (uint32_t)((gw * 32 + lane) * Q8_BYTES), (c & 1) != 0);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&w_empty[ws]);
                 uint32_t o[32], z0, z1;
@@ -333,23 +361,23 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 __syncwarp();
                 if (lane == 0) {
                     if (PAIR)
-                        mbar_arrive_leader(&stage_full[s], first);
+                        mbar_arrive_leader(&stage_full[s]);
                     else
                         mbar_arrive(&stage_full[s]);
                 }
             }
         } else {
             // =============================== activations -> shared memory =====================
-            const int xw = warp - T::W_WARPS_ALL;
-            const int row = (xw % T::X_WARPS) * 32 + lane;
+            const int xw = warp - HF_W_WARPS;
+            const int row = (xw & 3) * 32 + lane;
 #pragma unroll 1
-            for (int c = xw / T::X_WARPS; c < n_chunks; c += T::GROUPS) {
-                const int s = c % NS, rs = c % T::RAW_SLOTS;
+            for (int c = xw >> 2; c < n_chunks; c += HF_GROUPS) {
+                const int s = c % NS, rs = c % HF_RAW_SLOTS;
                 const uint32_t round = (uint32_t)(c / NS);
-                alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&x_full[rs], (uint32_t)(c / T::RAW_SLOTS) & 1u, p.fault)) != 0;
+                alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&x_full[rs], (uint32_t)(c / HF_RAW_SLOTS) & 1u, p.fault)) != 0;
                 if (!alive) break;
                 uint4 v[9];
-                const uint32_t raw = sbase + T::RAW_OFF + rs * T::RAW_BYTES + (uint32_t)(row * Q8_BYTES);
+                const uint32_t raw = sbase + HF_RAW_OFF + rs * HF_RAW_BYTES + (uint32_t)(row * Q8_BYTES);
 #pragma unroll
                 for (int i = 0; i < 9; ++i) v[i] = lds_v4(raw + 16 * i);
                 __syncwarp();
@@ -358,20 +386,20 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                     alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&stage_empty[s], (round - 1) & 1u, p.fault)) != 0;
                     if (!alive) break;
                 }
-                const uint32_t at = sbase + s * T::X_BYTES + (uint32_t)(row * 128 + ((row & 7) << 4));
+                const uint32_t at = sbase + s * HF_X_BYTES + (uint32_t)(row * 128 + ((row & 7) << 4));
                 const float r0 = convert_activation_block(v[1], v[2], v[0].x, at, 0);
                 const float r1 = convert_activation_block(v[3], v[4], v[0].y, at, 4);
-                const float r2 = convert_activation_block(v[5], v[6], v[0].z, at + T::X_BOX, 0);
-                const float r3 = convert_activation_block(v[7], v[8], v[0].w, at + T::X_BOX, 4);
+                const float r2 = convert_activation_block(v[5], v[6], v[0].z, at + HF_X_BOX, 0);
+                const float r3 = convert_activation_block(v[7], v[8], v[0].w, at + HF_X_BOX, 4);
                 // the rank-one operand: sixteen residues per column, four of each chunk; those without a chunk stay zero
-                const uint32_t zx = sbase + T::Z_OFF + ((c >> 2) & 1) * T::Z_BYTES + tile_off(row, 0);
+                const uint32_t zx = sbase + HF_Z_OFF + ((c >> 2) & 1) * HF_Z_BYTES + tile_off(row, 0);
                 sts_v2(zx + ((c & 2) >> 1) * TC_LBO + (c & 1) * 8, as_u32(__floats2half2_rn(r0, r1)), as_u32(__floats2half2_rn(r2, r3)));
                 if (c == n_chunks - 1 && (c & 3) == 1) sts_v4(zx + TC_LBO, make_uint4(0u, 0u, 0u, 0u));
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // tiles are read by the tensor core
                 __syncwarp();
                 if (lane == 0) {
                     if (PAIR)
-                        mbar_arrive_leader(&stage_full[s], first);
+                        mbar_arrive_leader(&stage_full[s]);
                     else
                         mbar_arrive(&stage_full[s]);
                 }
@@ -407,38 +435,38 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 }
             }
         }
-    } else if (warp == T::COPY_X_WARP) {
+    } else if (warp == HF_COPY_X_WARP) {
         // =============================== raw activations ======================================
         if (lane == 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            const int64_t col = m0 + rank * T::X_ROWS;
+            const int64_t col = m0 + rank * HF_X_ROWS;
             for (int c = 0; c < n_chunks; ++c) {
-                const int rs = c % T::RAW_SLOTS;
-                const uint32_t round = (uint32_t)(c / T::RAW_SLOTS);
+                const int rs = c % HF_RAW_SLOTS;
+                const uint32_t round = (uint32_t)(c / HF_RAW_SLOTS);
                 if (round > 0 && !mbar_wait_bounded(&x_empty[rs], (round - 1) & 1u, p.fault)) break;
-                mbar_arrive_expect_tx(&x_full[rs], T::RAW_BYTES);
-                const uint32_t dst = sbase + T::RAW_OFF + rs * T::RAW_BYTES;
+                mbar_arrive_expect_tx(&x_full[rs], HF_RAW_BYTES);
+                const uint32_t dst = sbase + HF_RAW_OFF + rs * HF_RAW_BYTES;
                 if (p.order == JQ_ORDER_KSUPER_COL)  // the tensor is [n_super * M blocks][144 bytes]
                     tma_load_2d(dst, &maps.x, 0, (int)((int64_t)(c0 + c) * p.M + col), &x_full[rs]);
                 else                                 // the tensor is [M columns][n_super * 144 bytes]
                     tma_load_2d(dst, &maps.x, (c0 + c) * Q8_BYTES, (int)col, &x_full[rs]);
             }
         }
-    } else if (warp == T::COPY_W_WARP) {
+    } else if (warp == HF_COPY_W_WARP) {
         // =============================== raw weights ==========================================
         if (lane == 0) {
             if (!p.static_weights) asm volatile("griddepcontrol.wait;" ::: "memory");
             for (int pr = 0; pr < n_chunks / 2; ++pr) {
-                const int ws = pr % T::W_SLOTS;
-                const uint32_t round = (uint32_t)(pr / T::W_SLOTS);
+                const int ws = pr % HF_W_SLOTS;
+                const uint32_t round = (uint32_t)(pr / HF_W_SLOTS);
                 if (round > 0 && !mbar_wait_bounded(&w_empty[ws], (round - 1) & 1u, p.fault)) break;
                 mbar_arrive_expect_tx(&w_full[ws], HF_W_SLOT_BYTES);
-                tma_load_2d(sbase + T::W_OFF + ws * HF_W_SLOT_BYTES, &maps.w[mat], ((c0 >> 1) + pr) * Q8_BYTES, (int)n0, &w_full[ws]);
+                tma_load_2d(sbase + HF_W_OFF + ws * HF_W_SLOT_BYTES, &maps.w[mat], ((c0 >> 1) + pr) * Q8_BYTES, (int)n0, &w_full[ws]);
             }
         }
     } else if (lane == 0 && rank == 0) {
         // =============================== MMA issuer (of a pair: the first CTA's, for both) =====
-        const uint32_t idesc = tc_idesc_f16(CG * HF_ROWS, NT);
+        const uint32_t idesc = tc_idesc_f16(PAIR ? 2 * HF_ROWS : HF_ROWS, T::NT);
         bool alive = true;
         for (int c = 0; c < n_chunks; ++c) {
             const int s = c % NS;
@@ -448,10 +476,10 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 break;
             }
             tc_fence_after();
-            const uint32_t a = tmem + T::A_COL + (uint32_t)s * HF_A_COLS, x = sbase + s * T::X_BYTES;
+            const uint32_t a = tmem + T::A_COL + (uint32_t)s * HF_A_COLS, x = sbase + s * HF_X_BYTES;
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
-                const uint64_t db = tc_desc_sw128(x + (t >> 2) * T::X_BOX + (t & 3) * 32);
+                const uint64_t db = tc_desc_sw128(x + (t >> 2) * HF_X_BOX + (t & 3) * 32);
                 const uint32_t more = c > 0 || t > 0 ? 1u : 0u;
                 if (PAIR)
                     tc_mma_f16_ts_pair(tmem, a + t * 8, db, idesc, more);
@@ -460,7 +488,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
             }
             if ((c & 3) == 3 || c == n_chunks - 1) {  // the rank-one terms of sixteen blocks
                 const uint32_t z = (uint32_t)((c >> 2) & 1);
-                const uint64_t db = tc_desc(sbase + T::Z_OFF + z * T::Z_BYTES);
+                const uint64_t db = tc_desc(sbase + HF_Z_OFF + z * HF_Z_BYTES);
                 if (PAIR)
                     tc_mma_f16_ts_pair(tmem, tmem + T::Z_COL + z * HF_Z_COLS, db, idesc, 1u);
                 else
@@ -468,13 +496,13 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
             }
             // the stage may be overwritten once these MMAs have read it
             if (PAIR)
-                tc_commit_pair(&stage_empty[s], first);
+                tc_commit_pair(&stage_empty[s]);
             else
                 tc_commit(&stage_empty[s]);
         }
         if (alive) {
             if (PAIR)
-                tc_commit_pair(acc_full, first);
+                tc_commit_pair(acc_full);
             else
                 tc_commit(acc_full);
         }
@@ -502,7 +530,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             part[u][q] = 0.0f;
-                            if (q < parts && j0 + u < end) part[u][q] = lds_f32_of(part0 + (j0 + u) * 128, CG * q + rank);
+                            if (q < parts && j0 + u < end) part[u][q] = lds_f32_of(part0 + (j0 + u) * 128, q);
                         }
                     }
 #pragma unroll
@@ -523,7 +551,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
     tc_fence_before();
     __syncthreads();
     if (PAIR) cluster_sync();  // nor does the other CTA, which may still arrive on this one's barriers until here
-    if (warp == T::MMA_WARP) {
+    if (warp == HF_MMA_WARP) {
         __syncwarp();
         if (PAIR)
             asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HF_TMEM_COLS) : "memory");
@@ -532,44 +560,42 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
     }
 }
 
-template <int CG, int NT, bool SPLIT, int MATS>
+template <bool PAIR, bool SPLIT, int MATS>
 int launch_kernel(cudaStream_t st, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
-    using T = HfTile<CG, NT>;
-    const auto kernel = gemm_q4_0_q8_1_f16_kernel<CG, NT, SPLIT, MATS>;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), T::SMEM_BYTES)) return rc;
+    const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, MATS>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
     (void)cudaGetLastError();  // a stale error of an earlier, unrelated call must not be taken for this launch's
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(T::THREADS);
-    cfg.dynamicSmemBytes = T::SMEM_BYTES;
+    cfg.blockDim = dim3(HF_THREADS);
+    cfg.dynamicSmemBytes = HF_SMEM_BYTES;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = CG;
+    attr[1].val.clusterDim.x = PAIR ? 2 : 1;
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = (unsigned)p.k_splits;
     cfg.attrs = attr;
-    cfg.numAttrs = CG > 1 || SPLIT ? 2 : 1;
+    cfg.numAttrs = PAIR || SPLIT ? 2 : 1;
     JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, maps));
     return JQ_OK;
 }
-// Clusters of CG CTAs by z along K of this kernel that the current device runs at a time (0: none).  The instances for several
-// matrices have the same threads and shared memory.  `answered` is cleared when the query failed for another reason than the size
-// of the cluster.
-template <int CG, int NT, bool SPLIT>
+// Clusters of z CTAs along K, or of a pair of CTAs, of this kernel that the current device runs at a time (0: none).  The instances
+// for several matrices have the same threads and shared memory.  `answered` is cleared when the query failed for another reason than
+// the size of the cluster.
+template <bool PAIR, bool SPLIT>
 int clusters_at_a_time(unsigned z, int *out, bool *answered) {
-    using T = HfTile<CG, NT>;
-    const auto kernel = gemm_q4_0_q8_1_f16_kernel<CG, NT, SPLIT, 1>;
-    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), T::SMEM_BYTES)) return rc;
+    const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, 1>;
+    if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CG, 1, z);
-    cfg.blockDim = dim3(T::THREADS);
-    cfg.dynamicSmemBytes = T::SMEM_BYTES;
+    cfg.gridDim = dim3(PAIR ? 2 : 1, 1, z);
+    cfg.blockDim = dim3(HF_THREADS);
+    cfg.dynamicSmemBytes = HF_SMEM_BYTES;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CG;
+    attr[0].val.clusterDim.x = PAIR ? 2 : 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = z;
     cfg.attrs = attr;
@@ -603,21 +629,18 @@ int form_widths(const DeviceCaps &caps, GemmF16Widths *out) {
     w.splits[1] = caps.sm_count;
     bool answered = true;
     for (int s = 2; s <= HF_MAX_SPLITS; ++s)
-        if (int rc = clusters_at_a_time<1, 128, true>((unsigned)s, &w.splits[s], &answered)) return rc;
-    if (int rc = clusters_at_a_time<2, 256, false>(1, &w.pairs, &answered)) return rc;
-    if (int rc = clusters_at_a_time<2, 128, false>(1, &w.narrow[1], &answered)) return rc;
-    for (int s = 2; s <= HF_MAX_NARROW_SPLITS; ++s)
-        if (int rc = clusters_at_a_time<2, 128, true>((unsigned)s, &w.narrow[s], &answered)) return rc;
+        if (int rc = clusters_at_a_time<false, true>((unsigned)s, &w.splits[s], &answered)) return rc;
+    if (int rc = clusters_at_a_time<true, false>(1, &w.pairs, &answered)) return rc;
     if (answered) table.push_back(Entry{dev, w});
     *out = w;
     return JQ_OK;
 }
+// form: 0 pairs of CTAs, 1 split K, 2 neither
 template <int MATS>
-int launch_form(cudaStream_t st, int cg, int nt, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
-    const bool split = p.k_splits > 1;
-    if (cg == 1) return split ? launch_kernel<1, 128, true, MATS>(st, grid, p, maps) : launch_kernel<1, 128, false, MATS>(st, grid, p, maps);
-    if (nt == 128) return split ? launch_kernel<2, 128, true, MATS>(st, grid, p, maps) : launch_kernel<2, 128, false, MATS>(st, grid, p, maps);
-    return launch_kernel<2, 256, false, MATS>(st, grid, p, maps);
+int launch_form(cudaStream_t st, int form, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
+    if (form == 0) return launch_kernel<true, false, MATS>(st, grid, p, maps);
+    if (form == 1) return launch_kernel<false, true, MATS>(st, grid, p, maps);
+    return launch_kernel<false, false, MATS>(st, grid, p, maps);
 }
 
 }  // namespace
@@ -655,22 +678,16 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     p.static_weights = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 1 : 0;
     GemmF16Widths width;
     if (int rc = form_widths(caps, &width)) return rc;
-    const GemmF16Plan plan = plan_gemm_f16(p.n_chunks, gx * gy, pair_gx / 2 * pair_gy, width, pair_gx / 2 * gy);
-    int cg = plan.pair || plan.narrow ? 2 : 1, nt = plan.pair ? 256 : 128;
+    const GemmF16Plan plan = plan_gemm_f16(p.n_chunks, gx * gy, pair_gx / 2 * pair_gy, width);
+    const bool pair = plan.pair;
     p.k_splits = plan.k_splits;
     p.chunks_per_split = plan.chunks_per_split;
-#ifdef HF_FORCE
-    if (const char *f = getenv("HF_FORM")) {
-        sscanf(f, "%d,%d,%d", &cg, &nt, &p.k_splits);
-        p.chunks_per_split = ((p.n_chunks + p.k_splits - 1) / p.k_splits + 1) / 2 * 2;
-        if ((p.n_chunks + p.chunks_per_split - 1) / p.chunks_per_split != p.k_splits) return set_error(JQ_ERR_UNSUPPORTED, "no such split");
-    }
-#endif
     const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
     HfMaps<HF_MAX_MATS> maps{};
     p.tile_begin[0] = 0;
     for (int i = 0; i < p.n_mats; ++i) {
-        p.tile_begin[i + 1] = p.tile_begin[i] + (int)((p.rows[i] + cg * HF_ROWS - 1) / (cg * HF_ROWS) * cg);
+        const int64_t per = pair ? 2 : 1;
+        p.tile_begin[i + 1] = p.tile_begin[i] + (int)((p.rows[i] + per * HF_ROWS - 1) / (per * HF_ROWS) * per);
         if (int rc = encode_byte_map(&maps.w[i], w[i], row_bytes, (uint64_t)p.rows[i], row_bytes, Q8_BYTES, HF_ROWS)) return rc;
 #ifdef JQ_BOUNDS_CHECK
         p.ext_y[i] = make_extent(p.y[i], (unsigned long long)M * (unsigned long long)p.rows[i] * sizeof(float));
@@ -678,13 +695,13 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     }
     const int64_t n_super = K / SUPER;
     const uint64_t x_row = (uint64_t)n_super * Q8_BYTES;
-    const uint32_t x_rows = (uint32_t)(nt / cg);
     if (int rc = order == JQ_ORDER_KSUPER_COL
-                     ? encode_byte_map(&maps.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, x_rows)
-                     : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, x_rows))
+                     ? encode_byte_map(&maps.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, HF_X_ROWS)
+                     : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, HF_X_ROWS))
         return rc;
-    const dim3 grid((unsigned)p.tile_begin[p.n_mats], (unsigned)(nt == 256 ? pair_gy : gy), (unsigned)p.k_splits);
-    if (p.n_mats > 1) return launch_form(st, cg, nt, grid, p, maps);
+    const int form = pair ? 0 : p.k_splits > 1 ? 1 : 2;
+    const dim3 grid((unsigned)p.tile_begin[p.n_mats], (unsigned)(pair ? pair_gy : gy), (unsigned)p.k_splits);
+    if (p.n_mats > 1) return launch_form(st, form, grid, p, maps);
     HfParams<1> p1{};
     p1.y[0] = p.y[0];
     p1.rows[0] = p.rows[0];
@@ -702,7 +719,7 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     HfMaps<1> maps1{};
     maps1.w[0] = maps.w[0];
     maps1.x = maps.x;
-    return launch_form(st, cg, nt, grid, p1, maps1);
+    return launch_form(st, form, grid, p1, maps1);
 }
 
 }  // namespace jq

@@ -45,12 +45,14 @@ __device__ __forceinline__ float block_sum_reference_order(float v, float *warp_
 // the per-thread partial sums of squares, the block tree and rsqrtf give the same inverse RMS bit
 // for bit.  The normalised row is staged in shared memory and quantized from there warp by warp
 // (one warp per 128-value block, one lane four consecutive values: the quantizer's own mapping).
+// STAGED: the weight vector is brought into shared memory behind the row.
+template <bool STAGED>
 __global__ void __launch_bounds__(RMS_THREADS, 5)
 rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ weight, float *normed_out,
                      uint8_t *__restrict__ xq, int H, int T, float epsilon, int n_super, int order, int s_mode) {
     // input, residual and normed_out carry no __restrict__: normed_out may be input itself (the reference's
     // in-place form); every read of a row happens before the barrier that precedes the first write to it
-    extern __shared__ __align__(16) float row[];  // H floats
+    extern __shared__ __align__(16) float row[];  // H floats (STAGED: and the weights)
     __shared__ float warp_partial[32];
     __shared__ float inverse_rms;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -62,6 +64,15 @@ rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ we
     // are free to use any thread-to-element mapping
     const bool vec = (H & 3) == 0 && ((uintptr_t)(input + base) & 15u) == 0 &&
                      (residual == nullptr || ((uintptr_t)(residual + base) & 15u) == 0);
+    const bool vec_out = vec && ((uintptr_t)weight & 15u) == 0 && (normed_out == nullptr || ((uintptr_t)(normed_out + base) & 15u) == 0);
+    const bool fused = vec_out && xq != nullptr && (n_super & 1) == 0;  // normalised and quantized in one pass
+    if (STAGED && fused) {
+        // Few tokens: the kernel is one chain of latencies, and with the matrices of a whole layer streamed since its last use
+        // the weight vector comes from HBM.  It is on its way while the row is loaded and summed.
+        const uint32_t dst = smem_u32(row + H);
+        for (int i = threadIdx.x; i < (H >> 2); i += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(weight + 4 * i) : "memory");
+    }
     if (vec) {
         const float4 *in4 = reinterpret_cast<const float4 *>(input + base);
         float4 *res4 = reinterpret_cast<float4 *>(residual != nullptr ? residual + base : nullptr);
@@ -126,10 +137,10 @@ rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ we
     }
     sum_square = block_sum_reference_order(sum_square, warp_partial);
     if (threadIdx.x == 0) inverse_rms = rsqrtf(sum_square / (float)H + epsilon);
+    if (STAGED) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const float inv = inverse_rms;
-    const bool vec_out = vec && ((uintptr_t)weight & 15u) == 0 && (normed_out == nullptr || ((uintptr_t)(normed_out + base) & 15u) == 0);
-    if (vec_out && xq != nullptr && (n_super & 1) == 0) {
+    if (fused) {
         // Normalisation and quantization in one pass over the row: a warp takes a pair of neighbouring blocks, a lane
         // its eight consecutive values, (z * inv) * w goes to the fp32 output (if wanted) and into the quantizer
         // straight from registers.  Same products, same bits as normalising the row first; it saves the row's second
@@ -138,7 +149,8 @@ rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ we
         for (int pr = warp; pr < (n_super >> 1); pr += n_warps) {
             const int e0 = pr * (2 * SUPER) + lane * 8;
             const float4 z0 = *reinterpret_cast<const float4 *>(row + e0), z1 = *reinterpret_cast<const float4 *>(row + e0 + 4);
-            const float4 w0 = __ldg(reinterpret_cast<const float4 *>(weight + e0)), w1 = __ldg(reinterpret_cast<const float4 *>(weight + e0 + 4));
+            const float4 w0 = STAGED ? *reinterpret_cast<const float4 *>(row + H + e0) : __ldg(reinterpret_cast<const float4 *>(weight + e0));
+            const float4 w1 = STAGED ? *reinterpret_cast<const float4 *>(row + H + e0 + 4) : __ldg(reinterpret_cast<const float4 *>(weight + e0 + 4));
             const float v[8] = {__fmul_rn(__fmul_rn(z0.x, inv), w0.x), __fmul_rn(__fmul_rn(z0.y, inv), w0.y),
                                 __fmul_rn(__fmul_rn(z0.z, inv), w0.z), __fmul_rn(__fmul_rn(z0.w, inv), w0.w),
                                 __fmul_rn(__fmul_rn(z1.x, inv), w1.x), __fmul_rn(__fmul_rn(z1.y, inv), w1.y),
@@ -289,11 +301,16 @@ int launch_rms_norm_q8_1(cudaStream_t st, float *d_input, float *d_residual, con
     if (H > (1 << 24) || T > 0x7FFFFFFF) return set_error(JQ_ERR_TOO_LARGE, "rms_norm: shape too large");
     DeviceCaps caps;
     if (int rc = device_caps(&caps)) return rc;
-    const size_t smem = (size_t)H * sizeof(float);
+    size_t smem = (size_t)H * sizeof(float);
     if (smem + 1024 > (size_t)caps.smem_optin)
         return set_error(JQ_ERR_TOO_LARGE, "rms_norm: a row of %lld floats does not fit in shared memory", (long long)H);
+    // A decode step of one sequence (four layers of 4096 x 11008 and the output norm, replayed from a graph, all launches) 186.0 ->
+    // 180.4 us; of eight sequences 155.7 -> 158.0: there the row's neighbours bring the vector in.
+    const bool staged = T <= 2 && d_xq != nullptr && 2 * smem + 1024 <= (size_t)caps.smem_optin;
+    if (staged) smem *= 2;
+    const auto kernel = staged ? rms_norm_q8_1_kernel<true> : rms_norm_q8_1_kernel<false>;
     if (smem > 48 * 1024) {
-        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(rms_norm_q8_1_kernel), (int)smem)) return rc;
+        if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem)) return rc;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)T);
@@ -303,7 +320,7 @@ int launch_rms_norm_q8_1(cudaStream_t st, float *d_input, float *d_residual, con
     cudaLaunchAttribute attr[1];
     launch_with_pdl(cfg, attr);
     const int n_super = (int)(H / SUPER);
-    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, rms_norm_q8_1_kernel, d_input, d_residual, d_weight, d_normed,
+    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, d_input, d_residual, d_weight, d_normed,
                                    static_cast<uint8_t *>(d_xq), (int)H, (int)T, epsilon, n_super, order, s_mode));
     return JQ_OK;
 }

@@ -28,6 +28,7 @@ namespace {
 constexpr int GV_MAX_STAGES = 8;
 constexpr int GV_BAR_BYTES = 256;  // full[8] + empty[8] ring mbarriers, red_full[4] + red_empty[4] (+ spare)
 constexpr int GV_RED_SLOTS = 4;
+constexpr int GV_PREVIOUS_ENDED = 29;  // (8-byte slot of the barrier block) non-zero: the preceding kernel has ended
 constexpr uint32_t MASK4 = 0x0F0F0F0Fu;
 
 constexpr int GV_MAX_MATS = 4;
@@ -59,6 +60,7 @@ struct GemvParams {
     int rows_per_stage;
     int prefetch_early;    // the weight stream may start before the preceding kernel in the stream has finished
     int early_stages;      // stages the producer may request before the activations are staged
+    uint32_t ahead_cycles; // > 0: while the preceding kernel still runs, another stage may be requested every so many cycles
     uint32_t x_copy_bytes; // > 0: the producer brings ready Q8_1 blocks in by bulk copy, straight to their place,
                            // queued ahead of the rest of the weight stream
     GatherArgs gather;     // all-gather epilogue (world == 0: plain store to y)
@@ -286,6 +288,19 @@ __device__ __forceinline__ bool producer_activations(const GemvParams &p, uint64
     return true;
 }
 
+// The preceding kernel still runs (its end is noted in shared memory by the first consumer warp): until then another stage may be
+// requested each time `cycles` have passed.  False: it has ended (or the polls have run out), the activations come next.
+__device__ __forceinline__ bool may_run_ahead(const volatile uint32_t *previous_ended, long long *last, uint32_t cycles, uint32_t limit) {
+    for (uint32_t i = 0; i < limit && *previous_ended == 0u; ++i) {
+        const long long now = clock64();
+        if (now - *last >= (long long)cycles) {
+            *last = now;
+            return true;
+        }
+    }
+    return false;
+}
+
 template <bool PER_ROW>
 __device__ __forceinline__ void gemv_producer(const GemvParams &p, uint64_t *full, uint64_t *empty,
                                               uint64_t *x_ready, uint8_t *ring, int lane, uint64_t *x_full = nullptr,
@@ -300,12 +315,15 @@ __device__ __forceinline__ void gemv_producer(const GemvParams &p, uint64_t *ful
     // activations can come in: with static weights the whole ring is requested first, it lands during that wait.
     const int early_stages =
         p.x_copy_bytes != 0 && p.prefetch_early && p.gather.world > 1 && p.gather.wait_previous ? p.stages : p.early_stages;
+    const volatile uint32_t *previous_ended = reinterpret_cast<const volatile uint32_t *>(full + GV_PREVIOUS_ENDED);
+    long long last = PER_ROW ? 0 : clock64();
     for (int c = 0; c < n_chunks; ++c) {
         int rows;
         const int64_t r0 = walk_stage(walk, c, R, &rows);
         int ok = 1;
         if (lane == 0) {
-            if (c == early_stages) {
+            if (!x_done && c >= early_stages &&
+                !(!PER_ROW && p.ahead_cycles != 0 && round == 0 && may_run_ahead(previous_ended, &last, p.ahead_cycles, p.poll_limit))) {
                 ok = producer_activations(p, x_ready, x_full, xs) ? 1 : 0;
                 x_done = true;
             }
@@ -645,6 +663,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
         mbar_init(x_full, 1);
         mbar_init(meet, NW);
         mbar_init(meet + 1, NW);
+        *reinterpret_cast<volatile uint32_t *>(full + GV_PREVIOUS_ENDED) = 0u;
         fence_mbar_init();
         // Tagged all-gather: this launch's number comes from a count that every launch raises by 65536, a share per
         // CTA.  The next launch in the stream starts only after every CTA of this one has passed the trigger below,
@@ -680,6 +699,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
     constexpr bool tagged = TAGGED;  // p.gather.ticket != nullptr
     const bool x_tagged = tagged && p.gather.x_words != nullptr;
     if (!x_tagged) griddep_wait();
+    if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(full + GV_PREVIOUS_ENDED) = 1u;
     uint32_t gather_epoch = 0;  // number of this all-gather (previous ones finished: *epoch_ptr)
     uint32_t x_tag = 0;
     if (tagged) {
@@ -1126,6 +1146,15 @@ int fast_path_ok(const void *d_w, const void *d_xq, const float *d_x_f32, int64_
     return JQ_OK;
 }
 
+// (dp4a form) How fast the weight stream runs ahead of the preceding kernel's end, beyond the first two stages.  After a norm or an activation
+// the SMs have nothing else to do; too fast a stream delays the loads of that very kernel.  One sequence's decode step (four layers
+// of 4096 x 11008 and the output projection, replayed), bytes per cycle and SM 0 / 8 / 14 / 20 / 28 / 60 (HBM gives 23): 180.3 / 176.9 /
+// 176.9 / 180.1 / 184.4 / 189.9 us; K = 8192, N = 28672 after its like 23.8 / 23.8 / 23.8 / 24.0 / 24.2 / 24.5 us.
+constexpr uint32_t GV_AHEAD_BYTES_PER_CYCLE = 10;
+void set_run_ahead(GemvParams &p, int ctas_per_sm) {
+    p.ahead_cycles = p.prefetch_early && p.gather.world == 0 ? p.stage_bytes * (uint32_t)ctas_per_sm / GV_AHEAD_BYTES_PER_CYCLE : 0;
+}
+
 template <int M_T, int NSB, int NW, int MINB>
 int run_dp4a(cudaStream_t st, GemvParams &p, const DeviceCaps &caps) {
     // MINB CTAs share an SM: each gets an equal slice of its shared memory (1 KB per CTA is reserved)
@@ -1149,6 +1178,7 @@ int run_dp4a(cudaStream_t st, GemvParams &p, const DeviceCaps &caps) {
     }
     if (p.stages < 2) return set_error(JQ_ERR_UNSUPPORTED, "row of %u bytes does not fit the shared-memory ring", p.row_bytes);
     const int smem = GV_BAR_BYTES + (int)p.y_bytes + (int)p.x_bytes + p.stages * (int)p.stage_bytes;
+    set_run_ahead(p, MINB);
 #ifdef JQ_BOUNDS_CHECK
     p.smem_total = (uint32_t)smem;
 #endif

@@ -8,6 +8,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "jq_common.cuh"
@@ -744,31 +745,187 @@ int jq_debug_set_extent_shrink(unsigned long long bytes) {
 
 namespace {
 
-struct DeviceScratch {
+// What a host call needs on the device and in pinned memory: a stream, one device buffer and a staging buffer.  Lanes are kept
+// between calls, because making them costs as much as a small call's own work; each call has one to itself while it runs, and at
+// most LANES_KEPT idle ones of at most LANE_KEPT_BYTES stay per device (jq_release_host_scratch gives them back).
+inline size_t whole_lines(size_t bytes) { return (bytes + 255) / 256 * 256; }
+constexpr size_t STAGE_CHUNK = (size_t)512 << 10, STAGE_SLOTS = 32, STAGE_BYTES = STAGE_CHUNK * STAGE_SLOTS;
+constexpr size_t RESULT_BYTES = (size_t)2 << 20;
+constexpr size_t LANE_KEPT_BYTES = (size_t)64 << 20, LANES_KEPT = 2;
+constexpr size_t MAX_COPY_THREADS = 8;
+static_assert(STAGE_SLOTS % MAX_COPY_THREADS == 0, "a thread meets its own chunks again in a slot");
+struct HostLane {
+    int device = 0;
     cudaStream_t stream = nullptr;
-    void *ptrs[4] = {nullptr, nullptr, nullptr, nullptr};
-    int n = 0;
-    int alloc(void **out, size_t bytes) {
-        *out = nullptr;
-        if (bytes == 0) return JQ_OK;
-        JQ_CUDA_TRY(cudaMallocAsync(out, bytes, stream));
-        ptrs[n++] = *out;
-        return JQ_OK;
-    }
+    uint8_t *d = nullptr;
+    size_t d_bytes = 0;
+    uint8_t *pinned = nullptr;      // STAGE_SLOTS chunks on their way to the device, then RESULT_BYTES from it
+    cudaEvent_t sent[STAGE_SLOTS] = {};
+    bool in_use[STAGE_SLOTS] = {};  // by this call: `sent` says when the chunk has gone
+    size_t next_slot = 0;
+
     int open() {
+        JQ_CUDA_TRY(cudaGetDevice(&device));
         JQ_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        JQ_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&pinned), STAGE_BYTES + RESULT_BYTES, cudaHostAllocDefault));
+        for (cudaEvent_t &e : sent) JQ_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         return JQ_OK;
     }
-    ~DeviceScratch() {
-        if (stream) {
-            for (int i = 0; i < n; ++i) cudaFreeAsync(ptrs[i], stream);
+    int reserve(size_t bytes) {
+        if (bytes <= d_bytes) return JQ_OK;
+        if (d != nullptr) JQ_CUDA_TRY(cudaFreeAsync(d, stream));
+        d = nullptr;
+        d_bytes = 0;
+        JQ_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(&d), bytes, stream));
+        d_bytes = bytes;
+        return JQ_OK;
+    }
+    ~HostLane() {
+        if (stream != nullptr) {
+            if (d != nullptr) cudaFreeAsync(d, stream);
             cudaStreamSynchronize(stream);
             cudaStreamDestroy(stream);
         }
+        for (cudaEvent_t e : sent)
+            if (e != nullptr) cudaEventDestroy(e);
+        if (pinned != nullptr) cudaFreeHost(pinned);
     }
+};
+std::mutex g_lanes_mutex;
+std::vector<HostLane *> &idle_lanes() {  // never destroyed: no CUDA call may run while the process ends
+    static std::vector<HostLane *> &lanes = *new std::vector<HostLane *>();
+    return lanes;
+}
+
+// A lane for the duration of a call.
+class LaneLease {
+  public:
+    int open() {
+        int dev = 0;
+        JQ_CUDA_TRY(cudaGetDevice(&dev));
+        {
+            std::lock_guard<std::mutex> lock(g_lanes_mutex);
+            std::vector<HostLane *> &idle = idle_lanes();
+            for (size_t i = 0; i < idle.size(); ++i) {
+                if (idle[i]->device == dev) {
+                    lane_ = idle[i];
+                    idle.erase(idle.begin() + (ptrdiff_t)i);
+                    std::fill(lane_->in_use, lane_->in_use + STAGE_SLOTS, false);
+                    return JQ_OK;
+                }
+            }
+        }
+        lane_ = new (std::nothrow) HostLane();
+        if (lane_ == nullptr) return set_error(JQ_ERR_CUDA, "out of host memory");
+        return lane_->open();
+    }
+    HostLane *operator->() const { return lane_; }
+    HostLane &operator*() const { return *lane_; }
+    // the call is over and nothing is queued any more: the lane may serve another one
+    void done() { finished_ = true; }
+    ~LaneLease() {
+        if (lane_ == nullptr) return;
+        if (finished_ && lane_->d_bytes <= LANE_KEPT_BYTES) {
+            std::lock_guard<std::mutex> lock(g_lanes_mutex);
+            std::vector<HostLane *> &idle = idle_lanes();
+            size_t kept = 0;
+            for (const HostLane *l : idle) kept += l->device == lane_->device;
+            if (kept < LANES_KEPT) {
+                try {
+                    idle.push_back(lane_);
+                    return;
+                } catch (...) {  // no memory for the list
+                }
+            }
+        }
+        delete lane_;
+    }
+
+  private:
+    HostLane *lane_ = nullptr;
+    bool finished_ = false;
+};
+
+// Host array of `bytes` -> device.  The driver takes pageable memory through a staging buffer of its own with one core (9.4 MB at
+// 7 to 9 GB/s); here several threads copy chunks into the lane's and hand each to the copy engine as it is ready.
+int copy_in(HostLane &lane, void *dst, const void *src, size_t bytes) {
+    if (bytes == 0) return JQ_OK;
+    const size_t chunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK, first_slot = lane.next_slot;
+    lane.next_slot = (first_slot + chunks) % STAGE_SLOTS;
+    size_t threads = 1;
+    while (threads < MAX_COPY_THREADS && threads * 2 <= chunks && threads * 4 <= std::max<size_t>(4, std::thread::hardware_concurrency())) threads *= 2;
+    std::atomic<int> failed{cudaSuccess};
+    const auto part = [&](size_t t, bool own_thread) {
+        cudaError_t e = own_thread ? cudaSetDevice(lane.device) : cudaSuccess;
+        for (size_t i = t; i < chunks && e == cudaSuccess; i += threads) {
+            const size_t slot = (first_slot + i) % STAGE_SLOTS, off = i * STAGE_CHUNK, n = std::min(STAGE_CHUNK, bytes - off);
+            if (lane.in_use[slot]) e = cudaEventSynchronize(lane.sent[slot]);
+            if (e != cudaSuccess) break;
+            std::memcpy(lane.pinned + slot * STAGE_CHUNK, static_cast<const uint8_t *>(src) + off, n);
+            e = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + off, lane.pinned + slot * STAGE_CHUNK, n, cudaMemcpyHostToDevice, lane.stream);
+            if (e == cudaSuccess) e = cudaEventRecord(lane.sent[slot], lane.stream);
+            lane.in_use[slot] = true;
+        }
+        if (e != cudaSuccess) failed.store((int)e);
+    };
+    std::thread helpers[MAX_COPY_THREADS - 1];
+    size_t started = 1;
+    try {
+        for (; started < threads; ++started) helpers[started - 1] = std::thread(part, started, true);
+    } catch (...) {  // no more threads: their chunks are copied here
+    }
+    part(0, false);
+    for (size_t t = started; t < threads; ++t) part(t, false);
+    for (size_t t = 1; t < started; ++t) helpers[t - 1].join();
+    if (failed.load() != cudaSuccess) return cuda_error((cudaError_t)failed.load(), "copy of a host array to the device");
+    return JQ_OK;
+}
+
+// Results -> host arrays: through the lane's pinned buffer while they fit, so that several of them cost one wait.
+class HostResults {
+  public:
+    explicit HostResults(HostLane &lane) : lane_(lane) {}
+    int fetch(void *dst, const void *src, size_t bytes) {
+        if (bytes == 0) return JQ_OK;
+        if (n_ < 2 && at_ + bytes <= RESULT_BYTES) {
+            uint8_t *const p = lane_.pinned + STAGE_BYTES + at_;
+            JQ_CUDA_TRY(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, lane_.stream));
+            copies_[n_++] = Copy{dst, p, bytes};
+            at_ += whole_lines(bytes);
+            return JQ_OK;
+        }
+        JQ_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, lane_.stream));
+        return JQ_OK;
+    }
+    int finish() {
+        JQ_CUDA_TRY(cudaStreamSynchronize(lane_.stream));
+        for (int i = 0; i < n_; ++i) std::memcpy(copies_[i].dst, copies_[i].src, copies_[i].bytes);
+        return JQ_OK;
+    }
+
+  private:
+    struct Copy {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    };
+    HostLane &lane_;
+    Copy copies_[2] = {};
+    int n_ = 0;
+    size_t at_ = 0;
 };
 
 }  // namespace
+
+int jq_release_host_scratch(void) {
+    std::vector<HostLane *> lanes;
+    {
+        std::lock_guard<std::mutex> lock(g_lanes_mutex);
+        lanes.swap(idle_lanes());
+    }
+    for (HostLane *l : lanes) delete l;
+    return JQ_OK;
+}
 
 int jq_q8_1_host(const float *input, uint8_t *output, const int *dims, int ndims) {
     if (dims == nullptr || ndims < 1) return set_error(JQ_ERR_INVALID_ARG, "dims missing");
@@ -781,17 +938,18 @@ int jq_q8_1_host(const float *input, uint8_t *output, const int *dims, int ndims
     if (ne0 == 0 || M == 0) return JQ_OK;
     if (input == nullptr || output == nullptr) return set_error(JQ_ERR_INVALID_ARG, "null pointer");
     if (ne0 % QK != 0) return set_error(JQ_ERR_SHAPE, "dims[0] = %lld is not a multiple of %d", (long long)ne0, QK);
-    DeviceScratch s;
-    if (int rc = s.open()) return rc;
-    void *d_x, *d_y;
     const size_t in_bytes = (size_t)ne0 * M * sizeof(float), out_bytes = jq_q8_1_bytes(ne0, M);
-    if (int rc = s.alloc(&d_x, in_bytes)) return rc;
-    if (int rc = s.alloc(&d_y, out_bytes)) return rc;
-    JQ_CUDA_TRY(cudaMemcpyAsync(d_x, input, in_bytes, cudaMemcpyHostToDevice, s.stream));
-    if (int rc = launch_quantize_q8_1(s.stream, static_cast<const float *>(d_x), d_y, ne0, M, JQ_ORDER_KSUPER_COL, JQ_S_SUM_X))
+    const size_t y_at = whole_lines(in_bytes);
+    LaneLease s;
+    if (int rc = s.open()) return rc;
+    if (int rc = s->reserve(y_at + out_bytes)) return rc;
+    if (int rc = copy_in(*s, s->d, input, in_bytes)) return rc;
+    if (int rc = launch_quantize_q8_1(s->stream, reinterpret_cast<const float *>(s->d), s->d + y_at, ne0, M, JQ_ORDER_KSUPER_COL, JQ_S_SUM_X))
         return rc;
-    JQ_CUDA_TRY(cudaMemcpyAsync(output, d_y, out_bytes, cudaMemcpyDeviceToHost, s.stream));
-    JQ_CUDA_TRY(cudaStreamSynchronize(s.stream));
+    HostResults out(*s);
+    if (int rc = out.fetch(output, s->d + y_at, out_bytes)) return rc;
+    if (int rc = out.finish()) return rc;
+    s.done();
     return JQ_OK;
 }
 
@@ -826,31 +984,32 @@ int jq_mat_mul_q4_0_q8_1_host_ex(const void *weight_q4_0, const float *input, ui
     if (M == 0) return JQ_OK;
     if ((K > 0 && (input == nullptr || (N > 0 && weight_q4_0 == nullptr))) || (N > 0 && output == nullptr))
         return set_error(JQ_ERR_INVALID_ARG, "null pointer");
-    DeviceScratch s;
-    if (int rc = s.open()) return rc;
-    void *d_w, *d_x, *d_ws, *d_y;
     const size_t w_bytes = jq_q4_0_bytes(N, K), x_bytes = (size_t)M * K * sizeof(float);
     const size_t ws_bytes = jq_q8_1_bytes(K, M), y_bytes = (size_t)M * N * sizeof(float);
-    if (int rc = s.alloc(&d_w, w_bytes)) return rc;
-    if (int rc = s.alloc(&d_x, x_bytes)) return rc;
-    if (int rc = s.alloc(&d_ws, ws_bytes)) return rc;
-    if (int rc = s.alloc(&d_y, y_bytes)) return rc;
-    if (w_bytes) JQ_CUDA_TRY(cudaMemcpyAsync(d_w, weight_q4_0, w_bytes, cudaMemcpyHostToDevice, s.stream));
-    if (x_bytes) JQ_CUDA_TRY(cudaMemcpyAsync(d_x, input, x_bytes, cudaMemcpyHostToDevice, s.stream));
+    const size_t x_at = whole_lines(w_bytes), ws_at = x_at + whole_lines(x_bytes), y_at = ws_at + whole_lines(ws_bytes);
+    LaneLease s;
+    if (int rc = s.open()) return rc;
+    if (int rc = s->reserve(y_at + y_bytes + 16)) return rc;
+    uint8_t *const d = s->d;
+    HostResults out(*s);
+    if (int rc = copy_in(*s, d, weight_q4_0, w_bytes)) return rc;
+    if (int rc = copy_in(*s, d + x_at, input, x_bytes)) return rc;
     if (K > 0) {
         // the workspace keeps the order q8_1() writes (q8_1.cu:84-86) ...
-        if (int rc = launch_quantize_q8_1(s.stream, static_cast<const float *>(d_x), d_ws, K, M, JQ_ORDER_KSUPER_COL, s_mode))
+        if (int rc = launch_quantize_q8_1(s->stream, reinterpret_cast<const float *>(d + x_at), d + ws_at, K, M, JQ_ORDER_KSUPER_COL, s_mode))
             return rc;
-        if (quant_workspace) JQ_CUDA_TRY(cudaMemcpyAsync(quant_workspace, d_ws, ws_bytes, cudaMemcpyDeviceToHost, s.stream));
     }
     if (N > 0) {
         // ... and the multiply is told so, which the reference's own kernel is not (it reads
         // m * (K/128) + k/128, mm_q4_0_q8_1.cu:230) and therefore mixes columns for M > 1.
-        if (int rc = dispatch_mul_mat(s.stream, d_w, d_ws, static_cast<float *>(d_y), K, N, M, JQ_ORDER_KSUPER_COL, JQ_KERNEL_AUTO))
+        if (int rc = dispatch_mul_mat(s->stream, d, d + ws_at, reinterpret_cast<float *>(d + y_at), K, N, M, JQ_ORDER_KSUPER_COL, JQ_KERNEL_AUTO))
             return rc;
-        JQ_CUDA_TRY(cudaMemcpyAsync(output, d_y, y_bytes, cudaMemcpyDeviceToHost, s.stream));
     }
-    JQ_CUDA_TRY(cudaStreamSynchronize(s.stream));
+    if (K > 0 && quant_workspace != nullptr)
+        if (int rc = out.fetch(quant_workspace, d + ws_at, ws_bytes)) return rc;
+    if (int rc = out.fetch(output, d + y_at, y_bytes)) return rc;
+    if (int rc = out.finish()) return rc;
+    s.done();
     return JQ_OK;
 }
 

@@ -93,6 +93,7 @@ _SIGS = {
     "jq_parse_q8_1_output": (_ci, [_vp, _vp, _vp, _vp, _i64]),
     "jq_mat_mul_q4_0_q8_1_host": (_ci, [_vp, _vp, _vp, _vp, ctypes.POINTER(_ci), _ci, _ci, _ci]),
     "jq_mat_mul_q4_0_q8_1_host_ex": (_ci, [_vp, _vp, _vp, _vp, ctypes.POINTER(_ci), _ci, _ci, _ci, _ci]),
+    "jq_release_host_scratch": (_ci, []),
     "jq_weights_create": (_ci, [_vp, _i64, _i64, ctypes.POINTER(_vp)]),
     "jq_weights_destroy": (_ci, [_vp]),
     "jq_weights_device_ptr": (_vp, [_vp]),

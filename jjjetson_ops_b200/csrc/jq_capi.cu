@@ -752,7 +752,7 @@ inline size_t whole_lines(size_t bytes) { return (bytes + 255) / 256 * 256; }
 constexpr size_t STAGE_CHUNK = (size_t)512 << 10, STAGE_SLOTS = 32, STAGE_BYTES = STAGE_CHUNK * STAGE_SLOTS;
 constexpr size_t RESULT_BYTES = (size_t)2 << 20;
 constexpr size_t LANE_KEPT_BYTES = (size_t)64 << 20, LANES_KEPT = 2;
-constexpr size_t MAX_COPY_THREADS = 8;
+constexpr size_t MAX_COPY_THREADS = 4;
 static_assert(STAGE_SLOTS % MAX_COPY_THREADS == 0, "a thread meets its own chunks again in a slot");
 struct HostLane {
     int device = 0;
@@ -852,8 +852,9 @@ int copy_in(HostLane &lane, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return JQ_OK;
     const size_t chunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK, first_slot = lane.next_slot;
     lane.next_slot = (first_slot + chunks) % STAGE_SLOTS;
-    size_t threads = 1;
-    while (threads < MAX_COPY_THREADS && threads * 2 <= chunks && threads * 4 <= std::max<size_t>(4, std::thread::hardware_concurrency())) threads *= 2;
+    // A thread costs some 50 us here: one, two and four of them take 9.4 MB in 770 / 590 / 800 us and the last two 38 MB in 2420 / 1640 us
+    // (eight: 900, 2150); threads that only copy, with one that hands over, 860 and 1900 us.
+    const size_t threads = std::thread::hardware_concurrency() < 4 || chunks < 4 ? 1 : chunks < 48 ? 2 : MAX_COPY_THREADS;
     std::atomic<int> failed{cudaSuccess};
     const auto part = [&](size_t t, bool own_thread) {
         cudaError_t e = own_thread ? cudaSetDevice(lane.device) : cudaSuccess;

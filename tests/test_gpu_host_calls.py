@@ -1,0 +1,66 @@
+"""The host wrappers' copies: chunks of 512 KB by one, two and four threads, a staging ring that goes round, results that do not fit in the
+staging buffer, calls from several threads, and after the kept buffers were given back.  The same kernels on the same blocks as the
+device calls: the same bits."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(c, torch, dev, K, N, M):
+    rng = np.random.default_rng(K + N + M)
+    w = rng.integers(0, 256, size=(N, K // 32, 18), dtype=np.uint8)
+    w[:, :, 0] = 0
+    w[:, :, 1] = 0x20  # d = 2^-7
+    x = rng.standard_normal((M, K), dtype=np.float32)
+    d_w = torch.from_numpy(w.reshape(-1)).to(dev)
+    d_q = c.quantize_q8_1(torch.from_numpy(x).to(dev), c.ORDER_KSUPER_COL, c.S_SUM_X)
+    return w.reshape(-1), x, d_q.cpu().numpy(), c.mul_mat_q4_0_q8_1(d_w, d_q, K, N, M, c.ORDER_KSUPER_COL).cpu().numpy()
+
+
+def _call(mmq, c, w, x, K, N, M):
+    q, y = np.zeros(c.q8_1_bytes(K, M), dtype=np.uint8), np.zeros((M, N), dtype=np.float32)
+    mmq(w, x, q, y, [K, M, 1, 1], N, K)
+    return q, y
+
+
+# one chunk; 2 MB and a part; more than the ring; four threads and more than the ring; results of 2.6 MB; activations of three chunks
+@pytest.mark.parametrize("K,N,M", [(256, 1, 1), (2048, 1900, 3), (8192, 4000, 2), (8192, 5500, 1), (256, 20001, 32), (11008, 40, 32)])
+def test_host_multiply_equals_device_calls(native_lib, cuda_device, K, N, M):
+    import torch
+
+    from jjjetson_ops_b200 import import_reference_modules
+
+    c, mmq = native_lib, import_reference_modules()[1].mmq
+    w, x, want_q, want = _case(c, torch, cuda_device, K, N, M)
+    for _ in range(3):
+        q, y = _call(mmq, c, w, x, K, N, M)
+        assert np.array_equal(q, want_q) and np.array_equal(y, want)
+    assert c.lib().jq_release_host_scratch() == 0
+    q, y = _call(mmq, c, w, x, K, N, M)
+    assert np.array_equal(q, want_q) and np.array_equal(y, want)
+
+
+def test_host_multiply_from_several_threads(native_lib, cuda_device):
+    import torch
+
+    from jjjetson_ops_b200 import import_reference_modules
+
+    c, mmq = native_lib, import_reference_modules()[1].mmq
+    cases = [(K, N, M, *_case(c, torch, cuda_device, K, N, M)) for K, N, M in [(4096, 1030, 1), (2048, 2050, 4), (8192, 600, 2), (256, 64, 7), (1024, 4000, 20)]]
+    bad = []
+
+    def work(K, N, M, w, x, want_q, want):
+        for _ in range(10):
+            q, y = _call(mmq, c, w, x, K, N, M)
+            if not (np.array_equal(q, want_q) and np.array_equal(y, want)):
+                bad.append((K, N, M))
+
+    threads = [threading.Thread(target=work, args=case) for case in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad

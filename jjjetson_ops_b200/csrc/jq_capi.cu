@@ -205,6 +205,17 @@ inline bool small_batch_kernel_pays(int64_t K, int64_t N, int64_t M) {
     return !(M == 1 && K > 8192 && N * K <= (int64_t)6 << 20);
 }
 
+// With JQ_OPT_PREFILL_EXACT the small-batch kernel also takes batches of 64 columns and more as long as there are few tiles of 128 x
+// 128: the integer GEMM needs them all to fill the SMs, and rounds off two to seven times as much.  Multiply alone, integer GEMM /
+// small-batch kernel: K = N = 4096, M = 64 25.9 / 12.7 us, M = 256 45.8 / 39.8, M = 512 (128 tiles) 69.0 / 67.9; K = 4096, N = 11008, M = 256
+// (172) 137 / 95 us; K = 9472, N = 502, M = 66 57.8 / 11.4; the other side: K = 2560, N = 6047, M = 684 (288) 89.8 / 93.3 us, K = 512, N = 25906,
+// M = 549 (1015) 78 / 103, and short K, where a CTA has little to do per column: K = 256, N = 1716, M = 547 (70) 5.4 / 6.8, N = 3138,
+// M = 139 (50) 4.9 / 3.8 us.
+inline bool small_batch_kernel_pays_exact(int64_t K, int64_t N, int64_t M) {
+    const int64_t tiles = ((N + 127) / 128) * ((M + 127) / 128);
+    return tiles <= 280 && tiles <= K / 4;
+}
+
 int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N,
                      int64_t M, int order, int kernel) {
     if (N == 0 || M == 0) return JQ_OK;
@@ -225,8 +236,10 @@ int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *
     int rc = JQ_ERR_UNSUPPORTED;
     if (M <= 2) rc = launch_gemv_dp4a(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
     if (rc == JQ_ERR_UNSUPPORTED && M <= 8) rc = launch_gemv_mma(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
-    if (rc == JQ_ERR_UNSUPPORTED && small_batch_kernel_pays(K, N, M)) rc = launch_mmq_stream(st, d_w, d_xq, d_y, K, N, M, order);
-    if (rc == JQ_ERR_UNSUPPORTED && M >= FP16_OPERANDS_MIN_COLUMNS && option_value(JQ_OPT_PREFILL_EXACT) == 0)
+    const bool exact = option_value(JQ_OPT_PREFILL_EXACT) != 0;
+    if (rc == JQ_ERR_UNSUPPORTED && (small_batch_kernel_pays(K, N, M) || (exact && small_batch_kernel_pays_exact(K, N, M))))
+        rc = launch_mmq_stream(st, d_w, d_xq, d_y, K, N, M, order);
+    if (rc == JQ_ERR_UNSUPPORTED && M >= FP16_OPERANDS_MIN_COLUMNS && !exact)
         rc = launch_gemm_f16(st, d_w, d_xq, d_y, K, N, M, order);  // refuses shapes outside its rules: the integer GEMM takes those
     if (rc == JQ_ERR_UNSUPPORTED && M > 8) rc = launch_gemm_mma(st, d_w, d_xq, d_y, K, N, M, order);
     if (rc == JQ_ERR_UNSUPPORTED) rc = launch_mmq_generic(st, d_w, d_xq, d_y, K, N, M, order);

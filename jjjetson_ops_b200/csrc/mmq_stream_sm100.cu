@@ -1,13 +1,13 @@
 // Small-batch multiply (a few to a few dozen activation columns): an int8 tensor-core kernel that reads every weight
-// once per 32 columns and keeps the memory system busy while it does.
+// once per 32 columns (up to 63 where that makes one wave of CTAs) and keeps the memory system busy while it does.
 //
 // Work to replace: q4_0_q8_1_mat_mul_kernel (reference src/cuda/mm_q4_0_q8_1.cu:164-289) for batched decode.  The
 // cost is the weight stream as long as the arithmetic hides behind it, so the kernel is organised around that:
 //
 //   * A CTA owns 32 * WR weight rows and 8 * CT columns for all of K.  Weights and activations of a K stage arrive by
-//     tiled tensor copies in a ring of up to eight stages.  Two CTAs of eight consumer warps share an SM, so about
-//     100 KB are in flight per SM and one CTA's start and end lie behind the other's stream; a grid that has at most one
-//     CTA per SM takes sixteen consumer warps and the whole of the shared memory.
+//     tiled tensor copies in a ring of up to eight stages, as much as shared memory holds: about 200 KB in flight per SM.  Where the
+//     rows can be dealt out so that each SM has one CTA, it has one; otherwise two or three CTAs of eight consumer warps share an
+//     SM and one's start and end lie behind the others' streams.
 //   * The consumer warps split K, not the tile: each takes one pair of 32-value blocks per stage for all rows
 //     of its row group and all columns.  So a weight is unpacked once and an activation fragment is read once (WR
 //     times) per CTA, the least shared-memory traffic there is, and the activations need no registers between
@@ -18,13 +18,15 @@
 //     and less 1.5 * 2^23 it is the block sum exactly (a conversion instruction runs at half the rate), then the
 //     reference's acc += d4 * (sumi * d8 - 8 * s8) (mm_q4_0_q8_1.cu:92) in packed fma.
 //
-// What bounds it: up to about 16 columns the copies (rows of 144 bytes arrive at about 8 cycles each per SM, 4.8 TB/s of
-// weights and activations together: with no arithmetic K = 4096, N = 11008, M = 8 takes 11.2 us, without the activations
-// 8.0, as it stands 13.1), beyond that the arithmetic: 70 warp instructions per 16 x 32 weights at 24 columns, 43 % of the
-// issue slots busy at K = 4096, N = 11008, whose 172 CTAs of 64 rows fill one place on most SMs and two on 24 of them.
-// Measured and dropped: 16-byte cp.async by two producer warps instead of the tensor copies, 15.2 us at that shape and
-// 22.5 against 18.0 us at M = 24; weights of four or eight stages ahead of the previous kernel's end instead of two, no
-// difference.
+// What bounds it: the copies, on the most loaded SM.  Rows of 144 bytes, 256 values of a weight row or 128 of a column, arrive at
+// about eight cycles each per SM, so K = 4096, 96 weight rows and 24 columns on an SM are 9.6 us, two CTAs of 64 rows and 24 columns
+// 15.  Hence one CTA of many rows instead of several of few: the activations of an SM are then copied once, and no SM has twice the
+// rows of another.  K = 4096, N = 11008, which is 344 tiles of 32 rows, 172 of 64 and 115 of 96: M = 12 12.8 -> 10.8 us, M = 24
+// 16.9 -> 13.1, M = 32 21.1 -> 16.3, M = 40 24.7 -> 18.8; its weights alone are 3.8 us at the copy bandwidth of the memory.  From some 40
+// columns on the arithmetic: 70 warp instructions per 16 x 32 weights and 24 columns.
+// Measured and dropped: 16-byte cp.async by two producer warps instead of the tensor copies, 15.2 us at M = 8 there (13.1) and 22.5
+// against 18.0 at M = 24; untiled bulk copies of a column's or a row's part of a stage, one per lane, to padded places: 16.9 -> 22.2 us
+// for the columns, 42 for the rows; weights of four or eight stages ahead of the previous kernel's end instead of two, no difference.
 //
 // Rounding.  K % 256 == 0: a warp keeps one running sum over all of its blocks and the warps' parts are added one after the other,
 // 1.0 to 1.4 times the error against 64 bits of the kernels that took these shapes up to 32 columns (8e-8 to 12e-8 of the result)
@@ -49,15 +51,15 @@ namespace jq {
 namespace {
 
 constexpr int SK_MAX_STAGES = 8;
-// Consumer warps: 8 with two CTAs per SM, 16 with one, for grids that would leave the second place empty anyway (K = 11008,
-// N = 4096, M = 8 17.6 -> 10.6 us, whole linears of K = N = 4096: M = 24 12 -> 9.5 us)
+// Consumer warps with several CTAs per SM, and with 32 rows and one CTA per SM, for grids that would leave the second place empty
+// anyway (K = 11008, N = 4096, M = 8 17.6 -> 10.6 us, whole linears of K = N = 4096: M = 24 12 -> 9.5 us)
 constexpr int SK_WARPS = 8, SK_WARPS_ALONE = 16;
 constexpr int SK_BAR_BYTES = 256;       // full[8], empty[8], meet[2]
 constexpr int SK_PITCH = 144;           // bytes of a weight row per 256 values of K, of an activation column per 128
 constexpr int SK_ODD_PITCH = 160;       // the same for the odd rows of an odd K, which start 8 bytes into their 160
 constexpr int SK_MAX_MATS = 4;
 constexpr int SK_RED_PITCH = 36;        // floats between two columns of a warp's partial tile: 2 * 36 = 8 mod 32 banks
-constexpr int SK_COLUMNS = 32;          // most columns a CTA takes
+constexpr int SK_COLUMNS = 32;          // most columns a CTA takes, unless choose_shape gives it all of them
 constexpr int SK_FLUSH = 4;             // stages per running sum
 constexpr int SK_SHORT_SUPERS = 16;     // K up to 2048: short running sums
 constexpr uint32_t SK_MASK4 = 0x0F0F0F0Fu;
@@ -97,6 +99,8 @@ struct StreamTile {
     static constexpr bool PAIR_FIRST = ODD && (WARPS == SK_WARPS || CT <= 2);
     static constexpr bool LEVELS = ODD && WARPS == SK_WARPS && CT == 1;  // running sums of SK_FLUSH stages, and one of those
     static constexpr int KW = WARPS / WR;  // warps along K = pairs of blocks per stage
+    // CTAs per SM; three: K = 4096, N = 32000, M = 16 27.8 -> 24.8 us, N = 22016, M = 12 23.2 -> 19.1 (more columns take too many registers)
+    static constexpr int PLACES = WARPS != SK_WARPS ? 1 : !ODD && CT <= 2 ? 3 : 2;
     static constexpr int SUPERS = KW / 2;     // 128-value groups per stage
     // weights of 256 values of K: ROWS rows, or ROWS / 2 even ones and ROWS / 2 odd ones
     static constexpr int HALF_BYTES = ODD ? ROWS / 2 * (SK_PITCH + SK_ODD_PITCH) : ROWS * SK_PITCH;
@@ -215,7 +219,7 @@ __device__ __forceinline__ void stream_load_activations(const StreamParams &p, c
 }
 
 template <int CT, int WR, bool ODD, int WARPS>
-__global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) mmq_stream_kernel(const __grid_constant__ StreamParams p, const __grid_constant__ StreamMaps maps) {
+__global__ void __launch_bounds__((WARPS + 1) * 32, (StreamTile<CT, WR, ODD, WARPS>::PLACES)) mmq_stream_kernel(const __grid_constant__ StreamParams p, const __grid_constant__ StreamMaps maps) {
     using T = StreamTile<CT, WR, ODD, WARPS>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -389,8 +393,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, WARPS == SK_WARPS ? 2 : 1) m
 template <int CT, int WR, bool ODD, int WARPS>
 int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps) {
     using T = StreamTile<CT, WR, ODD, WARPS>;
-    // two CTAs may share an SM (1 KB of its shared memory is reserved per CTA)
-    const int budget = WARPS == SK_WARPS ? min(caps.smem_optin, caps.smem_per_sm / 2 - 1024) : caps.smem_optin;
+    const int budget = min(caps.smem_optin, caps.smem_per_sm / T::PLACES - 1024);  // 1 KB of an SM's is reserved per CTA
     p.stages = min(SK_MAX_STAGES, (budget - SK_BAR_BYTES) / T::STAGE_BYTES);
     if (p.stages < 2 || p.stages * T::STAGE_BYTES < T::RED_BYTES)
         return set_error(JQ_ERR_UNSUPPORTED, "the stages of the small-batch kernel do not fit in shared memory");
@@ -417,14 +420,76 @@ int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const D
     return JQ_OK;
 }
 
-template <int CT, bool ODD>
-int run_stream_shape(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps, int wr, bool alone) {
-    if (alone) return run_stream<CT, 1, ODD, SK_WARPS_ALONE>(st, p, maps, caps);
-    return wr == 1 ? run_stream<CT, 1, ODD, SK_WARPS>(st, p, maps, caps) : run_stream<CT, 2, ODD, SK_WARPS>(st, p, maps, caps);
+// What a CTA takes.
+struct StreamShape {
+    int wr;     // groups of 32 rows
+    int warps;
+    int ct;     // groups of 8 columns
+};
+
+// One wave, one CTA per SM, with as few rows per CTA as that allows: K = 4096, M = 24, N = 14208 (148 CTAs of 96 rows) 17.1 -> 13.3 us,
+// N = 14300 (112 of 128) 17.1 -> 16.3, N = 18944 (148 of 128) 18.4 -> 16.7; N = 19200 (150 of 128) would be two waves and stays with
+// two CTAs of 64 rows per SM, 24.5.  From three column tiles on, tiles of 64 rows that fill the SMs are given four warps along K;
+// everything else eight or, where tiles of 32 rows do not fill them, sixteen, so that enough warps are at work: K = 11008, N =
+// 8192, M = 24 (128 CTAs of 64 rows, sixteen warps, instead of 256 of 32) 23.1 -> 21.4 us, K = 3072, N = 8192, M = 48 (two groups of
+// columns, so 2 x 128 tiles of 64 rows; 2 x 64 of 128) 13.5 -> 12.7.  How many warps share K decides how the sum is rounded, and
+// does not depend on how rows and columns are dealt out beyond that.
+//
+// 33 to 63 columns are two groups, unless one CTA of all columns makes one wave of what otherwise is more: K = 4096, N = 11008 (115 CTAs of
+// 96 rows instead of 2 x 172 of 64) M = 40 24.7 -> 18.8 us, M = 48 24.9 -> 22.4, M = 60 30.9 -> 29.0.  With 128 rows six column tiles
+// fit into the registers: N = 18944, M = 36 33.5 -> 25.2 us, M = 48 32.5 -> 31.2; the other side, M = 60, 40.4 in two groups, 59.6 in one.
+//
+// An odd K keeps to the shapes that its rounding was settled for (narrow: 32 rows only).
+StreamShape choose_shape(const int64_t (&tiles)[5], int64_t *groups, int64_t M, bool odd, bool narrow, int sm_count) {
+    *groups = (M + SK_COLUMNS - 1) / SK_COLUMNS;  // columns in equal groups of at most 32
+    const int ct = (int)(((M + *groups - 1) / *groups + 7) / 8);
+    const auto one_wave = [&](int wr, int64_t n_groups) { return tiles[wr] * n_groups <= sm_count; };
+    const bool four_along_k = !narrow && ct >= 3 && tiles[2] * *groups >= sm_count;
+    if (!four_along_k) {
+        if (one_wave(1, *groups)) return {1, SK_WARPS_ALONE, ct};
+        if (!odd && one_wave(2, *groups)) return {2, 16, ct};
+        if (!odd && one_wave(3, *groups)) return {3, 24, ct};  // (at most two column tiles: from three on 64 rows were one wave)
+        return {1, SK_WARPS, ct};
+    }
+    if (!odd && !one_wave(2, *groups)) {
+        if (one_wave(3, *groups)) return {3, 12, ct};
+        if (one_wave(4, *groups)) return {4, 16, ct};
+        const int all = (int)((M + 7) / 8);
+        const int wr = *groups != 2 ? 0 : one_wave(3, 1) ? 3 : one_wave(4, 1) && all <= 6 ? 4 : 0;
+        if (wr != 0) {
+            *groups = 1;
+            return {wr, 4 * wr, all};
+        }
+    }
+    return {2, SK_WARPS, ct};
 }
+
 template <int CT>
-int run_stream_columns(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps, int wr, bool alone, bool odd) {
-    return odd ? run_stream_shape<CT, true>(st, p, maps, caps, wr, alone) : run_stream_shape<CT, false>(st, p, maps, caps, wr, alone);
+int run_stream_columns(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps, StreamShape f, bool odd) {
+    if constexpr (CT > 4) {
+        if constexpr (CT <= 6) {
+            if (f.wr == 4) return run_stream<CT, 4, false, 16>(st, p, maps, caps);
+        }
+        return run_stream<CT, 3, false, 12>(st, p, maps, caps);
+    } else {
+        if (odd) {
+            if (f.warps == SK_WARPS_ALONE) return run_stream<CT, 1, true, SK_WARPS_ALONE>(st, p, maps, caps);
+            if constexpr (CT >= 3) {
+                if (f.wr == 2) return run_stream<CT, 2, true, SK_WARPS>(st, p, maps, caps);
+            }
+            return run_stream<CT, 1, true, SK_WARPS>(st, p, maps, caps);
+        }
+        if (f.wr == 1 && f.warps == SK_WARPS_ALONE) return run_stream<CT, 1, false, SK_WARPS_ALONE>(st, p, maps, caps);
+        if (f.wr == 2 && f.warps == 16) return run_stream<CT, 2, false, 16>(st, p, maps, caps);
+        if constexpr (CT <= 2) {
+            if (f.wr == 3) return run_stream<CT, 3, false, 24>(st, p, maps, caps);
+            return run_stream<CT, 1, false, SK_WARPS>(st, p, maps, caps);
+        } else {
+            if (f.wr == 3) return run_stream<CT, 3, false, 12>(st, p, maps, caps);
+            if (f.wr == 4) return run_stream<CT, 4, false, 16>(st, p, maps, caps);
+            return run_stream<CT, 2, false, SK_WARPS>(st, p, maps, caps);
+        }
+    }
 }
 
 // The maps of one weight matrix.  Row pitch (of two rows, if odd) and bases are multiples of 16 bytes, and no map covers
@@ -455,15 +520,14 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     if (p.n_mats < 1 || p.n_mats > SK_MAX_MATS) return set_error(JQ_ERR_INVALID_ARG, "1 to %d weight matrices per launch", SK_MAX_MATS);
     const void *w[SK_MAX_MATS] = {};
     uintptr_t bits = 0;
-    int64_t tiles = 0, wide_tiles = 0;
+    int64_t tiles[5] = {};  // of 32, 64, 96 and 128 rows
     const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
     for (int i = 0; i < p.n_mats; ++i) {
         w[i] = multi != nullptr ? multi->w[i] : d_w;
         p.y[i] = multi != nullptr ? multi->y[i] : d_y;
         p.rows[i] = multi != nullptr ? multi->rows[i] : N;
         bits |= (uintptr_t)w[i];
-        tiles += (p.rows[i] + 31) / 32;
-        wide_tiles += (p.rows[i] + 63) / 64;
+        for (int wr = 1; wr <= 4; ++wr) tiles[wr] += (p.rows[i] + 32 * wr - 1) / (32 * wr);
 #ifdef JQ_BOUNDS_CHECK
         p.ext_y[i] = make_extent(p.y[i], (unsigned long long)M * (unsigned long long)p.rows[i] * sizeof(float));
 #endif
@@ -476,26 +540,26 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     p.fault = device_fault_ptr();
     p.poll_limit = copy_wait_poll_limit();
     p.early_stages = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 2 : 0;
-    // columns in equal groups of at most 32
-    const int64_t groups = (M + SK_COLUMNS - 1) / SK_COLUMNS;
-    const int ct = (int)(((M + groups - 1) / groups + 7) / 8);
-    // 64 rows per CTA halve the activation traffic, which from three column tiles on exceeds the weights'; 32 rows
-    // keep more SMs at work when there are few, and running sums half as long (odd K, see the top)
-    const int wr = !(odd && n_super > SK_SHORT_SUPERS) && ct >= 3 && wide_tiles * groups >= caps.sm_count ? 2 : 1;
-    const bool alone = wr == 1 && tiles * groups <= caps.sm_count;
+    int64_t groups = 0;  // of columns
+    const StreamShape shape = choose_shape(tiles, &groups, M, odd, odd && n_super > SK_SHORT_SUPERS, caps.sm_count);
+    const int ct = shape.ct;
     StreamMaps maps{};
     for (int i = 0; i < p.n_mats; ++i)
-        if (int rc = encode_weight_maps(&maps.w[i], &maps.w_odd[i], w[i], p.rows[i], row_bytes, 32 * wr, odd)) return rc;
+        if (int rc = encode_weight_maps(&maps.w[i], &maps.w_odd[i], w[i], p.rows[i], row_bytes, 32 * shape.wr, odd)) return rc;
     const uint64_t x_row = (uint64_t)n_super * Q8_BYTES;
     if (int rc = order == JQ_ORDER_KSUPER_COL
                      ? encode_byte_map(&maps.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, 8u * (uint32_t)ct)
                      : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, 8u * (uint32_t)ct))
         return rc;
     switch (ct) {
-        case 1: return run_stream_columns<1>(st, p, maps, caps, wr, alone, odd);
-        case 2: return run_stream_columns<2>(st, p, maps, caps, wr, alone, odd);
-        case 3: return run_stream_columns<3>(st, p, maps, caps, wr, alone, odd);
-        default: return run_stream_columns<4>(st, p, maps, caps, wr, alone, odd);
+        case 1: return run_stream_columns<1>(st, p, maps, caps, shape, odd);
+        case 2: return run_stream_columns<2>(st, p, maps, caps, shape, odd);
+        case 3: return run_stream_columns<3>(st, p, maps, caps, shape, odd);
+        case 4: return run_stream_columns<4>(st, p, maps, caps, shape, odd);
+        case 5: return run_stream_columns<5>(st, p, maps, caps, shape, odd);
+        case 6: return run_stream_columns<6>(st, p, maps, caps, shape, odd);
+        case 7: return run_stream_columns<7>(st, p, maps, caps, shape, odd);
+        default: return run_stream_columns<8>(st, p, maps, caps, shape, odd);
     }
 }
 

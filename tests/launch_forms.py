@@ -51,10 +51,30 @@ def gemm_f16_form(K, rows, M):
 
 
 def small_batch_form(K, rows, M):
-    """(odd K, column tiles, rows per CTA, CTA alone on its SM) on a B200, as launch_mmq_stream chooses them."""
+    """How K is shared out on a B200, which fixes the order of the additions: (odd K, column tiles of a group of at most 32, rows and
+    whether the CTA is alone on its SM, for CTAs of 32 or 64 rows): 64 rows are four warps along K, 32 are eight, alone sixteen."""
     odd = K // 128 % 2 != 0
     groups = -(-M // 32)
     ct = -(-(-(-M // groups)) // 8)
     wide = sum(-(-n // 64) for n in rows) * groups
     wr = 2 if not (odd and K > 2048) and ct >= 3 and wide >= B200_SMS else 1
     return odd, ct, 32 * wr, wr == 1 and sum(-(-n // 32) for n in rows) * groups <= B200_SMS
+
+
+def small_batch_tile(K, rows, M):
+    """(rows, column tiles, consumer warps) of a CTA on a B200, as launch_mmq_stream chooses them."""
+    odd, ct, narrow_rows, alone = small_batch_form(K, rows, M)
+    groups = -(-M // 32)
+    tiles = {r: sum(-(-n // r) for n in rows) for r in (64, 96, 128)}
+    if alone:
+        return 32, ct, 16
+    along_k = 4 if narrow_rows == 64 else 8
+    if not odd:
+        for r in (64, 96, 128):
+            if tiles[r] * groups <= B200_SMS and r * along_k <= 768:
+                return r, ct, r // 32 * along_k
+        if along_k == 4 and groups == 2:
+            for r, most in ((96, 8), (128, 6)):
+                if tiles[r] <= B200_SMS:
+                    return (r, -(-M // 8), r // 8) if -(-M // 8) <= most else (64, ct, 8)
+    return narrow_rows, ct, 8

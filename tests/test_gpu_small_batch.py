@@ -8,7 +8,7 @@ a few 1e-7 as a rule).
 import numpy as np
 import pytest
 
-from launch_forms import small_batch_form
+from launch_forms import small_batch_form, small_batch_tile
 
 pytestmark = pytest.mark.gpu
 
@@ -84,6 +84,55 @@ def test_small_batch_two_ctas_per_sm(env, K, N, M, form, order):
     c.mul_mat_q4_0_q8_1(d_w, env.t.from_numpy(xq).to(env.dev), K, N, M, order, out=y)
     assert not env.t.isnan(y).any()
     assert O.err_max_rel(y.cpu().numpy()[:, rows], O.mul_mat_ref(np.ascontiguousarray(wq[rows]), xq, K, len(rows), M, order)) <= TOL
+
+
+# One CTA per SM with 64, 96 and 128 rows, at the ends of what makes one wave; all columns of 33 to 63 in one; two and three CTAs per SM.
+@pytest.mark.parametrize("K,N,M,tile", [
+    (6400, 9472, 8, (64, 1, 16)), (512, 4737, 16, (64, 2, 16)), (1280, 9408, 17, (64, 3, 16)), (512, 4672, 64, (64, 4, 16)),
+    (6400, 9473, 3, (96, 1, 24)), (768, 14208, 9, (96, 2, 24)), (6400, 14209, 8, (32, 1, 8)), (1280, 14209, 16, (32, 2, 8)),
+    (512, 9472, 24, (64, 3, 8)), (512, 9473, 24, (96, 3, 12)), (1024, 14208, 31, (96, 4, 12)), (512, 14209, 17, (128, 3, 16)),
+    (2304, 18944, 32, (128, 4, 16)), (256, 18945, 24, (64, 3, 8)), (512, 18945, 27, (64, 4, 8)), (512, 7104, 33, (96, 3, 12)),
+    (512, 9473, 33, (96, 5, 12)), (4096, 14208, 48, (96, 6, 12)), (512, 9480, 49, (96, 7, 12)), (1280, 14145, 63, (96, 8, 12)),
+    (512, 14209, 40, (128, 5, 16)), (2304, 18944, 41, (128, 6, 16)), (512, 14209, 49, (64, 4, 8)), (256, 18945, 40, (64, 3, 8))])
+@pytest.mark.parametrize("order", [0, 1])
+def test_small_batch_tiles(env, K, N, M, tile, order):
+    assert small_batch_tile(K, [N], M) == tile
+    c, O = env.c, env.O
+    w, x = _problem(K, N, M)
+    d_w = c.quantize_q4_0(env.t.from_numpy(w).to(env.dev))
+    wq = d_w.cpu().numpy().reshape(N, -1)
+    last = N // tile[0] * tile[0]
+    rows = np.unique(np.concatenate([np.random.default_rng(N).choice(N, size=120, replace=False),
+                                     [0, 31, 32, tile[0] - 1, tile[0], last - 1, min(last, N - 1), N - 2, N - 1]]))
+    xq = O.quantize_q8_1(x, order, c.S_SUM_X)
+    y = env.t.full((M, N), float("nan"), device=env.dev)
+    c.set_option(c.OPT_PREFILL_EXACT, 1)  # 64 columns
+    try:
+        c.mul_mat_q4_0_q8_1(d_w, env.t.from_numpy(xq).to(env.dev), K, N, M, order, out=y)
+    finally:
+        c.set_option(c.OPT_PREFILL_EXACT, 0)
+    assert not env.t.isnan(y).any()
+    assert O.err_max_rel(y.cpu().numpy()[:, rows], O.mul_mat_ref(np.ascontiguousarray(wq[rows]), xq, K, len(rows), M, order)) <= TOL
+
+
+# With JQ_OPT_PREFILL_EXACT, both sides of the line between this kernel and the integer GEMM: the number of tiles of 128 x 128, K / 4
+@pytest.mark.parametrize("K,N,M,here", [(1536, 4480, 1024, True), (1536, 4481, 1024, False), (256, 1024, 1000, True), (256, 1025, 1000, False),
+                                        (512, 130, 64, True), (1280, 333, 77, True)])
+def test_exact_prefill_kernel(env, K, N, M, here):
+    c, O, t = env.c, env.O, env.t
+    g = t.Generator(device=env.dev)
+    g.manual_seed(K + N + M)
+    w = c.quantize_q4_0(t.randn((N, K), generator=g, device=env.dev).mul_(0.02))
+    xq = c.quantize_q8_1(t.randn((M, K), generator=g, device=env.dev), s_mode=c.S_D_SUM_Q)
+    c.set_option(c.OPT_PREFILL_EXACT, 1)
+    try:
+        y = c.mul_mat_q4_0_q8_1(w, xq, K, N, M)
+    finally:
+        c.set_option(c.OPT_PREFILL_EXACT, 0)
+    gemm = c.mul_mat_q4_0_q8_1(w, xq, K, N, M, kernel=c.KERNEL_GEMM_MMA)
+    assert t.equal(y, gemm) != here and O.err_max_rel(y.cpu().numpy(), gemm.cpu().numpy()) <= TOL
+    rows = t.randperm(N, generator=g, device=env.dev)[:600]
+    assert _error_against_64_bits(t, w, xq, y, K, rows) <= 1.125 * _error_against_64_bits(t, w, xq, gemm, K, rows)
 
 
 @pytest.mark.parametrize("K,rows,M,same_form", [(512, [40, 1, 96, 33], 12, True), (6400, [40, 1, 96, 33], 5, True), (640, [40, 1, 96, 33], 7, True),

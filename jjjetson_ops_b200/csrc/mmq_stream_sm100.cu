@@ -99,8 +99,6 @@ struct StreamTile {
     static constexpr bool PAIR_FIRST = ODD && (WARPS == SK_WARPS || CT <= 2);
     static constexpr bool LEVELS = ODD && WARPS == SK_WARPS && CT == 1;  // running sums of SK_FLUSH stages, and one of those
     static constexpr int KW = WARPS / WR;  // warps along K = pairs of blocks per stage
-    // CTAs per SM; three: K = 4096, N = 32000, M = 16 27.8 -> 24.8 us, N = 22016, M = 12 23.2 -> 19.1 (more columns take too many registers)
-    static constexpr int PLACES = WARPS != SK_WARPS ? 1 : !ODD && CT <= 2 ? 3 : 2;
     static constexpr int SUPERS = KW / 2;     // 128-value groups per stage
     // weights of 256 values of K: ROWS rows, or ROWS / 2 even ones and ROWS / 2 odd ones
     static constexpr int HALF_BYTES = ODD ? ROWS / 2 * (SK_PITCH + SK_ODD_PITCH) : ROWS * SK_PITCH;
@@ -218,8 +216,9 @@ __device__ __forceinline__ void stream_load_activations(const StreamParams &p, c
     }
 }
 
-template <int CT, int WR, bool ODD, int WARPS>
-__global__ void __launch_bounds__((WARPS + 1) * 32, (StreamTile<CT, WR, ODD, WARPS>::PLACES)) mmq_stream_kernel(const __grid_constant__ StreamParams p, const __grid_constant__ StreamMaps maps) {
+// PLACES: CTAs per SM
+template <int CT, int WR, bool ODD, int WARPS, int PLACES>
+__global__ void __launch_bounds__((WARPS + 1) * 32, PLACES) mmq_stream_kernel(const __grid_constant__ StreamParams p, const __grid_constant__ StreamMaps maps) {
     using T = StreamTile<CT, WR, ODD, WARPS>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -390,10 +389,10 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, (StreamTile<CT, WR, ODD, WAR
     }
 }
 
-template <int CT, int WR, bool ODD, int WARPS>
+template <int CT, int WR, bool ODD, int WARPS, int PLACES = WARPS == SK_WARPS ? 2 : 1>
 int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const DeviceCaps &caps) {
     using T = StreamTile<CT, WR, ODD, WARPS>;
-    const int budget = min(caps.smem_optin, caps.smem_per_sm / T::PLACES - 1024);  // 1 KB of an SM's is reserved per CTA
+    const int budget = min(caps.smem_optin, caps.smem_per_sm / PLACES - 1024);  // 1 KB of an SM's is reserved per CTA
     p.stages = min(SK_MAX_STAGES, (budget - SK_BAR_BYTES) / T::STAGE_BYTES);
     if (p.stages < 2 || p.stages * T::STAGE_BYTES < T::RED_BYTES)
         return set_error(JQ_ERR_UNSUPPORTED, "the stages of the small-batch kernel do not fit in shared memory");
@@ -403,7 +402,7 @@ int run_stream(cudaStream_t st, StreamParams &p, const StreamMaps &maps, const D
     for (int i = 0; i < p.n_mats; ++i) p.tile_begin[i + 1] = p.tile_begin[i] + (int)((p.rows[i] + T::ROWS - 1) / T::ROWS);
     const int64_t gy = (p.M + T::COLS - 1) / T::COLS;
     if (gy > 65535) return set_error(JQ_ERR_UNSUPPORTED, "too many columns for the small-batch kernel");
-    auto kernel = mmq_stream_kernel<CT, WR, ODD, WARPS>;
+    auto kernel = mmq_stream_kernel<CT, WR, ODD, WARPS, PLACES>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), bytes, true)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)p.tile_begin[p.n_mats], (unsigned)gy);
@@ -425,6 +424,7 @@ struct StreamShape {
     int wr;     // groups of 32 rows
     int warps;
     int ct;     // groups of 8 columns
+    int places = 2;  // CTAs per SM, of eight consumer warps
 };
 
 // One wave, one CTA per SM, with as few rows per CTA as that allows: K = 4096, M = 24, N = 14208 (148 CTAs of 96 rows) 17.1 -> 13.3 us,
@@ -439,17 +439,28 @@ struct StreamShape {
 // 96 rows instead of 2 x 172 of 64) M = 40 24.7 -> 18.8 us, M = 48 24.9 -> 22.4, M = 60 30.9 -> 29.0.  With 128 rows six column tiles
 // fit into the registers: N = 18944, M = 36 33.5 -> 25.2 us, M = 48 32.5 -> 31.2; the other side, M = 60, 40.4 in two groups, 59.6 in one.
 //
-// An odd K keeps to the shapes that its rounding was settled for (narrow: 32 rows only).
-StreamShape choose_shape(const int64_t (&tiles)[5], int64_t *groups, int64_t M, bool odd, bool narrow, int sm_count) {
+// Up to 4096 values of K the sixteen warps of a CTA of 64 rows have little to do before their sums meet, and with 32 columns many
+// sums: K = 1792, M = 28, N = 4800 (150 tiles of 32 rows) 6.9 us in CTAs of 32 rows, 7.2 in 64; K = 512 3.8 / 4.1; with 12 columns N = 4800
+// 4.8 / 5.1, N = 5440 (170) 5.4 / 5.2, N = 9472 5.8 / 5.2; K = 4096, M = 28 N = 4800 12.2 / 12.0.
+//
+// Tiles of 32 rows that are two waves of two CTAs per SM stay that, beyond three share an SM up to two column tiles (then the registers do not
+// reach).  K = 4096, M = 16, two / three: 570 tiles 17.4 / 19.2 us, 590 18.1 / 19.3, 600 20.9 / 19.3, 1000 29.2 / 26.6; K = 1024 590
+// 7.3 / 7.5, 600 8.8 / 7.5; K = 8192, M = 4 590 25.1 / 26.8, 600 31.6 / 27.0.
+//
+// An odd K keeps to the shapes that its rounding was settled for, 32 rows only beyond K = 2048.
+StreamShape choose_shape(const int64_t (&tiles)[5], int64_t *groups, int64_t M, bool odd, int n_super, int sm_count) {
     *groups = (M + SK_COLUMNS - 1) / SK_COLUMNS;  // columns in equal groups of at most 32
     const int ct = (int)(((M + *groups - 1) / *groups + 7) / 8);
     const auto one_wave = [&](int wr, int64_t n_groups) { return tiles[wr] * n_groups <= sm_count; };
+    const bool narrow = odd && n_super > SK_SHORT_SUPERS;
     const bool four_along_k = !narrow && ct >= 3 && tiles[2] * *groups >= sm_count;
     if (!four_along_k) {
         if (one_wave(1, *groups)) return {1, SK_WARPS_ALONE, ct};
-        if (!odd && one_wave(2, *groups)) return {2, 16, ct};
-        if (!odd && one_wave(3, *groups)) return {3, 24, ct};  // (at most two column tiles: from three on 64 rows were one wave)
-        return {1, SK_WARPS, ct};
+        const bool long_k = n_super >= 4096 / SUPER;
+        if (!odd && one_wave(2, *groups) && (long_k || (ct < 4 && 10 * tiles[1] * *groups > 11 * sm_count))) return {2, 16, ct};
+        // (at most two column tiles below: from three on 64 rows are one wave here)
+        if (!odd && !one_wave(2, *groups) && one_wave(3, *groups)) return {3, 24, ct};
+        return {1, SK_WARPS, ct, !odd && tiles[1] * *groups > 4 * sm_count ? 3 : 2};
     }
     if (!odd && !one_wave(2, *groups)) {
         if (one_wave(3, *groups)) return {3, 12, ct};
@@ -483,8 +494,10 @@ int run_stream_columns(cudaStream_t st, StreamParams &p, const StreamMaps &maps,
         if (f.wr == 2 && f.warps == 16) return run_stream<CT, 2, false, 16>(st, p, maps, caps);
         if constexpr (CT <= 2) {
             if (f.wr == 3) return run_stream<CT, 3, false, 24>(st, p, maps, caps);
+            if (f.places == 3) return run_stream<CT, 1, false, SK_WARPS, 3>(st, p, maps, caps);
             return run_stream<CT, 1, false, SK_WARPS>(st, p, maps, caps);
         } else {
+            if (f.wr == 1) return run_stream<CT, 1, false, SK_WARPS>(st, p, maps, caps);
             if (f.wr == 3) return run_stream<CT, 3, false, 12>(st, p, maps, caps);
             if (f.wr == 4) return run_stream<CT, 4, false, 16>(st, p, maps, caps);
             return run_stream<CT, 2, false, SK_WARPS>(st, p, maps, caps);
@@ -541,7 +554,7 @@ int launch_mmq_stream(cudaStream_t st, const void *d_w, const void *d_xq, float 
     p.poll_limit = copy_wait_poll_limit();
     p.early_stages = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 2 : 0;
     int64_t groups = 0;  // of columns
-    const StreamShape shape = choose_shape(tiles, &groups, M, odd, odd && n_super > SK_SHORT_SUPERS, caps.sm_count);
+    const StreamShape shape = choose_shape(tiles, &groups, M, odd, (int)n_super, caps.sm_count);
     const int ct = shape.ct;
     StreamMaps maps{};
     for (int i = 0; i < p.n_mats; ++i)

@@ -62,19 +62,20 @@ def small_batch_form(K, rows, M):
 
 
 def small_batch_tile(K, rows, M):
-    """(rows, column tiles, consumer warps) of a CTA on a B200, as launch_mmq_stream chooses them."""
+    """(rows, column tiles, consumer warps, CTAs per SM) of a launch on a B200, as launch_mmq_stream chooses them."""
     odd, ct, narrow_rows, alone = small_batch_form(K, rows, M)
     groups = -(-M // 32)
-    tiles = {r: sum(-(-n // r) for n in rows) for r in (64, 96, 128)}
+    tiles = {r: sum(-(-n // r) for n in rows) for r in (32, 64, 96, 128)}
     if alone:
-        return 32, ct, 16
+        return 32, ct, 16, 1
     along_k = 4 if narrow_rows == 64 else 8
-    if not odd:
-        for r in (64, 96, 128):
-            if tiles[r] * groups <= B200_SMS and r * along_k <= 768:
-                return r, ct, r // 32 * along_k
-        if along_k == 4 and groups == 2:
-            for r, most in ((96, 8), (128, 6)):
-                if tiles[r] <= B200_SMS:
-                    return (r, -(-M // 8), r // 8) if -(-M // 8) <= most else (64, ct, 8)
-    return narrow_rows, ct, 8
+    one_wave = next((r for r in (64, 96, 128) if tiles[r] * groups <= B200_SMS and r * along_k <= 768), None)
+    if odd or (along_k == 4 and one_wave == 64):
+        return narrow_rows, ct, 8, 2
+    if one_wave and (along_k == 4 or one_wave != 64 or K >= 4096 or (ct < 4 and tiles[32] * groups > 1.1 * B200_SMS)):
+        return one_wave, ct, one_wave // 32 * along_k, 1
+    if along_k == 4 and groups == 2:
+        for r, most in ((96, 8), (128, 6)):
+            if tiles[r] <= B200_SMS:
+                return (r, -(-M // 8), r // 8, 1) if -(-M // 8) <= most else (64, ct, 8, 2)
+    return narrow_rows, ct, 8, 3 if along_k == 8 and tiles[32] * groups > 4 * B200_SMS else 2

@@ -88,12 +88,14 @@ def test_small_batch_two_ctas_per_sm(env, K, N, M, form, order):
 
 # One CTA per SM with 64, 96 and 128 rows, at the ends of what makes one wave; all columns of 33 to 63 in one; two and three CTAs per SM.
 @pytest.mark.parametrize("K,N,M,tile", [
-    (6400, 9472, 8, (64, 1, 16)), (512, 4737, 16, (64, 2, 16)), (1280, 9408, 17, (64, 3, 16)), (512, 4672, 64, (64, 4, 16)),
-    (6400, 9473, 3, (96, 1, 24)), (768, 14208, 9, (96, 2, 24)), (6400, 14209, 8, (32, 1, 8)), (1280, 14209, 16, (32, 2, 8)),
-    (512, 9472, 24, (64, 3, 8)), (512, 9473, 24, (96, 3, 12)), (1024, 14208, 31, (96, 4, 12)), (512, 14209, 17, (128, 3, 16)),
-    (2304, 18944, 32, (128, 4, 16)), (256, 18945, 24, (64, 3, 8)), (512, 18945, 27, (64, 4, 8)), (512, 7104, 33, (96, 3, 12)),
-    (512, 9473, 33, (96, 5, 12)), (4096, 14208, 48, (96, 6, 12)), (512, 9480, 49, (96, 7, 12)), (1280, 14145, 63, (96, 8, 12)),
-    (512, 14209, 40, (128, 5, 16)), (2304, 18944, 41, (128, 6, 16)), (512, 14209, 49, (64, 4, 8)), (256, 18945, 40, (64, 3, 8))])
+    (6400, 9472, 8, (64, 1, 16, 1)), (512, 5185, 16, (64, 2, 16, 1)), (1280, 9408, 17, (64, 3, 16, 1)), (4096, 4672, 64, (64, 4, 16, 1)),
+    (512, 5184, 16, (32, 2, 8, 2)), (512, 4672, 64, (32, 4, 8, 2)), (1280, 4800, 17, (32, 3, 8, 2)),
+    (6400, 9473, 3, (96, 1, 24, 1)), (768, 14208, 9, (96, 2, 24, 1)), (6400, 14209, 8, (32, 1, 8, 2)), (1280, 18944, 16, (32, 2, 8, 2)),
+    (6400, 18945, 8, (32, 1, 8, 3)), (1280, 18945, 16, (32, 2, 8, 3)),
+    (512, 9472, 24, (64, 3, 8, 2)), (512, 9473, 24, (96, 3, 12, 1)), (1024, 14208, 31, (96, 4, 12, 1)), (512, 14209, 17, (128, 3, 16, 1)),
+    (2304, 18944, 32, (128, 4, 16, 1)), (256, 18945, 24, (64, 3, 8, 2)), (512, 18945, 27, (64, 4, 8, 2)), (512, 7104, 33, (96, 3, 12, 1)),
+    (512, 9473, 33, (96, 5, 12, 1)), (4096, 14208, 48, (96, 6, 12, 1)), (512, 9480, 49, (96, 7, 12, 1)), (1280, 14145, 63, (96, 8, 12, 1)),
+    (512, 14209, 40, (128, 5, 16, 1)), (2304, 18944, 41, (128, 6, 16, 1)), (512, 14209, 49, (64, 4, 8, 2)), (256, 18945, 40, (64, 3, 8, 2))])
 @pytest.mark.parametrize("order", [0, 1])
 def test_small_batch_tiles(env, K, N, M, tile, order):
     assert small_batch_tile(K, [N], M) == tile

@@ -30,6 +30,8 @@ constexpr int GV_BAR_BYTES = 256;  // full[8] + empty[8] ring mbarriers, red_ful
 constexpr int GV_RED_SLOTS = 4;
 constexpr int GV_PREVIOUS_ENDED = 29;  // (8-byte slot of the barrier block) non-zero: the preceding kernel has ended
 constexpr uint32_t MASK4 = 0x0F0F0F0Fu;
+constexpr int GV_MAGIC_I = 0x4B400000;  // bit pattern of 1.5 * 2^23: an integer sum added to it reads as a float, less 1.5 * 2^23, exactly
+constexpr float GV_MAGIC_F = 12582912.0f;
 
 constexpr int GV_MAX_MATS = 4;
 
@@ -941,7 +943,85 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
 // its high nibbles weights 16+4t.. (a2/a3) -- exactly the k ranges the fragment layout asks of it.
 // Partial fp32 sums of the NW warps are added in a fixed order through shared memory.
 // ------------------------------------------------------------------------------------------------
-template <int KBW, int NW>
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<uint64_t &>(d))
+        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t &>(d))
+        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)),
+          "l"(reinterpret_cast<const uint64_t &>(c)));
+    return d;
+}
+
+// Activations of the blocks [kb0, kb0 + KBW), from memory (READY) or from where they were staged: B fragments (column g) and scales
+// (columns 2t, 2t + 1); zeros for a block or a column that is not there.  Staged ones are read without a test, the last block or column
+// in place of one that is not there: with tests the shared-memory loads came one after the other, 1 us.  kb0 and KBW are multiples
+// of four, a group of 144 bytes.
+template <int KBW, bool READY>
+__device__ __forceinline__ void load_fragments(const GemvParams &p, const uint8_t *xs, int kb0, int g, int t, uint32_t (&xb0)[KBW],
+                                               uint32_t (&xb1)[KBW], float (&xd0)[KBW], float (&xd1)[KBW], float (&xm0)[KBW], float (&xm1)[KBW]) {
+    uint4 heads[KBW / 4][2];
+#pragma unroll
+    for (int i = 0; i < KBW / 4; ++i) {
+        const int ks = min((kb0 >> 2) + i, p.n_super - 1);
+        const bool there = (kb0 >> 2) + i < p.n_super;
+        const auto group = [&](int m) {
+            m = min(m, p.M - 1);
+            return READY ? p.xq + (size_t)q8_block_index(ks, m, p.n_super, p.M, p.order) * Q8_BYTES
+                         : xs + (size_t)m * p.x_pitch + (size_t)ks * Q8_BYTES;
+        };
+        const auto load4 = [&](const uint8_t *src, int m) {
+            if constexpr (!READY) return *reinterpret_cast<const uint4 *>(src);
+            else return there && m < p.M && JQ_IN_EXTENT(p.ext_x, src, 16, p.fault) ? __ldg(reinterpret_cast<const uint4 *>(src)) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        const auto load1 = [&](const uint8_t *src) {
+            if constexpr (!READY) return *reinterpret_cast<const uint32_t *>(src);
+            else return there && g < p.M && JQ_IN_EXTENT(p.ext_x, src, 4, p.fault) ? __ldg(reinterpret_cast<const uint32_t *>(src)) : 0u;
+        };
+        heads[i][0] = load4(group(2 * t), 2 * t);
+        heads[i][1] = load4(group(2 * t + 1), 2 * t + 1);
+        const uint8_t *qs = group(g) + Q8_QS_OFFSET + 4 * t;
+#pragma unroll
+        for (int sub = 0; sub < 4; ++sub) {
+            xb0[4 * i + sub] = load1(qs + QK * sub);
+            xb1[4 * i + sub] = load1(qs + QK * sub + 16);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < KBW / 4; ++i) {
+        const bool there = (kb0 >> 2) + i < p.n_super;
+        const uint32_t ds[2][4] = {{heads[i][0].x, heads[i][0].y, heads[i][0].z, heads[i][0].w},
+                                   {heads[i][1].x, heads[i][1].y, heads[i][1].z, heads[i][1].w}};
+#pragma unroll
+        for (int sub = 0; sub < 4; ++sub) {
+            const int j = 4 * i + sub;
+            const uint32_t s0 = there && 2 * t < p.M ? ds[0][sub] : 0u, s1 = there && 2 * t + 1 < p.M ? ds[1][sub] : 0u;
+            if (!there || g >= p.M) xb0[j] = xb1[j] = 0u;
+            xd0[j] = half_bits_to_float(s0 & 0xFFFFu);
+            xm0[j] = -8.0f * half_bits_to_float(s0 >> 16);
+            xd1[j] = half_bits_to_float(s1 & 0xFFFFu);
+            xm1[j] = -8.0f * half_bits_to_float(s1 >> 16);
+        }
+    }
+}
+
+// What bounds it: K = 4096, N = 22016, M = 8 (148 CTAs of 149 rows) took 15.4 us, of which the copies alone, with no
+// arithmetic, 11.1 (HBM at 7.2 TB/s in between) and the start 2.9: the wait for the preceding kernel, the activations and the fragments.
+// Ready blocks (READY) therefore go from memory to the registers of the warp that uses them (staged in shared memory by all for all:
+// 1.2 us more), their place in shared memory is one more stage of weights, and the arithmetic has no test per pair of blocks, so
+// that the loads of one pair go past the sums of another, and runs on integer sums that start from 1.5 * 2^23 (a conversion
+// instruction runs at half the rate) and packed fma: the same operations, the same bits.  M = 8, before / after: N = 4096 5.9 / 5.3 us,
+// N = 11008 9.4 / 8.4, N = 22016 15.4 / 14.1; K = 6144, N = 16384 19.8 / 16.5; K = 1024, N = 12000 7.4 / 5.6; with the quantizer inside, K =
+// 4096, N = 32000, M = 3 21.2 / 19.6.  Up to K = 2048 (eight warps, some with no block) a test per pair is the better form: K = 1024,
+// N = 30000, M = 6 13.5 without, 11.9 with it.
+// READY: the activations are Q8_1 blocks, else fp32 that is quantized here.
+template <int KBW, int NW, bool READY>
 __global__ void __launch_bounds__((NW + 2) * 32, 1) gemv_mma_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -1008,43 +1088,31 @@ __global__ void __launch_bounds__((NW + 2) * 32, 1) gemv_mma_kernel(const GemvPa
         return;
     }
 
-    stage_activations<NW>(p, xs, x_ready, warp, lane);
-    if (threadIdx.x == 0) trace_stamp(p, 4);  // activations staged
-
     const int g = lane >> 2, t = lane & 3;
-    const int nb = p.K / QK;
+    const int nb = p.K / QK;  // a multiple of eight
     const int kb0 = warp * KBW;
-    const uint32_t xs_addr = smem_u32(xs);
+    constexpr int GROUP = NW == 8 ? 2 : KBW % 8 == 0 ? 8 : 4;  // blocks under one test: all there or all not
     const uint32_t ring_addr = smem_u32(ring);
     // B fragments (column g) and scales (columns 2t, 2t+1) of this warp's K slice.
     uint32_t xb0[KBW], xb1[KBW];
     float xd0[KBW], xd1[KBW], xm0[KBW], xm1[KBW];
+    if constexpr (READY) {
+        load_fragments<KBW, true>(p, xs, kb0, g, t, xb0, xb1, xd0, xd1, xm0, xm1);
+        // the producer goes on with the weights when these have landed
+        uint32_t landed = 0u;
 #pragma unroll
-    for (int j = 0; j < KBW; ++j) {
-        const int kb = kb0 + j;
-        xb0[j] = xb1[j] = 0u;
-        xd0[j] = xd1[j] = xm0[j] = xm1[j] = 0.0f;
-        if (kb < nb) {
-            const int ks = kb >> 2, sub = kb & 3;
-            if (g < p.M) {
-                const uint32_t b = xs_addr + (uint32_t)g * p.x_pitch + (uint32_t)ks * Q8_BYTES + Q8_QS_OFFSET + sub * QK;
-                xb0[j] = lds_u32(b + 4u * t);
-                xb1[j] = lds_u32(b + 4u * (t + 4));
-            }
-            if (2 * t < p.M) {
-                const uint32_t ds = lds_u32(xs_addr + (uint32_t)(2 * t) * p.x_pitch + (uint32_t)ks * Q8_BYTES + 4u * sub);
-                xd0[j] = half_bits_to_float(ds & 0xFFFFu);
-                xm0[j] = -8.0f * half_bits_to_float(ds >> 16);
-            }
-            if (2 * t + 1 < p.M) {
-                const uint32_t ds = lds_u32(xs_addr + (uint32_t)(2 * t + 1) * p.x_pitch + (uint32_t)ks * Q8_BYTES + 4u * sub);
-                xd1[j] = half_bits_to_float(ds & 0xFFFFu);
-                xm1[j] = -8.0f * half_bits_to_float(ds >> 16);
-            }
-        }
+        for (int j = 0; j < KBW; ++j) landed |= xb0[j] | xb1[j] | __float_as_uint(xd0[j]) | __float_as_uint(xd1[j]);
+        landed = __shfl_xor_sync(0xFFFFFFFFu, landed, 1);
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0]; // after %1" ::"r"(smem_u32(x_ready)), "r"(landed) : "memory");
+        if (threadIdx.x == 0) trace_stamp(p, 4);  // activations there
+    } else {
+        stage_activations<NW>(p, xs, x_ready, warp, lane);
+        if (threadIdx.x == 0) trace_stamp(p, 4);  // activations staged
+        load_fragments<KBW, false>(p, xs, kb0, g, t, xb0, xb1, xd0, xd1, xm0, xm1);
     }
 
-    const int zero4[4] = {0, 0, 0, 0};
+    const int magic4[4] = {GV_MAGIC_I, GV_MAGIC_I, GV_MAGIC_I, GV_MAGIC_I};
+    const float2 minus = make_float2(-GV_MAGIC_F, -GV_MAGIC_F);
 
     for (int c = 0; c < n_chunks; ++c) {
         const int s = c % p.stages;
@@ -1054,18 +1122,21 @@ __global__ void __launch_bounds__((NW + 2) * 32, 1) gemv_mma_kernel(const GemvPa
         if (threadIdx.x == 0 && c == n_chunks - 1) trace_stamp(p, 6);  // last stage landed
         const uint32_t stage = ring_addr + (uint32_t)s * p.stage_bytes;
 
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};  // (row g, col 2t), (g, 2t+1), (g+8, 2t), (g+8, 2t+1)
+        float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // (row g, columns 2t and 2t + 1), (row g + 8, the same)
         const uint32_t row_lo = stage + (uint32_t)g * p.row_stride;
         const uint32_t row_hi = stage + (uint32_t)(g + 8) * p.row_stride;
 #pragma unroll
-        for (int jp = 0; jp < KBW / 2; ++jp) {
-            const int kbe = kb0 + 2 * jp;  // even block, 4-byte aligned start at byte 18*kbe
-            if (kbe < nb) {
+        for (int grp = 0; grp < KBW / GROUP; ++grp) {
+            if (kb0 + grp * GROUP >= nb) break;  // (uniform in the warp)
+#pragma unroll
+            for (int pair = 0; pair < GROUP / 2; ++pair) {
+                const int jb = grp * GROUP + 2 * pair;
                 uint32_t a_even[4], a_odd[4];
                 float d_even[2], d_odd[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const uint32_t pr = (h == 0 ? row_lo : row_hi) + (uint32_t)kbe * Q4_BYTES;
+                    // even block, 4-byte aligned start at byte 18 * block
+                    const uint32_t pr = (h == 0 ? row_lo : row_hi) + (uint32_t)(kb0 + jb) * Q4_BYTES;
                     const uint32_t u0 = lds_u32(pr + 4u * t), u1 = lds_u32(pr + 4u * t + 4u), u2 = lds_u32(pr + 4u * t + 20u);
                     const uint32_t we = __funnelshift_r(u0, u1, 16);  // word t of the even block
                     a_even[h] = we & MASK4;              // a0 / a1: weights 4t..4t+3
@@ -1075,23 +1146,18 @@ __global__ void __launch_bounds__((NW + 2) * 32, 1) gemv_mma_kernel(const GemvPa
                     d_even[h] = half_bits_to_float(lds_u16(pr));
                     d_odd[h] = half_bits_to_float(lds_u16(pr + Q4_BYTES));
                 }
-                int ce[4], co[4];
-                {
-                    const uint32_t bfrag[2] = {xb0[2 * jp], xb1[2 * jp]};
-                    mma_u8s8_16832(ce, a_even, bfrag, zero4);
-                }
-                acc[0] = fmaf(d_even[0], fmaf((float)ce[0], xd0[2 * jp], xm0[2 * jp]), acc[0]);
-                acc[1] = fmaf(d_even[0], fmaf((float)ce[1], xd1[2 * jp], xm1[2 * jp]), acc[1]);
-                acc[2] = fmaf(d_even[1], fmaf((float)ce[2], xd0[2 * jp], xm0[2 * jp]), acc[2]);
-                acc[3] = fmaf(d_even[1], fmaf((float)ce[3], xd1[2 * jp], xm1[2 * jp]), acc[3]);
-                if (kbe + 1 < nb) {
-                    const uint32_t bfrag[2] = {xb0[2 * jp + 1], xb1[2 * jp + 1]};
-                    mma_u8s8_16832(co, a_odd, bfrag, zero4);
-                    acc[0] = fmaf(d_odd[0], fmaf((float)co[0], xd0[2 * jp + 1], xm0[2 * jp + 1]), acc[0]);
-                    acc[1] = fmaf(d_odd[0], fmaf((float)co[1], xd1[2 * jp + 1], xm1[2 * jp + 1]), acc[1]);
-                    acc[2] = fmaf(d_odd[1], fmaf((float)co[2], xd0[2 * jp + 1], xm0[2 * jp + 1]), acc[2]);
-                    acc[3] = fmaf(d_odd[1], fmaf((float)co[3], xd1[2 * jp + 1], xm1[2 * jp + 1]), acc[3]);
-                }
+                const auto block = [&](const uint32_t (&a)[4], const float (&d)[2], int j) {
+                    const uint32_t bfrag[2] = {xb0[j], xb1[j]};
+                    int sums[4];
+                    mma_u8s8_16832(sums, a, bfrag, magic4);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float2 sum = add2(make_float2(__int_as_float(sums[2 * h]), __int_as_float(sums[2 * h + 1])), minus);  // exact
+                        acc[h] = fma2(make_float2(d[h], d[h]), fma2(sum, make_float2(xd0[j], xd1[j]), make_float2(xm0[j], xm1[j])), acc[h]);
+                    }
+                };
+                block(a_even, d_even, jb);
+                block(a_odd, d_odd, jb + 1);
             }
         }
         __syncwarp();
@@ -1102,8 +1168,8 @@ __global__ void __launch_bounds__((NW + 2) * 32, 1) gemv_mma_kernel(const GemvPa
         const uint32_t rround = (uint32_t)(c / GV_RED_SLOTS);
         if (rround > 0 && !mbar_wait_bounded(&red_empty[slot], (rround - 1) & 1u, p.fault, p.poll_limit)) return;
         float *mine = red + ((size_t)slot * NW + warp) * 128;
-        *reinterpret_cast<float2 *>(&mine[g * 8 + 2 * t]) = make_float2(acc[0], acc[1]);
-        *reinterpret_cast<float2 *>(&mine[(g + 8) * 8 + 2 * t]) = make_float2(acc[2], acc[3]);
+        *reinterpret_cast<float2 *>(&mine[g * 8 + 2 * t]) = acc[0];
+        *reinterpret_cast<float2 *>(&mine[(g + 8) * 8 + 2 * t]) = acc[1];
         __syncwarp();
         if (lane == 0) mbar_arrive(&red_full[slot]);
     }
@@ -1206,7 +1272,7 @@ int run_mma(cudaStream_t st, GemvParams &p, const DeviceCaps &caps) {
 #ifdef JQ_BOUNDS_CHECK
     p.smem_total = (uint32_t)smem;
 #endif
-    auto kernel = gemv_mma_kernel<KBW, NW>;
+    auto kernel = p.x_f32 == nullptr ? gemv_mma_kernel<KBW, NW, true> : gemv_mma_kernel<KBW, NW, false>;
     if (int rc = ensure_smem_attr(kernel, smem)) return rc;
     const int64_t want = (p.N + 15) / 16;
     const int grid = (int)min((int64_t)caps.sm_count, max((int64_t)1, want));
@@ -1390,9 +1456,10 @@ int launch_gemv_mma(cudaStream_t st, const void *d_w, const void *d_xq, const fl
         // quantization (cfg2 M = 4: 10.8 us; 11.0 us with two stages requested earlier)
         p.prefetch_early = 0;
         p.early_stages = 1 << 30;
+    } else {
+        p.x_bytes = 0;  // ready blocks go straight to the registers (by the producer's bulk copies, as in the dp4a
+                        // kernel: K = 4096, N = 11008, M = 8 10.5 against 9.3 us with the warps' own loads to shared memory)
     }
-    // (ready blocks by the producer's bulk copies, as in the dp4a kernel, were measured slower here: cfg2 M = 8 on
-    // ready blocks 10.5 against 9.3 us with the warps' own loads)
     if (int rc = apply_multi(p, multi, nullptr)) return rc;
     const int nb = (int)(K / QK);
     if (nb <= 8 * 8) return run_mma<8, 8>(st, p, caps);

@@ -202,6 +202,24 @@ def test_small_batch_is_as_exact_as_the_generic_kernel(env, K, N, M):
     assert _error_against_64_bits(t, w, xq, y, K, rows) <= 1.125 * _error_against_64_bits(t, w, xq, before, K, rows)
 
 
+# The decode kernel for 3 to 8 columns on ready blocks: warps with all, some and none of their blocks (8 of 8, 12 of 16 warps); ends of rows
+# and columns; both orders; against the same kernel with the quantizer inside, which sums in the same order: the same bits.
+@pytest.mark.parametrize("K,N,M", [(256, 1, 3), (768, 17, 4), (2048, 2400, 8), (2304, 15, 3), (3072, 2401, 5), (4096, 2370, 8), (4096, 16, 4),
+                                   (4352, 33, 3), (5376, 2369, 7), (6144, 40, 8), (4608, 31, 6)])
+@pytest.mark.parametrize("order", [0, 1])
+def test_decode_batch_on_ready_blocks(env, K, N, M, order):
+    c, O, t = env.c, env.O, env.t
+    w, x = _problem(K, N, M)
+    wq = O.quantize_q4_0(w)
+    xq = O.quantize_q8_1(x, order, c.S_SUM_X)
+    d_w, d_x = t.from_numpy(wq).to(env.dev), t.from_numpy(xq).to(env.dev)
+    y = t.full((M, N), float("nan"), device=env.dev)
+    c.mul_mat_q4_0_q8_1(d_w, d_x, K, N, M, order, kernel=c.KERNEL_GEMV_MMA, out=y)
+    assert O.err_max_rel(y.cpu().numpy(), O.mul_mat_ref(wq, xq, K, N, M, order)) <= TOL
+    if M <= 4 and K <= 4096:
+        assert t.equal(y, c.linear_q4_0(d_w, t.from_numpy(x).to(env.dev), N, s_mode=c.S_SUM_X))
+
+
 @pytest.mark.parametrize("K,N,M", [(4224, 4800, 45), (8192, 9600, 24), (11008, 600, 8), (4096, 9600, 1), (4096, 9600, 6)])
 def test_poll_limit_of_one_waits_for_copies(env, K, N, M):
     """The shortest limit that can be set: a kernel does not give up on its own copies, and so cannot end before them."""

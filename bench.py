@@ -1039,7 +1039,7 @@ def measure_extras(torch, capi, synth, dev, peaks):
         try:
             t = bench_linear(4096, 4096, 512, steps=50)
             out["cfg3_M512_exact"] = {"us": t * 1e6, "TOPS": o / t / 1e12, "frac_int8_peak": o / t / 1e12 / int8_peak,
-                                      "kernel": "JQ_OPT_PREFILL_EXACT: quantize launch + exact-integer mma.sync GEMM"}
+                                      "kernel": "JQ_OPT_PREFILL_EXACT: quantize launch + exact-integer mma.sync kernel"}
             out["cfg5_chain_M128_exact"] = bench_layer_chain(torch, capi, synth, dev, peaks, 128)
         finally:
             capi.set_option(capi.OPT_PREFILL_EXACT, 0)

@@ -192,10 +192,10 @@ constexpr int64_t FP16_OPERANDS_MIN_COLUMNS = 64;
 
 // The small-batch kernel takes what the decode kernels above it refuse, up to 63 columns, and every batch whose K is an
 // odd multiple of 128 (the GEMMs need K % 256 == 0).  Multiply alone, cold weights, what was taken before / this kernel:
-// K = 4096, N = 11008, M = 16 18.7 / 14.1 us, M = 24 27.8 / 17.8 us (passes of eight columns), M = 48 44.7 / 26.0 us (integer
+// K = 4096, N = 11008, M = 16 18.7 / 10.8 us, M = 24 27.8 / 13.1 us (passes of eight columns), M = 48 44.7 / 22.4 us (integer
 // GEMM); K = 11008, N = 4096, M = 8 61.6 / 11.0 us (generic kernel); K = 1408, N = 1003, M = 1 3.4 / 2.8 us, M = 48
 // 13.9 / 3.9 us; K = 4224, N = 11008, M = 2 24.2 / 14.1 us (generic kernel).  Where the decode kernel runs (3 to 8 columns,
-// K <= 6144) it is the faster one at K = 4096: N = 11008 9.5 against 13.1 us.
+// K <= 6144) it is the faster one at K = 4096: N = 11008 8.4 us for 8 columns, 11.0 here for 9.
 // One column of a long odd K and few rows stays with the generic kernel: a CTA's stages of K are a chain however few the rows,
 // and there a warp per row still has an SM almost to itself.  Quantizer and multiply, generic / small-batch kernel: K = 10880,
 // N = 64 11.2 / 13.8 us, N = 600 12.8 / 14.2 us; K = 8320, N = 300 10.5 / 11.5 us, N = 800 11.1 / 11.5 us (with static weights

@@ -18,6 +18,7 @@ namespace jq {
 namespace {
 
 constexpr int RMS_THREADS = 256;  // the reference's block size; the summation order depends on it
+constexpr size_t RMS_STATIC_BYTES = 1024;  // more than the kernel's static shared memory and what the device reserves per block
 
 // Block sum with the reference's tree (include/cuda_utils.cuh:19-27, 49-65): shuffle-down inside
 // each warp, one partial per warp through shared memory, shuffle-down over the partials in warp 0.
@@ -302,14 +303,15 @@ int launch_rms_norm_q8_1(cudaStream_t st, float *d_input, float *d_residual, con
     DeviceCaps caps;
     if (int rc = device_caps(&caps)) return rc;
     size_t smem = (size_t)H * sizeof(float);
-    if (smem + 1024 > (size_t)caps.smem_optin)
+    if (smem + RMS_STATIC_BYTES > (size_t)caps.smem_optin)
         return set_error(JQ_ERR_TOO_LARGE, "rms_norm: a row of %lld floats does not fit in shared memory", (long long)H);
     // A decode step of one sequence (four layers of 4096 x 11008 and the output norm, replayed from a graph, all launches) 186.0 ->
     // 180.4 us; of eight sequences 155.7 -> 158.0: there the row's neighbours bring the vector in.
-    const bool staged = T <= 2 && d_xq != nullptr && 2 * smem + 1024 <= (size_t)caps.smem_optin;
+    const bool staged = T <= 2 && d_xq != nullptr && 2 * smem + RMS_STATIC_BYTES <= (size_t)caps.smem_optin;
     if (staged) smem *= 2;
     const auto kernel = staged ? rms_norm_q8_1_kernel<true> : rms_norm_q8_1_kernel<false>;
-    if (smem > 48 * 1024) {
+    // without being asked for, a block has 48 KB, of which the kernel's static variables take a part
+    if (smem + RMS_STATIC_BYTES > 48 * 1024) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem)) return rc;
     }
     cudaLaunchConfig_t cfg = {};

@@ -334,3 +334,35 @@ def test_multi_linear_equals_separate_linears(native_lib, oracle, cuda_device, M
         c.linear_q4_0_multi(wq, Ns, x=x, xq=xq, K=K, M=M)  # both kinds of input
     with pytest.raises(c.JqError):
         c.linear_q4_0_multi(wq * 5, list(Ns) * 5, x=x)  # more than four matrices
+
+
+RMS_EDGE_WORKER = r"""
+import sys
+sys.path.insert(0, sys.argv[1])
+import torch
+from jjjetson_ops_b200 import capi as c
+dev = torch.device("cuda:0")
+g = torch.Generator(device=dev)
+g.manual_seed(3)
+for T, H in ((2, 6144), (1, 6144), (3, 12288), (1, 12288)):
+    x, r = torch.randn((T, H), generator=g, device=dev), torch.randn((T, H), generator=g, device=dev)
+    w = 1.0 + 0.1 * torch.randn(H, generator=g, device=dev)
+    z = x.double() + r.double()
+    want = z * torch.rsqrt((z * z).mean(dim=1, keepdim=True) + 1e-5) * w.double()
+    normed = torch.empty_like(x)
+    xq = c.rms_norm_q8_1(x, w, 1e-5, residual=r, normed=normed)
+    # in units of 2**-24: 48 additions per thread, 8 levels of the tree and the squares' own (2) count half, 29; rsqrtf 2 ulp, 4; z and two products, 3
+    assert ((normed.double() - want).abs() <= 40 * 2.0**-24 * want.abs()).all(), (T, H)
+    assert torch.equal(xq[: c.q8_1_bytes(H, T)], c.quantize_q8_1(normed, c.ORDER_COL_KSUPER, c.S_D_SUM_Q)[: c.q8_1_bytes(H, T)]), (T, H)
+print("edges ok")
+"""
+
+
+def test_rms_norm_rows_of_48_kb(native_lib, cuda_device):
+    """Rows (and row and weights together, for one and two tokens) of 48 KB: with the kernel's static variables just more than a block
+    has without asking.  In a process of its own, because a wider row before would have raised the limit."""
+    import subprocess
+    import sys
+
+    done = subprocess.run([sys.executable, "-c", RMS_EDGE_WORKER, ROOT], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and "edges ok" in done.stdout, done.stdout + done.stderr

@@ -169,27 +169,27 @@ __device__ __forceinline__ uint32_t h2_high_scale(uint32_t v, __half2 scale) {
     return as_u32(__hmul2(__hfma2(as_h2(v), as_h2(H2_SIXTEENTH), as_h2(H2_MINUS_72)), scale));
 }
 
+// The kernel has an instance for one matrix and one for up to four.  What is looked up by matrix is addressable (__grid_constant__:
+// by value, such a look-up takes a copy in local memory, 128 bytes per thread of the instances for several matrices) ...
 template <int MATS>
-struct HfMaps {
-    CUtensorMap w[MATS];
-    CUtensorMap x;
-};
-
-// The kernel has an instance for one matrix and one for up to four, and takes these by value: a look-up by matrix needs
-// them addressable (__grid_constant__), and then fields are read again in every turn of the conversion loop.
-template <int MATS>
-struct HfParams {
+struct HfMats {
     // Up to four weight matrices that share K and the activations: the CTAs with blockIdx.x in [tile_begin[i],
     // tile_begin[i + 1]) have 128 rows each of matrix i (whole pairs of CTAs, if they work in pairs), which goes to y[i],
     // an [M][rows[i]] array.
+    CUtensorMap w[MATS];
+    CUtensorMap x;
     float *y[MATS];
     int64_t rows[MATS];
     int tile_begin[MATS + 1];
     int n_mats;
-    int *fault;
 #ifdef JQ_BOUNDS_CHECK
     Extent ext_y[MATS];  // range-checked debug build (the operand loads are tensor copies: their maps bound them)
 #endif
+};
+
+// ... and the rest is not: fields of an addressable parameter are read again in every turn of the conversion loop.
+struct HfParams {
+    int *fault;
     int64_t M;
     int n_chunks;        // K / 128
     int order;
@@ -252,17 +252,17 @@ __device__ __forceinline__ float convert_activation_block(const uint4 &lo, const
 
 // the matrix this CTA works on
 template <int MATS>
-__device__ __forceinline__ int hf_matrix(const HfParams<MATS> &p) {
+__device__ __forceinline__ int hf_matrix(const HfMats<MATS> &mats) {
     int mat = 0;
     if (MATS > 1) {
-        while (mat + 1 < p.n_mats && (int)blockIdx.x >= p.tile_begin[mat + 1]) ++mat;
+        while (mat + 1 < mats.n_mats && (int)blockIdx.x >= mats.tile_begin[mat + 1]) ++mat;
     }
     return mat;
 }
 
 template <bool PAIR, bool SPLIT, int MATS>
 __global__ void __launch_bounds__(HF_THREADS, 1)
-gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps<MATS> maps) {
+gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS> mats) {
     using T = HfTile<PAIR>;
     constexpr int NS = HF_STAGES;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -280,8 +280,8 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
-    const int mat = hf_matrix(p);
-    const int64_t n0 = (int64_t)((int)blockIdx.x - (MATS > 1 ? p.tile_begin[mat] : 0)) * HF_ROWS;  // this CTA's weight rows
+    const int mat = hf_matrix(mats);
+    const int64_t n0 = (int64_t)((int)blockIdx.x - (MATS > 1 ? mats.tile_begin[mat] : 0)) * HF_ROWS;  // this CTA's weight rows
     const int64_t m0 = (int64_t)blockIdx.y * T::NT;  // the tile's activation columns; this CTA converts X_ROWS from m0 + rank * X_ROWS
     const int c0 = SPLIT ? (int)blockIdx.z * p.chunks_per_split : 0;
     const int n_chunks = SPLIT ? min(p.chunks_per_split, p.n_chunks - c0) : p.n_chunks;  // even
@@ -413,9 +413,9 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
             tc_fence_after();
             asm volatile("griddepcontrol.wait;" ::: "memory");  // (long past: orders the stores to y after the previous kernel)
             finished = true;
-            const int out = hf_matrix(p);
-            float *const y = p.y[out];
-            const int64_t N = p.rows[out], n = n0 + gw * 32 + lane;
+            const int out = hf_matrix(mats);
+            float *const y = mats.y[out];
+            const int64_t N = mats.rows[out], n = n0 + gw * 32 + lane;
 #pragma unroll
             for (int blk = 0; blk < T::BLOCKS; ++blk) {
                 const int col = ((warp >> 2) * T::BLOCKS + blk) * 32;
@@ -430,7 +430,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                     float *at = y + (m0 + col) * N + n;
 #pragma unroll
                     for (int j = 0; j < 32; ++j, at += N) {
-                        if (m0 + col + j < p.M && n < N && JQ_IN_EXTENT(p.ext_y[out], at, sizeof(float), p.fault)) *at = __uint_as_float(v[j]);
+                        if (m0 + col + j < p.M && n < N && JQ_IN_EXTENT(mats.ext_y[out], at, sizeof(float), p.fault)) *at = __uint_as_float(v[j]);
                     }
                 }
             }
@@ -447,9 +447,9 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 mbar_arrive_expect_tx(&x_full[rs], HF_RAW_BYTES);
                 const uint32_t dst = sbase + HF_RAW_OFF + rs * HF_RAW_BYTES;
                 if (p.order == JQ_ORDER_KSUPER_COL)  // the tensor is [n_super * M blocks][144 bytes]
-                    tma_load_2d(dst, &maps.x, 0, (int)((int64_t)(c0 + c) * p.M + col), &x_full[rs]);
+                    tma_load_2d(dst, &mats.x, 0, (int)((int64_t)(c0 + c) * p.M + col), &x_full[rs]);
                 else                                 // the tensor is [M columns][n_super * 144 bytes]
-                    tma_load_2d(dst, &maps.x, (c0 + c) * Q8_BYTES, (int)col, &x_full[rs]);
+                    tma_load_2d(dst, &mats.x, (c0 + c) * Q8_BYTES, (int)col, &x_full[rs]);
             }
         }
     } else if (warp == HF_COPY_W_WARP) {
@@ -461,7 +461,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
                 const uint32_t round = (uint32_t)(pr / HF_W_SLOTS);
                 if (round > 0 && !mbar_wait_bounded(&w_empty[ws], (round - 1) & 1u, p.fault)) break;
                 mbar_arrive_expect_tx(&w_full[ws], HF_W_SLOT_BYTES);
-                tma_load_2d(sbase + HF_W_OFF + ws * HF_W_SLOT_BYTES, &maps.w[mat], ((c0 >> 1) + pr) * Q8_BYTES, (int)n0, &w_full[ws]);
+                tma_load_2d(sbase + HF_W_OFF + ws * HF_W_SLOT_BYTES, &mats.w[mat], ((c0 >> 1) + pr) * Q8_BYTES, (int)n0, &w_full[ws]);
             }
         }
     } else if (lane == 0 && rank == 0) {
@@ -515,9 +515,9 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
         cluster_sync();
         if (finished) {
             const int gw = warp & 3;
-            const int out = hf_matrix(p);
-            float *const y = p.y[out];
-            const int64_t N = p.rows[out], n = n0 + gw * 32 + lane;
+            const int out = hf_matrix(mats);
+            float *const y = mats.y[out];
+            const int64_t N = mats.rows[out], n = n0 + gw * 32 + lane;
             const int end = 32 * (z + 1) / parts;
 #pragma unroll
             for (int blk = 0; blk < T::BLOCKS; ++blk) {
@@ -539,7 +539,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
 #pragma unroll
                         for (int q = 1; q < HF_MAX_SPLITS; ++q) v += part[u][q];
                         const int64_t m = m0 + ((warp >> 2) * T::BLOCKS + blk) * 32 + j0 + u;
-                        if (j0 + u < end && m < p.M && n < N && JQ_IN_EXTENT(p.ext_y[out], y + m * N + n, sizeof(float), p.fault)) y[m * N + n] = v;
+                        if (j0 + u < end && m < p.M && n < N && JQ_IN_EXTENT(mats.ext_y[out], y + m * N + n, sizeof(float), p.fault)) y[m * N + n] = v;
                     }
                 }
             }
@@ -561,7 +561,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams<MATS> p, const __grid_constant__ HfMaps
 }
 
 template <bool PAIR, bool SPLIT, int MATS>
-int launch_kernel(cudaStream_t st, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
+int launch_kernel(cudaStream_t st, dim3 grid, const HfParams &p, const HfMats<MATS> &mats) {
     const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, MATS>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
     (void)cudaGetLastError();  // a stale error of an earlier, unrelated call must not be taken for this launch's
@@ -579,7 +579,7 @@ int launch_kernel(cudaStream_t st, dim3 grid, const HfParams<MATS> &p, const HfM
     attr[1].val.clusterDim.z = (unsigned)p.k_splits;
     cfg.attrs = attr;
     cfg.numAttrs = PAIR || SPLIT ? 2 : 1;
-    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, maps));
+    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, mats));
     return JQ_OK;
 }
 // Clusters of z CTAs along K, or of a pair of CTAs, of this kernel that the current device runs at a time (0: none).  The instances
@@ -637,10 +637,10 @@ int form_widths(const DeviceCaps &caps, GemmF16Widths *out) {
 }
 // form: 0 pairs of CTAs, 1 split K, 2 neither
 template <int MATS>
-int launch_form(cudaStream_t st, int form, dim3 grid, const HfParams<MATS> &p, const HfMaps<MATS> &maps) {
-    if (form == 0) return launch_kernel<true, false, MATS>(st, grid, p, maps);
-    if (form == 1) return launch_kernel<false, true, MATS>(st, grid, p, maps);
-    return launch_kernel<false, false, MATS>(st, grid, p, maps);
+int launch_form(cudaStream_t st, int form, dim3 grid, const HfParams &p, const HfMats<MATS> &mats) {
+    if (form == 0) return launch_kernel<true, false, MATS>(st, grid, p, mats);
+    if (form == 1) return launch_kernel<false, true, MATS>(st, grid, p, mats);
+    return launch_kernel<false, false, MATS>(st, grid, p, mats);
 }
 
 }  // namespace
@@ -650,18 +650,19 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     // a weight row's pitch, K / 32 * 18 bytes, must be a multiple of 16 for the tensor copies
     if (K % (2 * SUPER) != 0) return set_error(JQ_ERR_UNSUPPORTED, "fp16-operand tcgen05 GEMM needs K %% 256 == 0 (K = %lld)", (long long)K);
     const void *w[HF_MAX_MATS] = {};
-    HfParams<HF_MAX_MATS> p{};
-    p.n_mats = multi != nullptr ? multi->n : 1;
-    if (p.n_mats < 1 || p.n_mats > HF_MAX_MATS) return set_error(JQ_ERR_INVALID_ARG, "1 to %d weight matrices per launch", HF_MAX_MATS);
+    HfParams p{};
+    HfMats<HF_MAX_MATS> mats{};
+    mats.n_mats = multi != nullptr ? multi->n : 1;
+    if (mats.n_mats < 1 || mats.n_mats > HF_MAX_MATS) return set_error(JQ_ERR_INVALID_ARG, "1 to %d weight matrices per launch", HF_MAX_MATS);
     uintptr_t bits = (uintptr_t)d_xq;
     int64_t gx = 0, pair_gx = 0;  // CTAs along the weight rows, on their own and in pairs
-    for (int i = 0; i < p.n_mats; ++i) {
+    for (int i = 0; i < mats.n_mats; ++i) {
         w[i] = multi != nullptr ? multi->w[i] : d_w;
-        p.y[i] = multi != nullptr ? multi->y[i] : d_y;
-        p.rows[i] = multi != nullptr ? multi->rows[i] : N;
+        mats.y[i] = multi != nullptr ? multi->y[i] : d_y;
+        mats.rows[i] = multi != nullptr ? multi->rows[i] : N;
         bits |= (uintptr_t)w[i];
-        gx += (p.rows[i] + HF_ROWS - 1) / HF_ROWS;
-        pair_gx += (p.rows[i] + 2 * HF_ROWS - 1) / (2 * HF_ROWS) * 2;
+        gx += (mats.rows[i] + HF_ROWS - 1) / HF_ROWS;
+        pair_gx += (mats.rows[i] + 2 * HF_ROWS - 1) / (2 * HF_ROWS) * 2;
     }
     if ((bits & 15u) != 0) return set_error(JQ_ERR_UNSUPPORTED, "fp16-operand tcgen05 GEMM needs 16-byte aligned operands");
     if (N == 0 || M == 0) return JQ_OK;
@@ -683,43 +684,34 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     p.k_splits = plan.k_splits;
     p.chunks_per_split = plan.chunks_per_split;
     const uint32_t row_bytes = (uint32_t)(K / QK * Q4_BYTES);
-    HfMaps<HF_MAX_MATS> maps{};
-    p.tile_begin[0] = 0;
-    for (int i = 0; i < p.n_mats; ++i) {
+    mats.tile_begin[0] = 0;
+    for (int i = 0; i < mats.n_mats; ++i) {
         const int64_t per = pair ? 2 : 1;
-        p.tile_begin[i + 1] = p.tile_begin[i] + (int)((p.rows[i] + per * HF_ROWS - 1) / (per * HF_ROWS) * per);
-        if (int rc = encode_byte_map(&maps.w[i], w[i], row_bytes, (uint64_t)p.rows[i], row_bytes, Q8_BYTES, HF_ROWS)) return rc;
+        mats.tile_begin[i + 1] = mats.tile_begin[i] + (int)((mats.rows[i] + per * HF_ROWS - 1) / (per * HF_ROWS) * per);
+        if (int rc = encode_byte_map(&mats.w[i], w[i], row_bytes, (uint64_t)mats.rows[i], row_bytes, Q8_BYTES, HF_ROWS)) return rc;
 #ifdef JQ_BOUNDS_CHECK
-        p.ext_y[i] = make_extent(p.y[i], (unsigned long long)M * (unsigned long long)p.rows[i] * sizeof(float));
+        mats.ext_y[i] = make_extent(mats.y[i], (unsigned long long)M * (unsigned long long)mats.rows[i] * sizeof(float));
 #endif
     }
     const int64_t n_super = K / SUPER;
     const uint64_t x_row = (uint64_t)n_super * Q8_BYTES;
     if (int rc = order == JQ_ORDER_KSUPER_COL
-                     ? encode_byte_map(&maps.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, HF_X_ROWS)
-                     : encode_byte_map(&maps.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, HF_X_ROWS))
+                     ? encode_byte_map(&mats.x, d_xq, Q8_BYTES, (uint64_t)n_super * (uint64_t)M, Q8_BYTES, Q8_BYTES, HF_X_ROWS)
+                     : encode_byte_map(&mats.x, d_xq, x_row, (uint64_t)M, x_row, Q8_BYTES, HF_X_ROWS))
         return rc;
     const int form = pair ? 0 : p.k_splits > 1 ? 1 : 2;
-    const dim3 grid((unsigned)p.tile_begin[p.n_mats], (unsigned)(pair ? pair_gy : gy), (unsigned)p.k_splits);
-    if (p.n_mats > 1) return launch_form(st, form, grid, p, maps);
-    HfParams<1> p1{};
-    p1.y[0] = p.y[0];
-    p1.rows[0] = p.rows[0];
-    p1.n_mats = 1;
-    p1.fault = p.fault;
+    const dim3 grid((unsigned)mats.tile_begin[mats.n_mats], (unsigned)(pair ? pair_gy : gy), (unsigned)p.k_splits);
+    if (mats.n_mats > 1) return launch_form(st, form, grid, p, mats);
+    HfMats<1> one{};
+    one.w[0] = mats.w[0];
+    one.x = mats.x;
+    one.y[0] = mats.y[0];
+    one.rows[0] = mats.rows[0];
+    one.n_mats = 1;
 #ifdef JQ_BOUNDS_CHECK
-    p1.ext_y[0] = p.ext_y[0];
+    one.ext_y[0] = mats.ext_y[0];
 #endif
-    p1.M = p.M;
-    p1.n_chunks = p.n_chunks;
-    p1.order = p.order;
-    p1.k_splits = p.k_splits;
-    p1.chunks_per_split = p.chunks_per_split;
-    p1.static_weights = p.static_weights;
-    HfMaps<1> maps1{};
-    maps1.w[0] = maps.w[0];
-    maps1.x = maps.x;
-    return launch_form(st, form, grid, p1, maps1);
+    return launch_form(st, form, grid, p, one);
 }
 
 }  // namespace jq

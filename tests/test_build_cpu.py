@@ -1,6 +1,8 @@
 """What the build does with and without torch, with the compiler replaced by a list of its command lines."""
 import importlib.util
 import os
+import re
+import subprocess
 
 import pytest
 
@@ -39,3 +41,11 @@ def test_another_torch_is_another_build(commands, monkeypatch):
     monkeypatch.setattr(_build.importlib.metadata, "version", lambda name: "0.0.0")
     _build.build_all()
     assert len(commands) == 2
+
+
+def test_the_fp16_operand_gemm_keeps_nothing_in_local_memory(tmp_path):
+    """As the compiler reports it: no instance has a stack frame (a look-up by matrix in a by-value parameter takes one) or spills."""
+    done = subprocess.run([_build._nvcc(), *_build.NVCC_FLAGS, "-Xptxas", "-v", "-I", _build.INCLUDE_DIR, "-cubin", "-o", str(tmp_path / "x.cubin"),
+                           os.path.join(_build.CSRC, "mmq_gemm_f16_sm100.cu")], capture_output=True, text=True, check=True)
+    frames = re.findall(r"(\d+) bytes stack frame, (\d+) bytes spill stores, (\d+) bytes spill loads", done.stdout + done.stderr)
+    assert len(frames) == 6 and set(frames) == {("0", "0", "0")}

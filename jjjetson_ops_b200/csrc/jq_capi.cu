@@ -758,9 +758,10 @@ int jq_debug_set_extent_shrink(unsigned long long bytes) {
 
 namespace {
 
-// What a host call needs on the device and in pinned memory: a stream, one device buffer and a staging buffer.  Lanes are kept
-// between calls, because making them costs as much as a small call's own work; each call has one to itself while it runs, and at
-// most LANES_KEPT idle ones of at most LANE_KEPT_BYTES stay per device (jq_release_host_scratch gives them back).
+// What a host call needs on the device and in pinned memory: a stream, one device buffer and a staging buffer.  Each call has such a
+// lane to itself while it runs.  LANES_KEPT of at most LANE_KEPT_BYTES are kept per device between calls, because making them costs
+// more than a small call's own work (jq_release_host_scratch gives the idle ones back).  Further calls at the same time get one
+// without a staging buffer, which would take longer to make than it saves, and so does a call that cannot have one.
 inline size_t whole_lines(size_t bytes) { return (bytes + 255) / 256 * 256; }
 constexpr size_t STAGE_CHUNK = (size_t)512 << 10, STAGE_SLOTS = 32, STAGE_BYTES = STAGE_CHUNK * STAGE_SLOTS;
 constexpr size_t RESULT_BYTES = (size_t)2 << 20;
@@ -769,19 +770,23 @@ constexpr size_t MAX_COPY_THREADS = 4;
 static_assert(STAGE_SLOTS % MAX_COPY_THREADS == 0, "a thread meets its own chunks again in a slot");
 struct HostLane {
     int device = 0;
+    bool kept = false;              // one of the device's LANES_KEPT
     cudaStream_t stream = nullptr;
     uint8_t *d = nullptr;
     size_t d_bytes = 0;
-    uint8_t *pinned = nullptr;      // STAGE_SLOTS chunks on their way to the device, then RESULT_BYTES from it
+    uint8_t *pinned = nullptr;      // (or none) STAGE_SLOTS chunks on their way to the device, then RESULT_BYTES from it
     cudaEvent_t sent[STAGE_SLOTS] = {};
     bool in_use[STAGE_SLOTS] = {};  // by this call: `sent` says when the chunk has gone
     size_t next_slot = 0;
 
     int open() {
-        JQ_CUDA_TRY(cudaGetDevice(&device));
         JQ_CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        JQ_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&pinned), STAGE_BYTES + RESULT_BYTES, cudaHostAllocDefault));
+        if (!kept) return JQ_OK;
         for (cudaEvent_t &e : sent) JQ_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        if (cudaHostAlloc(reinterpret_cast<void **>(&pinned), STAGE_BYTES + RESULT_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+            (void)cudaGetLastError();
+            pinned = nullptr;
+        }
         return JQ_OK;
     }
     int reserve(size_t bytes) {
@@ -805,6 +810,7 @@ struct HostLane {
     }
 };
 std::mutex g_lanes_mutex;
+size_t g_kept_lanes[MAX_DEVICES];  // idle or at work
 std::vector<HostLane *> &idle_lanes() {  // never destroyed: no CUDA call may run while the process ends
     static std::vector<HostLane *> &lanes = *new std::vector<HostLane *>();
     return lanes;
@@ -816,6 +822,7 @@ class LaneLease {
     int open() {
         int dev = 0;
         JQ_CUDA_TRY(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= MAX_DEVICES) return set_error(JQ_ERR_UNSUPPORTED, "device index %d out of range", dev);
         {
             std::lock_guard<std::mutex> lock(g_lanes_mutex);
             std::vector<HostLane *> &idle = idle_lanes();
@@ -827,9 +834,12 @@ class LaneLease {
                     return JQ_OK;
                 }
             }
+            lane_ = new (std::nothrow) HostLane();
+            if (lane_ == nullptr) return set_error(JQ_ERR_CUDA, "out of host memory");
+            lane_->device = dev;
+            lane_->kept = g_kept_lanes[dev] < LANES_KEPT;
+            g_kept_lanes[dev] += lane_->kept;
         }
-        lane_ = new (std::nothrow) HostLane();
-        if (lane_ == nullptr) return set_error(JQ_ERR_CUDA, "out of host memory");
         return lane_->open();
     }
     HostLane *operator->() const { return lane_; }
@@ -838,18 +848,16 @@ class LaneLease {
     void done() { finished_ = true; }
     ~LaneLease() {
         if (lane_ == nullptr) return;
-        if (finished_ && lane_->d_bytes <= LANE_KEPT_BYTES) {
+        if (lane_->kept) {
             std::lock_guard<std::mutex> lock(g_lanes_mutex);
-            std::vector<HostLane *> &idle = idle_lanes();
-            size_t kept = 0;
-            for (const HostLane *l : idle) kept += l->device == lane_->device;
-            if (kept < LANES_KEPT) {
+            if (finished_ && lane_->d_bytes <= LANE_KEPT_BYTES) {
                 try {
-                    idle.push_back(lane_);
+                    idle_lanes().push_back(lane_);
                     return;
                 } catch (...) {  // no memory for the list
                 }
             }
+            --g_kept_lanes[lane_->device];
         }
         delete lane_;
     }
@@ -863,6 +871,10 @@ class LaneLease {
 // 7 to 9 GB/s); here several threads copy chunks into the lane's and hand each to the copy engine as it is ready.
 int copy_in(HostLane &lane, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return JQ_OK;
+    if (lane.pinned == nullptr) {
+        JQ_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, lane.stream));
+        return JQ_OK;
+    }
     const size_t chunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK, first_slot = lane.next_slot;
     lane.next_slot = (first_slot + chunks) % STAGE_SLOTS;
     // A thread costs some 50 us here: one, two and four of them take 9.4 MB in 770 / 590 / 800 us and the last two 38 MB in 2420 / 1640 us
@@ -901,7 +913,7 @@ class HostResults {
     explicit HostResults(HostLane &lane) : lane_(lane) {}
     int fetch(void *dst, const void *src, size_t bytes) {
         if (bytes == 0) return JQ_OK;
-        if (n_ < 2 && at_ + bytes <= RESULT_BYTES) {
+        if (lane_.pinned != nullptr && n_ < 2 && at_ + bytes <= RESULT_BYTES) {
             uint8_t *const p = lane_.pinned + STAGE_BYTES + at_;
             JQ_CUDA_TRY(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, lane_.stream));
             copies_[n_++] = Copy{dst, p, bytes};
@@ -936,6 +948,7 @@ int jq_release_host_scratch(void) {
     {
         std::lock_guard<std::mutex> lock(g_lanes_mutex);
         lanes.swap(idle_lanes());
+        for (const HostLane *l : lanes) --g_kept_lanes[l->device];
     }
     for (HostLane *l : lanes) delete l;
     return JQ_OK;

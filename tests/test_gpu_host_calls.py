@@ -1,7 +1,9 @@
 """The host wrappers' copies: chunks of 512 KB by one, two and four threads, a staging ring that goes round, results that do not fit in the
 staging buffer, calls from several threads, and after the kept buffers were given back.  The same kernels on the same blocks as the
 device calls: the same bits."""
+import ctypes
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -64,3 +66,46 @@ def test_host_multiply_from_several_threads(native_lib, cuda_device):
     for t in threads:
         t.join()
     assert not bad
+
+
+def _best(times, f):
+    """The shortest of several calls, in seconds: whoever else uses the host's cores only adds to it."""
+    best = float("inf")
+    for _ in range(times):
+        t0 = time.perf_counter()
+        f()
+        best = min(best, time.perf_counter() - t0)
+    return best
+
+
+def test_more_callers_than_kept_sets_make_no_staging(native_lib, cuda_device):
+    """Eight callers at once: six of them have a set for the one call, without the pinned memory that takes milliseconds to make and unmake."""
+    import torch
+
+    c = native_lib
+    K, N, M = 256, 64, 1
+    w, x, want_q, want = _case(c, torch, cuda_device, K, N, M)
+    calls, callers, bad = 40, 8, []
+
+    def call(q, y):  # (other Python threads run meanwhile)
+        return c.lib().jq_mat_mul_q4_0_q8_1_host(w.ctypes.data, x.ctypes.data, q.ctypes.data, y.ctypes.data, (ctypes.c_int * 4)(K, M, 1, 1), 4, N, K)
+
+    def work():
+        q, y = np.zeros_like(want_q), np.zeros_like(want)
+        for _ in range(calls):
+            q[:], y[:] = 0, 0
+            if call(q, y) != 0 or not (np.array_equal(q, want_q) and np.array_equal(y, want)):
+                bad.append(1)
+
+    def together():
+        threads = [threading.Thread(target=work) for _ in range(callers)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+
+    work()
+    alone = _best(20, lambda: call(np.zeros_like(want_q), np.zeros_like(want)))
+    assert not bad
+    # 45 us alone, 400 for a call of each of eight; with pinned memory for each call 5000
+    assert _best(3, together) / calls <= 40 * alone and not bad

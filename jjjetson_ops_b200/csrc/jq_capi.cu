@@ -798,10 +798,15 @@ struct HostLane {
         d_bytes = bytes;
         return JQ_OK;
     }
+    void release_buffer() {
+        if (d != nullptr) cudaFreeAsync(d, stream);
+        cudaStreamSynchronize(stream);
+        d = nullptr;
+        d_bytes = 0;
+    }
     ~HostLane() {
         if (stream != nullptr) {
-            if (d != nullptr) cudaFreeAsync(d, stream);
-            cudaStreamSynchronize(stream);
+            release_buffer();
             cudaStreamDestroy(stream);
         }
         for (cudaEvent_t e : sent)
@@ -849,8 +854,10 @@ class LaneLease {
     ~LaneLease() {
         if (lane_ == nullptr) return;
         if (lane_->kept) {
+            // of a large call's lane the device buffer alone is given back: making the pinned memory again takes longer than the call
+            if (lane_->d_bytes > LANE_KEPT_BYTES) lane_->release_buffer();
             std::lock_guard<std::mutex> lock(g_lanes_mutex);
-            if (finished_ && lane_->d_bytes <= LANE_KEPT_BYTES) {
+            if (finished_) {
                 try {
                     idle_lanes().push_back(lane_);
                     return;

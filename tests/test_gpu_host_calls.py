@@ -109,3 +109,21 @@ def test_more_callers_than_kept_sets_make_no_staging(native_lib, cuda_device):
     assert not bad
     # 45 us alone, 400 for a call of each of eight; with pinned memory for each call 5000
     assert _best(3, together) / calls <= 40 * alone and not bad
+
+
+def test_buffers_beyond_what_is_kept(native_lib, cuda_device):
+    """68 MB on the device, more than is kept: right, again and again, and without making the pinned memory anew each time."""
+    import torch
+
+    from jjjetson_ops_b200 import import_reference_modules
+
+    c, mmq = native_lib, import_reference_modules()[1].mmq
+    best = []
+    for K, N, M in ((8192, 14336, 1), (8192, 14800, 1)):
+        w, x, want_q, want = _case(c, torch, cuda_device, K, N, M)
+        for _ in range(3):
+            q, y = _call(mmq, c, w, x, K, N, M)
+            assert np.array_equal(q, want_q) and np.array_equal(y, want)
+        best.append(_best(10, lambda: _call(mmq, c, w, x, K, N, M)))
+    # 2.2 ms for 66 MB, 3.7 for 68, which are allocated and given back by each call; 17 with the pinned memory and the events
+    assert best[1] <= 4 * best[0]

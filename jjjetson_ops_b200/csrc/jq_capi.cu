@@ -259,6 +259,16 @@ void *mapped_alias(const void *host_ptr) {
     return attr.devicePointer;
 }
 
+// Memory that the driver has to stage when it copies it: neither page-locked nor its own.
+bool pageable(const void *host_ptr) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, host_ptr) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;
+    }
+    return attr.type == cudaMemoryTypeUnregistered;
+}
+
 // Coalesced copy, used to write a small result straight into mapped host memory: for tens of KB
 // one kernel is much quicker than a separate copy-engine transfer.
 // With a single block it can also publish a completion ticket in mapped host memory, which the
@@ -874,11 +884,11 @@ class LaneLease {
     bool finished_ = false;
 };
 
-// Host array of `bytes` -> device.  The driver takes pageable memory through a staging buffer of its own with one core (9.4 MB at
+// Host array of `bytes` -> device.  Page-locked memory is copied as it is.  The driver takes pageable memory through a staging buffer of its own with one core (9.4 MB at
 // 7 to 9 GB/s); here several threads copy chunks into the lane's and hand each to the copy engine as it is ready.
 int copy_in(HostLane &lane, void *dst, const void *src, size_t bytes) {
     if (bytes == 0) return JQ_OK;
-    if (lane.pinned == nullptr) {
+    if (lane.pinned == nullptr || !pageable(src)) {
         JQ_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, lane.stream));
         return JQ_OK;
     }
@@ -914,13 +924,13 @@ int copy_in(HostLane &lane, void *dst, const void *src, size_t bytes) {
     return JQ_OK;
 }
 
-// Results -> host arrays: through the lane's pinned buffer while they fit, so that several of them cost one wait.
+// Results -> host arrays: pageable ones through the lane's pinned buffer while they fit, so that several of them cost one wait.
 class HostResults {
   public:
     explicit HostResults(HostLane &lane) : lane_(lane) {}
     int fetch(void *dst, const void *src, size_t bytes) {
         if (bytes == 0) return JQ_OK;
-        if (lane_.pinned != nullptr && n_ < 2 && at_ + bytes <= RESULT_BYTES) {
+        if (lane_.pinned != nullptr && n_ < 2 && at_ + bytes <= RESULT_BYTES && pageable(dst)) {
             uint8_t *const p = lane_.pinned + STAGE_BYTES + at_;
             JQ_CUDA_TRY(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, lane_.stream));
             copies_[n_++] = Copy{dst, p, bytes};

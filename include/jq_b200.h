@@ -338,8 +338,9 @@ int jq_mat_mul_q4_0_q8_1_host_ex(const void *weight_q4_0, const float *input, ui
                                  float *output, const int *input_dims, int ndims, int nrows_out,
                                  int ncols_k, int s_mode);
 
-/* The host wrappers above keep what they need on the device and in pinned memory from one call to the next: at most two idle sets
- * per device, each of at most 64 MB on the device and 18 MB pinned.  This gives the idle ones back. */
+/* The host wrappers above keep what they need on the device and in pinned memory from one call to the next: at most two sets per
+ * device, each of at most 64 MB on the device and 18 MB pinned, in the device's primary context only.  This gives the idle ones
+ * back. */
 int jq_release_host_scratch(void);
 
 /* Weights kept resident on the current device, for callers that run many multiplies. */

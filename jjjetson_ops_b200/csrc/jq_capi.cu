@@ -9,7 +9,10 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
+
+#include <cuda.h>
 
 #include "jq_common.cuh"
 
@@ -768,10 +771,91 @@ int jq_debug_set_extent_shrink(unsigned long long bytes) {
 
 namespace {
 
+// The driver's context calls, looked up through the runtime, which has none of its own.
+struct ContextCalls {
+    CUresult (*current)(CUcontext *) = nullptr;
+    CUresult (*device)(CUdevice *) = nullptr;
+    CUresult (*id)(CUcontext, unsigned long long *) = nullptr;
+    CUresult (*primary_state)(CUdevice, unsigned *, int *) = nullptr;
+    CUresult (*primary_retain)(CUcontext *, CUdevice) = nullptr;
+    CUresult (*primary_release)(CUdevice) = nullptr;
+    CUresult (*push)(CUcontext) = nullptr;
+    CUresult (*pop)(CUcontext *) = nullptr;
+    bool found = false;
+};
+const ContextCalls &context_calls() {
+    static const ContextCalls calls = [] {
+        ContextCalls c;
+        c.found = true;
+        const auto find = [&](const char *name, auto *fn) {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+            if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) {
+                (void)cudaGetLastError();
+                c.found = false;
+            } else {
+                *fn = reinterpret_cast<std::remove_pointer_t<decltype(fn)>>(f);
+            }
+        };
+        find("cuCtxGetCurrent", &c.current);
+        find("cuCtxGetDevice", &c.device);
+        find("cuCtxGetId", &c.id);
+        find("cuDevicePrimaryCtxGetState", &c.primary_state);
+        find("cuDevicePrimaryCtxRetain", &c.primary_retain);
+        find("cuDevicePrimaryCtxRelease", &c.primary_release);
+        find("cuCtxPushCurrent", &c.push);
+        find("cuCtxPopCurrent", &c.pop);
+        return c;
+    }();
+    return calls;
+}
+// A device's primary context, if there is one now (id 0: there is none), alive as long as this object.  A device that was reset has
+// another one, with another id.
+struct PrimaryContext {
+    CUdevice device;
+    CUcontext context = nullptr;
+    unsigned long long id = 0;
+    explicit PrimaryContext(CUdevice d) : device(d) {
+        const ContextCalls &cu = context_calls();
+        unsigned flags = 0;
+        int active = 0;
+        if (cu.primary_state(device, &flags, &active) != CUDA_SUCCESS || !active || cu.primary_retain(&context, device) != CUDA_SUCCESS)
+            context = nullptr;
+        else if (cu.id(context, &id) != CUDA_SUCCESS)
+            id = 0;
+    }
+    PrimaryContext(const PrimaryContext &) = delete;
+    ~PrimaryContext() {
+        if (context != nullptr) context_calls().primary_release(device);
+    }
+};
+// What the calling thread works on.
+struct HostContext {
+    int device = 0;
+    CUdevice cu_device = 0;
+    unsigned long long primary = 0;  // id of the device's primary context, 0 if the thread works in another one
+    int find() {
+        JQ_CUDA_TRY(cudaGetDevice(&device));
+        if (device < 0 || device >= MAX_DEVICES) return set_error(JQ_ERR_UNSUPPORTED, "device index %d out of range", device);
+        const ContextCalls &cu = context_calls();
+        if (!cu.found) return JQ_OK;
+        CUcontext here = nullptr;
+        if (cu.current(&here) != CUDA_SUCCESS || here == nullptr) {  // the thread's first call: what the runtime would do by itself
+            JQ_CUDA_TRY(cudaSetDevice(device));
+            if (cu.current(&here) != CUDA_SUCCESS || here == nullptr) return JQ_OK;
+        }
+        if (cu.device(&cu_device) != CUDA_SUCCESS) return JQ_OK;
+        const PrimaryContext p(cu_device);
+        if (p.context == here) primary = p.id;
+        return JQ_OK;
+    }
+};
+
 // What a host call needs on the device and in pinned memory: a stream, one device buffer and a staging buffer.  Each call has such a
 // lane to itself while it runs.  LANES_KEPT of at most LANE_KEPT_BYTES are kept per device between calls, because making them costs
 // more than a small call's own work (jq_release_host_scratch gives the idle ones back).  Further calls at the same time get one
-// without a staging buffer, which would take longer to make than it saves, and so does a call that cannot have one.
+// without a staging buffer, which would take longer to make than it saves, and so does a call that cannot have one and a call in another
+// context than the device's primary one: nothing tells the library when such a context ends.
 inline size_t whole_lines(size_t bytes) { return (bytes + 255) / 256 * 256; }
 constexpr size_t STAGE_CHUNK = (size_t)512 << 10, STAGE_SLOTS = 32, STAGE_BYTES = STAGE_CHUNK * STAGE_SLOTS;
 constexpr size_t RESULT_BYTES = (size_t)2 << 20;
@@ -781,6 +865,8 @@ static_assert(STAGE_SLOTS % MAX_COPY_THREADS == 0, "a thread meets its own chunk
 struct HostLane {
     int device = 0;
     bool kept = false;              // one of the device's LANES_KEPT
+    CUdevice cu_device = 0;         // (kept lanes) the device's primary context
+    unsigned long long context = 0;
     cudaStream_t stream = nullptr;
     uint8_t *d = nullptr;
     size_t d_bytes = 0;
@@ -814,6 +900,12 @@ struct HostLane {
         d = nullptr;
         d_bytes = 0;
     }
+    // its context has gone, and all of it with it
+    void forget() {
+        stream = nullptr;
+        d = pinned = nullptr;
+        std::fill(sent, sent + STAGE_SLOTS, nullptr);
+    }
     ~HostLane() {
         if (stream != nullptr) {
             release_buffer();
@@ -835,25 +927,34 @@ std::vector<HostLane *> &idle_lanes() {  // never destroyed: no CUDA call may ru
 class LaneLease {
   public:
     int open() {
-        int dev = 0;
-        JQ_CUDA_TRY(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= MAX_DEVICES) return set_error(JQ_ERR_UNSUPPORTED, "device index %d out of range", dev);
+        HostContext here;
+        if (int rc = here.find()) return rc;
         {
             std::lock_guard<std::mutex> lock(g_lanes_mutex);
             std::vector<HostLane *> &idle = idle_lanes();
-            for (size_t i = 0; i < idle.size(); ++i) {
-                if (idle[i]->device == dev) {
-                    lane_ = idle[i];
-                    idle.erase(idle.begin() + (ptrdiff_t)i);
+            for (size_t i = 0; here.primary != 0 && i < idle.size();) {
+                HostLane *const l = idle[i];
+                if (l->device != here.device) {
+                    ++i;
+                    continue;
+                }
+                idle.erase(idle.begin() + (ptrdiff_t)i);
+                if (l->context == here.primary) {
+                    lane_ = l;
                     std::fill(lane_->in_use, lane_->in_use + STAGE_SLOTS, false);
                     return JQ_OK;
                 }
+                l->forget();
+                delete l;
+                --g_kept_lanes[here.device];
             }
             lane_ = new (std::nothrow) HostLane();
             if (lane_ == nullptr) return set_error(JQ_ERR_CUDA, "out of host memory");
-            lane_->device = dev;
-            lane_->kept = g_kept_lanes[dev] < LANES_KEPT;
-            g_kept_lanes[dev] += lane_->kept;
+            lane_->device = here.device;
+            lane_->cu_device = here.cu_device;
+            lane_->context = here.primary;
+            lane_->kept = here.primary != 0 && g_kept_lanes[here.device] < LANES_KEPT;
+            g_kept_lanes[here.device] += lane_->kept;
         }
         return lane_->open();
     }
@@ -967,7 +1068,14 @@ int jq_release_host_scratch(void) {
         lanes.swap(idle_lanes());
         for (const HostLane *l : lanes) --g_kept_lanes[l->device];
     }
-    for (HostLane *l : lanes) delete l;
+    for (HostLane *l : lanes) {
+        const PrimaryContext primary(l->cu_device);
+        if (primary.id != l->context) l->forget();
+        const bool pushed = primary.context != nullptr && context_calls().push(primary.context) == CUDA_SUCCESS;
+        delete l;
+        CUcontext popped = nullptr;
+        if (pushed) context_calls().pop(&popped);
+    }
     return JQ_OK;
 }
 

@@ -150,3 +150,66 @@ def test_page_locked_arrays_are_copied_as_they_are(native_lib, cuda_device):
     lw = locked(w)
     pageable, direct = (_best(40, lambda: _call(mmq, c, v, x, K, N, M)) for v in (w, lw))
     assert direct <= 0.7 * pageable  # 25 MB: 0.50 against 1.0 ms
+
+
+CONTEXTS_WORKER = r"""
+import ctypes, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np, torch
+from jjjetson_ops_b200 import capi as c
+from oracle import jq_oracle as O
+O.build()
+lib, cu = c.lib(), ctypes.CDLL("libcuda.so.1")
+rt = ctypes.CDLL([line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line][0])
+
+def quantize(seed, K=1024, M=3000):  # 12 MB in, 3.4 MB out
+    x = np.random.default_rng(seed).standard_normal((M, K), dtype=np.float32)
+    q = np.zeros(c.q8_1_bytes(K, M), np.uint8)
+    assert lib.jq_q8_1_host(x.ctypes.data, q.ctypes.data, (ctypes.c_int * 2)(K, M), 2) == 0, lib.jq_last_error()
+    assert np.array_equal(q, O.quantize_q8_1(x, O.ORDER_KSUPER_COL, O.S_SUM_X)), seed
+
+def multiply(K, N, M):
+    rng = np.random.default_rng(N)
+    w, x = O.quantize_q4_0(rng.standard_normal((N, K), dtype=np.float32)), rng.standard_normal((M, K), dtype=np.float32)
+    q, y = np.zeros(c.q8_1_bytes(K, M), np.uint8), np.zeros((M, N), np.float32)
+    assert lib.jq_mat_mul_q4_0_q8_1_host(w.ctypes.data, x.ctypes.data, q.ctypes.data, y.ctypes.data, (ctypes.c_int * 4)(K, M, 1, 1), 4, N, K) == 0
+    assert O.err_max_rel(y, O.mul_mat_ref(w, O.quantize_q8_1(x, O.ORDER_KSUPER_COL, O.S_SUM_X), K, N, M, O.ORDER_KSUPER_COL)) <= 1e-5
+
+class Own:
+    def __enter__(self):
+        self.context = ctypes.c_void_p()
+        assert cu.cuInit(0) == 0 and cu.cuCtxCreate_v2(ctypes.byref(self.context), 0, 0) == 0
+    def __exit__(self, *_):
+        assert cu.cuCtxDestroy_v2(self.context) == 0
+
+with Own():
+    multiply(256, 64, 1)
+    multiply(4096, 2000, 1)
+    multiply(1408, 1003, 20)
+    quantize(1)
+quantize(2)
+with Own():
+    quantize(3)
+quantize(4)
+with Own():
+    assert lib.jq_release_host_scratch() == 0
+    quantize(5)
+quantize(6)
+assert rt.cudaDeviceReset() == 0
+quantize(7)
+quantize(8)
+assert rt.cudaDeviceReset() == 0 and lib.jq_release_host_scratch() == 0
+quantize(9)
+print("contexts ok")
+"""
+
+
+def test_host_calls_in_other_contexts(native_lib, cuda_device):
+    """Nothing is kept of a context of the caller's own, which may end unseen, nor used when the device has been reset."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", CONTEXTS_WORKER, root], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and "contexts ok" in done.stdout, done.stdout + done.stderr

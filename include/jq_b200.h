@@ -110,7 +110,11 @@ int jq_get_option(int option, int *value_out);
  * The tcgen05 GEMM uses its slice differently: SM clock stamps of CTA (0,0) for the first 128
  * blocks of K, four groups of 128 rows x 8 columns (accumulator seen complete / previous block
  * accumulated / buffer handed back, one column per drain warp; then MMA issue time in column 0
- * and stage publication per producer warp in columns 1-3). */
+ * and stage publication per producer warp in columns 1-3).  The fp16-operand GEMM stamps SM clocks
+ * of its first CTA for the first 64 stages: rows 0-63 the first weight warp, rows 64-127 the first
+ * activation warp (the stages that the first producer group converts; columns: loop top, raw bytes
+ * landed, -, operand stage free, converted, published), rows 128-191 the MMA thread (stage seen
+ * full, MMAs and commit issued). */
 int jq_trace_enable(void *d_buf, int64_t n_launches);
 
 const char *jq_status_string(int status);

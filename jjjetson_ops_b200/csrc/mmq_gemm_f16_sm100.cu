@@ -197,7 +197,13 @@ struct HfParams {
     // [z * chunks_per_split, ...) each; their partial tiles meet in shared memory.
     int k_splits, chunks_per_split;
     int static_weights;  // the weight copies may start before the previous kernel in the stream has finished
+    unsigned long long *trace;  // tracing aid (or nullptr): SM clock stamps of the first CTA, rows of 8
 };
+// TRACE: an instance of its own, so that the others have neither the test nor the registers
+template <bool TRACE>
+__device__ __forceinline__ void hf_stamp(const HfParams &p, int who, int c, int slot) {
+    if (TRACE && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && c < 64) p.trace[(who * 64 + c) * 8 + slot] = (unsigned long long)clock64();
+}
 
 __device__ __forceinline__ void sts_v2(uint32_t addr, uint32_t a, uint32_t b) {
     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
@@ -260,7 +266,7 @@ __device__ __forceinline__ int hf_matrix(const HfMats<MATS> &mats) {
     return mat;
 }
 
-template <bool PAIR, bool SPLIT, int MATS>
+template <bool PAIR, bool SPLIT, int MATS, bool TRACE = false>
 __global__ void __launch_bounds__(HF_THREADS, 1)
 gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS> mats) {
     using T = HfTile<PAIR>;
@@ -334,8 +340,11 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
             for (int c = warp >> 2; c < n_chunks; c += HF_GROUPS) {
                 const int s = c % NS, ws = (c >> 1) % HF_W_SLOTS;
                 const uint32_t round = (uint32_t)(c / NS);
+                const bool stamps = TRACE && tid == 0;
+                if (stamps) hf_stamp<TRACE>(p, 0, c, 0);
                 alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&w_full[ws], (uint32_t)((c >> 1) / HF_W_SLOTS) & 1u, p.fault)) != 0;
                 if (!alive) break;
+                if (stamps) hf_stamp<TRACE>(p, 0, c, 1);
                 uint32_t ww[18];
                 load_q4_chunk(ww, sbase + HF_W_OFF + ws * HF_W_SLOT_BYTES + (uint32_t)((gw * 32 + lane) * Q8_BYTES), (c & 1) != 0);
                 __syncwarp();
@@ -346,6 +355,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                     alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&stage_empty[s], (round - 1) & 1u, p.fault)) != 0;
                     if (!alive) break;
                 }
+                if (stamps) hf_stamp<TRACE>(p, 0, c, 3);
                 tc_fence_after();
                 const uint32_t a = lanes + T::A_COL + (uint32_t)s * HF_A_COLS;
                 tmem_st32_nowait(a, o);
@@ -357,6 +367,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                 tmem_st2_nowait(zt + 2 * (c & 3), as_u32(__hmul2(as_h2(z0), m8)), as_u32(__hmul2(as_h2(z1), m8)));
                 if (c == n_chunks - 1 && (c & 3) == 1) tmem_st4_nowait(zt + 4, 0u, 0u, 0u, 0u);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                if (stamps) hf_stamp<TRACE>(p, 0, c, 4);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
@@ -365,6 +376,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                     else
                         mbar_arrive(&stage_full[s]);
                 }
+                if (stamps) hf_stamp<TRACE>(p, 0, c, 5);
             }
         } else {
             // =============================== activations -> shared memory =====================
@@ -374,8 +386,11 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
             for (int c = xw >> 2; c < n_chunks; c += HF_GROUPS) {
                 const int s = c % NS, rs = c % HF_RAW_SLOTS;
                 const uint32_t round = (uint32_t)(c / NS);
+                const bool stamps = TRACE && tid == HF_W_WARPS * 32;
+                if (stamps) hf_stamp<TRACE>(p, 1, c, 0);
                 alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&x_full[rs], (uint32_t)(c / HF_RAW_SLOTS) & 1u, p.fault)) != 0;
                 if (!alive) break;
+                if (stamps) hf_stamp<TRACE>(p, 1, c, 1);
                 uint4 v[9];
                 const uint32_t raw = sbase + HF_RAW_OFF + rs * HF_RAW_BYTES + (uint32_t)(row * Q8_BYTES);
 #pragma unroll
@@ -386,6 +401,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                     alive = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&stage_empty[s], (round - 1) & 1u, p.fault)) != 0;
                     if (!alive) break;
                 }
+                if (stamps) hf_stamp<TRACE>(p, 1, c, 3);
                 const uint32_t at = sbase + s * HF_X_BYTES + (uint32_t)(row * 128 + ((row & 7) << 4));
                 const float r0 = convert_activation_block(v[1], v[2], v[0].x, at, 0);
                 const float r1 = convert_activation_block(v[3], v[4], v[0].y, at, 4);
@@ -395,6 +411,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                 const uint32_t zx = sbase + HF_Z_OFF + ((c >> 2) & 1) * HF_Z_BYTES + tile_off(row, 0);
                 sts_v2(zx + ((c & 2) >> 1) * TC_LBO + (c & 1) * 8, as_u32(__floats2half2_rn(r0, r1)), as_u32(__floats2half2_rn(r2, r3)));
                 if (c == n_chunks - 1 && (c & 3) == 1) sts_v4(zx + TC_LBO, make_uint4(0u, 0u, 0u, 0u));
+                if (stamps) hf_stamp<TRACE>(p, 1, c, 4);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // tiles are read by the tensor core
                 __syncwarp();
                 if (lane == 0) {
@@ -403,6 +420,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                     else
                         mbar_arrive(&stage_full[s]);
                 }
+                if (stamps) hf_stamp<TRACE>(p, 1, c, 5);
             }
         }
 
@@ -475,6 +493,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                 alive = false;
                 break;
             }
+            hf_stamp<TRACE>(p, 2, c, 0);
             tc_fence_after();
             const uint32_t a = tmem + T::A_COL + (uint32_t)s * HF_A_COLS, x = sbase + s * HF_X_BYTES;
 #pragma unroll
@@ -499,6 +518,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
                 tc_commit_pair(&stage_empty[s]);
             else
                 tc_commit(&stage_empty[s]);
+            hf_stamp<TRACE>(p, 2, c, 1);
         }
         if (alive) {
             if (PAIR)
@@ -562,7 +582,7 @@ gemm_q4_0_q8_1_f16_kernel(const HfParams p, const __grid_constant__ HfMats<MATS>
 
 template <bool PAIR, bool SPLIT, int MATS>
 int launch_kernel(cudaStream_t st, dim3 grid, const HfParams &p, const HfMats<MATS> &mats) {
-    const auto kernel = gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, MATS>;
+    const auto kernel = p.trace != nullptr ? gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, MATS, true> : gemm_q4_0_q8_1_f16_kernel<PAIR, SPLIT, MATS>;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), HF_SMEM_BYTES)) return rc;
     (void)cudaGetLastError();  // a stale error of an earlier, unrelated call must not be taken for this launch's
     cudaLaunchConfig_t cfg = {};
@@ -677,6 +697,7 @@ int launch_gemm_f16(cudaStream_t st, const void *d_w, const void *d_xq, float *d
     p.n_chunks = (int)(K / SUPER);
     p.order = order;
     p.static_weights = option_value(JQ_OPT_STATIC_WEIGHTS) != 0 ? 1 : 0;
+    p.trace = static_cast<unsigned long long *>(next_trace_slot());
     GemmF16Widths width;
     if (int rc = form_widths(caps, &width)) return rc;
     const GemmF16Plan plan = plan_gemm_f16(p.n_chunks, gx * gy, pair_gx / 2 * pair_gy, width);

@@ -216,3 +216,30 @@ def test_gemm_f16_first_call_in_a_capture(env):
     assert gemm_f16_form(2048, [2048], 128) == 4 and gemm_f16_form(256, [18690], 130) == "pair"
     r = subprocess.run([sys.executable, "-c", FIRST_CALL], capture_output=True, text=True, cwd=ROOT, timeout=300)
     assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("K,rows,M", [(4096, [4096], 512), (4096, [1024], 64), (8192, [8192], 1024), (1024, [512, 128, 128], 100)])
+def test_trace_stamps_of_a_launch_are_ordered(env, K, rows, M):
+    """jq_trace_enable: single CTAs, a split K, pairs, several matrices.  Each of the first stages has its stamps in order, and the next
+    launch none."""
+    c, t = env.c, env.t
+    x = t.randn((M, K), device=env.dev)
+    ws = [c.quantize_q4_0(t.randn((n, K), device=env.dev)) for n in rows]
+    want = c.linear_q4_0_multi(ws, rows, x=x)
+    xq = c.quantize_q8_1(x, c.ORDER_COL_KSUPER, c.S_D_SUM_Q)
+    buf = t.zeros((2, 512, 8), dtype=t.int64, device=env.dev)
+    t.cuda.synchronize()
+    c.check(c.lib().jq_trace_enable(buf.data_ptr(), 1))
+    got = [c.linear_q4_0_multi(ws, rows, xq=xq, K=K, M=M) for _ in range(2)]
+    c.check(c.lib().jq_trace_enable(None, 0))
+    t.cuda.synchronize()
+    assert all(t.equal(a, b) for g in got for a, b in zip(g, want))
+    stamps = buf.cpu().numpy()
+    assert not stamps[1].any()
+    weights, activations, mma = stamps[0, :64], stamps[0, 64:128], stamps[0, 128:192]
+    n = int((mma[:, 0] != 0).sum())  # the first CTA's stages
+    assert n >= 2 and (mma[:n, :2] != 0).all() and (np.diff(mma[:n, :2].reshape(-1)) >= 0).all()
+    for who in (weights, activations):
+        own = [i for i in range(64) if who[i].any()]
+        assert own == list(range(0, n, 3))
+        assert (np.diff(who[own][:, [0, 1, 3, 4, 5]].reshape(-1)) >= 0).all() and (who[own, 4] <= mma[own, 0]).all()  # converted before it is seen

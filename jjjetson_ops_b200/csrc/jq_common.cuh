@@ -309,6 +309,28 @@ __device__ __forceinline__ void mma_u8s8_16832(int (&d)[4], const uint32_t (&a)[
           "r"(c[2]), "r"(c[3]));
 }
 
+// Two fp32 operations at a time.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<uint64_t &>(d))
+        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t &>(d))
+        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)),
+          "l"(reinterpret_cast<const uint64_t &>(c)));
+    return d;
+}
+
+// An integer sum that starts from MAGIC_I, the bit pattern of 1.5 * 2^23, reads as a float, and less MAGIC_F is the sum exactly (up to
+// 2^22; a conversion instruction runs at half the rate).
+constexpr int MAGIC_I = 0x4B400000;
+constexpr float MAGIC_F = 12582912.0f;
+
 // One 32-value group of the activation quantizer, as 8 lanes x 4 floats, following
 // quantize_q8_1_kernel (src/cuda/q8_1.cu:55-79,101-103) operation by operation so that the int8
 // values, fp16 d and fp16 sum come out bit-identical: max and sum by xor butterflies with

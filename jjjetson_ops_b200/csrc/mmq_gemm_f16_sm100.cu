@@ -6,9 +6,9 @@
 // batches.  The reference adds, per 32-wide block, d4 * (sumi * d8 - 8 * s8) (mm_q4_0_q8_1.cu:92).
 // With sumi = sum(q4 * q8) that is
 //     sum_i ((q4_i - 8) * d4) * (q8_i * d8)   +   (-8 * d4) * (s8 - d8 * sum_i q8_i)
-// The first term is a plain product of two fp16 matrices B[n][k] = (q4 - 8) * d4 and
-// A[m][k] = q8 * d8; the second is rank one per block and joins the same accumulator as one more
-// MMA per 128 values of K (operands s8 - d8 * sum(q8), computed in fp32, and -8 * d4, exact).  It
+// The first term is a plain product of two fp16 matrices A[n][k] = (q4 - 8) * d4 and
+// B[m][k] = q8 * d8; the second is rank one per block and joins the same accumulator as one more
+// MMA per 512 values of K (operands -8 * d4, exact, and s8 - d8 * sum(q8), computed in fp32).  It
 // vanishes up to the rounding of s8 when the quantizer stored s = d * sum(q), and carries the
 // quantisation residue when it stored the sum of the unquantised values.
 //
@@ -213,6 +213,51 @@ __device__ __forceinline__ void tmem_st2_nowait(uint32_t taddr, uint32_t a, uint
 }
 __device__ __forceinline__ void tmem_st4_nowait(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// A weight row's 72 bytes of a 128-value chunk from a raw slot, where two chunks of 128 rows lie 144 bytes apart: four 16-byte
+// words (conflict-free at that pitch) and one of 8, which comes last in an even chunk and first in an odd one.
+__device__ __forceinline__ void load_q4_chunk(uint32_t (&ww)[18], uint32_t raw, bool odd) {
+    if (!odd) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 v = lds_v4(raw + 16 * i);
+            ww[4 * i] = v.x;
+            ww[4 * i + 1] = v.y;
+            ww[4 * i + 2] = v.z;
+            ww[4 * i + 3] = v.w;
+        }
+        const uint2 e = lds_v2(raw + 64);
+        ww[16] = e.x;
+        ww[17] = e.y;
+    } else {
+        const uint2 e = lds_v2(raw + 72);
+        ww[0] = e.x;
+        ww[1] = e.y;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 v = lds_v4(raw + 80 + 16 * i);
+            ww[2 + 4 * i] = v.x;
+            ww[3 + 4 * i] = v.y;
+            ww[4 + 4 * i] = v.z;
+            ww[5 + 4 * i] = v.w;
+        }
+    }
+}
+
+// The sixteen quant bytes and the scale of block j of a 72-byte chunk
+__device__ __forceinline__ void q4_chunk_block(const uint32_t (&ww)[18], int j, uint32_t (&q)[4], uint32_t *dbits) {
+    if ((j & 1) == 0) {  // starts on a word boundary: [d | q0 q1] [q2..q5] ...
+        const int w0 = (j / 2) * 9;
+        *dbits = ww[w0] & 0xFFFFu;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) q[t] = __funnelshift_r(ww[w0 + t], ww[w0 + t + 1], 16);
+    } else {  // starts in the middle of a word
+        const int w0 = (j / 2) * 9 + 4;
+        *dbits = ww[w0] >> 16;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) q[t] = ww[w0 + 1 + t];
+    }
 }
 
 // Two blocks (64 values of K) of one weight row -> 32 words (q4 - 8) * d4: (values, of word t) 4t, 4t + 2 | 4t + 16, 4t + 18 |

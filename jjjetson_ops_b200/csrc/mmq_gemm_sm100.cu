@@ -50,8 +50,6 @@ struct GemmTile {
     static constexpr int MIN_CTAS = SMEM <= 100 * 1024 ? 2 : 1;
 };
 constexpr uint32_t MASK4 = 0x0F0F0F0Fu;
-constexpr int MAGIC_I = 0x4B400000;        // bit pattern of 1.5 * 2^23
-constexpr float MAGIC_F = 12582912.0f;
 
 __device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void *gmem_src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gmem_src) : "memory");
@@ -60,16 +58,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// d = a * b + c on two packed floats
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t &>(d))
-        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)),
-          "l"(reinterpret_cast<const uint64_t &>(c)));
-    return d;
 }
 
 // D(16x8, f32) += A(16x8, f16 row) * B(8x8, f16 col)
@@ -218,15 +206,15 @@ __global__ void __launch_bounds__(GM_THREADS, GemmTile<RT, CT>::MIN_CTAS) gemm_q
                 for (int j = 0; j < CT; ++j) {
                     int c4[4];
                     mma_u8s8_16832(c4, a_e, be[j], magic4);
-                    float2 lo = ffma2(make_float2(__int_as_float(c4[0]), __int_as_float(c4[1])), de[j], ce[j]);
-                    float2 hi = ffma2(make_float2(__int_as_float(c4[2]), __int_as_float(c4[3])), de[j], ce[j]);
-                    float2 a01 = ffma2(make_float2(d4e[0], d4e[0]), lo, make_float2(acc[i][j][0], acc[i][j][1]));
-                    float2 a23 = ffma2(make_float2(d4e[1], d4e[1]), hi, make_float2(acc[i][j][2], acc[i][j][3]));
+                    float2 lo = fma2(make_float2(__int_as_float(c4[0]), __int_as_float(c4[1])), de[j], ce[j]);
+                    float2 hi = fma2(make_float2(__int_as_float(c4[2]), __int_as_float(c4[3])), de[j], ce[j]);
+                    float2 a01 = fma2(make_float2(d4e[0], d4e[0]), lo, make_float2(acc[i][j][0], acc[i][j][1]));
+                    float2 a23 = fma2(make_float2(d4e[1], d4e[1]), hi, make_float2(acc[i][j][2], acc[i][j][3]));
                     mma_u8s8_16832(c4, a_o, bo[j], magic4);
-                    lo = ffma2(make_float2(__int_as_float(c4[0]), __int_as_float(c4[1])), d_o[j], co[j]);
-                    hi = ffma2(make_float2(__int_as_float(c4[2]), __int_as_float(c4[3])), d_o[j], co[j]);
-                    a01 = ffma2(make_float2(d4o[0], d4o[0]), lo, a01);
-                    a23 = ffma2(make_float2(d4o[1], d4o[1]), hi, a23);
+                    lo = fma2(make_float2(__int_as_float(c4[0]), __int_as_float(c4[1])), d_o[j], co[j]);
+                    hi = fma2(make_float2(__int_as_float(c4[2]), __int_as_float(c4[3])), d_o[j], co[j]);
+                    a01 = fma2(make_float2(d4o[0], d4o[0]), lo, a01);
+                    a23 = fma2(make_float2(d4o[1], d4o[1]), hi, a23);
                     acc[i][j][0] = a01.x;
                     acc[i][j][1] = a01.y;
                     acc[i][j][2] = a23.x;

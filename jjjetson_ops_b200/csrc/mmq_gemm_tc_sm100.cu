@@ -129,15 +129,6 @@ __device__ __forceinline__ void tc_stamp(const TcParams &p, int g, int kind, int
     }
 }
 
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t &>(d))
-        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)),
-          "l"(reinterpret_cast<const uint64_t &>(c)));
-    return d;
-}
-
 __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -306,8 +297,8 @@ gemm_q4_0_q8_1_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap w
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int e = hq * 4 + q;
-                    acc[2 * e] = ffma2(make_float2(__uint_as_float(d4[q].x), __uint_as_float(d4[q].y)), u[2 * e], acc[2 * e]);
-                    acc[2 * e + 1] = ffma2(make_float2(__uint_as_float(d4[q].z), __uint_as_float(d4[q].w)), u[2 * e + 1], acc[2 * e + 1]);
+                    acc[2 * e] = fma2(make_float2(__uint_as_float(d4[q].x), __uint_as_float(d4[q].y)), u[2 * e], acc[2 * e]);
+                    acc[2 * e + 1] = fma2(make_float2(__uint_as_float(d4[q].z), __uint_as_float(d4[q].w)), u[2 * e + 1], acc[2 * e + 1]);
                 }
             }
             if (kb == 0 && c > 0) {  // the previous stage's tables are no longer needed, nor its tiles
@@ -322,8 +313,8 @@ gemm_q4_0_q8_1_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap w
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
-                u[q] = ffma2(make_float2(__uint_as_float(v0[2 * q]), __uint_as_float(v0[2 * q + 1])), d8p, c8p);
-                u[16 + q] = ffma2(make_float2(__uint_as_float(v1[2 * q]), __uint_as_float(v1[2 * q + 1])), d8p, c8p);
+                u[q] = fma2(make_float2(__uint_as_float(v0[2 * q]), __uint_as_float(v0[2 * q + 1])), d8p, c8p);
+                u[16 + q] = fma2(make_float2(__uint_as_float(v1[2 * q]), __uint_as_float(v1[2 * q + 1])), d8p, c8p);
             }
             tc_fence_before();
             __syncwarp();
@@ -337,8 +328,8 @@ gemm_q4_0_q8_1_tc_kernel(const TcParams p, const __grid_constant__ CUtensorMap w
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
                 const uint4 d4 = lds_v4(d4_prev + e * 16);
-                acc[2 * e] = ffma2(make_float2(__uint_as_float(d4.x), __uint_as_float(d4.y)), u[2 * e], acc[2 * e]);
-                acc[2 * e + 1] = ffma2(make_float2(__uint_as_float(d4.z), __uint_as_float(d4.w)), u[2 * e + 1], acc[2 * e + 1]);
+                acc[2 * e] = fma2(make_float2(__uint_as_float(d4.x), __uint_as_float(d4.y)), u[2 * e], acc[2 * e]);
+                acc[2 * e + 1] = fma2(make_float2(__uint_as_float(d4.z), __uint_as_float(d4.w)), u[2 * e + 1], acc[2 * e + 1]);
             }
             // zero-point term: complete, because its MMAs were issued before the last block's, which has been seen
             tc_fence_after();

@@ -30,8 +30,6 @@ constexpr int GV_BAR_BYTES = 256;  // full[8] + empty[8] ring mbarriers, red_ful
 constexpr int GV_RED_SLOTS = 4;
 constexpr int GV_PREVIOUS_ENDED = 29;  // (8-byte slot of the barrier block) non-zero: the preceding kernel has ended
 constexpr uint32_t MASK4 = 0x0F0F0F0Fu;
-constexpr int GV_MAGIC_I = 0x4B400000;  // bit pattern of 1.5 * 2^23: an integer sum added to it reads as a float, less 1.5 * 2^23, exactly
-constexpr float GV_MAGIC_F = 12582912.0f;
 
 constexpr int GV_MAX_MATS = 4;
 
@@ -943,22 +941,6 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
 // its high nibbles weights 16+4t.. (a2/a3) -- exactly the k ranges the fragment layout asks of it.
 // Partial fp32 sums of the NW warps are added in a fixed order through shared memory.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("add.rn.f32x2 %0, %1, %2;"
-        : "=l"(reinterpret_cast<uint64_t &>(d))
-        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
-    return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t &>(d))
-        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)),
-          "l"(reinterpret_cast<const uint64_t &>(c)));
-    return d;
-}
-
 // Activations of the blocks [kb0, kb0 + KBW), from memory (READY) or from where they were staged: B fragments (column g) and scales
 // (columns 2t, 2t + 1); zeros for a block or a column that is not there.  Staged ones are read without a test, the last block or column
 // in place of one that is not there: with tests the shared-memory loads came one after the other, 1 us.  kb0 and KBW are multiples
@@ -1111,8 +1093,8 @@ __global__ void __launch_bounds__((NW + 2) * 32, 1) gemv_mma_kernel(const GemvPa
         load_fragments<KBW, false>(p, xs, kb0, g, t, xb0, xb1, xd0, xd1, xm0, xm1);
     }
 
-    const int magic4[4] = {GV_MAGIC_I, GV_MAGIC_I, GV_MAGIC_I, GV_MAGIC_I};
-    const float2 minus = make_float2(-GV_MAGIC_F, -GV_MAGIC_F);
+    const int magic4[4] = {MAGIC_I, MAGIC_I, MAGIC_I, MAGIC_I};
+    const float2 minus = make_float2(-MAGIC_F, -MAGIC_F);
 
     for (int c = 0; c < n_chunks; ++c) {
         const int s = c % p.stages;

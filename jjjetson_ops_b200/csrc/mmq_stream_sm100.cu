@@ -63,8 +63,6 @@ constexpr int SK_COLUMNS = 32;          // most columns a CTA takes, unless choo
 constexpr int SK_FLUSH = 4;             // stages per running sum
 constexpr int SK_SHORT_SUPERS = 16;     // K up to 2048: short running sums
 constexpr uint32_t SK_MASK4 = 0x0F0F0F0Fu;
-constexpr int SK_MAGIC_I = 0x4B400000;  // bit pattern of 1.5 * 2^23
-constexpr float SK_MAGIC_F = 12582912.0f;
 
 struct StreamMaps {
     CUtensorMap w[SK_MAX_MATS];
@@ -110,13 +108,6 @@ struct StreamTile {
     static_assert(ROWS / 2 * SK_PITCH % 128 == 0, "tensor copies land on 128-byte boundaries");
 };
 
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("add.rn.f32x2 %0, %1, %2;"
-        : "=l"(reinterpret_cast<uint64_t &>(d))
-        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
-    return d;
-}
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 d;
     asm("mul.rn.f32x2 %0, %1, %2;"
@@ -124,15 +115,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
         : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)));
     return d;
 }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t &>(d))
-        : "l"(reinterpret_cast<const uint64_t &>(a)), "l"(reinterpret_cast<const uint64_t &>(b)),
-          "l"(reinterpret_cast<const uint64_t &>(c)));
-    return d;
-}
-
 // Sums of the warps' parts, in an order that is always the same: one after the other, as a tree, or with what each addition
 // rounds off added up as well (Knuth's two-sum), so that only the result is rounded.
 template <int N>
@@ -165,8 +147,8 @@ __device__ __forceinline__ float sum_compensated(const float (&v)[N]) {
 
 // sumi * d8 - 8 * s8 of one block for the rows g and g + 8 and two columns
 __device__ __forceinline__ void block_terms(float2 (&t)[2], const uint32_t (&a)[4], const uint32_t (&b)[2], float2 d8, float2 m8s) {
-    const int magic4[4] = {SK_MAGIC_I, SK_MAGIC_I, SK_MAGIC_I, SK_MAGIC_I};
-    const float2 minus = make_float2(-SK_MAGIC_F, -SK_MAGIC_F);
+    const int magic4[4] = {MAGIC_I, MAGIC_I, MAGIC_I, MAGIC_I};
+    const float2 minus = make_float2(-MAGIC_F, -MAGIC_F);
     int c[4];
     mma_u8s8_16832(c, a, b, magic4);
     t[0] = fma2(add2(make_float2(__int_as_float(c[0]), __int_as_float(c[1])), minus), d8, m8s);  // the sum is exact
@@ -436,8 +418,9 @@ struct StreamShape {
 // does not depend on how rows and columns are dealt out beyond that.
 //
 // 33 to 63 columns are two groups, unless one CTA of all columns makes one wave of what otherwise is more: K = 4096, N = 11008 (115 CTAs of
-// 96 rows instead of 2 x 172 of 64) M = 40 24.7 -> 18.8 us, M = 48 24.9 -> 22.4, M = 60 30.9 -> 29.0.  With 128 rows six column tiles
-// fit into the registers: N = 18944, M = 36 33.5 -> 25.2 us, M = 48 32.5 -> 31.2; the other side, M = 60, 40.4 in two groups, 59.6 in one.
+// 96 rows instead of 2 x 172 of 64) M = 40 24.7 -> 18.8 us, M = 48 24.9 -> 22.4, M = 60 30.9 -> 29.0.  With 128 rows the limit
+// is six column tiles, for which the registers lack 44 bytes a thread (96 rows, seven or eight tiles: 56): N = 18944, M = 36 33.5 -> 25.2
+// us, M = 48 32.5 -> 31.2; the other side, M = 60, 40.4 in two groups, 59.6 in one.
 //
 // Up to 4096 values of K the sixteen warps of a CTA of 64 rows have little to do before their sums meet, and with 32 columns many
 // sums: K = 1792, M = 28, N = 4800 (150 tiles of 32 rows) 6.9 us in CTAs of 32 rows, 7.2 in 64; K = 512 3.8 / 4.1; with 12 columns N = 4800

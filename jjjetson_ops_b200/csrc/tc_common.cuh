@@ -112,15 +112,6 @@ __device__ __forceinline__ void tmem_st32_nowait(uint32_t taddr, const uint32_t 
         : "memory");
 }
 
-// D(fp32, TMEM) (+)= A(fp16 tile) x B(fp16 tile)^T, K = 16
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
 // All tensor-core operations this thread has issued so far arrive on the mbarrier when they complete.
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -152,52 +143,6 @@ __device__ __forceinline__ float lds_f32_of(uint32_t addr, int rank) {
 __device__ __forceinline__ void cluster_sync() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-
-// A weight row's 72 bytes of a 128-value chunk from a raw slot, where two chunks of 128 rows lie 144 bytes apart: four 16-byte
-// words (conflict-free at that pitch) and one of 8, which comes last in an even chunk and first in an odd one.
-__device__ __forceinline__ void load_q4_chunk(uint32_t (&ww)[18], uint32_t raw, bool odd) {
-    if (!odd) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 v = lds_v4(raw + 16 * i);
-            ww[4 * i] = v.x;
-            ww[4 * i + 1] = v.y;
-            ww[4 * i + 2] = v.z;
-            ww[4 * i + 3] = v.w;
-        }
-        const uint2 e = lds_v2(raw + 64);
-        ww[16] = e.x;
-        ww[17] = e.y;
-    } else {
-        const uint2 e = lds_v2(raw + 72);
-        ww[0] = e.x;
-        ww[1] = e.y;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 v = lds_v4(raw + 80 + 16 * i);
-            ww[2 + 4 * i] = v.x;
-            ww[3 + 4 * i] = v.y;
-            ww[4 + 4 * i] = v.z;
-            ww[5 + 4 * i] = v.w;
-        }
-    }
-}
-
-// The sixteen quant bytes and the scale of block j of a 72-byte chunk
-__device__ __forceinline__ void q4_chunk_block(const uint32_t (&ww)[18], int j, uint32_t (&q)[4], uint32_t *dbits) {
-    if ((j & 1) == 0) {  // starts on a word boundary: [d | q0 q1] [q2..q5] ...
-        const int w0 = (j / 2) * 9;
-        *dbits = ww[w0] & 0xFFFFu;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) q[t] = __funnelshift_r(ww[w0 + t], ww[w0 + t + 1], 16);
-    } else {  // starts in the middle of a word
-        const int w0 = (j / 2) * 9 + 4;
-        *dbits = ww[w0] >> 16;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) q[t] = ww[w0 + 1 + t];
-    }
 }
 
 }  // namespace jq

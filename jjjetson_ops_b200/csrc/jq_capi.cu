@@ -212,11 +212,23 @@ inline bool small_batch_kernel_pays(int64_t K, int64_t N, int64_t M) {
 // 128: the integer GEMM needs them all to fill the SMs, and rounds off two to seven times as much.  Multiply alone, integer GEMM /
 // small-batch kernel: K = N = 4096, M = 64 25.9 / 12.7 us, M = 256 45.8 / 39.8, M = 512 (128 tiles) 69.0 / 67.9; K = 4096, N = 11008, M = 256
 // (172) 137 / 95 us; K = 9472, N = 502, M = 66 57.8 / 11.4; the other side: K = 2560, N = 6047, M = 684 (288) 89.8 / 93.3 us, K = 512, N = 25906,
-// M = 549 (1015) 78 / 103, and short K, where a CTA has little to do per column: K = 256, N = 1716, M = 547 (70) 5.4 / 6.8, N = 3138,
-// M = 139 (50) 4.9 / 3.8 us.
-inline bool small_batch_kernel_pays_exact(int64_t K, int64_t N, int64_t M) {
-    const int64_t tiles = ((N + 127) / 128) * ((M + 127) / 128);
-    return tiles <= 280 && tiles <= K / 4;
+// M = 549 (1015) 78 / 103.
+// One wave of it, two CTAs of 64 rows and up to 32 columns per SM, is always the quicker one.  Beyond, an estimate of both decides, by
+// half waves of the one and waves of the other (of tiles of 128 x 128, or of 64 x 64 where those would fill less than four fifths of
+// the SMs): the integer GEMM gains where its tiles are just one wave.  Nanoseconds, fitted to 157 shapes, K 256 to 11008, within 2 % on
+// average (10 % at most), and of 500 drawn shapes one is 7 % and one 2 % slower than with the other kernel; integer GEMM / small-batch kernel, us: K = 1024, N = 2290, M = 950 (144 tiles) 20.9 / 25.3, K = 9216, N = 16610, M =
+// 114 (130) 150 / 162, K = 256, N = 1916, M = 479 (60) 5.2 / 6.7; the other side: K = 2304, N = 7095, M = 233 (112) 40.5 / 35.7, K = 1280, N =
+// 2163, M = 1661 (221) 48.4 / 43.9, K = 512, N = 3006, M = 258 (72) 8.3 / 7.7.
+inline bool small_batch_kernel_pays_exact(int64_t K, int64_t N, int64_t M, int sm_count) {
+    const auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+    const int64_t tiles = up(N, 128) * up(M, 128);
+    if (tiles > 280 || tiles > K / 4) return false;
+    const int64_t groups = up(M, 32), half_wave = up(up(N, 64) * groups, sm_count);
+    if (half_wave <= 2) return true;
+    const int64_t here = half_wave * (K * (474 * up(up(M, groups), 8) + 182) / 1000 + 780) + 1840 + K * 19 / 100;
+    const int64_t there = 5 * tiles >= 4 * sm_count ? up(tiles, sm_count) * (K * 158 / 10 + 650) + 3710
+                                                    : up(up(N, 64) * up(M, 64), sm_count) * (K * 536 / 100 + 600) + 1360 - K * 12 / 100;
+    return here <= there;
 }
 
 int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N,
@@ -240,7 +252,13 @@ int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *
     if (M <= 2) rc = launch_gemv_dp4a(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
     if (rc == JQ_ERR_UNSUPPORTED && M <= 8) rc = launch_gemv_mma(st, d_w, d_xq, nullptr, nullptr, d_y, K, N, M, order, 0);
     const bool exact = option_value(JQ_OPT_PREFILL_EXACT) != 0;
-    if (rc == JQ_ERR_UNSUPPORTED && (small_batch_kernel_pays(K, N, M) || (exact && small_batch_kernel_pays_exact(K, N, M))))
+    bool small_batch = small_batch_kernel_pays(K, N, M);
+    if (rc == JQ_ERR_UNSUPPORTED && exact && !small_batch) {
+        DeviceCaps caps;
+        if (int e = device_caps(&caps)) return e;
+        small_batch = small_batch_kernel_pays_exact(K, N, M, caps.sm_count);
+    }
+    if (rc == JQ_ERR_UNSUPPORTED && small_batch)
         rc = launch_mmq_stream(st, d_w, d_xq, d_y, K, N, M, order);
     if (rc == JQ_ERR_UNSUPPORTED && M >= FP16_OPERANDS_MIN_COLUMNS && !exact)
         rc = launch_gemm_f16(st, d_w, d_xq, d_y, K, N, M, order);  // refuses shapes outside its rules: the integer GEMM takes those

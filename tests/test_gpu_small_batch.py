@@ -117,9 +117,11 @@ def test_small_batch_tiles(env, K, N, M, tile, order):
     assert O.err_max_rel(y.cpu().numpy()[:, rows], O.mul_mat_ref(np.ascontiguousarray(wq[rows]), xq, K, len(rows), M, order)) <= TOL
 
 
-# With JQ_OPT_PREFILL_EXACT, both sides of the line between this kernel and the integer GEMM: the number of tiles of 128 x 128, K / 4
-@pytest.mark.parametrize("K,N,M,here", [(1536, 4480, 1024, True), (1536, 4481, 1024, False), (256, 1024, 1000, True), (256, 1025, 1000, False),
-                                        (512, 130, 64, True), (1280, 333, 77, True)])
+# With JQ_OPT_PREFILL_EXACT, both sides of the lines between this kernel and the integer GEMM: 280 tiles of 128 x 128, K / 4 of them, one wave
+# here (296 tiles of 64 x 32), and the estimates beyond
+@pytest.mark.parametrize("K,N,M,here", [(2048, 17920, 140, True), (2048, 17921, 140, False), (256, 8192, 64, True), (256, 8193, 64, False),
+                                        (256, 1216, 479, True), (256, 1217, 479, False), (1024, 2304, 950, False), (1024, 2305, 950, True),
+                                        (1024, 3776, 950, True), (1024, 3777, 950, False), (512, 130, 64, True), (1280, 333, 77, True)])
 def test_exact_prefill_kernel(env, K, N, M, here):
     c, O, t = env.c, env.O, env.t
     g = t.Generator(device=env.dev)

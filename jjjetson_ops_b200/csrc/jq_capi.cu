@@ -216,7 +216,8 @@ inline bool small_batch_kernel_pays(int64_t K, int64_t N, int64_t M) {
 // One wave of it, two CTAs of 64 rows and up to 32 columns per SM, is always the quicker one.  Beyond, an estimate of both decides, by
 // half waves of the one and waves of the other (of tiles of 128 x 128, or of 64 x 64 where those would fill less than four fifths of
 // the SMs): the integer GEMM gains where its tiles are just one wave.  Nanoseconds, fitted to 157 shapes, K 256 to 11008, within 2 % on
-// average (10 % at most), and of 500 drawn shapes one is 7 % and one 2 % slower than with the other kernel; integer GEMM / small-batch kernel, us: K = 1024, N = 2290, M = 950 (144 tiles) 20.9 / 25.3, K = 9216, N = 16610, M =
+// average (10 % at most); of 500 drawn shapes one is 2 % slower than with the other kernel.  (Near ties of a short K go to the integer
+// GEMM, which starts quicker behind the quantizer: K = 512, N = 11790, M = 97 13.2 / 15.2 us with it.)  Integer GEMM / small-batch kernel, us: K = 1024, N = 2290, M = 950 (144 tiles) 20.9 / 25.3, K = 9216, N = 16610, M =
 // 114 (130) 150 / 162, K = 256, N = 1916, M = 479 (60) 5.2 / 6.7; the other side: K = 2304, N = 7095, M = 233 (112) 40.5 / 35.7, K = 1280, N =
 // 2163, M = 1661 (221) 48.4 / 43.9, K = 512, N = 3006, M = 258 (72) 8.3 / 7.7.
 inline bool small_batch_kernel_pays_exact(int64_t K, int64_t N, int64_t M, int sm_count) {
@@ -228,7 +229,7 @@ inline bool small_batch_kernel_pays_exact(int64_t K, int64_t N, int64_t M, int s
     const int64_t here = half_wave * (K * (474 * up(up(M, groups), 8) + 182) / 1000 + 780) + 1840 + K * 19 / 100;
     const int64_t there = 5 * tiles >= 4 * sm_count ? up(tiles, sm_count) * (K * 158 / 10 + 650) + 3710
                                                     : up(up(N, 64) * up(M, 64), sm_count) * (K * 536 / 100 + 600) + 1360 - K * 12 / 100;
-    return here <= there;
+    return here + (K < 1024 ? here / 50 : 0) <= there;
 }
 
 int dispatch_mul_mat(cudaStream_t st, const void *d_w, const void *d_xq, float *d_y, int64_t K, int64_t N,

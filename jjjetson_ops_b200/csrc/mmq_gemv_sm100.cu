@@ -301,7 +301,7 @@ __device__ __forceinline__ bool may_run_ahead(const volatile uint32_t *previous_
     return false;
 }
 
-template <bool PER_ROW>
+template <bool PER_ROW, bool AHEAD = false>
 __device__ __forceinline__ void gemv_producer(const GemvParams &p, uint64_t *full, uint64_t *empty,
                                               uint64_t *x_ready, uint8_t *ring, int lane, uint64_t *x_full = nullptr,
                                               uint8_t *xs = nullptr) {
@@ -316,14 +316,14 @@ __device__ __forceinline__ void gemv_producer(const GemvParams &p, uint64_t *ful
     const int early_stages =
         p.x_copy_bytes != 0 && p.prefetch_early && p.gather.world > 1 && p.gather.wait_previous ? p.stages : p.early_stages;
     const volatile uint32_t *previous_ended = reinterpret_cast<const volatile uint32_t *>(full + GV_PREVIOUS_ENDED);
-    long long last = PER_ROW ? 0 : clock64();
+    long long last = AHEAD ? clock64() : 0;
     for (int c = 0; c < n_chunks; ++c) {
         int rows;
         const int64_t r0 = walk_stage(walk, c, R, &rows);
         int ok = 1;
         if (lane == 0) {
-            if (!x_done && c >= early_stages &&
-                !(!PER_ROW && p.ahead_cycles != 0 && round == 0 && may_run_ahead(previous_ended, &last, p.ahead_cycles, p.poll_limit))) {
+            if (AHEAD ? !x_done && c >= early_stages && !(round == 0 && may_run_ahead(previous_ended, &last, p.ahead_cycles, p.poll_limit))
+                      : c == early_stages) {
                 ok = producer_activations(p, x_ready, x_full, xs) ? 1 : 0;
                 x_done = true;
             }
@@ -640,7 +640,8 @@ __device__ __forceinline__ bool consumers_meet(uint64_t *bar, int lane, int *fau
     return mbar_wait_bounded(bar, 0u, fault, limit);
 }
 
-template <int M_T, int NSB, int NW, int MINB, bool TAGGED>
+// AHEAD: the weight stream runs ahead for as long as the preceding kernel lasts (runs_ahead says where)
+template <int M_T, int NSB, int NW, int MINB, bool TAGGED, bool AHEAD>
 __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
         mbar_init(x_full, 1);
         mbar_init(meet, NW);
         mbar_init(meet + 1, NW);
-        *reinterpret_cast<volatile uint32_t *>(full + GV_PREVIOUS_ENDED) = 0u;
+        if (AHEAD) *reinterpret_cast<volatile uint32_t *>(full + GV_PREVIOUS_ENDED) = 0u;
         fence_mbar_init();
         // Tagged all-gather: this launch's number comes from a count that every launch raises by 65536, a share per
         // CTA.  The next launch in the stream starts only after every CTA of this one has passed the trigger below,
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
         if (lane == 0) {
             if (!p.prefetch_early) griddep_wait();
             trace_stamp(p, 1);  // weight stream begins
-            gemv_producer<false>(p, full, empty, x_ready, ring, 0, x_full, xs);
+            gemv_producer<false, AHEAD>(p, full, empty, x_ready, ring, 0, x_full, xs);
             trace_stamp(p, 2);  // last copy issued
         }
         return;
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB) gemv_dp4a_kernel(const Ge
     constexpr bool tagged = TAGGED;  // p.gather.ticket != nullptr
     const bool x_tagged = tagged && p.gather.x_words != nullptr;
     if (!x_tagged) griddep_wait();
-    if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(full + GV_PREVIOUS_ENDED) = 1u;
+    if (AHEAD && threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(full + GV_PREVIOUS_ENDED) = 1u;
     uint32_t gather_epoch = 0;  // number of this all-gather (previous ones finished: *epoch_ptr)
     uint32_t x_tag = 0;
     if (tagged) {
@@ -1197,13 +1198,22 @@ int fast_path_ok(const void *d_w, const void *d_xq, const float *d_x_f32, int64_
 // (dp4a form) How fast the weight stream runs ahead of the preceding kernel's end, beyond the first two stages.  After a norm or an activation
 // the SMs have nothing else to do; too fast a stream delays the loads of that very kernel.  One sequence's decode step (four layers
 // of 4096 x 11008 and the output projection, replayed), bytes per cycle and SM 0 / 8 / 14 / 20 / 28 / 60 (HBM gives 23): 180.3 / 176.9 /
-// 176.9 / 180.1 / 184.4 / 189.9 us; K = 8192, N = 28672 after its like 23.8 / 23.8 / 23.8 / 24.0 / 24.2 / 24.5 us.
+// 176.9 / 180.1 / 184.4 / 189.9 us.
 constexpr uint32_t GV_AHEAD_BYTES_PER_CYCLE = 10;
-void set_run_ahead(GemvParams &p, int ctas_per_sm) {
-    p.ahead_cycles = p.prefetch_early && p.gather.world == 0 ? p.stage_bytes * (uint32_t)ctas_per_sm / GV_AHEAD_BYTES_PER_CYCLE : 0;
+// Where that pays.  Multiplies of ready blocks behind their like, the quantizer, RMSNorm and SwiGLU, 170 shapes; us behind RMSNorm | SwiGLU, without
+// / with it.  One column, K > 3200, from 36 million weights on: K = 4096, N = 22016 12.79 / 12.22 | 11.88 / 11.19, K = 3584, N = 11008 9.60 / 9.07 |
+// 8.21 / 7.54, K = 8192, N = 11008 14.99 / 14.50 | 11.60 / 11.10; the other side: K = 4096, N = 6144 7.38 / 7.55 | 6.05 / 6.24, K = 8192, N = 4096
+// 10.73 / 10.62 | 6.20 / 6.63 (a stage that was requested late is in the activations' way), K = 2048, N = 11008 7.55 / 7.96 | 6.66 / 7.10,
+// K = 8192 in long slabs, N = 22016 22.09 / 22.28 | 19.78 / 19.93, K = 11008, N = 4096 14.03 / 14.03 | 7.53 / 8.12.  Two columns, K > 4096, of few
+// rows: K = 8192, N = 4096 12.98 / 12.74 | 9.96 / 8.94, N = 16384 23.18 / 22.72 | 19.85 / 19.29; the other side: K = 5888, N = 28672 30.59 /
+// 30.73 | 27.45 / 27.91; K = 3072, N = 11008 11.27 / 11.10 | 8.88 / 9.12.
+inline bool runs_ahead(const GemvParams &p) {
+    if (!p.prefetch_early || p.gather.world != 0 || p.x_f32 != nullptr) return false;
+    if (p.M == 2) return p.K > 4096 && (p.N <= 12288 || (p.K >= 7168 && p.N < 24576));
+    return p.K > 3200 && p.K <= (p.N >= 16384 ? 6144 : 8192) && p.N * p.K >= (int64_t)36 << 20;
 }
 
-template <int M_T, int NSB, int NW, int MINB>
+template <int M_T, int NSB, int NW, int MINB, bool MAY_RUN_AHEAD = false>
 int run_dp4a(cudaStream_t st, GemvParams &p, const DeviceCaps &caps) {
     // MINB CTAs share an SM: each gets an equal slice of its shared memory (1 KB per CTA is reserved)
     const int64_t budget = min((int64_t)caps.smem_optin, (int64_t)caps.smem_per_sm / MINB - 1024);
@@ -1226,11 +1236,12 @@ int run_dp4a(cudaStream_t st, GemvParams &p, const DeviceCaps &caps) {
     }
     if (p.stages < 2) return set_error(JQ_ERR_UNSUPPORTED, "row of %u bytes does not fit the shared-memory ring", p.row_bytes);
     const int smem = GV_BAR_BYTES + (int)p.y_bytes + (int)p.x_bytes + p.stages * (int)p.stage_bytes;
-    set_run_ahead(p, MINB);
+    p.ahead_cycles = p.stage_bytes * (uint32_t)MINB / GV_AHEAD_BYTES_PER_CYCLE;
 #ifdef JQ_BOUNDS_CHECK
     p.smem_total = (uint32_t)smem;
 #endif
-    auto kernel = p.gather.ticket != nullptr ? gemv_dp4a_kernel<M_T, NSB, NW, MINB, true> : gemv_dp4a_kernel<M_T, NSB, NW, MINB, false>;
+    auto kernel = p.gather.ticket != nullptr ? gemv_dp4a_kernel<M_T, NSB, NW, MINB, true, false> : gemv_dp4a_kernel<M_T, NSB, NW, MINB, false, false>;
+    if (MAY_RUN_AHEAD && runs_ahead(p)) kernel = gemv_dp4a_kernel<M_T, NSB, NW, MINB, false, MAY_RUN_AHEAD>;
     if (int rc = ensure_smem_attr(kernel, smem)) return rc;
     const int64_t want = (p.N + p.rows_per_stage - 1) / p.rows_per_stage;
     const int grid = (int)min((int64_t)caps.sm_count * MINB, max((int64_t)1, want));
@@ -1397,12 +1408,12 @@ int launch_gemv_dp4a(cudaStream_t st, const void *d_w, const void *d_xq, const f
                 // that cost.  With ready-made Q8_1 input two CTAs of 8 warps per SM overlap better.
                 // (20 consumer warps instead of 16 fit the register file and change nothing: 6.22 us either way)
                 if (p.x_f32 != nullptr || x_words) return run_dp4a<1, 1, 16, 1>(st, p, caps);
-                return run_dp4a<1, 1, 8, 2>(st, p, caps);
+                return run_dp4a<1, 1, 8, 2, true>(st, p, caps);
             case 2:
                 // long slabs stream better with 12 consumer warps (K = 8192, N = 28672 on ready blocks: 22.9 -> 21.6 us),
                 // short ones start faster with 8 (N = 4096: 6.56 against 7.01 us)
-                if (N >= 16384) return run_dp4a<1, 2, 12, 1>(st, p, caps);
-                return run_dp4a<1, 2, 8, 1>(st, p, caps);
+                if (N >= 16384) return run_dp4a<1, 2, 12, 1, true>(st, p, caps);
+                return run_dp4a<1, 2, 8, 1, true>(st, p, caps);
             case 3: return run_dp4a<1, 3, 7, 1>(st, p, caps);  // (9 consumer warps: K = 11008, N = 4096 7.3 -> 9.6 us)
             case 4: return run_dp4a<1, 4, 7, 1>(st, p, caps);
             default: break;
@@ -1415,7 +1426,7 @@ int launch_gemv_dp4a(cudaStream_t st, const void *d_w, const void *d_xq, const f
                 // 9.10 us, multiply on ready blocks 8.42 / 8.32 / 8.58 / 9.00 us
                 if (p.x_f32 != nullptr) return run_dp4a<2, 1, 12, 1>(st, p, caps);
                 return run_dp4a<2, 1, 10, 1>(st, p, caps);
-            case 2: return run_dp4a<2, 2, 7, 1>(st, p, caps);
+            case 2: return run_dp4a<2, 2, 7, 1, true>(st, p, caps);
             default: break;
         }
     }

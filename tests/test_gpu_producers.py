@@ -336,6 +336,35 @@ def test_multi_linear_equals_separate_linears(native_lib, oracle, cuda_device, M
         c.linear_q4_0_multi(wq * 5, list(Ns) * 5, x=x)  # more than four matrices
 
 
+
+# Both sides of the lines where the decode kernel's weight stream runs ahead of the norm before it (one column: 36 * 2^20 weights, K > 3200,
+# the long slabs; two columns: 12288 rows, K >= 7168): the same bits as without, and as often as it is repeated
+@pytest.mark.parametrize("T,K,N", [(1, 4096, 9216), (1, 4096, 9215), (1, 3328, 11343), (1, 3072, 12289), (1, 6144, 16384), (1, 6400, 16384),
+                                   (1, 8192, 4608), (1, 8192, 16383), (1, 8192, 16384), (2, 4352, 12288), (2, 4352, 12289), (2, 7168, 24575),
+                                   (2, 8192, 300)])
+def test_multiply_behind_rms_norm_with_static_weights(native_lib, cuda_device, T, K, N):
+    import torch
+
+    c = native_lib
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(K + N)
+    w = c.quantize_q4_0(torch.randn((N, K), generator=g, device=cuda_device).mul_(0.02))
+    x, wn = torch.randn((T, K), generator=g, device=cuda_device), 1.0 + 0.1 * torch.randn(K, generator=g, device=cuda_device)
+    xq = torch.zeros(c.q8_1_bytes(K, T), dtype=torch.uint8, device=cuda_device)
+    ys = [torch.full((T, N), float("nan"), device=cuda_device) for _ in range(4)]
+    c.rms_norm_q8_1(x, wn, 1e-6, xq=xq)
+    want = c.mul_mat_q4_0_q8_1(w, xq, K, N, T)
+    torch.cuda.synchronize()
+    c.set_option(c.OPT_STATIC_WEIGHTS, 1)
+    try:
+        for y in ys:
+            c.rms_norm_q8_1(x, wn, 1e-6, xq=xq)
+            c.mul_mat_q4_0_q8_1(w, xq, K, N, T, out=y)
+    finally:
+        c.set_option(c.OPT_STATIC_WEIGHTS, 0)
+    assert all(torch.equal(y, want) for y in ys)
+
+
 RMS_EDGE_WORKER = r"""
 import sys
 sys.path.insert(0, sys.argv[1])

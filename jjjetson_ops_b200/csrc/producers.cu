@@ -18,6 +18,7 @@ namespace jq {
 namespace {
 
 constexpr int RMS_THREADS = 256;  // the reference's block size; the summation order depends on it
+constexpr int RMS_FEW_TOKENS = 2;
 constexpr size_t RMS_STATIC_BYTES = 1024;  // more than the kernel's static shared memory and what the device reserves per block
 
 // Block sum with the reference's tree (include/cuda_utils.cuh:19-27, 49-65): shuffle-down inside
@@ -46,17 +47,22 @@ __device__ __forceinline__ float block_sum_reference_order(float v, float *warp_
 // the per-thread partial sums of squares, the block tree and rsqrtf give the same inverse RMS bit
 // for bit.  The normalised row is staged in shared memory and quantized from there warp by warp
 // (one warp per 128-value block, one lane four consecutive values: the quantizer's own mapping).
-// STAGED: the weight vector is brought into shared memory behind the row.
-template <bool STAGED>
+// FEW: one or two tokens are one chain of latencies, and with the matrices of a model streamed since its last use the weight vector comes
+// from HBM.  It is on its way to L2 while the preceding kernel ends (a hint: no value is read before the wait) and to shared memory,
+// behind the row, while the row is loaded and summed.
+template <bool FEW>
 __global__ void __launch_bounds__(RMS_THREADS, 5)
 rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ weight, float *normed_out,
                      uint8_t *__restrict__ xq, int H, int T, float epsilon, int n_super, int order, int s_mode) {
     // input, residual and normed_out carry no __restrict__: normed_out may be input itself (the reference's
     // in-place form); every read of a row happens before the barrier that precedes the first write to it
-    extern __shared__ __align__(16) float row[];  // H floats (STAGED: and the weights)
+    extern __shared__ __align__(16) float row[];  // H floats (FEW: and the weights)
     __shared__ float warp_partial[32];
     __shared__ float inverse_rms;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (FEW) {
+        for (int i = threadIdx.x * 32; i < H; i += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(weight + i));
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int token = blockIdx.x;
     const int64_t base = (int64_t)token * H;
@@ -65,11 +71,7 @@ rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ we
     // are free to use any thread-to-element mapping
     const bool vec = (H & 3) == 0 && ((uintptr_t)(input + base) & 15u) == 0 &&
                      (residual == nullptr || ((uintptr_t)(residual + base) & 15u) == 0);
-    const bool vec_out = vec && ((uintptr_t)weight & 15u) == 0 && (normed_out == nullptr || ((uintptr_t)(normed_out + base) & 15u) == 0);
-    const bool fused = vec_out && xq != nullptr && (n_super & 1) == 0;  // normalised and quantized in one pass
-    if (STAGED && fused) {
-        // Few tokens: the kernel is one chain of latencies, and with the matrices of a whole layer streamed since its last use
-        // the weight vector comes from HBM.  It is on its way while the row is loaded and summed.
+    if (FEW && ((uintptr_t)weight & 15u) == 0) {
         const uint32_t dst = smem_u32(row + H);
         for (int i = threadIdx.x; i < (H >> 2); i += blockDim.x)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * i), "l"(weight + 4 * i) : "memory");
@@ -138,10 +140,11 @@ rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ we
     }
     sum_square = block_sum_reference_order(sum_square, warp_partial);
     if (threadIdx.x == 0) inverse_rms = rsqrtf(sum_square / (float)H + epsilon);
-    if (STAGED) asm volatile("cp.async.wait_all;" ::: "memory");
+    if (FEW) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const float inv = inverse_rms;
-    if (fused) {
+    const bool vec_out = vec && ((uintptr_t)weight & 15u) == 0 && (normed_out == nullptr || ((uintptr_t)(normed_out + base) & 15u) == 0);
+    if (vec_out && xq != nullptr && (n_super & 1) == 0) {
         // Normalisation and quantization in one pass over the row: a warp takes a pair of neighbouring blocks, a lane
         // its eight consecutive values, (z * inv) * w goes to the fp32 output (if wanted) and into the quantizer
         // straight from registers.  Same products, same bits as normalising the row first; it saves the row's second
@@ -150,8 +153,8 @@ rms_norm_q8_1_kernel(float *input, float *residual, const float *__restrict__ we
         for (int pr = warp; pr < (n_super >> 1); pr += n_warps) {
             const int e0 = pr * (2 * SUPER) + lane * 8;
             const float4 z0 = *reinterpret_cast<const float4 *>(row + e0), z1 = *reinterpret_cast<const float4 *>(row + e0 + 4);
-            const float4 w0 = STAGED ? *reinterpret_cast<const float4 *>(row + H + e0) : __ldg(reinterpret_cast<const float4 *>(weight + e0));
-            const float4 w1 = STAGED ? *reinterpret_cast<const float4 *>(row + H + e0 + 4) : __ldg(reinterpret_cast<const float4 *>(weight + e0 + 4));
+            const float4 w0 = FEW ? *reinterpret_cast<const float4 *>(row + H + e0) : __ldg(reinterpret_cast<const float4 *>(weight + e0));
+            const float4 w1 = FEW ? *reinterpret_cast<const float4 *>(row + H + e0 + 4) : __ldg(reinterpret_cast<const float4 *>(weight + e0 + 4));
             const float v[8] = {__fmul_rn(__fmul_rn(z0.x, inv), w0.x), __fmul_rn(__fmul_rn(z0.y, inv), w0.y),
                                 __fmul_rn(__fmul_rn(z0.z, inv), w0.z), __fmul_rn(__fmul_rn(z0.w, inv), w0.w),
                                 __fmul_rn(__fmul_rn(z1.x, inv), w1.x), __fmul_rn(__fmul_rn(z1.y, inv), w1.y),
@@ -306,10 +309,12 @@ int launch_rms_norm_q8_1(cudaStream_t st, float *d_input, float *d_residual, con
     if (smem + RMS_STATIC_BYTES > (size_t)caps.smem_optin)
         return set_error(JQ_ERR_TOO_LARGE, "rms_norm: a row of %lld floats does not fit in shared memory", (long long)H);
     // A decode step of one sequence (four layers of 4096 x 11008 and the output norm, replayed from a graph, all launches) 186.0 ->
-    // 180.4 us; of eight sequences 155.7 -> 158.0: there the row's neighbours bring the vector in.
-    const bool staged = T <= 2 && d_xq != nullptr && 2 * smem + RMS_STATIC_BYTES <= (size_t)caps.smem_optin;
-    if (staged) smem *= 2;
-    const auto kernel = staged ? rms_norm_q8_1_kernel<true> : rms_norm_q8_1_kernel<false>;
+    // 180.4 us; RMSNorm and multiply, K = 8192, N = 28672, 28.3 -> 26.6, K = 4096, N = 4096 6.39 -> 6.12; with the vector in L2 already
+    // it costs 0.1 us (K = 2048, N = 8192, two tokens 8.53 -> 8.83).  Eight sequences 155.7 -> 158.0: there the row's neighbours bring the vector in.
+    // (an odd number of blocks takes the two passes below, which read it as they go)
+    const bool few = T <= RMS_FEW_TOKENS && d_xq != nullptr && H % (2 * SUPER) == 0 && 2 * smem + RMS_STATIC_BYTES <= (size_t)caps.smem_optin;
+    if (few) smem *= 2;
+    const auto kernel = few ? rms_norm_q8_1_kernel<true> : rms_norm_q8_1_kernel<false>;
     // without being asked for, a block has 48 KB, of which the kernel's static variables take a part
     if (smem + RMS_STATIC_BYTES > 48 * 1024) {
         if (int rc = ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem)) return rc;

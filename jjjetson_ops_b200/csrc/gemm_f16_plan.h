@@ -25,8 +25,9 @@ struct GemmF16Plan {
 // The cheapest form by what a launch takes, in hundredths of a us: per wave of CTAs a fixed part and 68 for each 128-value stage
 // (79 where pairs of CTAs share 256 x 256: they convert as much per stage as single CTAs and multiply twice as much).  The fixed
 // part fills the pipeline and writes the tile, and adds up the parts where K is split.  A fit over 110 shapes (K 256 to 11008, N 64
-// to 32000, M 64 to 2048, the multiply alone, every form): within 5 % (one CTA and parts of K) and 8 % (pairs), and the form it names
-// takes 0.3 % more than the quickest one on average.  Both sides of the lines, the multiply alone, us:
+// to 32000, M 64 to 2048, the multiply alone, every form): the form it names takes 0.3 % more than the quickest one on average.  Against 116
+// shapes in a chain of launches, of the form it names: pairs 6 % off on average and 12 % at most (K = 8192, N = 28672, M = 2048 is 760 by
+// the estimate and takes 860 to 890, at the card's power limit), the others 11 %, mostly launches of a few us that take 1 to 1.5 less.  Both sides of the lines, the multiply alone, us:
 //   K = N = 4096, M = 512 (128 tiles): one 26.2, pairs 31.1 (64 on 74 places)
 //   K = N = 4096, M = 128 (32 tiles): four parts 12.4, three 15.5, six 21.2, because 32 clusters of six take two waves
 //   K = 8192, N = 1101, M = 167: six parts 15.6, eight 24.6

@@ -212,13 +212,13 @@ inline bool small_batch_kernel_pays(int64_t K, int64_t N, int64_t M) {
 // 128: the integer GEMM needs them all to fill the SMs, and rounds off two to seven times as much.  Multiply alone, integer GEMM /
 // small-batch kernel: K = N = 4096, M = 64 25.9 / 12.7 us, M = 256 45.8 / 39.8, M = 512 (128 tiles) 69.0 / 67.9; K = 4096, N = 11008, M = 256
 // (172) 137 / 95 us; K = 9472, N = 502, M = 66 57.8 / 11.4; the other side: K = 2560, N = 6047, M = 684 (288) 89.8 / 93.3 us, K = 512, N = 25906,
-// M = 549 (1015) 78 / 103.
+// M = 549 (1015) 78 / 103, and short K, where a CTA has little to do per column: K = 256, N = 1716, M = 547 (70) 5.4 / 6.8.
 // One wave of it, two CTAs of 64 rows and up to 32 columns per SM, is always the quicker one.  Beyond, an estimate of both decides, by
 // half waves of the one and waves of the other (of tiles of 128 x 128, or of 64 x 64 where those would fill less than four fifths of
 // the SMs): the integer GEMM gains where its tiles are just one wave.  Nanoseconds, fitted to 157 shapes, K 256 to 11008, within 2 % on
 // average (10 % at most); of 500 drawn shapes one is 2 % slower than with the other kernel.  (Near ties of a short K go to the integer
-// GEMM, which starts quicker behind the quantizer: K = 512, N = 11790, M = 97 13.2 / 15.2 us with it.)  Integer GEMM / small-batch kernel, us: K = 1024, N = 2290, M = 950 (144 tiles) 20.9 / 25.3, K = 9216, N = 16610, M =
-// 114 (130) 150 / 162, K = 256, N = 1916, M = 479 (60) 5.2 / 6.7; the other side: K = 2304, N = 7095, M = 233 (112) 40.5 / 35.7, K = 1280, N =
+// GEMM, which starts quicker behind the quantizer: K = 512, N = 11790, M = 97 13.2 / 15.2 us with it.)  Integer GEMM / small-batch kernel, us:
+// K = 1024, N = 2290, M = 950 (144 tiles) 20.9 / 25.3, K = 9216, N = 16610, M = 114 (130) 150 / 162, K = 256, N = 1916, M = 479 (60) 5.2 / 6.7; the other side: K = 2304, N = 7095, M = 233 (112) 40.5 / 35.7, K = 1280, N =
 // 2163, M = 1661 (221) 48.4 / 43.9, K = 512, N = 3006, M = 258 (72) 8.3 / 7.7.
 inline bool small_batch_kernel_pays_exact(int64_t K, int64_t N, int64_t M, int sm_count) {
     const auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
